@@ -114,6 +114,21 @@ def test_linear_float32_few_rows_are_bit_for_bit_the_same_rows_among_many(ops, f
     assert (got.double() - want).abs().max().item() < 2e-6 * math.sqrt(k) * 4
 
 
+@pytest.mark.parametrize("n,k", [(1, 4), (31, 128), (33, 132), (127, 1024), (129, 1056), (130, 1050), (260, 3000)])
+@pytest.mark.parametrize("m", [2, 4, 5, 17, 32, 33, 64, 65, 129])
+def test_linear_float32_at_the_edges_of_rows_tiles_and_runs(ops, m, n, k):
+    """Remainders of the few-rows kernel's 32 columns and of the tiles' 64 x 128, K of one run, of runs of unequal length
+    and of no multiple of 4; the first m of 129 rows are bit for bit the same whatever m is.  Bound: an element is at most
+    8 sums of chains of run_length(K) multiply-adds each, every one of which rounds by half a unit of what is there."""
+    g = torch.Generator().manual_seed(32)
+    x, w, b = torch.randn(129, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda(), torch.randn(n, generator=g).cuda()
+    got = ops.linear(x[:m].contiguous(), w, b)
+    assert torch.equal(got, ops.linear(x, w, b)[:m])
+    run = max(128, ((k + 7) // 8 + 31) // 32 * 32)
+    bound = (min(run, k) + 9) * 2.0 ** -24 * (x[:m].double().abs() @ w.double().abs().T + b.double().abs())
+    assert bool(((got.double() - P.linear(x[:m], w, b, torch.float64)).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 331, 240), (8, 512, 96), (9, 331, 240), (16, 512, 96), (33, 1000, 328), (200, 384, 64)])
 def test_linear_bfloat16(ops, m, n, k):
     g = torch.Generator().manual_seed(4)
@@ -430,6 +445,23 @@ def test_attention(ops, dtype, nheads, kvheads, hd, lens_before, num_new, window
     got = ops.attention(q, batch, view, nheads, kvheads, hd, scale, window)
     assert not torch.isnan(got).any()
     torch.testing.assert_close(got.float(), want.float(), **tol(dtype))
+
+
+@pytest.mark.parametrize("nheads,kvheads,hd,window", [(4, 2, 128, 0), (3, 1, 48, 70), (2, 2, 256, 0), (5, 1, 16, 0)])
+@pytest.mark.parametrize("num_new", [[2, 15], [16, 17], [63, 64], [65, 130]])
+def test_prefill_attention_float32_at_the_edges_of_its_tiles(ops, nheads, kvheads, hd, window, num_new):
+    """Tiles of 64 query rows, of which up to 16 take two rows a thread; queries by themselves and as the first columns of
+    a wider matrix."""
+    cache, view, batch = make_cache_case(torch.float32, nheads, kvheads, hd, [37, 200], num_new, 8, window)
+    g = torch.Generator().manual_seed(19)
+    qkv = torch.randn(sum(num_new), (nheads + 2 * kvheads) * hd, generator=g).cuda()
+    q = ops.rope_store(qkv, None, batch, view, nheads, kvheads, hd)
+    scale = 1.0 / math.sqrt(hd)
+    want = P.attention(q, batch, view, nheads, kvheads, hd, scale, window)
+    got = ops.attention(q, batch, view, nheads, kvheads, hd, scale, window)
+    torch.testing.assert_close(got, want.float(), **tol(torch.float32))
+    wide = torch.cat([q, torch.randn(q.shape[0], 4, generator=g).cuda()], 1)
+    assert torch.equal(ops.attention(wide, batch, view, nheads, kvheads, hd, scale, window), got)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
