@@ -31,7 +31,7 @@ constexpr int HD = HEAD_DIM;
 constexpr int BLK = 64;           // tokens per cache block
 constexpr int SPLIT = 256;        // keys per decode split
 constexpr int GC = 8;             // query heads of one kv head handled by one decode block
-constexpr int TQ = 16;            // query rows per prefill block
+constexpr int TQ = 64;            // query rows per float32 prefill block
 
 template <typename T> struct Vec;  // 16-byte vectors
 template <> struct Vec<float> { static constexpr int N = 4; };
@@ -121,124 +121,170 @@ __device__ __forceinline__ int block_of(const AttnArgs& a, int slot, int kb) {
 }
 
 // ---------------------------------------------------------------------------------------------------
-// prefill: grid (query tiles, heads), 128 threads; thread (r = tid / 8, c = tid % 8) owns row r of the
-// tile, scores of keys c, c+8, ... and output columns c, c+8, ...
+// float32 prefill: a block per (tile of TQ query rows, head), the longest tiles first.  Bound by the FMA pipe: thread
+// (ty = tid / 16, tx = tid % 16) holds RPT rows (ty, ty + 8, ...) by four keys (tx, tx + 16, ...) of the scores and the
+// same rows by HD / 16 columns of the result, so that 12 reads of 16 bytes serve 128 multiply-adds of the first product and
+// 4 RPT + HD / 4 reads 4 RPT HD / 16 of the second (a row and one key or column a thread, as here before, read shared
+// memory twice a multiply-add: 671 against 210 us for three prompts of 1,100 tokens together, 32 heads of 128).  Rows of q
+// and k are padded by four floats (no bank conflicts); the probabilities lie where the keys were, so that two blocks fit a
+// multiprocessor and one's copies run under the other's arithmetic.  Tiles of up to 16 rows (short prompts) take RPT = 2.
 // ---------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(128) attn_prefill_kernel(AttnArgs a, const int* __restrict__ tiles) {
-  extern __shared__ float smem[];
-  float* qs = smem;                        // [TQ][HD + 1]
-  float* ks = qs + TQ * (HD + 1);          // [BLK][HD + 1]
-  float* vs = ks + BLK * (HD + 1);         // [BLK][HD]
-  float* ps = vs + BLK * HD;               // [TQ][BLK + 1]
+constexpr int QSTRIDE = HD + 4, PSTRIDE = BLK + 4;
+constexpr int KEY_FLOATS = BLK * (QSTRIDE > PSTRIDE ? QSTRIDE : PSTRIDE);  // keys, then probabilities
+constexpr size_t F32_PREFILL_SMEM = (size_t)(TQ * QSTRIDE + KEY_FLOATS + BLK * HD) * sizeof(float);
 
-  const int tid = threadIdx.x, r = tid >> 3, c = tid & 7;
-  const int seq = tiles[2 * blockIdx.x], r0 = tiles[2 * blockIdx.x + 1];
-  const int head = blockIdx.y;
+__device__ __forceinline__ void copy16_f32(float* smem, const float* gmem, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
+}
+
+template <int RPT>
+__device__ __forceinline__ void prefill_f32_tile(const AttnArgs& a, float* smem, int head, int row0, int rows_here, int p_first,
+                                                 int len, int slot) {
+  float* qs = smem;                // [TQ][QSTRIDE]
+  float* ks = qs + TQ * QSTRIDE;   // [BLK][QSTRIDE], then the probabilities [TQ][PSTRIDE]
+  float* vs = ks + KEY_FLOATS;     // [BLK][HD]
+  float* ps = ks;
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const int kvh = head / (a.nheads / a.kvheads);
-  const int row_begin = a.first_row[seq];
-  const int n_new = a.first_row[seq + 1] - row_begin;
-  const int len = a.len_after[seq];
-  const int len_before = len - n_new;
-  const int slot = a.slots[seq];
-  const int rows_here = min(TQ, n_new - r0);
-  const T* q = (const T*)a.q;
-  const T* kc = (const T*)a.keys;
-  const T* vc = (const T*)a.values;
-
-  for (int i = tid; i < TQ * HD; i += 128) {
-    const int rr = i / HD, d = i - rr * HD;
-    qs[rr * (HD + 1) + d] =
-        rr < rows_here ? to_f32(q[(size_t)(row_begin + r0 + rr) * a.q_stride + (size_t)head * HD + d]) : 0.f;
+  const float* q = (const float*)a.q + (size_t)row0 * a.q_stride + (size_t)head * HD;
+  const float* kc = (const float*)a.keys;
+  const float* vc = (const float*)a.values;
+  for (int i = tid; i < RPT * 8 * (HD / 4); i += 128) {  // every row of queries starts on 16 bytes (check_queries)
+    const int r = i / (HD / 4), d = (i - r * (HD / 4)) * 4;
+    copy16_f32(qs + r * QSTRIDE + d, q + (size_t)min(r, rows_here - 1) * a.q_stride + d, r < rows_here);
   }
-  const int p_first = len_before + r0;
   const int p_last = p_first + rows_here - 1;
-  const int my_pos = p_first + r;
-  const bool row_ok = r < rows_here;
-  const int kb_lo = first_visible(a, p_first) / BLK;
-  const int kb_hi = p_last / BLK;
-  const int my_first = first_visible(a, my_pos);
+  const int kb_lo = first_visible(a, p_first) / BLK, kb_hi = p_last / BLK;
   const float2 dist = a.distance ? a.distance[head] : make_float2(0.f, 0.f);
 
-  float m = -INFINITY, l = 0.f;
-  float acc[HD / 8];
+  float m[RPT], l[RPT], acc[RPT][HD / 16];
 #pragma unroll
-  for (int j = 0; j < HD / 8; ++j) acc[j] = 0.f;
-
+  for (int i = 0; i < RPT; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < HD / 16; ++c) acc[i][c] = 0.f;
+  }
   for (int kb = kb_lo; kb <= kb_hi; ++kb) {
     const int blk = block_of(a, slot, kb);
     if (blk < 0) continue;  // uniform over the block: a block that left the window
+    __syncthreads();        // everyone is done with the probabilities and values of the block before
+    const float* kbase = kc + ((size_t)blk * a.kvheads + kvh) * BLK * HD;
+    const float* vbase = vc + ((size_t)blk * a.kvheads + kvh) * BLK * HD;
+    for (int i = tid; i < BLK * (HD / 4); i += 128) {
+      const int key = i / (HD / 4), d = (i - key * (HD / 4)) * 4;
+      copy16_f32(ks + key * QSTRIDE + d, kbase + (size_t)key * HD + d, kb * BLK + key < len);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int i = tid; i < BLK * (HD / 4); i += 128) {
+      const int key = i / (HD / 4), d = (i - key * (HD / 4)) * 4;
+      copy16_f32(vs + key * HD + d, vbase + (size_t)key * HD + d, kb * BLK + key < len);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();
-    const T* kbase = kc + ((size_t)blk * a.kvheads + kvh) * BLK * HD;
-    const T* vbase = vc + ((size_t)blk * a.kvheads + kvh) * BLK * HD;
-    constexpr int VN = Vec<T>::N;
-    for (int i = tid; i < BLK * HD / VN; i += 128) {
-      const int key = (i * VN) / HD, d = (i * VN) - key * HD;
-      const bool valid = kb * BLK + key < len;
-      float kv[VN], vv[VN];
-      if (valid) {
-        load_vec<T>(kbase + (size_t)key * HD + d, kv);
-        load_vec<T>(vbase + (size_t)key * HD + d, vv);
+    float s[RPT][4];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+    for (int d = 0; d < HD; d += 4) {
+      float4 kx[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kx[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * QSTRIDE + d);
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const float4 qx = *reinterpret_cast<const float4*>(qs + (ty + 8 * i) * QSTRIDE + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(qx.x, kx[j].x, s[i][j]);
+          s[i][j] = fmaf(qx.y, kx[j].y, s[i][j]);
+          s[i][j] = fmaf(qx.z, kx[j].z, s[i][j]);
+          s[i][j] = fmaf(qx.w, kx[j].w, s[i][j]);
+        }
+      }
+    }
+    __syncthreads();  // the keys have been read: their place takes the probabilities
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = ty + 8 * i, my_pos = p_first + r, my_first = first_visible(a, my_pos);
+      float tile_max = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int kpos = kb * BLK + tx + 16 * j;
+        const bool visible = r < rows_here && kpos <= my_pos && kpos >= my_first;
+        float v = visible ? (a.softcap > 0.f ? a.softcap * tanhf(s[i][j] * a.scale / a.softcap) : s[i][j] * a.scale) : -INFINITY;
+        if (a.distance && visible) v -= dist.x * log1pf(dist.y * (float)(my_pos - kpos));
+        s[i][j] = v;
+        tile_max = fmaxf(tile_max, v);
       }
 #pragma unroll
-      for (int e = 0; e < VN; ++e) {
-        ks[key * (HD + 1) + d + e] = valid ? kv[e] : 0.f;
-        vs[key * HD + d + e] = valid ? vv[e] : 0.f;
+      for (int o = 8; o > 0; o >>= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, o));
+      const float m_new = fmaxf(m[i], tile_max);
+      const float m_use = m_new == -INFINITY ? 0.f : m_new;
+      const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_use);
+      float psum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_use);
+        psum += p;
+        ps[r * PSTRIDE + tx + 16 * j] = p;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
+      l[i] = l[i] * alpha + psum;
+      m[i] = m_new;
+#pragma unroll
+      for (int c = 0; c < HD / 16; ++c) acc[i][c] *= alpha;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+#pragma unroll 1
+    for (int key = 0; key < BLK; key += 4) {
+      float4 p[RPT];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) p[i] = *reinterpret_cast<const float4*>(ps + (ty + 8 * i) * PSTRIDE + key);
+      const float* vr = vs + key * HD + tx;
+#pragma unroll
+      for (int c = 0; c < HD / 16; ++c) {
+        const float v0 = vr[16 * c], v1 = vr[HD + 16 * c], v2 = vr[2 * HD + 16 * c], v3 = vr[3 * HD + 16 * c];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          acc[i][c] = fmaf(p[i].x, v0, acc[i][c]);
+          acc[i][c] = fmaf(p[i].y, v1, acc[i][c]);
+          acc[i][c] = fmaf(p[i].z, v2, acc[i][c]);
+          acc[i][c] = fmaf(p[i].w, v3, acc[i][c]);
+        }
       }
     }
-    __syncthreads();
-    float s[8];
-    float tile_max = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int key = c + 8 * i;
-      const int kpos = kb * BLK + key;
-      float dot = 0.f;
-      const float* qr = qs + r * (HD + 1);
-      const float* kr = ks + key * (HD + 1);
-#pragma unroll 8
-      for (int d = 0; d < HD; ++d) dot = fmaf(qr[d], kr[d], dot);
-      const bool visible = row_ok && kpos <= my_pos && kpos >= my_first;
-      s[i] = visible ? (a.softcap > 0.f ? a.softcap * tanhf(dot * a.scale / a.softcap) : dot * a.scale) : -INFINITY;
-      if (a.distance && visible) s[i] -= dist.x * log1pf(dist.y * (float)(my_pos - kpos));
-      tile_max = fmaxf(tile_max, s[i]);
-    }
-    tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 1));
-    tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 2));
-    tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 4));
-    const float m_new = fmaxf(m, tile_max);
-    const float m_use = m_new == -INFINITY ? 0.f : m_new;
-    const float alpha = m == -INFINITY ? 0.f : expf(m - m_use);
-    float psum = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float p = s[i] == -INFINITY ? 0.f : expf(s[i] - m_use);
-      psum += p;
-      ps[r * (BLK + 1) + c + 8 * i] = p;
-    }
-    psum += __shfl_xor_sync(0xffffffffu, psum, 1);
-    psum += __shfl_xor_sync(0xffffffffu, psum, 2);
-    psum += __shfl_xor_sync(0xffffffffu, psum, 4);
-    l = l * alpha + psum;
-    m = m_new;
-    __syncwarp();  // the 8 threads of a row are in one warp; ps[r] is read only by them
-#pragma unroll
-    for (int j = 0; j < HD / 8; ++j) acc[j] *= alpha;
-    const float* pr = ps + r * (BLK + 1);
-    for (int key = 0; key < BLK; ++key) {
-      const float p = pr[key];
-      const float* vr = vs + key * HD + c;
-#pragma unroll
-      for (int j = 0; j < HD / 8; ++j) acc[j] = fmaf(p, vr[8 * j], acc[j]);
-    }
   }
-  if (row_ok) {
-    T* o = (T*)a.out + (size_t)(row_begin + r0 + r) * a.nheads * HD + (size_t)head * HD;
-    if (a.sink != nullptr) l += expf(a.sink[head] - (m == -INFINITY ? 0.f : m));
-    const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
-    for (int j = 0; j < HD / 8; ++j) o[c + 8 * j] = from_f32<T>(acc[j] * inv);
+  for (int i = 0; i < RPT; ++i) {
+    const int r = ty + 8 * i;
+    if (r >= rows_here) continue;
+    float* o = (float*)a.out + (size_t)(row0 + r) * a.nheads * HD + (size_t)head * HD;
+    float sum = l[i];
+    if (a.sink != nullptr) sum += expf(a.sink[head] - (m[i] == -INFINITY ? 0.f : m[i]));
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+#pragma unroll
+    for (int c = 0; c < HD / 16; ++c) o[tx + 16 * c] = acc[i][c] * inv;
   }
+}
+
+__global__ void __launch_bounds__(128, 2) attn_prefill_f32_kernel(AttnArgs a, const int* __restrict__ tiles, int n_tiles) {
+  extern __shared__ __align__(16) float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int head = blockIdx.x % a.nheads, tile = n_tiles - 1 - blockIdx.x / a.nheads;
+  const int seq = tiles[2 * tile], r0 = tiles[2 * tile + 1];
+  const int row_begin = a.first_row[seq], n_new = a.first_row[seq + 1] - row_begin, len = a.len_after[seq];
+  const int rows_here = min(TQ, n_new - r0), slot = a.slots[seq];
+  const int p_first = len - n_new + r0;
+  if (rows_here <= 16)
+    prefill_f32_tile<2>(a, smem, head, row_begin + r0, rows_here, p_first, len, slot);
+  else
+    prefill_f32_tile<8>(a, smem, head, row_begin + r0, rows_here, p_first, len, slot);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -678,14 +724,14 @@ static int attention_prefill(const void* q, void* out, int dtype, const void* ke
     return fms_launch_status("attention_prefill");
   }
   if (dtype != FMS_F32) return fms_fail("attention_prefill: unsupported dtype code %d", dtype);
-  const size_t smem = (size_t)(TQ * (HD + 1) + BLK * (HD + 1) + BLK * HD + TQ * (BLK + 1)) * sizeof(float);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fms_fail("attention_prefill: shared memory of %zu bytes refused: %s", smem, cudaGetErrorString(e));
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32_PREFILL_SMEM);
+    if (e != cudaSuccess) return fms_fail("attention_prefill: shared memory of %zu bytes refused: %s", F32_PREFILL_SMEM, cudaGetErrorString(e));
     configured = true;
   }
-  attn_prefill_kernel<float><<<dim3(n_tiles, nheads), 128, smem, stream>>>(a, tiles);
+  if ((long)n_tiles * nheads > 0x7fffffffL) return fms_fail("attention_prefill: %ld thread blocks", (long)n_tiles * nheads);
+  fms_launch(attn_prefill_f32_kernel, dim3((unsigned)(n_tiles * nheads)), dim3(128), F32_PREFILL_SMEM, stream, a, tiles, n_tiles);
   return fms_launch_status("attention_prefill");
 }
 
