@@ -68,6 +68,14 @@ struct AttnArgs {
   // key, r1 * ln(1 + r2 * (query position - key position))
   const float2* distance;
   long q_stride;  // values from one token's queries to the next's (nheads * HD, or the row of a wider matrix); set by every entry
+  // not null: keys and values are no cache but rows of a matrix, position p of sequence s in row key_base[s] + p, head h's
+  // in columns h * kv_cols .. + HD of the two matrices; the results' rows are out_stride values apart (tcgen05 prefill only)
+  const int* key_base = nullptr;
+  int kv_cols = 0;
+  long out_stride = 0;
+  // with key_base, not null: a row's result is multiplied by the sigmoid of gate[row * gate_stride + head]
+  const __nv_bfloat16* gate = nullptr;
+  long gate_stride = 0;
 };
 
 // The first position that the query at `pos` sees (its last is pos).  It never decreases as pos grows, so a tile of
@@ -656,6 +664,26 @@ int launch_decode(const char* what, const AttnArgs& a, int dtype, int n_seqs, in
   }
   return fms_launch_status(what);
 }
+#if FMS_ATTENTION_TC
+int launch_prefill_tc(const char* what, const CUtensorMap& map_k, const CUtensorMap& map_v, const AttnArgs& a, const int* tiles,
+                      int n_tiles, int* error_flag, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+    if (e != cudaSuccess) return fms_fail("%s: shared memory of %zu bytes refused: %s", what, TC_SMEM, cudaGetErrorString(e));
+    configured = true;
+  }
+  const int group = a.nheads / a.kvheads;
+  const int gh = tc_heads_per_block(group);
+  const long blocks = (long)n_tiles * a.kvheads * ((group + gh - 1) / gh);
+  if (blocks > 0x7fffffffL) return fms_fail("%s: %ld thread blocks", what, blocks);
+  fms_launch(a.distance ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>, dim3((unsigned)blocks), dim3(192), TC_SMEM, stream,
+             map_k, map_v, a, tiles, n_tiles, error_flag);
+  return fms_launch_status(what);
+}
+#endif
 }  // namespace
 
 FMS_API int fms_attn_head_dim() { return HD; }
@@ -692,21 +720,7 @@ static int attention_prefill(const void* q, void* out, int dtype, const void* ke
     CUtensorMap map_k, map_v;
     const long rows = (long)pool_blocks * kvheads * BLK;
     if (make_map(&map_k, keys, rows, HD, BLK) || make_map(&map_v, values, rows, HD, BLK)) return 1;
-    static bool configured_tc = false;
-    if (!configured_tc) {
-      cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-      if (e != cudaSuccess) return fms_fail("attention_prefill: shared memory of %zu bytes refused: %s", TC_SMEM, cudaGetErrorString(e));
-      configured_tc = true;
-    }
-    const int group = nheads / kvheads;
-    const int gh = tc_heads_per_block(group);
-    const long blocks = (long)n_tiles * kvheads * ((group + gh - 1) / gh);
-    if (blocks > 0x7fffffffL) return fms_fail("attention_prefill: %ld thread blocks", blocks);
-    fms_launch(a.distance ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>, dim3((unsigned)blocks), dim3(192), TC_SMEM,
-               stream, map_k, map_v, a, tiles, n_tiles, error_flag);
-    return fms_launch_status("attention_prefill");
+    return launch_prefill_tc("attention_prefill", map_k, map_v, a, tiles, n_tiles, error_flag, stream);
   }
 #endif
   if (dtype == FMS_BF16) {
@@ -743,6 +757,35 @@ FMS_API int fms_attention_prefill(const void* q, void* out, int dtype, const voi
   return attention_prefill(q, out, dtype, keys, values, table, table_stride, block_tokens, slots, first_row, len_after,
                            tiles, n_tiles, nheads, kvheads, head_dim, scale, window, pool_blocks, table_rows, error_flag,
                            nullptr, stream);
+}
+
+// Prefill attention with a key and a value head for every query head, over keys and values that lie in the rows of a matrix
+// instead of a cache: position p of sequence s in row key_base[s] + p (0 <= that < rows for every position a query of s
+// sees), kv_stride values from row to row, kv_cols from head to head.  bfloat16, head sizes that the tcgen05 kernel has.
+// sink as above, or null; gate (bfloat16, a logit a row and head, gate_stride values from row to row): or null.
+FMS_API int fms_attention_prefill_rows(const void* q, long q_stride, void* out, long out_stride, const void* keys, const void* values,
+                                       long kv_stride, int kv_cols, long rows, const int* key_base, const int* first_row,
+                                       const int* len_after, const int* tiles, int n_tiles, int nheads, int head_dim, float scale,
+                                       int window, const float* sink, const void* gate, long gate_stride, int* error_flag,
+                                       cudaStream_t stream) {
+  if (n_tiles <= 0) return 0;
+#if FMS_ATTENTION_TC
+  if (check_args("attention_prefill_rows", nheads, nheads, head_dim, BLK)) return 1;
+  if (check_mask("attention_prefill_rows", window, 0, 0.f)) return 1;
+  if (check_queries(q, FMS_BF16, q_stride, nheads)) return 1;
+  if (!(scale > 0.f)) return fms_fail("attention_prefill_rows: the scale of the scores is %g; it must be positive", (double)scale);
+  if (rows <= 0 || rows > 0x7fffffffL || kv_stride % 8 || kv_cols % 64 || (uintptr_t)keys % 16 || (uintptr_t)values % 16 ||
+      kv_stride < (long)(nheads - 1) * kv_cols + HD || out_stride < (long)nheads * HD || out_stride % 8 || (uintptr_t)out % 16)
+    return fms_fail("attention_prefill_rows: %ld rows of %ld values, %d heads %d values apart", rows, kv_stride, nheads, kv_cols);
+  AttnArgs a{q, out, keys, values, nullptr, 0, nullptr, first_row, len_after, nheads, nheads, scale, window, 0, 0, sink, 0, 0.f, nullptr,
+             q_stride, key_base, kv_cols, out_stride, (const __nv_bfloat16*)gate, gate_stride};
+  CUtensorMap map_k, map_v;
+  const int cols = (nheads - 1) * kv_cols + HD;
+  if (make_map(&map_k, keys, rows, cols, BLK, kv_stride) || make_map(&map_v, values, rows, cols, BLK, kv_stride)) return 1;
+  return launch_prefill_tc("attention_prefill_rows", map_k, map_v, a, tiles, n_tiles, error_flag, stream);
+#else
+  return fms_fail("attention_prefill_rows: head size %d has no tcgen05 kernel", HD);
+#endif
 }
 
 // The same with a sink per head in the softmax's denominator (sink: [nheads] float32 on the device).

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
   const int n_new = a.first_row[seq + 1] - row_begin;
   const int len = a.len_after[seq];
   const int len_before = len - n_new;
-  const int slot = a.slots[seq];
+  const int slot = a.key_base ? 0 : a.slots[seq];
   const int pos_here = min(pp, n_new - r0);
   const int p_first = len_before + r0, p_last = p_first + pos_here - 1;
   const int kb_lo = first_visible(a, p_first) / BLK;
@@ -127,18 +127,20 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
     if (elect_one()) {
       for (int i = 0; i < nblocks && !*failed; ++i) {
         const int s = i % TC_STAGES;
-        const int blk = block_of(a, slot, kb_lo + i);
+        const int blk = a.key_base ? 0 : block_of(a, slot, kb_lo + i);
         unsigned char* kdst = kv + (size_t)s * 2 * TC_KV_TILE;
         unsigned char* vdst = kdst + TC_KV_TILE;
-        const int row = (max(blk, 0) * a.kvheads + kvh) * BLK;  // first row of the block in the [positions, HD] view
+        // first row and column of the block in the [positions, HD] view of the cache, or in the matrix
+        const int row = a.key_base ? a.key_base[seq] + (kb_lo + i) * BLK : (max(blk, 0) * a.kvheads + kvh) * BLK;
+        const int col = a.key_base ? kvh * a.kv_cols : 0;
         if (!wait_or_abort(&k_empty[s], ((i / TC_STAGES) & 1) ^ 1, failed)) break;
         mbar_arrive_expect_tx(&k_full[s], TC_KV_TILE);
 #pragma unroll
-        for (int c = 0; c < HD / 64; ++c) tma_load_2d(kdst + c * (BLK * 128), &map_k, c * 64, row, &k_full[s]);
+        for (int c = 0; c < HD / 64; ++c) tma_load_2d(kdst + c * (BLK * 128), &map_k, col + c * 64, row, &k_full[s]);
         if (!wait_or_abort(&v_empty[s], ((i / TC_STAGES) & 1) ^ 1, failed)) break;
         mbar_arrive_expect_tx(&v_full[s], TC_KV_TILE);
 #pragma unroll
-        for (int c = 0; c < HD / 64; ++c) tma_load_2d(vdst + c * (BLK * 128), &map_v, c * 64, row, &v_full[s]);
+        for (int c = 0; c < HD / 64; ++c) tma_load_2d(vdst + c * (BLK * 128), &map_v, col + c * 64, row, &v_full[s]);
       }
     }
   } else if (warp == 1) {
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
     bool ok = true;
     for (int i = 0; i < nblocks && ok; ++i) {
       const int kb = kb_lo + i, s = i % TC_STAGES;
-      const int blk = block_of(a, slot, kb);  // asked for here: it is needed after the exponentials
+      const int blk = a.key_base ? 0 : block_of(a, slot, kb);  // asked for here: it is needed after the exponentials
       if (tabled) {  // while the scores are on their way; distances of keys after a row count as 0 (they are masked)
         __syncwarp();
         float away[3];  // the distances of this lane's entries, at most 96 a head
@@ -319,9 +321,12 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
     if (ok && __all_sync(0xffffffffu, wait_or_abort(&o_done[(nblocks - 1) & 1], ((nblocks - 1) >> 1) & 1, failed))) {
       tc_fence_after();
       if (a.sink != nullptr && row_ok) l += exp2f(a.sink[kvh * group + g0 + gi] * LOG2E - (m_ref == -INFINITY ? 0.f : m_ref));
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if (a.gate != nullptr && row_ok)
+        inv /= 1.f + __expf(-__bfloat162float(a.gate[(size_t)(row_begin + r0 + pi) * a.gate_stride + kvh * group + g0 + gi]));
       __nv_bfloat16* o_row = (__nv_bfloat16*)a.out +
-                             ((size_t)(row_begin + r0 + (row_ok ? pi : 0)) * a.nheads + kvh * group + g0 + (row_ok ? gi : 0)) * HD;
+                             (size_t)(row_begin + r0 + (row_ok ? pi : 0)) * (a.key_base ? a.out_stride : (long)a.nheads * HD) +
+                             (size_t)(kvh * group + g0 + (row_ok ? gi : 0)) * HD;
 #pragma unroll
       for (int c0 = 0; c0 < HD; c0 += 32) {
         float o[32];

@@ -30,29 +30,34 @@ constexpr int KT = 32;      // keys brought into shared memory at a time
 constexpr int HG = 8;       // heads a block takes
 constexpr int THREADS = 256;
 
-// Value j (< 2 half) of a rotated run: pairs (2i, 2i + 1), or with `halves` (i, i + half), turned by position * inv_freq[i];
-// rot_mult multiplies sine and cosine (1 for a plain rotation).
+// A block a token: the token's sines and cosines once (a pair a thread, in shared memory) for all heads, then a pair of
+// every head's rotated run a thread.  Each head's query goes to a row of q_out of `q_width` values, its rotated part from
+// column q_rot on; with q_copy its unrotated part too, to the columns before (queries that stay in the heads' own space:
+// q_rot = dim).  [c | kr] of the token goes into the cache, c normed and kr turned.  Pairs are (2i, 2i + 1), or with
+// `halves` (i, i + half), turned by position * inv_freq[i]; rot_mult multiplies sines and cosines.  With a sine and a cosine
+// for every value of every head, as before, 2,048 tokens of 32 heads of 96 + 32 took 19.5 us.
 template <typename T>
-__device__ __forceinline__ float rotated(const T* src, int j, int half, int halves, float position, const float* inv_freq,
-                                         float rot_mult) {
-  const int pair = halves ? (j < half ? j : j - half) : j >> 1;
-  const bool second = halves ? j >= half : (j & 1);
-  float sn, cs;
-  sincosf(position * inv_freq[pair], &sn, &cs);
-  sn *= rot_mult;
-  cs *= rot_mult;
-  const float a = to_f32(src[halves ? pair : 2 * pair]), b = to_f32(src[halves ? pair + half : 2 * pair + 1]);
-  return second ? b * cs + a * sn : a * cs - b * sn;
+__device__ __forceinline__ void rotate_run(const T* src, T* dst, int i, int half, int halves, int rot, float2 turn) {
+  if (i < half) {
+    const int ja = halves ? i : 2 * i, jb = halves ? i + half : 2 * i + 1;
+    const float a = to_f32(src[ja]), b = to_f32(src[jb]);
+    dst[ja] = from_f32<T>(a * turn.y - b * turn.x);
+    dst[jb] = from_f32<T>(b * turn.y + a * turn.x);
+  } else {  // behind the rotated values: as they are
+    const int j = i + half;
+    if (j < rot) dst[j] = src[j];
+  }
 }
 
 template <typename T, typename TG>
 __global__ void __launch_bounds__(128) latent_prepare_kernel(
-    const T* __restrict__ proj, int proj_width, T* __restrict__ q_full, const TG* __restrict__ c_gain, float eps,
-    const float* __restrict__ inv_freq, int rot_dims, const int* __restrict__ positions,
+    const T* __restrict__ proj, int proj_width, T* __restrict__ q_out, int q_width, int q_rot, int q_copy,
+    const TG* __restrict__ c_gain, float eps, const float* __restrict__ inv_freq, int rot_dims, const int* __restrict__ positions,
     const int* __restrict__ position_ids, const int* __restrict__ token_seq, const int* __restrict__ slots,
     T* __restrict__ cache, const int* __restrict__ table, int table_stride, int block_tokens, int heads, int dim, int rot,
     int rank, int write_cache, int n_seqs, int n_slots, int n_blocks, int* __restrict__ error_flag, int halves,
     float rot_mult, const T* __restrict__ kv, int kv_width) {
+  extern __shared__ float2 turns[];  // [rot_dims / 2]: sine, cosine
   __shared__ float scratch[33];
   pdl_launch_dependents();
   pdl_wait();
@@ -61,18 +66,34 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(
   const int q_cols = heads * (dim + rot);
   const float position = (float)(position_ids ? ld_fresh(position_ids + t) : ld_fresh(positions + t));
   const int width = rank + rot;
+  const int half = rot_dims / 2, units = rot - half;  // of a run: its pairs, and the values behind them one by one
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    float sn, cs;
+    sincosf(position * inv_freq[i], &sn, &cs);
+    turns[i] = make_float2(sn * rot_mult, cs * rot_mult);
+  }
+  __syncthreads();
   // the rotated part of every head's query
-  const int half = rot_dims / 2;
-  for (int i = threadIdx.x; i < heads * rot; i += blockDim.x) {
-    const int h = i / rot, j = i - h * rot;
-    const T* src = row + (size_t)h * (dim + rot) + dim;
-    float v;
-    if (j < 2 * half) {
-      v = rotated(src, j, half, halves, position, inv_freq, rot_mult);
+  for (int i = threadIdx.x; i < heads * units; i += blockDim.x) {
+    const int h = i / units, u = i - h * units;
+    rotate_run(row + (size_t)h * (dim + rot) + dim, q_out + ((size_t)t * heads + h) * q_width + q_rot, u, half, halves, rot,
+               u < half ? turns[u] : make_float2(0.f, 0.f));
+  }
+  if (q_copy) {
+    constexpr int V = 16 / sizeof(T);
+    T* dst = q_out + (size_t)t * heads * q_width;
+    if (dim % V == 0 && rot % V == 0 && q_width % V == 0 && proj_width % V == 0 && (reinterpret_cast<uintptr_t>(proj) & 15) == 0) {
+      const int pieces = dim / V;
+      for (int i = threadIdx.x; i < heads * pieces; i += blockDim.x) {
+        const int h = i / pieces, d = (i - h * pieces) * V;
+        *reinterpret_cast<uint4*>(dst + (size_t)h * q_width + d) = *reinterpret_cast<const uint4*>(row + (size_t)h * (dim + rot) + d);
+      }
     } else {
-      v = to_f32(src[j]);
+      for (int i = threadIdx.x; i < heads * dim; i += blockDim.x) {
+        const int h = i / dim, d = i - h * dim;
+        dst[(size_t)h * q_width + d] = row[(size_t)h * (dim + rot) + d];
+      }
     }
-    q_full[((size_t)t * heads + h) * width + rank + j] = from_f32<T>(v);
   }
   if (!write_cache) return;
   const int seq = token_seq[t];
@@ -96,16 +117,30 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(
   }
   const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
   for (int d = threadIdx.x; d < rank; d += blockDim.x) dst[d] = from_f32<T>(to_f32(c[d]) * inv * to_f32(c_gain[d]));
-  const T* kr = c + rank;
-  for (int j = threadIdx.x; j < rot; j += blockDim.x) {
-    float v;
-    if (j < 2 * half) {
-      v = rotated(kr, j, half, halves, position, inv_freq, rot_mult);
-    } else {
-      v = to_f32(kr[j]);
-    }
-    dst[rank + j] = from_f32<T>(v);
+  for (int i = threadIdx.x; i < units; i += blockDim.x)
+    rotate_run(c + rank, dst + rank, i, half, halves, rot, i < half ? turns[i] : make_float2(0.f, 0.f));
+}
+
+// The cached rows of a step's sequences one behind the other: row r of `out` is position first[s] + r - start[s] of
+// sequence s for start[s] <= r < start[s + 1].  16-byte pieces; eight warps a block, a row a warp.
+__global__ void __launch_bounds__(256) latent_gather_kernel(const uint4* cache, const int* table, int table_stride, int block_tokens,
+                                                            const int* slots, const int* start, const int* first, int n_seqs,
+                                                            uint4* out, int pieces, int n_rows, int n_slots, int n_blocks) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= n_rows) return;
+  int lo = 0, hi = n_seqs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (start[mid] <= r) lo = mid; else hi = mid - 1;
   }
+  const int slot = slots[lo], pos = first[lo] + r - start[lo];
+  if (!FMS_IN(slot, n_slots) || !FMS_IN(pos / block_tokens, table_stride)) return;
+  const int blk = table[(size_t)slot * table_stride + pos / block_tokens];
+  const bool held = blk >= 0 && blk < n_blocks;  // a position without a block (none that a query sees): zeros
+  const uint4* src = cache + ((size_t)(held ? blk : 0) * block_tokens + pos % block_tokens) * pieces;
+  for (int i = lane; i < pieces; i += 32) out[(size_t)r * pieces + i] = held ? src[i] : make_uint4(0, 0, 0, 0);
 }
 
 // A run of columns of a wider matrix, normed row by row: out[t, :n] = x[t, off : off + n] / sqrt(mean(.^2) + eps) * gain
@@ -585,22 +620,36 @@ FMS_API int fms_latent_query_norm(const void* x, int dtype, int stride, int n, c
   return fms_launch_status("latent_query_norm");
 }
 
-FMS_API int fms_latent_prepare(const void* proj, int dtype, int proj_width, void* q_full, const void* c_gain, int gain_dtype,
-                               float eps, const float* inv_freq, int rot_dims, const int* positions,
-                               const int* position_ids, const int* token_seq, const int* slots, void* cache,
+// q_width, q_rot, q_copy: see the kernel (queries into the latent's space: rank + rot, rank, 0).
+FMS_API int fms_latent_prepare(const void* proj, int dtype, int proj_width, void* q_out, int q_width, int q_rot, int q_copy,
+                               const void* c_gain, int gain_dtype, float eps, const float* inv_freq, int rot_dims,
+                               const int* positions, const int* position_ids, const int* token_seq, const int* slots, void* cache,
                                const int* table, int table_stride, int block_tokens, int n_tokens, int heads, int dim,
                                int rot, int rank, int write_cache, int n_seqs, int n_slots, int n_blocks, int* error_flag,
                                int halves, float rot_mult, const void* kv, int kv_width, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  if (heads <= 0 || dim < 0 || rot < 0 || rank <= 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1))
-    return fms_fail("latent_prepare: heads %d, dim %d, rot %d (%d rotated), rank %d", heads, dim, rot, rot_dims, rank);
+  if (heads <= 0 || dim < 0 || rot < 0 || rank <= 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) || rot_dims > 8192 ||
+      q_rot < (q_copy ? dim : 0) || q_width < q_rot + rot)
+    return fms_fail("latent_prepare: heads %d, dim %d, rot %d (%d rotated), rank %d, rows of %d with the rotated part at %d", heads, dim,
+                    rot, rot_dims, rank, q_width, q_rot);
   FMS_DISPATCH_DTYPE(dtype, T, FMS_DISPATCH_DTYPE(gain_dtype, TG,
-                     fms_launch(latent_prepare_kernel<T, TG>, dim3(n_tokens), dim3(128), 0, stream, (const T*)proj,
-                                proj_width, (T*)q_full, (const TG*)c_gain, eps, inv_freq, rot_dims, positions,
-                                position_ids, token_seq, slots, (T*)cache, table, table_stride, block_tokens, heads, dim,
-                                rot, rank, write_cache, n_seqs, n_slots, n_blocks, error_flag, halves, rot_mult,
+                     fms_launch(latent_prepare_kernel<T, TG>, dim3(n_tokens), dim3(128), rot_dims / 2 * sizeof(float2), stream,
+                                (const T*)proj, proj_width, (T*)q_out, q_width, q_rot, q_copy, (const TG*)c_gain, eps, inv_freq,
+                                rot_dims, positions, position_ids, token_seq, slots, (T*)cache, table, table_stride, block_tokens,
+                                heads, dim, rot, rank, write_cache, n_seqs, n_slots, n_blocks, error_flag, halves, rot_mult,
                                 (const T*)kv, kv_width)));
   return fms_launch_status("latent_prepare");
+}
+
+// row_bytes: bytes of a cached row, a multiple of 16
+FMS_API int fms_latent_gather(const void* cache, int row_bytes, const int* table, int table_stride, int block_tokens, const int* slots,
+                              const int* start, const int* first, int n_seqs, void* out, int n_rows, int n_slots, int n_blocks,
+                              cudaStream_t stream) {
+  if (n_rows <= 0 || n_seqs <= 0) return 0;
+  if (row_bytes <= 0 || row_bytes % 16 || (uintptr_t)cache % 16 || (uintptr_t)out % 16) return fms_fail("latent_gather: rows of %d bytes", row_bytes);
+  fms_launch(latent_gather_kernel, dim3((n_rows + 7) / 8), dim3(256), 0, stream, (const uint4*)cache, table, table_stride, block_tokens,
+             slots, start, first, n_seqs, (uint4*)out, row_bytes / 16, n_rows, n_slots, n_blocks);
+  return fms_launch_status("latent_gather");
 }
 
 // n_splits == 1: every row takes all its keys in one block (a prompt's rows); else splits of fms_latent_split_tokens()

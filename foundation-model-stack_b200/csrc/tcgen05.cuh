@@ -197,12 +197,13 @@ EncodeTiled encode_tiled() {
   return fn;
 }
 
-// a [rows, K] bfloat16 matrix, K contiguous, loaded in boxes of `box_rows` rows x 64 k with the 128-byte swizzle
-int make_map(CUtensorMap* map, const void* base, long rows, int K, int box_rows = 128) {
+// a [rows, K] bfloat16 matrix, K contiguous, rows `stride` values apart (0: K), loaded in boxes of `box_rows` rows x 64 k
+// with the 128-byte swizzle
+int make_map(CUtensorMap* map, const void* base, long rows, int K, int box_rows = 128, long stride = 0) {
   EncodeTiled enc = encode_tiled();
   if (enc == nullptr) return fms_fail("gemm_tc: the driver does not export cuTensorMapEncodeTiled");
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  const cuuint64_t strides[1] = {(cuuint64_t)(stride ? stride : K) * 2};
   const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   const cuuint32_t elem[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,

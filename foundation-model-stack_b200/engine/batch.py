@@ -38,6 +38,7 @@ class Batch:
         self.want_rows: Optional[torch.Tensor] = None  # [n_wanted] int32 rows whose logits are returned
         self.n_wanted = 0
         self._tiles = {}
+        self.len_before_host: Optional[List[int]] = None  # lengths before the step, where the host made the batch of lists
         self.scratch = {}  # what a step's layers share (a table of rotation angles, ...); emptied when a step starts
 
     @staticmethod
@@ -97,6 +98,23 @@ class Batch:
                 base += n
             packed = torch.tensor([v for p in rows for v in p] + first, dtype=torch.int32).to(self.tokens.device)
             self._tiles[key] = (packed[: 2 * len(rows)].view(-1, 2), packed[2 * len(rows):])
+        return self._tiles[key]
+
+    def key_rows(self, window: int):
+        """(start, first, base: int32 [n_seqs + 1], [n_seqs], [n_seqs]; rows): the keys that a step of several tokens sees,
+        laid one sequence behind the other.  Sequence i's are the rows start[i] .. start[i + 1] and begin at its position
+        first[i] (0, or with a window the first of the cache block that holds the earliest key seen); its position p is row
+        base[i] + p."""
+        key = ("keys", window)
+        if key not in self._tiles:
+            start, first = [0], []
+            for before, n in zip(self.len_before_host, self.num_new):
+                first.append(max(0, before - window + 1) // 64 * 64 if window > 0 else 0)
+                start.append(start[-1] + before + n - first[-1])
+            base = [a - b for a, b in zip(start, first)]
+            packed = torch.tensor(start + first + base, dtype=torch.int32).to(self.tokens.device)
+            s = len(first)
+            self._tiles[key] = (packed[: s + 1], packed[s + 1: 2 * s + 1], packed[2 * s + 1:], start[-1])
         return self._tiles[key]
 
     def query_tiles(self, tile_rows: int) -> torch.Tensor:

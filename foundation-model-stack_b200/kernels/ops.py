@@ -70,7 +70,9 @@ _SIGNATURES = {
     "fms_gated_clamped": [_P, _P, _I, _I, _I, _F, _F, _P],
     "fms_latent_attention_prefill_bf16": [_P, _P, _P, _P, _L, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                                           _F, _I, _I, _I, _P, _I, _P, _P, _I, _P],
-    "fms_latent_prepare": [_P, _I, _I, _P, _P, _I, _F, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
+    "fms_latent_gather": [_P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _I, _I, _I, _P],
+    "fms_attention_prefill_rows": [_P, _L, _P, _L, _P, _P, _L, _I, _L, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P, _L, _P, _P],
+    "fms_latent_prepare": [_P, _I, _I, _P, _I, _I, _I, _P, _I, _F, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
                            _I, _I, _P, _I, _F, _P, _I, _P],
     "fms_latent_query_norm": [_P, _I, _I, _I, _P, _I, _F, _P, _I, _P],
     "fms_latent_attention": [_P, _P, _I, _P, _P, _L, _P, _I, _P, _I, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I,
@@ -1249,18 +1251,21 @@ USE_LATENT_MMA = os.environ.get("FMS_B200_LATENT_MMA", "1") != "0"  # 0: a promp
 
 def latent_prepare(proj: torch.Tensor, q_full: torch.Tensor, c_gain: torch.Tensor, eps: float, inv_freq: torch.Tensor,
                    rot_dims: int, batch, view, heads: int, dim: int, rot: int, rank: int, writes_cache: bool = True,
-                   halves: bool = False, rot_mult: float = 1.0, kv: Optional[torch.Tensor] = None) -> None:
+                   halves: bool = False, rot_mult: float = 1.0, kv: Optional[torch.Tensor] = None, own_space: bool = False) -> None:
     """From the fused projection [q heads (dim + rot each) | c (rank) | kr (rot) | ...] of a step's rows: norms c,
     rotates kr and every head's rot part by the row's position, writes [c | kr] into the cache at the row's place and
     the rotated query parts into q_full[:, h, rank:].  ``kv``: [c | kr] are the first columns of this matrix instead
     (queries that come from a projection of their own; ``proj`` then holds the query heads only).  ``halves``: value i
-    of a rotated run turns with value i + rot_dims / 2 instead of its neighbour; ``rot_mult`` multiplies sines and cosines."""
+    of a rotated run turns with value i + rot_dims / 2 instead of its neighbour; ``rot_mult`` multiplies sines and cosines.
+    ``own_space``: ``q_full`` is [tokens, heads, dim + rot] and takes every head's whole query, its rot part turned."""
+    if tuple(q_full.shape) != (proj.shape[0], heads, (dim if own_space else rank) + rot):
+        raise KernelError(f"latent_prepare: queries {tuple(q_full.shape)} for {heads} heads of {dim} + {rot}, rank {rank}")
     if kv is not None and (kv.dtype != proj.dtype or kv.shape[0] != proj.shape[0] or kv.shape[1] < rank + rot):
         raise KernelError("latent_prepare: the latent's matrix has the projection's dtype and rows, and rank + rot columns")
     if view.keys.dtype != proj.dtype or q_full.dtype != proj.dtype:
         raise KernelError(f"cache is {view.keys.dtype}, activations are {proj.dtype}")
-    _call("latent_attention", "fms_latent_prepare", _ptr(proj), _code(proj.dtype), proj.shape[1], _ptr(q_full), _ptr(c_gain),
-          _code(c_gain.dtype), float(eps), _ptr(inv_freq), int(rot_dims), _ptr(batch.positions),
+    _call("latent_attention", "fms_latent_prepare", _ptr(proj), _code(proj.dtype), proj.shape[1], _ptr(q_full),
+          q_full.shape[2], dim if own_space else rank, 1 if own_space else 0, _ptr(c_gain), _code(c_gain.dtype), float(eps), _ptr(inv_freq), int(rot_dims), _ptr(batch.positions),
           _ptr(getattr(batch, "position_ids", None)), _ptr(batch.token_seq), _ptr(batch.slots), _ptr(view.keys),
           _ptr(view.table), view.table.shape[1], view.block_tokens, proj.shape[0], heads, dim, rot, rank,
           1 if writes_cache else 0, batch.slots.shape[0], view.table.shape[0], view.keys.shape[0],
@@ -1276,6 +1281,62 @@ def latent_query_norm(proj: torch.Tensor, offset: int, n: int, gain: torch.Tenso
     out = torch.empty((proj.shape[0], n), dtype=proj.dtype, device=proj.device)
     _call("latent_attention", "fms_latent_query_norm", _ptr(proj) + offset * proj.element_size(), _code(proj.dtype),
           proj.shape[1], n, _ptr(gain), _code(gain.dtype), float(eps), _ptr(out), proj.shape[0], _stream())
+    return out
+
+
+# Bytes of keys and values that ``latent_attention_expanded`` makes at a time (heads are taken a few at a time beyond it)
+LATENT_EXPANDED_BYTES = 512 << 20
+# Nanoseconds that decide between the two forms of a prompt's latent attention.  In the latent's space a block walks a
+# sequence's keys at LATENT_WALK_NS a key, and a (query, key) pair of a head takes LATENT_PAIR_NS where all multiprocessors
+# are busy; making a key and a value of a head and attending over them takes LATENT_KEY_NS.  Measured with heads of 96 + 32
+# over a latent of 512, 32 heads, whole layers, latent's space / heads' space in us: a prompt of 64 tokens 45 / 41, of 256
+# 88 / 53, two of 2,048 together 873 / 209; 16 tokens onto 1,024 cached ones 244 / 68, onto 8,000 1,356 / 220; 64 tokens of
+# four sequences onto 1,000 each 211 / 106, of eight onto 1,000 each 219 / 138.
+LATENT_WALK_NS, LATENT_PAIR_NS, LATENT_KEY_NS = 160.0, 0.02, 0.44
+
+
+def latent_prefers_expanded(batch, window: int, heads: int) -> bool:
+    """Whether a step's rows attend over keys and values made of the cached latents (``latent_attention_expanded``) rather
+    than in the latent's space: unless so few queries share a key that its making does not pay."""
+    if batch.decode or getattr(batch, "len_before_host", None) is None:
+        return False
+    pairs = keys = longest = 0
+    for before, n in zip(batch.len_before_host, batch.num_new):
+        seen = min(before + n, window + n) if window > 0 else before + n
+        keys, longest = keys + seen, max(longest, seen)
+        pairs += n * min(before + (n + 1) // 2, seen)
+    return max(longest * LATENT_WALK_NS, pairs * heads * LATENT_PAIR_NS) > keys * heads * LATENT_KEY_NS
+
+
+def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor, sink: Optional[torch.Tensor], heads: int,
+                              head_dim: int, scale: float, window: int = 0, gate: Optional[torch.Tensor] = None,
+                              gate_offset: int = 0) -> torch.Tensor:
+    """The same attention in the heads' own space, for steps of many tokens: the cached rows [c | kr] that the step sees
+    are gathered, every head's keys and values made of them in one product, and the tcgen05 prefill kernel runs over those.
+    ``q`` [tokens, heads, head_dim]; ``expand`` [heads, 2 * head_dim, rank + rot]: head h's matrix that makes [key | value] of
+    a cached row; ``sink`` float32 or None; ``gate`` as in ``latent_attention``.  Returns [tokens, heads * head_dim]."""
+    n, width = q.shape[0], expand.shape[2]
+    if tuple(expand.shape[:2]) != (heads, 2 * head_dim) or view.keys.shape[-1] != width or q.dtype != torch.bfloat16 \
+            or (sink is not None and sink.dtype != torch.float32) or (gate is not None and gate.dtype != q.dtype):
+        raise KernelError(f"latent_attention_expanded: {heads} heads of {head_dim}, matrices {tuple(expand.shape)}, rows of {view.keys.shape[-1]}")
+    start, first, base, rows = batch.key_rows(window)
+    cached = torch.empty((rows, width), dtype=q.dtype, device=q.device)
+    _call("latent_attention", "fms_latent_gather", _ptr(view.keys), width * q.element_size(), _ptr(view.table), view.table.shape[1],
+          view.block_tokens, _ptr(batch.slots), _ptr(start), _ptr(first), batch.n_seqs, _ptr(cached), rows, view.table.shape[0],
+          view.keys.shape[0], _stream())
+    out = torch.empty((n, heads * head_dim), dtype=q.dtype, device=q.device)
+    lib = _attention_library(head_dim)
+    tiles = batch.query_tiles(attention_constants(head_dim, q.dtype, 1, 1)[1])
+    step = max(1, min(heads, LATENT_EXPANDED_BYTES // (rows * 2 * head_dim * q.element_size())))
+    for h in range(0, heads, step):
+        m = min(step, heads - h)
+        kv = linear(cached, expand[h:h + m].view(m * 2 * head_dim, width))
+        at = h * head_dim * q.element_size()
+        _call(lib, "fms_attention_prefill_rows", _ptr(q) + at, heads * head_dim, _ptr(out) + at, heads * head_dim, _ptr(kv),
+              _ptr(kv) + head_dim * kv.element_size(), kv.shape[1], 2 * head_dim, rows, _ptr(base), _ptr(batch.first_row),
+              _ptr(batch.len_after), _ptr(tiles), tiles.shape[0], m, head_dim, float(scale), int(window),
+              None if sink is None else _ptr(sink) + h * 4, None if gate is None else _ptr(gate) + (gate_offset + h) * gate.element_size(),
+              0 if gate is None else gate.shape[1], _ptr(error_flag(q.device)), _stream())
     return out
 
 

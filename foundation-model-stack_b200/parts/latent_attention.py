@@ -16,6 +16,10 @@ q_h . Wuk,h c = (Wuk,h^T q_h) . c, so the query is taken into the latent's space
 ``uk`` transposed once at load time), attention runs over the latent rows as they lie, and the head's result, a
 weighted sum of latents, goes through Wuv,h afterwards.  [Wq; Wdkv; Wg] is one fused projection.
 
+A step of many tokens of a bfloat16 model whose heads' keys and values are equally long (64 or 128 values) goes the other
+way where that is the shorter one (``ops.latent_prefers_expanded``): every head's keys and values are made of the cached rows
+in one product (``_expand``: [Wuk,h 0; 0 1; Wuv,h 0] takes a row [c | kr] to [k_h | v_h]), and attention runs over those.
+
 Options of the ``MixerSpec``: ``rot`` (rotated values per head), ``vdim``, ``rank``, ``rot_dims``; ``head_dim`` is the
 unrotated size, ``position.theta`` the rotation's base, ``scale`` the factor on the scores.  Further options, each of
 which leaves the above as it is when absent:
@@ -82,7 +86,7 @@ class LatentAttention(Part):
         self.declare("uk", (self.heads * self.dim, self.rank), role="matrix")
         self.declare("uv", (self.heads * self.vdim, self.rank), role="matrix")
         self.dense = self.add("dense", Linear(self.heads * self.vdim, spec.dim, False))
-        self._uk_t = self._uv = self._inv_freq = None
+        self._uk_t = self._uv = self._inv_freq = self._expand = self._sink = None
 
     def finalize(self, device, dtype) -> None:
         super().finalize(device, dtype)
@@ -90,6 +94,13 @@ class LatentAttention(Part):
         # [heads, rank, dim]: head h's matrix that takes its unrotated query into the latent's space
         self._uk_t = uk.view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
         self._uv = self.tensor("uv").view(self.heads, self.vdim, self.rank)
+        if self._expands(dtype):
+            self._expand = torch.zeros((self.heads, 2 * self.vdim, self.rank + self.rot), dtype=dtype, device=uk.device)
+            self._expand[:, : self.dim, : self.rank] = uk.view(self.heads, self.dim, self.rank)
+            self._expand[:, self.dim: self.vdim, self.rank:] = torch.eye(self.rot, dtype=dtype, device=uk.device)
+            self._expand[:, self.vdim:, : self.rank] = self._uv
+            if self.has_sink:
+                self._sink = self.tensor("sink").float().contiguous()
         from .position import rotary_inverse_frequencies, rotary_multiplier
 
         # every frequency in float64, rounded to float32 once
@@ -98,20 +109,30 @@ class LatentAttention(Part):
         self._inv_freq = freq.to(torch.float32).to(device).contiguous()
         self.rot_mult = rotary_multiplier(scaling)
 
+    def _expands(self, dtype) -> bool:
+        """Whether the heads' keys and values can be made of the cached rows for the prefill kernel."""
+        return (dtype == torch.bfloat16 and all(self.tensor(n).dtype == dtype for n in ("uk", "uv")) and self.scale > 0.0
+                and self.dim + self.rot == self.vdim and self.vdim in (64, 128) and (self.rank + self.rot) % 8 == 0)
+
     def cache_request(self):
         return KVRequest(1, self.rank + self.rot, 0, planes=1)
 
     def forward(self, x, batch, cache_view, writes_cache: bool = True):
         n, width = x.shape[0], self.rank + self.rot
         proj = self.in_proj.forward(x)
-        q_full = torch.empty((n, self.heads, width), dtype=proj.dtype, device=proj.device)
+        expanded = self._expand is not None and ops.latent_prefers_expanded(batch, self.window, self.heads)
+        q_full = torch.empty((n, self.heads, self.vdim if expanded else width), dtype=proj.dtype, device=proj.device)
         kv, queries = None, proj
         if self.q_rank:
             kv = proj
             queries = self.q_up.forward(ops.latent_query_norm(proj, width, self.q_rank, self.tensor("q_norm"), self.eps))
         ops.latent_prepare(queries, q_full, self.tensor("latent_norm"), self.eps, self._inv_freq, self.rot_dims, batch,
                            cache_view, self.heads, self.dim, self.rot, self.rank, writes_cache, halves=self.halves,
-                           rot_mult=self.rot_mult, kv=kv)
+                           rot_mult=self.rot_mult, kv=kv, own_space=expanded)
+        if expanded:
+            o = ops.latent_attention_expanded(q_full, batch, cache_view, self._expand, self._sink, self.heads, self.vdim, self.scale,
+                                              self.window, proj if self.has_gate else None, self.gate_col)
+            return self.dense.forward(o)
         if self.dim:
             ops.grouped_linear(queries, self._uk_t, self.heads, n, self.rank, self.dim, queries.shape[1], self.dim + self.rot,
                                q_full, self.heads * width, width)
@@ -126,7 +147,8 @@ class LatentAttention(Part):
         return self.dense.forward(o)
 
     def kernel_libraries(self, dtype):
-        return super().kernel_libraries(dtype) + ["latent_attention", "grouped"]
+        return super().kernel_libraries(dtype) + ["latent_attention", "grouped"] + (
+            [f"attention_hd{self.vdim}"] if self._expand is not None else [])
 
 
 register_mixer("latent_attention", LatentAttention)

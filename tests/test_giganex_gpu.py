@@ -429,6 +429,26 @@ def test_windowed_latent_attention_alone(dtype, shape):
         close(step_through(mixer, x.cuda(), cuts, dt), want, dtype, loose=2)
 
 
+@pytest.mark.parametrize("shape", [(3, 96, 32, 128, 24, 64, 1, 20), (2, 48, 16, 64, 40, 40, 0, 257), (4, 32, 32, 64, 16, 96, 1, 64),
+                                   (2, 96, 32, 128, 24, 512, 0, 1)])
+def test_windowed_latent_attention_in_the_heads_own_space(monkeypatch, shape):
+    """Only the cache blocks that a step's windows reach are gathered (earlier ones have been given back)."""
+    from fms_b200.kernels import ops
+
+    heads, dim, rd, vdim, qr, kr, scaled, window = shape
+    sc = {"factor": 8.0, "original": 96, "fast": 4.0, "slow": 1.0} if scaled else None
+    m = gm.latent(heads, dim, rd, vdim, qr, kr, 300.0, sc, 0.7 * (dim + rd) ** -0.5, window, None)["mixer"]
+    g = torch.Generator().manual_seed(sum(shape))
+    w = latent_tensors(g, 40, m)
+    mixer = latent_mixer(m, 40, w, 1e-5, torch.bfloat16)
+    x = torch.randn(331, 40, generator=g).to(torch.bfloat16)
+    want = pg.latent_attention(x.double(), {k: v.double() for k, v in w.items()}, "", m, 1e-5)
+    monkeypatch.setattr(ops, "latent_prefers_expanded", lambda batch, *_: not batch.decode)
+    for cuts in ([331], [63, 1, 1, 63, 2, 128, 73], [129, 202]):
+        close(step_through(mixer, x.cuda(), cuts, torch.bfloat16), want, "bf16", loose=2)
+
+
+
 @pytest.mark.parametrize("dtype", ["fp32", "bf16"])
 @pytest.mark.parametrize("rank", [24, 64])
 def test_one_key_just_inside_and_just_outside_a_window(dtype, rank):

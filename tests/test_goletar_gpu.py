@@ -204,6 +204,28 @@ def test_latent_attention_alone(dtype, shape):
         close(step_through(mixer, x.cuda(), cuts, dt), want, dtype)
 
 
+@pytest.mark.parametrize("shape", [(3, 96, 32, 128, 64, 32), (2, 48, 16, 64, 40, 10), (5, 0, 64, 64, 72, 64), (1, 128, 0, 128, 512, 0)])
+@pytest.mark.parametrize("at_a_time", [1, 1 << 29])
+def test_latent_attention_in_the_heads_own_space(monkeypatch, shape, at_a_time):
+    """Keys and values made of the cached rows (heads of 64 and 128; all at a time and one by one), onto what is cached
+    already, beside the form in the latent's space; tiles of 128 positions, blocks of 64 keys."""
+    from fms_b200.kernels import ops
+
+    heads, dim, rot, vdim, rank, dims = shape
+    m = gm.latent(heads, dim, rot, vdim, rank, 300.0, None, rot_dims=dims)["mixer"]
+    g = torch.Generator().manual_seed(sum(shape))
+    w = latent_tensors(g, 40, m)
+    mixer = latent_mixer(m, 40, w, 1e-5, torch.bfloat16)
+    x = torch.randn(331, 40, generator=g).to(torch.bfloat16)
+    d = {k: v.double() for k, v in w.items()}
+    want, _ = pg.latent_attention(x.double(), m, 1e-5, d["q"], d["dkv"], d["norm"], d["uk"], d["uv"], d["sink"], d["g"], d["o"])
+    monkeypatch.setattr(ops, "latent_prefers_expanded", lambda batch, *_: not batch.decode)
+    monkeypatch.setattr(ops, "LATENT_EXPANDED_BYTES", at_a_time)
+    for cuts in ([331], [63, 1, 1, 63, 2, 128, 73], [129, 202]):
+        close(step_through(mixer, x.cuda(), cuts, torch.bfloat16), want, "bf16")
+
+
+
 def test_latent_attention_sink_and_a_far_key():
     """Weights made so that a fault shows: head 0's sink is so large that it takes all of the softmax, head 1's
     so small that it takes nothing, and the keys' rotated part is scaled up so that every query has a few keys far
