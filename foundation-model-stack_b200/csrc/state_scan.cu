@@ -543,59 +543,71 @@ __global__ void linear_prepare_kernel(const T* proj, int stride, float* out, int
   else out[i] = v[0];
 }
 
-// Exponential gates under a running maximum, a warp per (sequence, head).  gate_raw: column h of the rows is head h's
+// Exponential gates under a running maximum, a block per (sequence, head).  gate_raw: column h of the rows is head h's
 // input gate before its bias, column heads + h its forget gate; bias [2 heads] float32; cap > 0:
 //   i = cap tanh((raw_i + bias_i) / cap);  f = logsigmoid(cap tanh((raw_f + bias_f) / cap))
 //   m' = max(f + m, i);  a = exp(f + m - m');  b = exp(i - m');  gates[t, h] = (a, b, exp(-m'))
 // norm_state holds per slot and head the normalizer n (dim values) and then m, zeros for a new sequence.  m is left at
 // its value after the step's last row; n as it was before the step is copied to norm_in [sequences, heads, dim], from
 // where every block of the scan reads it (the scan's blocks do not all run at once, and one of them writes the new n
-// into norm_state).  The lanes take a token each for the gates and exponentials; the maxima are walked in order.
+// into norm_state).  A thread a token for the gates and the exponentials, as many tokens at a time as the block has threads, the
+// next ones on their way meanwhile; only the walk over the maxima, an addition and a comparison a token, is one thread's.  (With
+// a warp for all three, 1,700 tokens of two sequences took 67 us.)
+constexpr int GATE_THREADS = 256;
+
 template <typename T>
-__global__ void exp_gates_kernel(const T* gate_raw, int stride, const float* bias, float cap, float* norm_state,
-                                 float* norm_in, float* gates, const int* first_row, const int* slots, int heads, int dim,
-                                 int write_state, int n_seqs, int n_slots) {
+__global__ void __launch_bounds__(GATE_THREADS) exp_gates_kernel(const T* gate_raw, int stride, const float* bias, float cap,
+                                                                 float* norm_state, float* norm_in, float* gates,
+                                                                 const int* first_row, const int* slots, int heads, int dim,
+                                                                 int write_state, int n_slots) {
+  __shared__ __align__(16) float si[GATE_THREADS], sf[GATE_THREADS], sm[GATE_THREADS + 1];  // sm[j]: the maximum before token j
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (unit >= n_seqs * heads) return;
-  const int seq = unit / heads, head = unit - seq * heads;
+  const int tid = threadIdx.x, width = blockDim.x;
+  const int unit = blockIdx.x, seq = unit / heads, head = unit - seq * heads;
   const int slot = __ldcg(slots + seq);
   if (!FMS_IN(slot, n_slots)) return;
   const int lo = first_row[seq], hi = first_row[seq + 1];
   float* st = norm_state + ((size_t)slot * heads + head) * (dim + 1);
-  float m = st[dim];
-  for (int e = lane; e < dim; e += 32) norm_in[(size_t)unit * dim + e] = st[e];
+  for (int e = tid; e < dim; e += width) norm_in[(size_t)unit * dim + e] = st[e];
   const float bi = bias[head], bf = bias[heads + head];
-  for (int base = lo; base < hi; base += 32) {
-    const int t = base + lane;
-    float gi = 0.f, gf = 0.f;
+  if (tid == 0) sm[0] = st[dim];
+  float raw_i = 0.f, raw_f = 0.f;
+  auto load = [&](int t) {
     if (t < hi) {
-      gi = cap * tanhf((to_f32(gate_raw[(size_t)t * stride + head]) + bi) / cap);
-      const float z = cap * tanhf((to_f32(gate_raw[(size_t)t * stride + heads + head]) + bf) / cap);
-      gf = z < 0.f ? z - log1pf(expf(z)) : -log1pf(expf(-z));
+      raw_i = to_f32(gate_raw[(size_t)t * stride + head]);
+      raw_f = to_f32(gate_raw[(size_t)t * stride + heads + head]);
     }
-    float before = 0.f, after = 0.f;
-    const int cn = min(32, hi - base);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {  // unrolled: the shuffles are issued ahead and only m waits for the step before
-      const float ij = __shfl_sync(0xffffffffu, gi, j), fj = __shfl_sync(0xffffffffu, gf, j);
-      const float next = j < cn ? fmaxf(fj + m, ij) : m;
-      if (lane == j) {
-        before = m;
-        after = next;
+  };
+  load(lo + tid);
+  for (int base = lo; base < hi; base += width) {
+    const int t = base + tid, cn = min(width, hi - base);
+    const float gi = cap * tanhf((raw_i + bi) / cap), z = cap * tanhf((raw_f + bf) / cap);
+    const float gf = z < 0.f ? z - log1pf(expf(z)) : -log1pf(expf(-z));
+    si[tid] = gi;
+    sf[tid] = gf;
+    load(t + width);
+    __syncthreads();
+    if (tid == 0) {
+      float m = sm[0];
+#pragma unroll 8
+      for (int j = 0; j < cn; ++j) {
+        m = fmaxf(sf[j] + m, si[j]);
+        sm[j + 1] = m;
       }
-      m = next;
     }
+    __syncthreads();
     if (t < hi) {
+      const float before = sm[tid], after = sm[tid + 1];
       float* g = gates + ((size_t)t * heads + head) * 3;
       g[0] = expf(gf + before - after);
       g[1] = expf(gi - after);
       g[2] = expf(-after);
     }
+    __syncthreads();
+    if (tid == 0) sm[0] = sm[cn];
   }
-  if (write_state && lane == 0) st[dim] = m;
+  if (write_state && tid == 0) st[dim] = sm[0];
 }
 
 // What a scan under one decay a key channel reads, made ready for every token at once: q | k | v in float32 (q times
@@ -1081,6 +1093,20 @@ FMS_API int fms_gla_prepare(const void* proj, int dtype, int stride, int u_col, 
   return fms_launch_status("gla_prepare");
 }
 
+// What a scan under exponential gates reads: gates [tokens, heads, 3], norm_in [sequences, heads, dim]; see the kernel.
+FMS_API int fms_exp_gates(const void* gate_raw, int dtype, int gate_stride, const float* gate_bias, float cap, float* norm_state,
+                          float* norm_in, float* gates, const int* first_row, const int* slots, int n_tokens, int n_seqs, int heads,
+                          int dim, int write_state, int n_slots, cudaStream_t stream) {
+  if (n_seqs <= 0 || n_tokens <= 0) return 0;
+  if (!gate_raw || !gate_bias || !gates || !norm_in || !norm_state || !(cap > 0.f) || heads <= 0 || dim <= 0)
+    return fms_fail("exp_gates: gates without bias, scratch, normalizer or cap");
+  const int threads = n_tokens <= 32 * n_seqs ? 32 : GATE_THREADS;
+  FMS_DISPATCH_DTYPE(dtype, T, fms_launch(exp_gates_kernel<T>, dim3(n_seqs * heads), dim3(threads), 0, stream, (const T*)gate_raw,
+                                          gate_stride, gate_bias, cap, norm_state, norm_in, gates, first_row, slots, heads, dim,
+                                          write_state, n_slots));
+  return fms_launch_status("exp_gates");
+}
+
 // qkv [tokens, 2 heads * dim + heads * vdim] float32.  With gate_raw (columns [i: heads | f: heads] of rows of
 // gate_stride values, bias [2 heads], cap): exponential gates, with normalizer and running maximum in norm_state
 // [slots, heads, dim + 1]; gates [tokens, heads, 3] and norm_in [sequences, heads, dim] are float32 scratch of the
@@ -1098,9 +1124,9 @@ FMS_API int fms_decay_scan(const float* qkv, const void* gate_raw, int dtype, in
   if (!gated && !channel && !decay) return fms_fail("decay_scan: neither gates nor decays");
   const long row_w = 2L * heads * dim + (long)heads * vdim;
   if (gated) {
-    FMS_DISPATCH_DTYPE(dtype, T, fms_launch(exp_gates_kernel<T>, dim3((n_seqs * heads + 3) / 4), dim3(128), 0, stream,
-                                            (const T*)gate_raw, gate_stride, gate_bias, cap, norm_state, norm_in, gates,
-                                            first_row, slots, heads, dim, write_state, n_seqs, n_slots));
+    if (fms_exp_gates(gate_raw, dtype, gate_stride, gate_bias, cap, norm_state, norm_in, gates, first_row, slots, n_tokens, n_seqs, heads,
+                      dim, write_state, n_slots, stream))
+      return 1;
   }
   // under fixed decays a token is two multiply-adds a state value and one sum: 16 threads a column group (half the
   // rows a thread, twice the blocks) pay up to twice as many blocks as under gates (a prompt of 2,048 tokens, 32 heads

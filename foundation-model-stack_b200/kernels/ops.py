@@ -91,6 +91,9 @@ _SIGNATURES = {
     "fms_gla_chunked": [_P, _I, _I, _I, _I, _P, _I, _P, _F, _F, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "fms_gla_decode": [_P, _I, _I, _I, _I, _P, _I, _P, _F, _F, _P, _P, _I, _P, _F, _P, _I, _I, _I, _I, _I, _I, _P],
     "fms_linear_prepare": [_P, _I, _I, _P, _I, _I, _I, _F, _I, _P],
+    "fms_exp_gates": [_P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "fms_chunk_scan": [_I, _P, _P, _P, _L, _P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
+                       _I, _I, _I, _I, _I, _I, _P],
     "fms_decay_scan": [_P, _P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_attention_prefill_sink": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
                                    _P],
@@ -911,6 +914,43 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
     return out
 
 
+CHUNK_SCAN_FROM = 64  # tokens of a sequence in one step from which a scan under one decay a head runs run by run
+CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
+
+
+def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int):
+    """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, decode steps and
+    short prompts (which go token by token), a capture that has not seen the batch before (the runs come from the host)."""
+    if batch.decode or not batch.num_new or max(batch.num_new) < CHUNK_SCAN_FROM:
+        return None
+    lib = load_library("chunk_scan")
+    if not lib.fms_chunk_scan_takes(int(dim), int(vdim), heads // key_heads):
+        return None
+    chunk = int(lib.fms_chunk_scan_tokens())
+    if ("chunks", chunk) not in batch._tiles and torch.cuda.is_current_stream_capturing():
+        return None
+    return batch.row_chunks(chunk)
+
+
+def _chunk_scan(kind: int, q: int, k: int, v: int, row: int, plan, batch, state: torch.Tensor, o: torch.Tensor, heads: int,
+                key_heads: int, dim: int, vdim: int, writes_state: bool, decay=None, gates=None, norm_in=None, norm_state=None,
+                dt_raw: Optional[int] = None, dt_dtype: int = F32, dt_stride: int = 0, dt_bias=None, a_log=None, d_skip=None) -> None:
+    """``fms_chunk_scan`` with its scratch; q, k, v, dt_raw: addresses."""
+    global launches
+    runs, first_run = plan
+    n, chunk, dev = runs.shape[0], 64, state.device
+    per_pass = max(1, min(n, CHUNK_STATE_BYTES // (heads * vdim * dim * 4)))
+    new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)  # noqa: E731
+    scores, states, totals = new(per_pass, key_heads, chunk, chunk), new(per_pass, heads, vdim, dim), new(per_pass, heads)
+    norms = new(per_pass, heads, dim) if kind == 1 else None
+    carry = new(2, heads, vdim, dim) if per_pass < n else None
+    _call("chunk_scan", "fms_chunk_scan", kind, q, k, v, row, _ptr(runs), _ptr(first_run), n, per_pass, _ptr(batch.slots), batch.n_seqs,
+          _ptr(decay), _ptr(gates), _ptr(norm_in), _ptr(norm_state), dt_raw, dt_dtype, dt_stride, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
+          _ptr(state), _ptr(carry), _ptr(scores), _ptr(states), _ptr(norms), _ptr(totals), _ptr(o), heads, key_heads, dim, vdim,
+          1 if writes_state else 0, state.shape[0], _stream())
+    launches += 4 * ((n + per_pass - 1) // per_pass) - 1
+
+
 def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                    d_skip: torch.Tensor, state: torch.Tensor, batch, heads: int, vdim: int, n_state: int, groups: int,
                    writes_state: bool = True) -> torch.Tensor:
@@ -922,6 +962,13 @@ def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bia
             or tuple(state.shape[1:]) != (heads, vdim, n_state):
         raise KernelError("selective_scan: xbc float32 [tokens, x | B | C], state float32 [slots, heads, vdim, state]")
     y = torch.empty((n, heads * vdim), dtype=torch.float32, device=xbc.device)
+    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups)
+    if plan is not None:
+        x, b = _ptr(xbc), _ptr(xbc) + heads * vdim * 4
+        _chunk_scan(2, b + groups * n_state * 4, b, x, xbc.shape[1], plan, batch, state, y, heads, groups, n_state, vdim, writes_state,
+                    dt_raw=_ptr(proj) + dt_offset * proj.element_size(), dt_dtype=_code(proj.dtype), dt_stride=proj.shape[1],
+                    dt_bias=dt_bias, a_log=a_log, d_skip=d_skip)
+        return y
     _call("state_scan", "fms_selective_scan", _ptr(xbc), _ptr(proj) + dt_offset * proj.element_size(), _code(proj.dtype),
           proj.shape[1], _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(y), _ptr(batch.first_row),
           _ptr(batch.slots), batch.n_seqs, heads, vdim, n_state, groups, 1 if writes_state else 0, state.shape[0],
@@ -1073,6 +1120,16 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
     norm_in = torch.empty((batch.n_seqs, heads, dim), dtype=torch.float32, device=proj.device) if gated else None
     gate_ptr = _ptr(proj) + gate_offset * proj.element_size() if gated else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads) if not gated or vdim == 128 else None
+    if plan is not None:
+        if gated:
+            _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], _ptr(gate_bias), float(gate_cap),
+                  _ptr(norm_state), _ptr(norm_in), _ptr(gates), _ptr(batch.first_row), _ptr(batch.slots), n, batch.n_seqs, heads, dim,
+                  1 if writes_state else 0, state.shape[0], _stream())
+        q = _ptr(qkv)
+        _chunk_scan(1 if gated else 0, q, q + heads * dim * 4, q + 2 * heads * dim * 4, cols, plan, batch, state, o, heads, heads, dim, vdim,
+                    writes_state, decay=decay, gates=gates, norm_in=norm_in, norm_state=norm_state)
+        return o
     _call("state_scan", "fms_decay_scan", _ptr(qkv), gate_ptr, _code(proj.dtype), proj.shape[1], _ptr(gate_bias),
           float(gate_cap), _ptr(gates), _ptr(norm_in), _ptr(decay), _ptr(state), _ptr(norm_state), _ptr(o), _ptr(batch.first_row),
           _ptr(batch.slots), n, batch.n_seqs, heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())

@@ -84,7 +84,7 @@ class _DecayedStateMixer(Part):
         self._norm = self.tensor("norm").float().contiguous()
 
     def kernel_libraries(self, dtype):
-        return super().kernel_libraries(dtype) + ["state_scan"]
+        return super().kernel_libraries(dtype) + ["state_scan", "chunk_scan"]
 
 
 class LightningAttention(_DecayedStateMixer):

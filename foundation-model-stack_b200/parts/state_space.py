@@ -98,7 +98,7 @@ class SelectiveStateSpace(Part):
         return self.dense.forward(y)
 
     def kernel_libraries(self, dtype):
-        return super().kernel_libraries(dtype) + ["state_scan"]
+        return super().kernel_libraries(dtype) + ["state_scan", "chunk_scan"]
 
 
 class GatedDeltaRule(Part):
