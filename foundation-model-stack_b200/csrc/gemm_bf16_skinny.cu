@@ -19,7 +19,8 @@
 //           act(gate) * up (fms/modules/feedforward.py:291-292) without the [M, 2 hidden] round trip.
 //
 // GROUPED: the rows of x are sorted into groups (offsets on the device), each with a matrix of its own, and a block belongs
-// to one group (blockIdx.y); a group's rows are at most 8 and a group without rows reads nothing.
+// to one group (blockIdx.y); a group's rows are at most 8 and a group without rows reads nothing.  STRIDED: every row has a run
+// of x and of y in every group, at a stride of the group's (a product a head).
 //
 // The weights of the first ring stages are requested before the kernel waits for the kernel before it
 // (programmatic dependent launch): weights do not depend on it, so the stream of weights from memory does
@@ -48,15 +49,18 @@ struct RopeArgs {
 };
 
 // What the ROWS16 epilogue does beyond the product: nothing, or y = act(v) * table[tokens[m]] (table set), or what `unit`
-// says: the square of relu, act(v), or v * scale, capped by cap * tanh(. / cap) where cap > 0.  offsets: GROUPED only.
-enum Unit { UNIT_NONE = 0, UNIT_SQUARES = 1, UNIT_ACT = 2, UNIT_CAP = 3 };
+// says: the square of relu, act(v), or v * scale, capped by cap * tanh(. / cap) where cap > 0.  The GLU8 epilogue: act(gate) * up,
+// or with UNIT_CLAMPED g * sigmoid(scale * g) * (u + 1), g = min(gate, cap), u = up within +-cap.  offsets: GROUPED only.
+enum Unit { UNIT_NONE = 0, UNIT_SQUARES = 1, UNIT_ACT = 2, UNIT_CAP = 3, UNIT_CLAMPED = 4 };
 struct RowArgs {
   const __nv_bfloat16* table;  // [vocab, N]
   const int* tokens;           // [M]
   int vocab, unit;
   const int* offsets;          // [groups + 1]
   float scale, cap;
+  long x_row = 0, x_group = 0, y_row = 0, y_group = 0;  // STRIDED: values from row to row and from group to group
 };
+enum Groups { ALONE = 0, GROUPED = 1, STRIDED = 2 };
 
 __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
@@ -88,8 +92,14 @@ __device__ __forceinline__ float activate(float g, int act) {
   }
 }
 
+// the gated unit of the routed experts: see grouped.cu
+__device__ __forceinline__ float clamped_unit(float gate, float up, float limit, float alpha) {
+  const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
+  return g * (1.f / (1.f + expf(-alpha * g))) * (u + 1.f);
+}
+
 // NT: tiles of 8 batch rows (M <= 8 NT).  RT: tiles per block.  D: ring stages.
-template <int NT, int RT, int MODE, int D, typename TOut, bool GROUPED>
+template <int NT, int RT, int MODE, int D, typename TOut, int GROUPS>
 __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloat16* __restrict__ x,
                                                                 const __nv_bfloat16* __restrict__ w,
                                                                 const __nv_bfloat16* __restrict__ bias,
@@ -105,7 +115,13 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, c = lane & 3;
   const int n_rows = MODE == GLU8 ? 2 * hidden : N;  // rows of w
-  if (GROUPED) {  // which weights are read depends on the kernel before
+  const size_t x_row = GROUPS == STRIDED ? (size_t)extra.x_row : (size_t)K;
+  if (GROUPS == STRIDED) {
+    x += (size_t)blockIdx.y * extra.x_group;
+    w += (size_t)blockIdx.y * n_rows * K;
+    y += (size_t)blockIdx.y * extra.y_group;
+  }
+  if (GROUPS == GROUPED) {  // which weights are read depends on the kernel before
     pdl_wait();
     const int r_lo = __ldcg(extra.offsets + blockIdx.y), r_hi = __ldcg(extra.offsets + blockIdx.y + 1);
     M = min(r_hi - r_lo, 8 * NT);
@@ -127,7 +143,7 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
     xok[j] = j * 8 + g < M;
-    xp[j] = x + (size_t)(xok[j] ? j * 8 + g : 0) * K + 8 * c;
+    xp[j] = x + (size_t)(xok[j] ? j * 8 + g : 0) * x_row + 8 * c;
   }
   float acc[RT][NT][4];
 #pragma unroll
@@ -165,7 +181,7 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
 #pragma unroll
   for (int i = 0; i < D; ++i) issue_w(i);  // weights: before the wait for the kernel that produces x
   cp_async_commit();
-  if (!GROUPED) pdl_wait();
+  if (GROUPS != GROUPED) pdl_wait();
 #pragma unroll
   for (int i = 0; i < D; ++i) issue_x(i);
   cp_async_commit();
@@ -225,7 +241,7 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
           gate += __bfloat162float(bias[row]);
           up += __bfloat162float(bias[hidden + row]);
         }
-        if (FMS_IN((size_t)m * hidden + row, (size_t)M * hidden)) y[(size_t)m * hidden + row] = from_f32<TOut>(activate(gate, act) * up);
+        if (FMS_IN((size_t)m * hidden + row, (size_t)M * hidden)) y[(size_t)m * hidden + row] = from_f32<TOut>(extra.unit == UNIT_CLAMPED ? clamped_unit(gate, up, extra.cap, extra.scale) : activate(gate, act) * up);
       }
     }
   } else if (MODE == QKV_ROPE) {
@@ -293,19 +309,20 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
           v *= extra.scale;
           if (extra.cap > 0.f) v = extra.cap * tanhf(v / extra.cap);
         }
-        if (FMS_IN((size_t)m * N + row, (size_t)M * N)) y[(size_t)m * N + row] = from_f32<TOut>(v);
+        if (GROUPS == STRIDED) y[(size_t)m * extra.y_row + row] = from_f32<TOut>(v);
+        else if (FMS_IN((size_t)m * N + row, (size_t)M * N)) y[(size_t)m * N + row] = from_f32<TOut>(v);
       }
     }
   }
 }
 
-template <int NT, int RT, int MODE, typename TOut, bool GROUPED = false>
+template <int NT, int RT, int MODE, typename TOut, int GROUPS = ALONE>
 int launch_typed(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int hidden, int act,
                  cudaStream_t stream, const RopeArgs& rope = RopeArgs{}, const RowArgs& extra = RowArgs{}, int groups = 1) {
   constexpr int LOADS = RT * 2 + NT;
   constexpr int D = LOADS <= 2 ? 7 : (LOADS == 3 ? 5 : (LOADS == 4 ? 4 : 3));  // 56 to 72 KB of ring per block
   constexpr size_t smem = (size_t)D * LOADS * THREADS * sizeof(uint4);
-  auto kernel = linear_skinny_kernel<NT, RT, MODE, D, TOut, GROUPED>;
+  auto kernel = linear_skinny_kernel<NT, RT, MODE, D, TOut, GROUPS>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -378,16 +395,31 @@ FMS_API int fms_token_gate_bf16_skinny(const void* x, const void* w, const void*
 }
 
 // Groups of at most 8 rows: for the rows offsets[g] .. offsets[g + 1] of x [rows, K], w [groups, N (or 2 N), K],
-// kind 0: y = x w^T; 2: its square where positive, else 0; 3: silu(gate) * up with w[g] = [gate; up].  y [rows, N].
+// kind 0: y = x w^T; 2: its square where positive, else 0; with w[g] = [gate; up] 1: the clamped unit under limit and alpha,
+// 3: silu(gate) * up.  y [rows, N].
 FMS_API int fms_grouped_bf16_skinny(const void* x, const void* w, void* y, const int* offsets, int groups, int N, int K, int kind,
-                                    cudaStream_t stream) {
+                                    float limit, float alpha, cudaStream_t stream) {
   if (groups <= 0 || N <= 0) return 0;
-  if (groups > 65535 || K <= 0 || K % 8 || !offsets || (kind != 0 && kind != 2 && kind != 3))
+  if (groups > 65535 || K <= 0 || K % 8 || !offsets || kind < 0 || kind > 3)
     return fms_fail("grouped_bf16_skinny: %d groups, K %d, kind %d", groups, K, kind);
-  const RowArgs extra{nullptr, nullptr, 0, kind == 2 ? UNIT_SQUARES : UNIT_NONE, offsets, 1.f, 0.f};
-  if (kind == 3)
-    return launch_typed<1, 2, GLU8, __nv_bfloat16, true>(x, w, nullptr, y, 8, 2 * N, K, N, 0, stream, RopeArgs{}, extra, groups);
-  return launch_typed<1, 1, ROWS16, __nv_bfloat16, true>(x, w, nullptr, y, 8, N, K, 0, 0, stream, RopeArgs{}, extra, groups);
+  const RowArgs extra{nullptr, nullptr, 0, kind == 2 ? UNIT_SQUARES : (kind == 1 ? UNIT_CLAMPED : UNIT_NONE), offsets, alpha, limit};
+  if (kind == 1 || kind == 3)
+    return launch_typed<1, 2, GLU8, __nv_bfloat16, GROUPED>(x, w, nullptr, y, 8, 2 * N, K, N, 0, stream, RopeArgs{}, extra, groups);
+  return launch_typed<1, 1, ROWS16, __nv_bfloat16, GROUPED>(x, w, nullptr, y, 8, N, K, 0, 0, stream, RopeArgs{}, extra, groups);
+}
+
+// A product a group for up to 8 rows: y[r, g * y_group + :N] = x[r, g * x_group + :K] w[g]^T, w [groups, N, K]; rows of x
+// x_row values apart and of y y_row.
+FMS_API int fms_strided_bf16_skinny(const void* x, const void* w, void* y, int M, int groups, int N, int K, long x_row, long x_group,
+                                    long y_row, long y_group, cudaStream_t stream) {
+  if (M <= 0 || groups <= 0 || N <= 0) return 0;
+  if (M > 8 || groups > 65535 || K <= 0 || K % 8 || x_row % 8 || x_group % 8 || (uintptr_t)x % 16)
+    return fms_fail("strided_bf16_skinny: %d rows, %d groups, K %d, rows %ld and groups %ld values apart", M, groups, K, x_row, x_group);
+  RowArgs extra{nullptr, nullptr, 0, UNIT_NONE, nullptr, 1.f, 0.f};
+  extra.x_row = x_row; extra.x_group = x_group; extra.y_row = y_row; extra.y_group = y_group;
+  // short rows of w: 32 of them a block, so that a block has something to read
+  if (K <= 256 && N >= 64) return launch_typed<1, 2, ROWS16, __nv_bfloat16, STRIDED>(x, w, nullptr, y, M, N, K, 0, 0, stream, RopeArgs{}, extra, groups);
+  return launch_typed<1, 1, ROWS16, __nv_bfloat16, STRIDED>(x, w, nullptr, y, M, N, K, 0, 0, stream, RopeArgs{}, extra, groups);
 }
 
 // The fused projection of an attention layer for up to 8 tokens: [q | k | v] = x [M, K] w[(nheads + 2 kvheads) head_dim, K]^T

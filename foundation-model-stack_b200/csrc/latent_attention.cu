@@ -25,7 +25,7 @@ __device__ __forceinline__ int ld_fresh(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_fresh(const float* p) { return __ldcg(p); }
 
 namespace {
-constexpr int SPLIT = 256;  // keys of one split of a decode step: fixed, so a sequence's sums depend on its length only
+constexpr int SPLIT = 256;  // keys of one split of a decode step
 constexpr int KT = 32;      // keys brought into shared memory at a time
 constexpr int HG = 8;       // heads a block takes
 constexpr int THREADS = 256;
@@ -207,6 +207,7 @@ struct LatentArgs {
   int table_stride, block_tokens, heads, rank, rot, n_splits, n_seqs, n_slots, n_blocks;
   float scale;
   int window;  // > 0: the row at position p sees the keys p - window + 1 .. p only
+  int split;  // keys of a split: a multiple of 32
 };
 
 // One block per (row, split of keys, group of HG heads).  Keys come KT at a time into shared memory as float32; a warp
@@ -233,9 +234,9 @@ __global__ void __launch_bounds__(THREADS) latent_attention_kernel(LatentArgs a)
   if (!FMS_IN(slot, a.n_slots)) return;
   const bool whole = a.n_splits == 1;  // one split takes all keys and writes the result itself
   const int seen = a.window > 0 ? max(0, pos - a.window + 1) : 0;  // the first key this row sees
-  const int hi = whole ? pos + 1 : min(pos + 1, split * SPLIT + SPLIT);
+  const int hi = whole ? pos + 1 : min(pos + 1, (split + 1) * a.split);
   if (hi <= seen) return;  // a split before the window: the merge does not look at it
-  const int lo = max(whole ? 0 : split * SPLIT, seen / KT * KT);  // tiles stay aligned; keys before `seen` are masked
+  const int lo = max(whole ? 0 : split * a.split, seen / KT * KT);  // tiles stay aligned; keys before `seen` are masked
   const T* q = (const T*)a.q + ((size_t)t * a.heads + h0) * width;
   for (int i = threadIdx.x; i < nh * width; i += THREADS) qs[i] = to_f32(q[i]);
   float acc[NACC];
@@ -336,21 +337,58 @@ template <typename T, typename TS>
 __global__ void __launch_bounds__(128) latent_combine_kernel(LatentArgs a) {
   pdl_launch_dependents();
   pdl_wait();
+  // what every split counts for, once for all values of the row; then a thread four values, the splits' partial rows four
+  // ahead (an exponential a value and split, one dependent load after the other, took as long as the attention itself)
+  constexpr int HELD = 1024;
+  __shared__ float weight[HELD];
+  __shared__ float factor;
   const int t = blockIdx.x, h = blockIdx.y;
   const int pos = ld_fresh(a.positions + t);
-  const int used = min(a.n_splits, pos / SPLIT + 1);
-  const int s_lo = a.window > 0 ? min(max(0, pos - a.window + 1) / SPLIT, used - 1) : 0;  // splits before the window hold nothing
+  const int used = min(a.n_splits, pos / a.split + 1);
+  const int s_lo = a.window > 0 ? min(max(0, pos - a.window + 1) / a.split, used - 1) : 0;  // splits before the window hold nothing
   const size_t at = ((size_t)t * a.heads + h) * a.n_splits;
+  const bool held = used - s_lo <= HELD;
   float m = a.sink ? to_f32(((const TS*)a.sink)[h]) : -INFINITY;
-  for (int s = s_lo; s < used; ++s) m = fmaxf(m, a.part_ml[2 * (at + s)]);
-  float denom = a.sink ? expf(to_f32(((const TS*)a.sink)[h]) - m) : 0.f;
-  for (int s = s_lo; s < used; ++s) denom += a.part_ml[2 * (at + s) + 1] * expf(a.part_ml[2 * (at + s)] - m);
-  float f = 1.f / denom;
-  if (a.gate) f *= 1.f / (1.f + expf(-to_f32(((const T*)a.gate)[(size_t)t * a.gate_stride + h])));
+  const int lane = threadIdx.x & 31;
+  for (int s = s_lo + lane; s < used; s += 32) m = fmaxf(m, a.part_ml[2 * (at + s)]);  // every warp alike
+  m = warp_max(m);
+  if (threadIdx.x < 32) {
+    float denom = 0.f;
+    for (int s = s_lo + lane; s < used; s += 32) {
+      const float w = expf(a.part_ml[2 * (at + s)] - m);
+      denom += a.part_ml[2 * (at + s) + 1] * w;
+      if (held) weight[s - s_lo] = w;
+    }
+    denom = warp_sum(denom);
+    if (a.sink) denom += expf(to_f32(((const TS*)a.sink)[h]) - m);
+    float f = 1.f / denom;
+    if (a.gate) f *= 1.f / (1.f + expf(-to_f32(((const T*)a.gate)[(size_t)t * a.gate_stride + h])));
+    if (lane == 0) factor = f;
+  }
+  __syncthreads();
+  const float f = factor;
   T* o = (T*)a.out + ((size_t)t * a.heads + h) * a.rank;
+  const float* part = a.part_o + (at + s_lo) * a.rank;
+  const int n = used - s_lo;
+  if (held && a.rank % 4 == 0) {
+    for (int d = threadIdx.x * 4; d < a.rank; d += blockDim.x * 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int s = 0; s < n; ++s) {
+        const float4 x = *reinterpret_cast<const float4*>(part + (size_t)s * a.rank + d);
+        const float w = weight[s];
+        v = make_float4(fmaf(x.x, w, v.x), fmaf(x.y, w, v.y), fmaf(x.z, w, v.z), fmaf(x.w, w, v.w));
+      }
+      o[d] = from_f32<T>(v.x * f);
+      o[d + 1] = from_f32<T>(v.y * f);
+      o[d + 2] = from_f32<T>(v.z * f);
+      o[d + 3] = from_f32<T>(v.w * f);
+    }
+    return;
+  }
   for (int d = threadIdx.x; d < a.rank; d += blockDim.x) {
     float v = 0.f;
-    for (int s = s_lo; s < used; ++s) v = fmaf(a.part_o[(at + s) * a.rank + d], expf(a.part_ml[2 * (at + s)] - m), v);
+    for (int s = 0; s < n; ++s) v = fmaf(part[(size_t)s * a.rank + d], held ? weight[s] : expf(a.part_ml[2 * (at + s_lo + s)] - m), v);
     o[d] = from_f32<T>(v * f);
   }
 }
@@ -363,7 +401,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(LatentArgs a) {
 // flash-attention kernel) and the sum; (C) warp w adds P . c for 16 rows and a quarter of the latent's columns
 // (rank / 4, its share of the accumulator in registers), c being read as it lies in the key tile.
 // With n_splits > 1 (a decode step: tq = 1, the block's rows are one token's heads) block z takes the keys of split z
-// (SPLIT keys) and leaves its unnormed sums, maximum and sum for latent_combine_kernel.
+// (a.split keys) and leaves its unnormed sums, maximum and sum for latent_combine_kernel.
 constexpr int MR = 32, MK = 32;
 
 __device__ __forceinline__ void lat_mma(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -414,8 +452,8 @@ __global__ void __launch_bounds__(256) latent_prefill_mma_kernel(LatentArgs a, c
   const int last_pos = ld_fresh(a.positions + first + ntok - 1);
   const int first_pos = ld_fresh(a.positions + first);
   const int seen = a.window > 0 ? max(0, first_pos - a.window + 1) : 0;  // the first key that any row of the tile sees
-  const int kt_lo = max(a.n_splits > 1 ? split * (SPLIT / MK) : 0, seen / MK);
-  const int n_kt = a.n_splits > 1 ? min(last_pos / MK + 1, (split + 1) * (SPLIT / MK)) : last_pos / MK + 1;
+  const int kt_lo = max(a.n_splits > 1 ? split * (a.split / MK) : 0, seen / MK);
+  const int n_kt = a.n_splits > 1 ? min(last_pos / MK + 1, (split + 1) * (a.split / MK)) : last_pos / MK + 1;
   if (kt_lo >= n_kt) return;  // a split beyond the sequence or before the window: the merge does not look at it
   if (tid < MR) {
     const int tok = tid / hb, hh = tid - tok * hb;
@@ -668,6 +706,7 @@ FMS_API int fms_latent_attention(const void* q, void* out, int dtype, const void
   a.table_stride = table_stride; a.block_tokens = block_tokens; a.heads = heads; a.rank = rank; a.rot = rot;
   a.n_splits = n_splits; a.n_seqs = n_seqs; a.n_slots = n_slots; a.n_blocks = n_blocks; a.scale = scale;
   a.window = window > 0 ? window : 0;
+  a.split = SPLIT;
   FMS_DISPATCH_DTYPE(dtype, T, FMS_DISPATCH_DTYPE(sink ? sink_dtype : dtype, TS, return launch_attention<T, TS>(a, n_tokens, stream)));
   return 0;
 }
@@ -680,9 +719,10 @@ FMS_API int fms_latent_attention_prefill_bf16(const void* q, void* out, const vo
                                               int block_tokens, const int* slots, const int* first_row,
                                               const int* positions, const int* tiles, int n_tiles, int tile_tokens,
                                               int heads_per_block, int heads, int rank, int rot, float scale, int n_seqs,
-                                              int n_slots, int n_blocks, const int* token_seq, int n_splits, float* part_o,
-                                              float* part_ml, int window, cudaStream_t stream) {
+                                              int n_slots, int n_blocks, const int* token_seq, int n_splits, int split_tokens,
+                                              float* part_o, float* part_ml, int window, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
+  if (n_splits > 1 && (split_tokens <= 0 || split_tokens % MK)) return fms_fail("latent_attention_prefill: splits of %d keys", split_tokens);
   if (n_splits < 1 || (n_splits > 1 && (tile_tokens != 1 || part_o == nullptr || part_ml == nullptr || token_seq == nullptr)))
     return fms_fail("latent_attention_prefill: %d splits need one token a tile and scratch", n_splits);
   const int width = rank + rot;
@@ -694,6 +734,7 @@ FMS_API int fms_latent_attention_prefill_bf16(const void* q, void* out, const vo
   a.table_stride = table_stride; a.block_tokens = block_tokens; a.heads = heads; a.rank = rank; a.rot = rot;
   a.n_splits = n_splits; a.n_seqs = n_seqs; a.n_slots = n_slots; a.n_blocks = n_blocks; a.scale = scale;
   a.window = window > 0 ? window : 0;
+  a.split = split_tokens;
   const int rowb = width * 2 + 16;
   const size_t smem = (size_t)(MR + 2 * MK) * rowb + MR * (MK + 1) * 4 + MR * (MK * 2 + 16) + MR * 16;
   dim3 grid(n_tiles, (heads + heads_per_block - 1) / heads_per_block, n_splits);

@@ -63,74 +63,154 @@ template <int CPT> __device__ __forceinline__ void load_channels(const __nv_bflo
   }
 }
 
-// A thread takes CPT consecutive channels of CONV_TOKENS consecutive rows; TMAX bounds the taps (4 or MAX_TAPS).
-template <typename T, int CPT, int TMAX>
+// A thread takes CPT consecutive channels of `groups` times CONV_TOKENS consecutive rows; TMAX bounds the taps (4 or MAX_TAPS), and
+// EXACT: the taps are TMAX.  Bound by the bytes of x and out.  Several groups of rows share the taps and the rows between them, and
+// where all rows lie inside one sequence, as nearly all do, nothing is looked up a token.
+template <typename T, int CPT, int TMAX, bool EXACT>
 __global__ void __launch_bounds__(CONV_THREADS) causal_conv_kernel(const T* x, int stride, const float* w, const float* bias,
                                                                    const float* tail, const int* token_seq,
                                                                    const int* first_row, const int* slots, float* out,
-                                                                   int n_tokens, int channels, int taps, int act,
-                                                                   int n_seqs, int n_slots) {
+                                                                   int n_tokens, int channels, int n_taps, int act,
+                                                                   int n_seqs, int n_slots, int groups) {
   pdl_launch_dependents();
   pdl_wait();
-  const int t0 = blockIdx.x * CONV_TOKENS, c = (blockIdx.y * CONV_THREADS + threadIdx.x) * CPT;
+  const int taps = EXACT ? TMAX : n_taps;
+  const int begin = blockIdx.x * CONV_TOKENS * groups, c = (blockIdx.y * CONV_THREADS + threadIdx.x) * CPT;
   if (c >= channels) return;
-  // everything the thread reads is asked for at once: the tile's rows and the taps - 1 before them, the taps, and
-  // where each of the tile's tokens belongs
-  float xs[CONV_TOKENS + TMAX - 1][CPT];  // xs[r]: row t0 - (taps - 1) + r
-#pragma unroll
-  for (int r = 0; r < CONV_TOKENS + TMAX - 1; ++r) {
-    const int t = t0 - (taps - 1) + r;
-    if (r < CONV_TOKENS + taps - 1 && t >= 0 && t < n_tokens) load_channels<CPT>(x + (size_t)t * stride + c, xs[r]);
-    else {
-#pragma unroll
-      for (int k = 0; k < CPT; ++k) xs[r][k] = 0.f;
-    }
-  }
+  const int end = min(begin + CONV_TOKENS * groups, n_tokens);
   float wt[CPT][TMAX], b[CPT];
 #pragma unroll
   for (int k = 0; k < CPT; ++k) {
+    if (EXACT && TMAX == 4) {  // the launch has looked at the alignment
+      const float4 v = *reinterpret_cast<const float4*>(w + (size_t)(c + k) * 4);
+      wt[k][0] = v.x; wt[k][1] = v.y; wt[k][2] = v.z; wt[k][3] = v.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < TMAX; ++j) wt[k][j] = j < taps ? w[(size_t)(c + k) * taps + j] : 0.f;
+      for (int j = 0; j < TMAX; ++j) wt[k][j] = j < taps ? w[(size_t)(c + k) * taps + j] : 0.f;
+    }
     b[k] = bias ? bias[c + k] : 0.f;
   }
-  int local[CONV_TOKENS], slot[CONV_TOKENS];
-#pragma unroll
-  for (int i = 0; i < CONV_TOKENS; ++i) {
-    local[i] = -1;
-    slot[i] = 0;
-    if (t0 + i < n_tokens) {
-      const int seq = token_seq[t0 + i];
-      if (FMS_IN(seq, n_seqs)) {
-        local[i] = t0 + i - first_row[seq];  // the row's place among its sequence's rows of this step
-        slot[i] = __ldcg(slots + seq);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < CONV_TOKENS; ++i) {
-    if (local[i] < 0 || !FMS_IN(slot[i], n_slots)) continue;
-    const float* tl = tail + (size_t)slot[i] * (taps - 1) * channels;
-    float acc[CPT];
-#pragma unroll
-    for (int k = 0; k < CPT; ++k) acc[k] = b[k];
-#pragma unroll
-    for (int j = 0; j < TMAX; ++j) {
-      if (j < taps) {
-        const int back = taps - 1 - j;  // how many rows before this one
-#pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-          const float v = back <= local[i] ? xs[i + j][k] : tl[(size_t)(taps - 1 + local[i] - back) * channels + c + k];
-          acc[k] = fmaf(wt[k][j], v, acc[k]);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < CPT; ++k) acc[k] = act ? acc[k] * sigmoid_f(acc[k]) : acc[k];
-    float* o = out + (size_t)(t0 + i) * channels + c;
-    if constexpr (CPT == 4) *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  float xs[CONV_TOKENS + TMAX - 1][CPT];  // xs[r]: row t0 - (taps - 1) + r
+  auto load_row = [&](int t, float (&v)[CPT]) {
+    if (t >= 0 && t < n_tokens) load_channels<CPT>(x + (size_t)t * stride + c, v);
     else {
 #pragma unroll
-      for (int k = 0; k < CPT; ++k) o[k] = acc[k];
+      for (int k = 0; k < CPT; ++k) v[k] = 0.f;
+    }
+  };
+  auto finish = [&](int t, const float (&acc)[CPT]) {
+    float r[CPT];
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) r[k] = act ? acc[k] * sigmoid_f(acc[k]) : acc[k];
+    float* o = out + (size_t)t * channels + c;
+    if constexpr (CPT == 4) *reinterpret_cast<float4*>(o) = make_float4(r[0], r[1], r[2], r[3]);
+    else {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) o[k] = r[k];
+    }
+  };
+  const int seq0 = token_seq[begin], seq1 = token_seq[end - 1];
+  if (EXACT && seq0 == seq1 && FMS_IN(seq0, n_seqs) && begin - first_row[seq0] >= taps - 1) {
+#pragma unroll
+    for (int r = 0; r < TMAX - 1; ++r) load_row(begin - (TMAX - 1) + r, xs[r]);
+#pragma unroll 1
+    for (int t0 = begin; t0 < end; t0 += CONV_TOKENS) {
+#pragma unroll
+      for (int i = 0; i < CONV_TOKENS; ++i) load_row(t0 + i, xs[TMAX - 1 + i]);
+#pragma unroll
+      for (int i = 0; i < CONV_TOKENS; ++i) {
+        if (t0 + i >= end) break;
+        float acc[CPT];
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+          acc[k] = b[k];
+#pragma unroll
+          for (int j = 0; j < TMAX; ++j) acc[k] = fmaf(wt[k][j], xs[i + j][k], acc[k]);
+        }
+        finish(t0 + i, acc);
+      }
+#pragma unroll
+      for (int r = 0; r < TMAX - 1; ++r)
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) xs[r][k] = xs[CONV_TOKENS + r][k];
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int t0 = begin; t0 < end; t0 += CONV_TOKENS) {
+#pragma unroll
+    for (int r = 0; r < CONV_TOKENS + TMAX - 1; ++r)
+      if (r < CONV_TOKENS + taps - 1) load_row(t0 - (taps - 1) + r, xs[r]);
+#pragma unroll
+    for (int i = 0; i < CONV_TOKENS; ++i) {
+      if (t0 + i >= end) break;
+      const int seq = token_seq[t0 + i];
+      if (!FMS_IN(seq, n_seqs)) continue;
+      const int local = t0 + i - first_row[seq];  // the row's place among its sequence's rows of this step
+      const int slot = __ldcg(slots + seq);
+      if (!FMS_IN(slot, n_slots)) continue;
+      const float* tl = tail + (size_t)slot * (taps - 1) * channels;
+      float acc[CPT];
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) acc[k] = b[k];
+#pragma unroll
+      for (int j = 0; j < TMAX; ++j) {
+        if (j < taps) {
+          const int back = taps - 1 - j;  // how many rows before this one
+#pragma unroll
+          for (int k = 0; k < CPT; ++k) {
+            const float v = back <= local ? xs[i + j][k] : tl[(size_t)(taps - 1 + local - back) * channels + c + k];
+            acc[k] = fmaf(wt[k][j], v, acc[k]);
+          }
+        }
+      }
+      finish(t0 + i, acc);
+    }
+  }
+}
+
+// A decode step: one row a sequence.  The thread that makes a channel's value also leaves its tail, so that one kernel does what a
+// prompt's two do (the tail of a prompt is read by other blocks than the one that could write it).
+template <typename T, int CPT, int TMAX>
+__global__ void __launch_bounds__(CONV_THREADS) causal_conv_decode_kernel(const T* x, int stride, const float* w, const float* bias,
+                                                                          float* tail, const int* token_seq, const int* slots, float* out,
+                                                                          int channels, int taps, int act, int write_state, int n_seqs,
+                                                                          int n_slots) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int c = (blockIdx.x * CONV_THREADS + threadIdx.x) * CPT, t = blockIdx.y;
+  if (c >= channels) return;
+  const int seq = token_seq[t];
+  if (!FMS_IN(seq, n_seqs)) return;
+  const int slot = __ldcg(slots + seq);
+  if (!FMS_IN(slot, n_slots)) return;
+  float* tl = tail + (size_t)slot * (taps - 1) * channels + c;
+  float xs[TMAX][CPT], wt[CPT][TMAX];
+#pragma unroll
+  for (int j = 0; j < TMAX; ++j) {
+    if (j < taps - 1) load_channels<CPT>(tl + (size_t)j * channels, xs[j]);
+    else if (j == taps - 1) load_channels<CPT>(x + (size_t)t * stride + c, xs[j]);
+  }
+  float acc[CPT];
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    acc[k] = bias ? bias[c + k] : 0.f;
+#pragma unroll
+    for (int j = 0; j < TMAX; ++j) wt[k][j] = j < taps ? w[(size_t)(c + k) * taps + j] : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < TMAX; ++j)
+    if (j < taps) {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) acc[k] = fmaf(wt[k][j], xs[j][k], acc[k]);
+    }
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    out[(size_t)t * channels + c + k] = act ? acc[k] * sigmoid_f(acc[k]) : acc[k];
+    if (write_state) {
+#pragma unroll
+      for (int j = 0; j + 1 < TMAX; ++j)
+        if (j < taps - 1) tl[(size_t)j * channels + k] = xs[j + 1][k];
     }
   }
 }
@@ -842,6 +922,66 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = t;
 }
 
+// Groups of up to NI * 4 * TPU values, four at a time a thread, all of a thread's values and gates asked for at once and kept:
+// what the kernel behind (any size) reads twice, and the gate's sigmoid before the norm, once.  Bound by the bytes of x, gate and
+// out (2,048 rows of 8 groups of 1,024 values: 44 us; 77 with the rows read twice and a block of 256 threads a group).
+template <typename T, int TPU, int NI>
+__global__ void __launch_bounds__(TPU == 32 ? 128 : TPU) gated_group_rmsnorm_once_kernel(const float* x, const T* gate, int gate_stride,
+                                                                                         int gate_mode, const float* weight,
+                                                                                         int weight_period, float eps, float factor,
+                                                                                         T* out, int n_tokens, int width, int gs) {
+  __shared__ float scratch[33];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x % TPU;
+  const size_t unit = (size_t)blockIdx.x * (blockDim.x / TPU) + (threadIdx.x / TPU);
+  const int per_row = width / gs;
+  if (unit >= (size_t)n_tokens * per_row) return;  // TPU > 32: one unit a block, so the whole block alike
+  const size_t t = unit / per_row;
+  const int c0 = (int)(unit - t * per_row) * gs;
+  const float* xr = x + t * width + c0;
+  const T* gr = gate ? gate + t * gate_stride + c0 : nullptr;
+  float v[NI][4], z[NI][4];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int e = (i * TPU + lane) * 4;
+    if (e < gs) {
+      ld4(xr + e, v[i]);
+      if (gate_mode != 0) ld4(gr + e, z[i]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[i][k] = z[i][k] = 0.f;
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (gate_mode == 1) v[i][k] *= z[i][k] * sigmoid_f(z[i][k]);
+      ss = fmaf(v[i][k], v[i][k], ss);
+    }
+  float total;
+  if constexpr (TPU == 32) total = warp_sum(ss);
+  else total = block_sum(ss, scratch);
+  const float inv = 1.f / sqrtf(total / (float)gs + eps);
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int e = (i * TPU + lane) * 4;
+    if (e >= gs) continue;
+    float w[4];
+    ld4(weight + (c0 + e) % weight_period, w);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float r = v[i][k] * inv * w[k];
+      if (gate_mode == 2) r *= sigmoid_f(z[i][k]);
+      if (gate_mode == 3) r *= z[i][k] * sigmoid_f(z[i][k]);
+      v[i][k] = r * factor;
+    }
+    st4(out + t * width + c0 + e, v[i]);
+  }
+}
+
 // TPU threads per (token, group): a warp, or a block of 256 where the groups are long; VEC values a thread at a time
 // (4 where the sizes and addresses allow it)
 template <typename T, int TPU, int VEC>
@@ -912,16 +1052,35 @@ FMS_API int fms_causal_conv(const void* x, int dtype, int stride, const float* w
   if (taps < 1 || taps > MAX_TAPS) return fms_fail("causal_conv: %d taps (1..%d)", taps, MAX_TAPS);
   const size_t item = dtype == FMS_BF16 ? 2 : 4;
   const bool four = channels % 4 == 0 && stride % 4 == 0 && (uintptr_t)x % (4 * item) == 0 && (uintptr_t)out % 16 == 0;
-  const int cpt = four ? 4 : 1;
-  const dim3 grid((n_tokens + CONV_TOKENS - 1) / CONV_TOKENS, (channels / cpt + CONV_THREADS - 1) / CONV_THREADS);
-#define FMS_CONV(CPT, TMAX)                                                                                          \
-  fms_launch(causal_conv_kernel<T, CPT, TMAX>, grid, dim3(CONV_THREADS), 0, stream, (const T*)x, stride, w, bias,     \
-             (const float*)tail, token_seq, first_row, slots, out, n_tokens, channels, taps, act, n_seqs, n_slots)
+  const unsigned across = (channels / (four ? 4 : 1) + CONV_THREADS - 1) / CONV_THREADS;
+  if (n_tokens == n_seqs && n_tokens <= 65535) {  // every sequence brings at least one row, so each brings one
+    const bool four_tail = four && (uintptr_t)tail % 16 == 0;
+    const dim3 grid((channels / (four_tail ? 4 : 1) + CONV_THREADS - 1) / CONV_THREADS, n_tokens);
+#define FMS_CONV(CPT, TMAX)                                                                                                        \
+  fms_launch(causal_conv_decode_kernel<T, CPT, TMAX>, grid, dim3(CONV_THREADS), 0, stream, (const T*)x, stride, w, bias, tail, token_seq, \
+             slots, out, channels, taps, act, write_state, n_seqs, n_slots)
+    FMS_DISPATCH_DTYPE(dtype, T, {
+      if (four_tail && taps <= 4) FMS_CONV(4, 4);
+      else if (four_tail) FMS_CONV(4, MAX_TAPS);
+      else if (taps <= 4) FMS_CONV(1, 4);
+      else FMS_CONV(1, MAX_TAPS);
+    });
+#undef FMS_CONV
+    return fms_launch_status("causal_conv");
+  }
+  const bool exact = four && taps == 4 && (uintptr_t)w % 16 == 0;
+  // four groups of rows a block where that still leaves every multiprocessor four blocks
+  const int groups = exact && (long)(n_tokens / (4 * CONV_TOKENS)) * across >= 4 * 148 ? 4 : 1;
+  const dim3 grid((n_tokens + CONV_TOKENS * groups - 1) / (CONV_TOKENS * groups), across);
+#define FMS_CONV(CPT, TMAX, EXACT)                                                                                          \
+  fms_launch(causal_conv_kernel<T, CPT, TMAX, EXACT>, grid, dim3(CONV_THREADS), 0, stream, (const T*)x, stride, w, bias,     \
+             (const float*)tail, token_seq, first_row, slots, out, n_tokens, channels, taps, act, n_seqs, n_slots, groups)
   FMS_DISPATCH_DTYPE(dtype, T, {
-    if (four && taps <= 4) FMS_CONV(4, 4);
-    else if (four) FMS_CONV(4, MAX_TAPS);
-    else if (taps <= 4) FMS_CONV(1, 4);
-    else FMS_CONV(1, MAX_TAPS);
+    if (exact) FMS_CONV(4, 4, true);
+    else if (four && taps <= 4) FMS_CONV(4, 4, false);
+    else if (four) FMS_CONV(4, MAX_TAPS, false);
+    else if (taps <= 4) FMS_CONV(1, 4, false);
+    else FMS_CONV(1, MAX_TAPS, false);
     if (write_state && taps > 1)
       fms_launch(conv_tail_kernel<T>, dim3((channels + 127) / 128, n_seqs), dim3(128), 0, stream, (const T*)x, stride, tail,
                  first_row, slots, channels, taps, n_seqs, n_slots);
@@ -1172,7 +1331,19 @@ FMS_API int fms_gated_group_rmsnorm(const float* x, const void* gate, int dtype,
   FMS_DISPATCH_DTYPE(dtype, T, fms_launch(gated_group_rmsnorm_kernel<T, TPU, VEC>, dim3((unsigned)(BLOCKS)), dim3(THREADS), 0,  \
                                           stream, x, (const T*)gate, gate_stride, gate_mode, weight, weight_period, eps, \
                                           factor, (T*)out, n_tokens, width, group_size))
-  if (group_size >= 512) {
+#define FMS_NORM_ONCE(TPU, NI, BLOCKS, THREADS)                                                                          \
+  FMS_DISPATCH_DTYPE(dtype, T, fms_launch(gated_group_rmsnorm_once_kernel<T, TPU, NI>, dim3((unsigned)(BLOCKS)), dim3(THREADS), 0, \
+                                          stream, x, (const T*)gate, gate_stride, gate_mode, weight, weight_period, eps, \
+                                          factor, (T*)out, n_tokens, width, group_size))
+  const bool once = four && weight_period % 4 == 0 && (uintptr_t)weight % 16 == 0 && group_size <= 4096;
+  if (once) {
+    // a warp a group, except where few long groups would leave most of the multiprocessors without one
+    if (group_size <= 128) FMS_NORM_ONCE(32, 1, (units + 3) / 4, 128);
+    else if (group_size <= 256) FMS_NORM_ONCE(32, 2, (units + 3) / 4, 128);
+    else if (group_size <= 1024 && units >= 8 * 148) FMS_NORM_ONCE(32, 8, (units + 3) / 4, 128);
+    else if (group_size <= 1024) FMS_NORM_ONCE(256, 1, units, 256);
+    else FMS_NORM_ONCE(256, 4, units, 256);
+  } else if (group_size >= 512) {
     if (four) FMS_NORM(256, 4, units, 256);
     else FMS_NORM(256, 1, units, 256);
   } else {
@@ -1180,5 +1351,6 @@ FMS_API int fms_gated_group_rmsnorm(const float* x, const void* gate, int dtype,
     else FMS_NORM(32, 1, (units + 3) / 4, 128);
   }
 #undef FMS_NORM
+#undef FMS_NORM_ONCE
   return fms_launch_status("gated_group_rmsnorm");
 }

@@ -45,7 +45,8 @@ _SIGNATURES = {
     "fms_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _P],
     "fms_linear_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     "fms_token_gate_bf16_skinny": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "fms_grouped_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "fms_grouped_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _F, _F, _P],
+    "fms_strided_bf16_skinny": [_P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _L, _P],
     "fms_linear_act_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     "fms_linear_cap_bf16_skinny": [_P, _P, _P, _I, _I, _I, _F, _F, _P],
     "fms_glu_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
@@ -69,7 +70,7 @@ _SIGNATURES = {
     "fms_relu_squared": [_P, _I, _L, _P],
     "fms_gated_clamped": [_P, _P, _I, _I, _I, _F, _F, _P],
     "fms_latent_attention_prefill_bf16": [_P, _P, _P, _P, _L, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
-                                          _F, _I, _I, _I, _P, _I, _P, _P, _I, _P],
+                                          _F, _I, _I, _I, _P, _I, _I, _P, _P, _I, _P],
     "fms_latent_gather": [_P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _I, _I, _I, _P],
     "fms_attention_prefill_rows": [_P, _L, _P, _L, _P, _P, _L, _I, _L, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P, _L, _P, _P],
     "fms_latent_prepare": [_P, _I, _I, _P, _I, _I, _I, _P, _I, _F, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
@@ -92,7 +93,7 @@ _SIGNATURES = {
     "fms_gla_decode": [_P, _I, _I, _I, _I, _P, _I, _P, _F, _F, _P, _P, _I, _P, _F, _P, _I, _I, _I, _I, _I, _I, _P],
     "fms_linear_prepare": [_P, _I, _I, _P, _I, _I, _I, _F, _I, _P],
     "fms_exp_gates": [_P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
-    "fms_chunk_scan": [_I, _P, _P, _P, _L, _P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
+    "fms_chunk_scan": [_I, _P, _P, _P, _L, _P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
                        _I, _I, _I, _I, _I, _I, _P],
     "fms_decay_scan": [_P, _P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_attention_prefill_sink": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
@@ -914,14 +915,19 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
     return out
 
 
-CHUNK_SCAN_FROM = 64  # tokens of a sequence in one step from which a scan under one decay a head runs run by run
 CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
+CHUNK_SCAN_FROM = 256  # tokens of the longest sequence of a step from which a scan under one decay a head goes run by run
+
+
+def chunk_scan_pays(batch, heads: int, vdim: int) -> bool:
+    """Whether a step's scan goes run by run (``fms_chunk_scan``) or token by token."""
+    return max(batch.num_new) >= CHUNK_SCAN_FROM
 
 
 def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int):
     """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, decode steps and
     short prompts (which go token by token), a capture that has not seen the batch before (the runs come from the host)."""
-    if batch.decode or not batch.num_new or max(batch.num_new) < CHUNK_SCAN_FROM:
+    if batch.decode or not batch.num_new or not chunk_scan_pays(batch, heads, vdim):
         return None
     lib = load_library("chunk_scan")
     if not lib.fms_chunk_scan_takes(int(dim), int(vdim), heads // key_heads):
@@ -942,13 +948,14 @@ def _chunk_scan(kind: int, q: int, k: int, v: int, row: int, plan, batch, state:
     per_pass = max(1, min(n, CHUNK_STATE_BYTES // (heads * vdim * dim * 4)))
     new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)  # noqa: E731
     scores, states, totals = new(per_pass, key_heads, chunk, chunk), new(per_pass, heads, vdim, dim), new(per_pass, heads)
+    factors, flags = new(per_pass, heads, 4, chunk), torch.empty((per_pass, heads), dtype=torch.int32, device=dev)
     norms = new(per_pass, heads, dim) if kind == 1 else None
     carry = new(2, heads, vdim, dim) if per_pass < n else None
     _call("chunk_scan", "fms_chunk_scan", kind, q, k, v, row, _ptr(runs), _ptr(first_run), n, per_pass, _ptr(batch.slots), batch.n_seqs,
           _ptr(decay), _ptr(gates), _ptr(norm_in), _ptr(norm_state), dt_raw, dt_dtype, dt_stride, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
-          _ptr(state), _ptr(carry), _ptr(scores), _ptr(states), _ptr(norms), _ptr(totals), _ptr(o), heads, key_heads, dim, vdim,
+          _ptr(state), _ptr(carry), _ptr(scores), _ptr(factors), _ptr(totals), _ptr(states), _ptr(norms), _ptr(flags), _ptr(o), heads, key_heads, dim, vdim,
           1 if writes_state else 0, state.shape[0], _stream())
-    launches += 4 * ((n + per_pass - 1) // per_pass) - 1
+    launches += 3 * ((n + per_pass - 1) // per_pass) - 1
 
 
 def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
@@ -1181,6 +1188,13 @@ def grouped_linear(x: torch.Tensor, weight: torch.Tensor, groups: int, rows: int
         yv = torch.as_strided(y, (groups, rows, n_out), (y_group_offset, y_row_stride, 1), y.storage_offset())
         torch.bmm(xv, weight.transpose(1, 2), out=yv)
         return y
+    if x.dtype == torch.bfloat16 and rows <= SKINNY_ROWS and k % 8 == 0 and x_row_stride % 8 == 0 and x_group_offset % 8 == 0 \
+            and _ptr(x) % 16 == 0 and groups <= 65535:
+        # a decode step of few rows: the weight-streaming kernel, a block per group and run of its matrix's rows (8 rows, 32
+        # groups of 512 x 96: 4.7 us, of 128 x 512: 3.5; 18 each with a warp a row of the matrix)
+        _call("gemm_bf16_skinny", "fms_strided_bf16_skinny", _ptr(x), _ptr(weight), _ptr(y), rows, groups, n_out, k, x_row_stride,
+              x_group_offset, y_row_stride, y_group_offset, _stream())
+        return y
     _call("grouped", "fms_grouped_linear", _ptr(x), _ptr(weight), _ptr(y), _code(x.dtype), None, None, None, groups, rows,
           n_out, k, x_row_stride, x_group_offset, y_row_stride, y_group_offset, 0, 0.0, 0.0,
           1 if rows <= GROUPED_FEW_ROWS else 0, _stream())
@@ -1276,10 +1290,10 @@ def routed_linear(rows: torch.Tensor, weight: torch.Tensor, routing: Routing, gl
               _stream())
         return out
     y = torch.empty((n, n_out), dtype=rows.dtype, device=rows.device)
-    if rows.dtype == torch.bfloat16 and n <= SKINNY_ROWS * routing.top and k % 8 == 0 and (silu or not glu):
+    if rows.dtype == torch.bfloat16 and n <= SKINNY_ROWS * routing.top and k % 8 == 0:
         # up to eight tokens, so up to eight rows an expert: the weight-streaming kernel, a block per group and run of rows
         _call("gemm_bf16_skinny", "fms_grouped_bf16_skinny", _ptr(rows), _ptr(weight), _ptr(y), _ptr(routing.offsets),
-              routing.experts, n_out, k, 3 if glu else (2 if relu_squared else 0), _stream())
+              routing.experts, n_out, k, (3 if silu else 1) if glu else (2 if relu_squared else 0), float(limit), float(alpha), _stream())
         return y
     _call("grouped", "fms_grouped_linear", _ptr(rows), _ptr(weight), _ptr(y), _code(rows.dtype), _ptr(routing.offsets),
           _ptr(routing.tile_first), _ptr(routing.group_of_row), routing.experts, n, n_out, k, k, 0, n_out, 0,
@@ -1303,6 +1317,7 @@ def route_gather(ys: torch.Tensor, routing: Routing, every: Optional[torch.Tenso
 
 # ---- attention over cached latents -------------------------------------------------------------------
 _latent_split = None
+LATENT_SHORT_SPLIT = 64  # keys of a split of the tensor-core kernel in a decode step of few sequences
 USE_LATENT_MMA = os.environ.get("FMS_B200_LATENT_MMA", "1") != "0"  # 0: a prompt's rows through the float32 kernel too
 
 
@@ -1413,10 +1428,14 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
             and (rank + rot) % 32 == 0 and (gate is None or gate.dtype == torch.bfloat16)):
         # both products on the tensor cores, 32 rows a block: a prompt's rows as tokens x heads over all their keys; a
         # decode step's as one token's heads over one split of the keys, merged afterwards
-        n_splits, part_o, part_ml = 1, None, None
+        n_splits, part_o, part_ml, split = 1, None, None, _latent_split
         if batch.decode:
             heads_per_block = 32
-            n_splits = max(1, (batch.max_len_after + _latent_split - 1) // _latent_split)
+            # a block walks its split's keys one tile after the other (0.15 us a key): where the splits would leave
+            # multiprocessors without a block, splits of 64 keys instead of 256 (8 x 1,024 keys: 35 -> 19 us)
+            if n * ((batch.max_len_after + split - 1) // split) * ((heads + 31) // 32) < 148:
+                split = LATENT_SHORT_SPLIT
+            n_splits = max(1, (batch.max_len_after + split - 1) // split)
             if n_splits > 1:
                 part_o = torch.empty((n, heads, n_splits, rank), dtype=torch.float32, device=q_full.device)
                 part_ml = torch.empty((n, heads, n_splits, 2), dtype=torch.float32, device=q_full.device)
@@ -1431,7 +1450,7 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
               0 if gate is None else gate.shape[1], _ptr(sink), _code(sink.dtype) if sink is not None else F32,
               _ptr(view.table), view.table.shape[1], view.block_tokens, _ptr(batch.slots), _ptr(batch.first_row),
               _ptr(batch.positions), _ptr(tiles), tiles.shape[0], tile_tokens, heads_per_block, heads, rank, rot,
-              float(scale), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _ptr(batch.token_seq), n_splits,
+              float(scale), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _ptr(batch.token_seq), n_splits, split,
               _ptr(part_o), _ptr(part_ml), int(window), _stream())
         if n_splits > 1:
             launches += 1

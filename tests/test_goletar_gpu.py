@@ -456,3 +456,23 @@ def test_trace_program_replays_a_batch(folders, oracles, tmp_path):
     for t in range(4):
         want = [wa[66 + t]] + ([wb[5 + t]] if t % 2 else [])
         close(read(t + 1), torch.stack(want), "fp32")
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8])
+@pytest.mark.parametrize("groups,n_out,k", [(3, 512, 96), (5, 40, 8), (2, 128, 512), (4, 70, 264)])
+def test_a_product_a_group_of_few_rows(rows, groups, n_out, k):
+    """The weight-streaming kernel over strided groups: rows of x and of y that lie inside wider ones; columns of no multiple of its
+    16 and 32 rows of the matrix, K of no multiple of its 32.  Bound: float32 sums of bfloat16 products, rounded to bfloat16."""
+    from fms_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(rows + n_out)
+    wide, gap = groups * (k + 8) + 16, groups * n_out + 24
+    x = torch.randn(rows, wide, generator=g).to(torch.bfloat16).cuda()
+    w = torch.randn(groups, n_out, k, generator=g).to(torch.bfloat16).cuda()
+    y = torch.full((rows, gap), 7.0, dtype=torch.bfloat16).cuda()
+    ops.grouped_linear(x, w, groups, rows, n_out, k, wide, k + 8, y, gap, n_out)
+    xs = torch.stack([x[:, i * (k + 8): i * (k + 8) + k] for i in range(groups)]).double()
+    want = torch.einsum("grk,gnk->grn", xs, w.double())
+    got = y[:, : groups * n_out].view(rows, groups, n_out).transpose(0, 1).double()
+    bound = 2.0 ** -8 * want.abs() + (k + 8) * 2.0 ** -24 * torch.einsum("grk,gnk->grn", xs.abs(), w.double().abs())
+    assert bool(((got - want).abs() <= bound).all()) and bool((y[:, groups * n_out:] == 7.0).all())
