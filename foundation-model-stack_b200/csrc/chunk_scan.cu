@@ -14,13 +14,13 @@
 //                  registers: leaves the state before every run
 //   chunk_outputs  o of every run and head, all runs at once
 //
-// The products are float32 products on the tensor cores: every operand is the sum of three bfloat16 (8 bits of it each, 24 in
-// all), and the six products of parts that matter are added in float32 (what is left out is 2^-24 of a product and less, as much as
-// float32 rounds).  On the FMA pipe shared memory returns its 128 bytes a cycle as slowly as the pipe multiplies (8 x 8 elements a
-// thread), and a single prompt's states are few warps' work.  Products of decays are taken as products (no logarithms: a decay of
-// zero and a run of tiny ones need no case), and a token's values never touch earlier tokens' rows, not even times zero.  The
-// states of the runs of one pass lie in at most pass_runs runs' worth of scratch; longer steps take several passes, between which the
-// one sequence that a boundary cuts has its state in `carry`.
+// Bound by the FMA pipe and by what shared memory returns to registers: 8 x 8 elements a thread, two elements a multiply-add
+// instruction (fma.rn.f32x2, the same roundings).  (On the tensor cores, with three bfloat16 parts a value and six products of
+// parts, the results were ten times further from 64 bits, 9e-7 instead of 8e-8 of a row, and no sooner there.)
+// Products of decays are taken as products (no logarithms: a decay of zero and a run of tiny ones need no case), and a token's
+// values never touch earlier tokens' rows, not even times zero.  The states of the runs of one pass lie in at most pass_runs runs'
+// worth of scratch; longer steps take several passes, between which the one sequence that a boundary cuts has its state in
+// `carry`.
 //
 // KIND 0: a = decay[head], b = 1.  KIND 1: (a, b, e) = gates[token, head]; a normalizer n_t = a n + b k beside S, and o is divided
 // by max(|n . q|, e) + 1e-6.  KIND 2: a = exp(-exp(a_log) dt), b = dt = softplus(raw + bias), and o += d_skip v; key heads
@@ -31,7 +31,8 @@ namespace {
 constexpr int C = 64;        // tokens of a run
 constexpr int COLS = 128;    // value columns of a block of outputs: one head of 128 values or two of 64
 constexpr int DIM = 128;     // key channels
-constexpr int ROW128 = 128 + 8, ROW64 = 64 + 8;  // strides of tiles of 128 and of 64 values a row
+constexpr int SLICE = 32, SROW = SLICE + 4;  // of the scores: channels brought into shared memory at a time
+constexpr int TROW = C + 4, CROW = COLS + 4; // rows of 64 tokens, of 128 columns, padded by four floats
 
 struct ChunkArgs {
   const float* q;  // token t, key head g: q + t * row + g * dim; k alike; v: v + t * row + head * vdim
@@ -53,10 +54,10 @@ struct ChunkArgs {
   int dt_is_bf16;
   float* state;    // [slots, heads, vdim, dim]
   float* carry;    // [2, heads, vdim, dim], written by every other pass, or null (one pass)
-  float* scores;   // scratch: [runs of a pass, key heads, C, C], element [s][t], quarters with s > t left out
+  float* scores;   // scratch: [runs of a pass, key heads, C, C], element [s][t]
   float* factors;  // scratch: [runs of a pass, heads, 4, C]: a, b, G, D(C, .)
   float* totals;   // scratch: [runs of a pass, heads]: G_C
-  float* states;   // scratch: [runs of a pass, heads, vdim, dim]
+  float* states;   // scratch: [runs of a pass, heads * vdim / COLS, dim, COLS]
   float* norms;    // scratch, KIND 1: [runs of a pass, heads, dim]
   int* flags;      // scratch: [runs of a pass, heads]: a value of the run's is not finite
   float* o;        // [tokens, heads * vdim]
@@ -64,79 +65,65 @@ struct ChunkArgs {
   int run_lo, run_hi, pass;  // this pass
 };
 
-// ---- float32 operands in three bfloat16 parts, tiles in shared memory [part][row][stride] ------------------------------
-typedef __nv_bfloat16 bf16;
-constexpr int PARTS = 3;
+__device__ __forceinline__ void copy16(float* smem, const float* gmem, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ uint32_t pack(float x, float y) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-  return *reinterpret_cast<const uint32_t*>(&v);
+typedef unsigned long long f32x2;  // two floats side by side in registers
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
-// two neighbouring values into the parts' words
-__device__ __forceinline__ void split2(float x, float y, uint32_t (&w)[PARTS]) {
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 swapped(f32x2 v) {
+  float a, b;
+  unpack2(v, a, b);
+  return pack2(b, a);
+}
+// acc [rows 2 i, 2 i + 1][columns j, j ^ 1] += a [rows] x b [columns]: one step of an outer product of 8 rows (two runs of
+// four, RS apart) by 2 P columns (runs of four, CS apart)
+template <int P, int RS, int CS>
+__device__ __forceinline__ void outer_step(const float* a, const float* b, f32x2 (&acc)[4][2 * P]) {
+  f32x2 x[4], y[P], z[P];
 #pragma unroll
-  for (int p = 0; p < PARTS; ++p) {
-    w[p] = pack(x, y);
-    x -= __uint_as_float(w[p] << 16);  // exact: the remainder has fewer bits than the value
-    y -= __uint_as_float(w[p] & 0xffff0000u);
+  for (int i = 0; i < 2; ++i) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(a + RS * i);
+    x[2 * i] = v.x;
+    x[2 * i + 1] = v.y;
   }
-}
-// four neighbouring values at `at` of a tile whose parts lie `part` elements apart
-__device__ __forceinline__ void put4(bf16* at, int part, float4 v) {
-  uint32_t a[PARTS], b[PARTS];
-  split2(v.x, v.y, a);
-  split2(v.z, v.w, b);
 #pragma unroll
-  for (int p = 0; p < PARTS; ++p) *reinterpret_cast<uint2*>(at + p * part) = make_uint2(a[p], b[p]);
-}
-template <bool TRANS>
-__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const bf16* p) {
-  if (TRANS)
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-  else
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-}
-// The 16 x 16 operand A at (m, k): stored [m][k], or [k][m] (ACROSS).  Rows of every tile are 16 bytes longer than a multiple of 64 of
-// them: the eight rows of a matrix meet different banks.
-template <bool ACROSS>
-__device__ __forceinline__ void load_a(uint32_t (&r)[4], const bf16* tile, int stride, int m, int k, int lane) {
-  if (ACROSS) ldmatrix4<true>(r, tile + (k + (lane & 7) + ((lane >> 4) << 3)) * stride + m + ((lane >> 3) & 1) * 8);
-  else ldmatrix4<false>(r, tile + (m + (lane & 15)) * stride + k + (lane >> 4) * 8);
-}
-// The operands B of two neighbouring 8 columns at (n, k): stored [n][k], or [k][n] (ACROSS)
-template <bool ACROSS>
-__device__ __forceinline__ void load_b(uint32_t (&r)[4], const bf16* tile, int stride, int n, int k, int lane) {
-  if (ACROSS) ldmatrix4<true>(r, tile + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * stride + n + (lane >> 4) * 8);
-  else ldmatrix4<false>(r, tile + (n + (lane & 7) + ((lane >> 4) << 3)) * stride + k + ((lane >> 3) & 1) * 8);
-}
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// acc [MT x 16 rows][NT x 8 columns] += A[m0 .., ka ..] B[kb .., n0 ..] for 16 k: six products of parts, the smallest first.
-// Element e of a lane: row lane / 4 + 8 (e / 2), column 2 (lane % 4) + e % 2 of its 16 x 8.
-template <int MT, int NT, bool A_ACROSS, bool B_ACROSS>
-__device__ __forceinline__ void step16(float (&acc)[MT][NT][4], const bf16* a, int a_part, int a_stride, int m0, int ka, const bf16* b,
-                                       int b_part, int b_stride, int n0, int kb, int lane) {
-  uint32_t x[PARTS][MT][4];
-#pragma unroll
-  for (int p = 0; p < PARTS; ++p)
-#pragma unroll
-    for (int i = 0; i < MT; ++i) load_a<A_ACROSS>(x[p][i], a + p * a_part, a_stride, m0 + 16 * i, ka, lane);
-#pragma unroll
-  for (int j = 0; j < NT; j += 2) {
-    uint32_t y[PARTS][4];
-#pragma unroll
-    for (int p = 0; p < PARTS; ++p) load_b<B_ACROSS>(y[p], b + p * b_part, b_stride, n0 + 8 * j, kb, lane);
-    constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};
-#pragma unroll
-    for (int t = 0; t < 6; ++t)
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) mma(acc[i][j + h], x[PA[t]][i], y[PB[t]][2 * h], y[PB[t]][2 * h + 1]);
+  for (int j = 0; j < P / 2; ++j) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(b + CS * j);
+    y[2 * j] = v.x;
+    y[2 * j + 1] = v.y;
+    z[2 * j] = swapped(v.x);
+    z[2 * j + 1] = swapped(v.y);
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      acc[i][2 * j] = fma2(x[i], y[j], acc[i][2 * j]);
+      acc[i][2 * j + 1] = fma2(x[i], z[j], acc[i][2 * j + 1]);
+    }
+}
+template <int P>
+__device__ __forceinline__ void outer_unpack(const f32x2 (&acc)[4][2 * P], float (&out)[8][2 * P]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      unpack2(acc[i][2 * j], out[2 * i][2 * j], out[2 * i + 1][2 * j + 1]);
+      unpack2(acc[i][2 * j + 1], out[2 * i][2 * j + 1], out[2 * i + 1][2 * j]);
+    }
 }
 
 // (a, b) of a token and head; beyond the run's end (1, 0), which changes nothing
@@ -156,29 +143,28 @@ __device__ __forceinline__ float2 token_gates(const ChunkArgs& g, int t, int end
   return make_float2((float)exp(-exp((double)g.a_log[head]) * dt), (float)dt);
 }
 
-// ---- scores: [s][t] of 64 x 64 a block, a warp 32 x 32; the factors of the key head's heads, a warp a head ------------------
-constexpr size_t SCORES_SMEM = (size_t)2 * PARTS * C * ROW128 * sizeof(bf16);
-
+// ---- scores: 64 x 64 a block, 8 x 4 a thread; the factors of the key head's heads, a warp a head ----------------------------
 template <int KIND>
 __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
-  extern __shared__ __align__(16) bf16 tiles[];
-  bf16* ks = tiles;                        // [PARTS][C][ROW128]
-  bf16* qs = tiles + PARTS * C * ROW128;
+  __shared__ __align__(16) float sm[2][2][C][SROW];
   pdl_launch_dependents();
   pdl_wait();
-  const int run = g.run_lo + blockIdx.x, kh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int run = g.run_lo + blockIdx.x, kh = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
   const int row0 = g.runs[2 * run], end = g.runs[2 * run + 1], rows = end - row0;
   const float* q = g.q + (size_t)row0 * g.row + (size_t)kh * DIM;
   const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
-#pragma unroll 4
-  for (int i = tid; i < C * (DIM / 4); i += 128) {
-    const int t = i / (DIM / 4), d = (i % (DIM / 4)) * 4;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    put4(ks + t * ROW128 + d, C * ROW128, t < rows ? *reinterpret_cast<const float4*>(k + (size_t)t * g.row + d) : zero);
-    put4(qs + t * ROW128 + d, C * ROW128, t < rows ? *reinterpret_cast<const float4*>(q + (size_t)t * g.row + d) : zero);
-  }
+  auto issue = [&](int d0, int buf) {
+    for (int i = tid; i < C * (SLICE / 4); i += 128) {
+      const int t = i / (SLICE / 4), d = (i % (SLICE / 4)) * 4;
+      const size_t at = (size_t)min(t, rows - 1) * g.row + d0 + d;
+      copy16(&sm[buf][0][t][d], q + at, t < rows);
+      copy16(&sm[buf][1][t][d], k + at, t < rows);
+    }
+    copies_commit();
+  };
+  issue(0, 0);
   const int shared = g.heads / g.key_heads;
-  for (int head = kh * shared + warp; head < (kh + 1) * shared; head += 4) {  // a lane two neighbouring tokens
+  for (int head = kh * shared + (tid >> 5); head < (kh + 1) * shared; head += 4) {  // a lane two neighbouring tokens
     const float2 w0 = token_gates<KIND>(g, row0 + 2 * lane, end, head), w1 = token_gates<KIND>(g, row0 + 2 * lane + 1, end, head);
     float upto = w0.x * w1.x, behind = upto;  // inclusive products over this lane's tokens and all earlier, all later ones
 #pragma unroll
@@ -200,143 +186,164 @@ __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
       g.flags[(size_t)blockIdx.x * g.heads + head] = 0;
     }
   }
-  __syncthreads();
-  const int s0 = (warp >> 1) * 32, t0 = (warp & 1) * 32;
-  if (s0 > t0) return;  // tokens behind every query of this quarter: never read
-  float acc[2][4][4] = {};
+  const int ty = tid >> 4, tx = tid & 15;  // tokens t = ty * 8 + i, s = tx + 16 j
+  float acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 #pragma unroll 1
-  for (int d = 0; d < DIM; d += 16)
-    step16<2, 4, false, false>(acc, ks, C * ROW128, ROW128, s0, d, qs, C * ROW128, ROW128, t0, d, lane);
+  for (int d0 = 0; d0 < DIM; d0 += SLICE) {
+    const int buf = (d0 / SLICE) & 1;
+    if (d0 + SLICE < DIM) {
+      issue(d0 + SLICE, buf ^ 1);
+      copies_wait<1>();
+    } else {
+      copies_wait<0>();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < SLICE; d += 4) {
+      float4 kx[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kx[j] = *reinterpret_cast<const float4*>(&sm[buf][1][tx + 16 * j][d]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 qx = *reinterpret_cast<const float4*>(&sm[buf][0][ty * 8 + i][d]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[i][j] = fmaf(qx.x, kx[j].x, acc[i][j]);
+          acc[i][j] = fmaf(qx.y, kx[j].y, acc[i][j]);
+          acc[i][j] = fmaf(qx.z, kx[j].z, acc[i][j]);
+          acc[i][j] = fmaf(qx.w, kx[j].w, acc[i][j]);
+        }
+      }
+    }
+    __syncthreads();
+  }
   float* out = g.scores + ((size_t)blockIdx.x * g.key_heads + kh) * C * C;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; e += 2)
-        *reinterpret_cast<float2*>(out + (s0 + 16 * i + (lane >> 2) + 4 * e) * C + t0 + 8 * j + 2 * (lane & 3)) = make_float2(acc[i][j][e], acc[i][j][e + 1]);
+    for (int i = 0; i < 8; i += 4)
+      *reinterpret_cast<float4*>(out + (tx + 16 * j) * C + ty * 8 + i) = make_float4(acc[i][j], acc[i + 1][j], acc[i + 2][j], acc[i + 3][j]);
 }
 
-// ---- the states before every run: VT value columns x 128 key channels a block, a warp 32 x 32 (VT = 32: 32 x 16) -----------------
-// A sequence's runs in order, the state in registers as the tensor cores leave it; the next run's keys and values are on their
-// way from global memory (in registers) meanwhile.  VT = 32 where 64 would leave multiprocessors without a block.
-template <int VT> constexpr size_t STATES_SMEM = (size_t)PARTS * C * (ROW128 + VT + 8) * sizeof(bf16);
+// ---- the states before every run: 128 key channels x VT value columns a block, 8 x VT / 8 a thread ------------------------
+// A sequence's runs in order, the state and a run's own part of it in registers; the next run's keys and values are on their
+// way meanwhile.  VT = 64, or 32 where that gives a single prompt's blocks to more multiprocessors.
+template <int VT> constexpr size_t STATES_SMEM = (size_t)2 * C * (DIM + VT) * sizeof(float);
 
 template <int VDIM, int KIND, int VT>
-__global__ void __launch_bounds__(256) chunk_states_kernel(ChunkArgs g) {
-  constexpr int WARPS_D = 8 / (VT / 32), NT = DIM / WARPS_D / 8, VROW = VT + 8, NK = C * DIM / 4 / 256, NV = C * VT / 4 / 256;
-  extern __shared__ __align__(16) bf16 tiles[];
-  bf16* ks = tiles;                        // [PARTS][C][ROW128]
-  bf16* vs = tiles + PARTS * C * ROW128;   // [PARTS][C][VROW], times D(C, s)
+__global__ void __launch_bounds__(128, 2) chunk_states_kernel(ChunkArgs g) {
+  constexpr int P = VT / 16;  // pairs of columns a thread
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float weight[C];
   pdl_launch_dependents();
   pdl_wait();
-  const int seq = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int seq = blockIdx.y, tid = threadIdx.x;
   const int lo = max(g.first_run[seq], g.run_lo), hi = min(g.first_run[seq + 1], g.run_hi);
   if (lo >= hi) return;
   const int slot = __ldcg(g.slots + seq);
   if (!FMS_IN(slot, g.n_slots)) return;
   const bool begins = lo == g.first_run[seq], ends = hi == g.first_run[seq + 1];
   const int col0 = blockIdx.x * VT, head = col0 / VDIM, kh = head / (g.heads / g.key_heads);  // columns over all heads
-  float4 pk[NK], pv[NV];
-  float pw[NV], total_next = 0.f;
-  auto fetch = [&](int run) {
+  auto issue = [&](int run, int buf) {
+    float* ks = sm + buf * C * (DIM + VT);
+    float* vs = ks + C * DIM;
     const int row0 = g.runs[2 * run], rows = g.runs[2 * run + 1] - row0;
     const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
     const float* v = g.v + (size_t)row0 * g.row + col0;
-    const float* w = g.factors + (((size_t)(run - g.run_lo) * g.heads + head) * 4 + 3) * C;
-#pragma unroll
-    for (int n = 0; n < NK; ++n) {
-      const int i = tid + 256 * n, t = i / (DIM / 4), d = (i % (DIM / 4)) * 4;
-      pk[n] = t < rows ? *reinterpret_cast<const float4*>(k + (size_t)t * g.row + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < C * (DIM / 4); i += 128) {
+      const int t = i / (DIM / 4), d = (i % (DIM / 4)) * 4;
+      copy16(ks + t * DIM + d, k + (size_t)min(t, rows - 1) * g.row + d, t < rows);
     }
-#pragma unroll
-    for (int n = 0; n < NV; ++n) {
-      const int i = tid + 256 * n, t = i / (VT / 4), c = (i % (VT / 4)) * 4;
-      pv[n] = t < rows ? *reinterpret_cast<const float4*>(v + (size_t)t * g.row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-      pw[n] = w[t];
+    for (int i = tid; i < C * (VT / 4); i += 128) {
+      const int t = i / (VT / 4), c = (i % (VT / 4)) * 4;
+      copy16(vs + t * VT + c, v + (size_t)min(t, rows - 1) * g.row + c, t < rows);
     }
-    total_next = g.totals[(size_t)(run - g.run_lo) * g.heads + head];
+    copies_commit();
   };
-  fetch(lo);
-  const int c0 = (warp / WARPS_D) * 32, d0 = (warp % WARPS_D) * (NT * 8);
+  issue(lo, 0);
+  const int td = (tid >> 3) * 4, tv = (tid & 7) * 4;  // channels td .. + 3 and td + 64 .., columns tv .. + 3 and tv + 32 ..
   const size_t per_seq = (size_t)g.heads * VDIM * DIM;
-  // element e of tile (i, j): column c0 + 16 i + lane / 4 + 8 (e / 2), channel d0 + 8 j + 2 (lane % 4) + e % 2
-  const size_t mine = (size_t)(col0 + c0 + (lane >> 2)) * DIM + d0 + 2 * (lane & 3);
-  const float* from = (begins ? g.state + (size_t)slot * per_seq : g.carry + (g.pass & 1) * per_seq) + mine;
-  float S[2][NT][4];
+  const float* from = (begins ? g.state + (size_t)slot * per_seq : g.carry + (g.pass & 1) * per_seq) + (size_t)col0 * DIM;
+  float S[8][2 * P];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < 2 * P; ++j)
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const float2 x = *reinterpret_cast<const float2*>(from + (size_t)(16 * i + 4 * e) * DIM + 8 * j);
-        S[i][j][e] = x.x;
-        S[i][j][e + 1] = x.y;
-      }
-  const bool norms = KIND == 1 && col0 % VDIM == 0 && tid < DIM;  // this thread walks the normalizer's channel tid
+    for (int i = 0; i < 8; i += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(from + (size_t)(tv + (j & 3) + (j >> 2) * 32) * DIM + td + (i >> 2) * 64);
+      S[i][j] = x.x;
+      S[i + 1][j] = x.y;
+      S[i + 2][j] = x.z;
+      S[i + 3][j] = x.w;
+    }
+  const bool norms = KIND == 1 && col0 % VDIM == 0;  // this block walks the head's normalizer: thread d its channel d
   float n = 0.f;
-  float* n_at = KIND == 1 ? g.norm_in + ((size_t)seq * g.heads + head) * DIM + (tid % DIM) : nullptr;
+  float* n_at = KIND == 1 ? g.norm_in + ((size_t)seq * g.heads + head) * DIM + tid : nullptr;
   if (norms) n = *n_at;
 #pragma unroll 1
   for (int run = lo; run < hi; ++run) {
-    const int local = run - g.run_lo;
-    const float total = total_next;
-    int bad = 0;
-#pragma unroll
-    for (int m = 0; m < NK; ++m) {
-      const int i = tid + 256 * m;
-      put4(ks + (i / (DIM / 4)) * ROW128 + (i % (DIM / 4)) * 4, C * ROW128, pk[m]);
+    const int local = run - g.run_lo, buf = (run - lo) & 1;
+    if (run + 1 < hi) {
+      issue(run + 1, buf ^ 1);
+      copies_wait<1>();
+    } else {
+      copies_wait<0>();
     }
-#pragma unroll
-    for (int m = 0; m < NV; ++m) {
-      const int i = tid + 256 * m;
-      const float4 x = pv[m];
-      const float w = pw[m];
-      bad |= !(fabsf(x.x) <= 3.3e38f && fabsf(x.y) <= 3.3e38f && fabsf(x.z) <= 3.3e38f && fabsf(x.w) <= 3.3e38f);
-      put4(vs + (i / (VT / 4)) * VROW + (i % (VT / 4)) * 4, C * VROW, make_float4(x.x * w, x.y * w, x.z * w, x.w * w));
+    const float total = g.totals[(size_t)local * g.heads + head];
+    if (tid < C) weight[tid] = g.factors[(((size_t)local * g.heads + head) * 4 + 3) * C + tid];
+    __syncthreads();
+    const float* ks = sm + buf * C * (DIM + VT);
+    float* vs = sm + buf * C * (DIM + VT) + C * DIM;
+    int bad = 0;
+    for (int i = tid; i < C * (VT / 4); i += 128) {
+      const float w = weight[i / (VT / 4)];
+      float4* p = reinterpret_cast<float4*>(vs) + i;
+      const float4 x = *p;
+      bad |= !(fabsf(x.x) <= 3.4028235e38f && fabsf(x.y) <= 3.4028235e38f && fabsf(x.z) <= 3.4028235e38f && fabsf(x.w) <= 3.4028235e38f);
+      *p = make_float4(x.x * w, x.y * w, x.z * w, x.w * w);
     }
     if (__syncthreads_or(bad) && tid == 0) g.flags[(size_t)local * g.heads + head] = 1;
-    if (run + 1 < hi) fetch(run + 1);
-    // what is before the run goes out
-    float* out = g.states + (size_t)local * per_seq + mine;
+    // what is before the run goes out, [dim][COLS] of the block of heads that outputs takes together
+    float* out = g.states + ((size_t)local * (g.heads * VDIM / COLS) + col0 / COLS) * DIM * COLS + col0 % COLS + tv;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+      for (int j = 0; j < 2 * P; j += 4)
+        *reinterpret_cast<float4*>(out + (size_t)(td + (i & 3) + (i >> 2) * 64) * COLS + (j >> 2) * 32) =
+            make_float4(S[i][j], S[i][j + 1], S[i][j + 2], S[i][j + 3]);
+    f32x2 acc[4][2 * P];
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) *reinterpret_cast<float2*>(out + (size_t)(16 * i + 4 * e) * DIM + 8 * j) = make_float2(S[i][j][e], S[i][j][e + 1]);
-    float T[2][NT][4] = {};
-#pragma unroll 1
-    for (int s = 0; s < C; s += 16)
-      step16<2, NT, true, true>(T, vs, C * VROW, VROW, c0, s, ks, C * ROW128, ROW128, d0, s, lane);
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int j = 0; j < 2 * P; ++j) acc[i][j] = 0;
+#pragma unroll 8
+    for (int s = 0; s < C; ++s) outer_step<P, 64, 32>(ks + s * DIM + td, vs + s * VT + tv, acc);
+    float T[8][2 * P];
+    outer_unpack<P>(acc, T);
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[i][j][e] = fmaf(total, S[i][j][e], T[i][j][e]);
+      for (int j = 0; j < 2 * P; ++j) S[i][j] = fmaf(total, S[i][j], T[i][j]);
     if (norms) {
       g.norms[((size_t)local * g.heads + head) * DIM + tid] = n;
-      const float* w = g.factors + (((size_t)local * g.heads + head) * 4 + 3) * C;
       float own = 0.f;
 #pragma unroll 8
-      for (int s = 0; s < C; ++s) {  // rows beyond the run's end are zeros; the three parts add up to the value
-        const bf16* at = ks + s * ROW128 + tid;
-        own = fmaf(w[s], __bfloat162float(at[0]) + (__bfloat162float(at[C * ROW128]) + __bfloat162float(at[2 * C * ROW128])), own);
-      }
+      for (int s = 0; s < C; ++s) own = fmaf(weight[s], ks[s * DIM + tid], own);  // rows beyond the run's end are zeros
       n = fmaf(total, n, own);
     }
-    __syncthreads();  // the tiles are free
+    __syncthreads();  // the stage and the weights are free
   }
   if (!ends || g.write_state) {
-    float* to = (ends ? g.state + (size_t)slot * per_seq : g.carry + ((g.pass + 1) & 1) * per_seq) + mine;
+    float* to = (ends ? g.state + (size_t)slot * per_seq : g.carry + ((g.pass + 1) & 1) * per_seq) + (size_t)col0 * DIM;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < 2 * P; ++j)
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; e += 2) *reinterpret_cast<float2*>(to + (size_t)(16 * i + 4 * e) * DIM + 8 * j) = make_float2(S[i][j][e], S[i][j][e + 1]);
+      for (int i = 0; i < 8; i += 4)
+        *reinterpret_cast<float4*>(to + (size_t)(tv + (j & 3) + (j >> 2) * 32) * DIM + td + (i >> 2) * 64) =
+            make_float4(S[i][j], S[i + 1][j], S[i + 2][j], S[i + 3][j]);
   }
   if (norms) {
     *n_at = n;
@@ -344,21 +351,22 @@ __global__ void __launch_bounds__(256) chunk_states_kernel(ChunkArgs g) {
   }
 }
 
-// ---- outputs: 64 tokens x 128 value columns a block, a warp 32 x 32 -----------------------------------------------------
-// First q against the state before the run, 64 channels at a time, then the run's own tokens: P as [s][t], a thread a token t
-// walking s downwards.  A warp's 32 columns belong to one head; it takes the tokens up to its last row, earlier rows with zeros
-// of P (or, where a value is not finite, by selection).
-constexpr int Q_TILE = PARTS * C * ROW64, S_TILE = PARTS * COLS * ROW64, P_TILE = PARTS * C * ROW64, V_TILE = PARTS * C * ROW128;
+// ---- outputs: 64 tokens x 128 value columns a block, 8 x 8 a thread ---------------------------------------------------
+// First q against the state before the run, 16 channels at a time (q transposed on its way through registers, the state by
+// asynchronous copies), then the run's own tokens: P^T, a thread a token t walking s downwards.  A warp's 64 columns belong to one
+// head; it takes the tokens up to its last row, earlier rows with zeros of P (or, where a value is not finite, by selection).
+constexpr int OSLICE = 16;
 template <int VDIM>
-constexpr size_t OUT_SMEM = sizeof(bf16) * (size_t)(Q_TILE + S_TILE > COLS / VDIM * P_TILE + V_TILE ? Q_TILE + S_TILE : COLS / VDIM * P_TILE + V_TILE);
+constexpr size_t OUT_SMEM = (size_t)(C * CROW + COLS / VDIM * C * TROW) * sizeof(float);
+static_assert(2 * OSLICE * (TROW + CROW) <= C * CROW, "the slices lie where the values go afterwards");
 
 template <int VDIM, int KIND>
-__global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(ChunkArgs g) {
+__global__ void __launch_bounds__(128, VDIM == 128 ? 4 : 3) chunk_outputs_kernel(ChunkArgs g) {
   constexpr int HB = COLS / VDIM;
-  extern __shared__ __align__(16) bf16 tiles[];
-  bf16* qs = tiles;                // [PARTS][C][ROW64], then P: [HB][PARTS][C][ROW64], row s, column t
-  bf16* ss = tiles + Q_TILE;       // [PARTS][COLS][ROW64]
-  bf16* vs = tiles + HB * P_TILE;  // [PARTS][C][ROW128], afterwards
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;                                 // [2][OSLICE][TROW], then the values [C][CROW] over both
+  float* ss = sm + 2 * OSLICE * TROW;             // [2][OSLICE][CROW]
+  float* Pt = sm + C * CROW;                      // [HB][C][TROW]: row s, column t
   __shared__ float as[HB][C], bs[HB][C], G[HB][C], nq[KIND == 1 ? C : 1];
   pdl_launch_dependents();
   pdl_wait();
@@ -366,129 +374,140 @@ __global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(ChunkArgs g) {
   const int row0 = g.runs[2 * run], rows = g.runs[2 * run + 1] - row0;
   const int kh = head0 / (g.heads / g.key_heads);
   const float* q = g.q + (size_t)row0 * g.row + (size_t)kh * DIM;
-  const float* S = g.states + ((size_t)local * g.heads + head0) * VDIM * DIM;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (tid < HB * C) {
-    const float* f = g.factors + ((size_t)local * g.heads + head0 + tid / C) * 4 * C + tid % C;
-    as[tid / C][tid % C] = f[0];
-    bs[tid / C][tid % C] = f[C];
-    G[tid / C][tid % C] = f[2 * C];
-  }
-  const int t0 = (warp >> 2) * 32, c0 = (warp & 3) * 32, my_head = c0 / VDIM;
-  float acc[2][4][4] = {};
-#pragma unroll 1
-  for (int d0 = 0; d0 < DIM; d0 += 64) {
-    if (d0) __syncthreads();
+  const float* S = g.states + ((size_t)local * gridDim.y + blockIdx.y) * DIM * COLS;
+  float4 pq[2];
+  auto fetch_q = [&](int d0) {
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int i = tid + 256 * n, t = i / 16, d = (i % 16) * 4;
-      put4(qs + t * ROW64 + d, C * ROW64, t < rows ? *reinterpret_cast<const float4*>(q + (size_t)t * g.row + d0 + d) : zero);
+    for (int i = 0; i < 2; ++i) {
+      const int t = (tid >> 2) + 32 * i;
+      pq[i] = t < rows ? *reinterpret_cast<const float4*>(q + (size_t)t * g.row + d0 + (tid & 3) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+  };
+  auto put_q = [&](int buf) {
+    float* p = qs + buf * OSLICE * TROW + (tid & 3) * 4 * TROW + (tid >> 2);
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const int i = tid + 256 * n, c = i / 16, d = (i % 16) * 4;
-      put4(ss + c * ROW64 + d, COLS * ROW64, *reinterpret_cast<const float4*>(S + (size_t)c * DIM + d0 + d));
+    for (int i = 0; i < 2; ++i) {
+      p[32 * i] = pq[i].x;
+      p[32 * i + TROW] = pq[i].y;
+      p[32 * i + 2 * TROW] = pq[i].z;
+      p[32 * i + 3 * TROW] = pq[i].w;
     }
-    __syncthreads();
-#pragma unroll 1
-    for (int d = 0; d < 64; d += 16)
-      step16<2, 4, false, false>(acc, qs, C * ROW64, ROW64, t0, d, ss, COLS * ROW64, ROW64, c0, d, lane);
+  };
+  auto issue_s = [&](int d0, int buf) {
+    float* p = ss + buf * OSLICE * CROW;
+    for (int i = tid; i < OSLICE * (COLS / 4); i += 128) {
+      const int d = i / (COLS / 4), c = (i % (COLS / 4)) * 4;
+      copy16(p + d * CROW + c, S + (size_t)(d0 + d) * COLS + c, true);
+    }
+    copies_commit();
+  };
+  issue_s(0, 0);
+  fetch_q(0);
+  for (int i = tid; i < HB * C; i += 128) {
+    const float* f = g.factors + ((size_t)local * g.heads + head0 + i / C) * 4 * C + i % C;
+    as[i / C][i % C] = f[0];
+    bs[i / C][i % C] = f[C];
+    G[i / C][i % C] = f[2 * C];
   }
-  __syncthreads();  // q and the state have been read; P and the values go where they were
+  put_q(0);
+  __syncthreads();
   float p_sum = 0.f;
-  if (tid < HB * C) {  // P[s][t] = b_s a_(s+1) .. a_t (q_t . k_s)
+  if (tid < HB * C) {  // P^T[s][t] = b_s a_(s+1) .. a_t (q_t . k_s)
     const int h = tid / C, t = tid % C;
     const float* raw = g.scores + ((size_t)local * g.key_heads + kh) * C * C + t;
-    bf16* p = qs + h * P_TILE + t;
+    float* p = Pt + h * C * TROW + t;
     float e = 1.f;
 #pragma unroll 8
     for (int s = C - 1; s >= 0; --s) {
-      float w = 0.f;
-      if (s <= t) {
-        w = raw[s * C] * (e * bs[h][s]);
-        e *= as[h][s];
-      }
+      const float x = raw[s * C];
+      const float w = s <= t ? x * (e * bs[h][s]) : 0.f;
+      if (s <= t) e *= as[h][s];
+      p[s * TROW] = w;
       p_sum += w;
-      uint32_t parts[PARTS];
-      split2(w, 0.f, parts);
-#pragma unroll
-      for (int k = 0; k < PARTS; ++k) reinterpret_cast<uint16_t*>(p + k * C * ROW64)[s * ROW64] = (uint16_t)parts[k];
     }
   }
+  const int tm = (warp >> 1) * 32 + (lane >> 3) * 4, tn = (warp & 1) * 64 + (lane & 7) * 4;
+  const int my_head = (warp & 1) * 64 / VDIM;  // of the block's
+  f32x2 acc2[4][8];
 #pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    const int i = tid + 256 * n, t = i / 32, c = (i % 32) * 4;
-    put4(vs + t * ROW128 + c, C * ROW128, t < rows ? *reinterpret_cast<const float4*>(g.v + (size_t)(row0 + t) * g.row + (size_t)head0 * VDIM + c) : zero);
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc2[i][j] = 0;
+  float own_nq = 0.f;  // KIND 1, threads 0..63: q_t . n
+  const float* n_before = KIND == 1 ? g.norms + ((size_t)local * g.heads + head0) * DIM : nullptr;
+#pragma unroll 1
+  for (int d0 = 0; d0 < DIM; d0 += OSLICE) {
+    const int buf = (d0 / OSLICE) & 1;
+    const bool more = d0 + OSLICE < DIM;
+    copies_wait<0>();
+    __syncthreads();  // this slice is there, and everyone is done with the one before it
+    if (more) {
+      issue_s(d0 + OSLICE, buf ^ 1);
+      fetch_q(d0 + OSLICE);
+    }
+    const float* x = qs + buf * OSLICE * TROW;
+    const float* y = ss + buf * OSLICE * CROW;
+#pragma unroll
+    for (int d = 0; d < OSLICE; ++d) outer_step<4, 16, 32>(x + d * TROW + tm, y + d * CROW + tn, acc2);
+    if (KIND == 1 && tid < C) {
+#pragma unroll
+      for (int d = 0; d < OSLICE; ++d) own_nq = fmaf(x[d * TROW + tid], n_before[d0 + d], own_nq);
+    }
+    if (more) put_q(buf ^ 1);
   }
+  __syncthreads();  // the slices are free: the values go there
+  for (int i = tid; i < C * (COLS / 4); i += 128) {
+    const int t = i / (COLS / 4), c = (i % (COLS / 4)) * 4;
+    copy16(sm + t * CROW + c, g.v + (size_t)(row0 + min(t, rows - 1)) * g.row + (size_t)head0 * VDIM + c, t < rows);
+  }
+  copies_commit();
   // G_t times what the state gives
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < 4; ++i) {
+    const float g0 = G[my_head][tm + (i >> 1) * 16 + (i & 1) * 2], g1 = G[my_head][tm + (i >> 1) * 16 + (i & 1) * 2 + 1];
 #pragma unroll
-    for (int e = 0; e < 4; e += 2) {
-      const float x = G[my_head][t0 + 16 * i + (lane >> 2) + 4 * e];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j][e] *= x;
-        acc[i][j][e + 1] *= x;
-      }
-    }
-  if (KIND == 1) {  // n_t . q_t = G_t (n . q_t) + the sum of the row of P: a warp eight tokens
-    const float4 x = reinterpret_cast<const float4*>(g.norms + ((size_t)local * g.heads + head0) * DIM)[lane];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int t = warp * 8 + i;
-      const float4 y = t < rows ? reinterpret_cast<const float4*>(q + (size_t)t * g.row)[lane] : zero;
-      const float sum = warp_sum(fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, x.w * y.w))));
-      if (lane == 0) nq[t] = G[0][t] * sum;
-    }
+    for (int j = 0; j < 8; ++j) acc2[i][j] = fma2(acc2[i][j], pack2(g0, g1), 0ull);
   }
+  if (KIND == 1 && tid < C) nq[tid] = fmaf(G[0][tid], own_nq, p_sum);  // n_t . q_t
   const bool bad = g.flags[(size_t)local * g.heads + head0 + my_head] != 0;
+  copies_wait<0>();
   __syncthreads();
-  if (KIND == 1 && tid < C) nq[tid] += p_sum;
+  const float* p = Pt + my_head * C * TROW + tm;
+  const int reach = (warp >> 1) * 32 + 32;
+  float acc[8][8];
   if (!bad) {
-#pragma unroll 1
-    for (int s = 0; s < t0 + 32; s += 16)
-      step16<2, 4, true, true>(acc, qs + my_head * P_TILE, C * ROW64, ROW64, t0, s, vs, C * ROW128, ROW128, c0, s, lane);
-  } else {  // rarely: value by value, earlier rows left out
-    const bf16* P = qs + my_head * P_TILE;
-    const float* v = g.v + (size_t)row0 * g.row + (size_t)head0 * VDIM + c0;
+#pragma unroll 8
+    for (int s = 0; s < reach; ++s) outer_step<4, 16, 32>(p + s * TROW, sm + s * CROW + tn, acc2);
+    outer_unpack<4>(acc2, acc);
+  } else {
+    outer_unpack<4>(acc2, acc);
+    for (int s = 0; s < reach; ++s)
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 8; ++i)
+        if (s <= tm + (i & 3) + (i >> 2) * 16) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int t = t0 + 16 * i + (lane >> 2) + 8 * (e >> 1);
-        for (int s = 0; s <= min(t, rows - 1); ++s) {
-          const bf16* at = P + s * ROW64 + t;
-          const float p = __bfloat162float(at[0]) + (__bfloat162float(at[C * ROW64]) + __bfloat162float(at[2 * C * ROW64]));
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j][e] = fmaf(p, v[(size_t)s * g.row + 8 * j + 2 * (lane & 3) + (e & 1)], acc[i][j][e]);
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(p[s * TROW + (i & 3) + (i >> 2) * 16], sm[s * CROW + tn + (j & 3) + (j >> 2) * 32], acc[i][j]);
         }
-      }
   }
-  if (KIND == 1) __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < 8; ++i) {
+    const int t = tm + (i & 3) + (i >> 2) * 16;
+    if (t >= rows) continue;
+    float scale = 1.f, skip = 0.f;
+    if (KIND == 1) scale = 1.f / (fmaxf(fabsf(nq[t]), g.gates[((size_t)(row0 + t) * g.heads + head0) * 3 + 2]) + 1e-6f);
+    if (KIND == 2) skip = g.d_skip[head0 + my_head];
+    float* out = g.o + (size_t)(row0 + t) * g.heads * VDIM + (size_t)head0 * VDIM + tn;
 #pragma unroll
-    for (int e = 0; e < 4; e += 2) {
-      const int t = t0 + 16 * i + (lane >> 2) + 4 * e;
-      if (t >= rows) continue;
-      float scale = 1.f, skip = 0.f;
-      if (KIND == 1) scale = 1.f / (fmaxf(fabsf(nq[t]), g.gates[((size_t)(row0 + t) * g.heads + head0) * 3 + 2]) + 1e-6f);
-      if (KIND == 2) skip = g.d_skip[head0 + my_head];
-      const size_t at = (size_t)head0 * VDIM + c0 + 2 * (lane & 3);
-      float* out = g.o + (size_t)(row0 + t) * g.heads * VDIM + at;
-      const float* v = g.v + (size_t)(row0 + t) * g.row + at;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2 x = make_float2(acc[i][j][e], acc[i][j][e + 1]);
-        if (KIND == 1) x = make_float2(x.x * scale, x.y * scale);
-        if (KIND == 2) {
-          const float2 y = *reinterpret_cast<const float2*>(v + 8 * j);
-          x = make_float2(fmaf(skip, y.x, x.x), fmaf(skip, y.y, x.y));
-        }
-        *reinterpret_cast<float2*>(out + 8 * j) = x;
+    for (int j = 0; j < 8; j += 4) {
+      float4 x = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+      if (KIND == 1) x = make_float4(x.x * scale, x.y * scale, x.z * scale, x.w * scale);
+      if (KIND == 2) {
+        const float4 v = *reinterpret_cast<const float4*>(sm + t * CROW + tn + (j >> 2) * 32);
+        x = make_float4(fmaf(skip, v.x, x.x), fmaf(skip, v.y, x.y), fmaf(skip, v.z, x.z), fmaf(skip, v.w, x.w));
       }
+      *reinterpret_cast<float4*>(out + (j >> 2) * 32) = x;
     }
+  }
 }
 
 template <int VDIM, int KIND, int VT>
@@ -499,7 +518,7 @@ int launch_states(const ChunkArgs& g, cudaStream_t stream) {
     if (e != cudaSuccess) return fms_fail("chunk_scan: shared memory refused: %s", cudaGetErrorString(e));
     configured = true;
   }
-  fms_launch(chunk_states_kernel<VDIM, KIND, VT>, dim3(g.heads * VDIM / VT, g.n_seqs), dim3(256), STATES_SMEM<VT>, stream, g);
+  fms_launch(chunk_states_kernel<VDIM, KIND, VT>, dim3(g.heads * VDIM / VT, g.n_seqs), dim3(128), STATES_SMEM<VT>, stream, g);
   return 0;
 }
 
@@ -511,7 +530,6 @@ int launch_passes(ChunkArgs g, int n_runs, int pass_runs, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(chunk_outputs_kernel<VDIM, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUT_SMEM<VDIM>);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_scores_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCORES_SMEM);
     if (e != cudaSuccess) return fms_fail("chunk_scan: shared memory refused: %s", cudaGetErrorString(e));
     configured = true;
   }
@@ -520,9 +538,9 @@ int launch_passes(ChunkArgs g, int n_runs, int pass_runs, cudaStream_t stream) {
     g.run_lo = lo;
     g.run_hi = lo + pass_runs < n_runs ? lo + pass_runs : n_runs;
     const int n = g.run_hi - lo;
-    fms_launch(chunk_scores_kernel<KIND>, dim3(n, g.key_heads), dim3(128), SCORES_SMEM, stream, g);
+    fms_launch(chunk_scores_kernel<KIND>, dim3(n, g.key_heads), dim3(128), 0, stream, g);
     if (columns_32(g, VDIM) ? launch_states<VDIM, KIND, 32>(g, stream) : launch_states<VDIM, KIND, 64>(g, stream)) return 1;
-    fms_launch(chunk_outputs_kernel<VDIM, KIND>, dim3(n, g.heads * VDIM / COLS), dim3(256), OUT_SMEM<VDIM>, stream, g);
+    fms_launch(chunk_outputs_kernel<VDIM, KIND>, dim3(n, g.heads * VDIM / COLS), dim3(128), OUT_SMEM<VDIM>, stream, g);
     if (fms_launch_status("chunk_scan")) return 1;
   }
   return 0;
