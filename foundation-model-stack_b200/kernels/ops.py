@@ -916,12 +916,19 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
 
 
 CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
-CHUNK_SCAN_FROM = 256  # tokens of the longest sequence of a step from which a scan under one decay a head goes run by run
+# A scan under one decay a head goes run by run where the longest sequence of a step has CHUNK_SCAN_FROM tokens and, with heads
+# of 64 values, also a CHUNK_SCAN_SHARE-th of the step's: the walk takes a sequence's tokens one after the other, but a step
+# of many sequences fills the multiprocessors all the same.  Whole layers, walk / runs in us (gated with a normalizer, fixed decays,
+# state space with heads of 64): one prompt of 200 tokens 156 / 142, 127 / 136, 191 / 185; of 256 183 / 142, 141 / 137, 221 / 185;
+# of 2,048 1,623 / 635, 893 / 566, 1,457 / 863; eight of 2,048 tokens together, the longest 391, 697 / 651, 603 / 598, 858 / 859;
+# eight of 1,000 together, the longest 190, 361 / 314, 315 / 285, 455 / 486.
+CHUNK_SCAN_FROM, CHUNK_SCAN_SHARE = 256, 5
 
 
 def chunk_scan_pays(batch, heads: int, vdim: int) -> bool:
     """Whether a step's scan goes run by run (``fms_chunk_scan``) or token by token."""
-    return max(batch.num_new) >= CHUNK_SCAN_FROM
+    longest = max(batch.num_new)
+    return longest >= CHUNK_SCAN_FROM and (vdim > 64 or CHUNK_SCAN_SHARE * longest >= sum(batch.num_new))
 
 
 def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int):
