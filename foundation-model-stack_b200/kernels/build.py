@@ -2,7 +2,8 @@
 
 Each ``csrc/*.cu`` becomes a shared library of its own, compiled by ``nvcc`` directly (no torch headers:
 the kernels take raw pointers and a stream) and loaded with ``ctypes``.  The attention source is
-compiled once per head size a model needs.  A library is named after a hash of its source, the shared
+compiled once per head size a model needs.  ``launcher.cpp``, which takes tensors to those entries, is the one Python
+extension among them (the host's C++ compiler, torch's and Python's headers).  A library is named after a hash of its source, the shared
 header and the flags, so it is rebuilt exactly when one of them changes.  Libraries are kept in
 ``csrc/_build`` inside the package when that folder can be written, else in a per-user folder under the
 system's temporary directory.  What is missing is compiled at first use; meanwhile a line is printed
@@ -12,10 +13,13 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -46,6 +50,7 @@ PLAIN_LIBRARIES = {
     "grouped": ("grouped.cu", []),
     "latent_attention": ("latent_attention.cu", []),
 }
+LAUNCHER = "launcher"
 
 _TAG = "_checked" if DEBUG_BOUNDS else ""
 _loaded: Dict[str, ctypes.CDLL] = {}
@@ -96,6 +101,8 @@ def _pick_build_dir() -> str:
 
 
 def _spec(name: str) -> Tuple[str, List[str]]:
+    if name == LAUNCHER:
+        return "launcher.cpp", []
     if name in PLAIN_LIBRARIES:
         return PLAIN_LIBRARIES[name]
     if name.startswith("attention_hd"):
@@ -106,7 +113,34 @@ def _spec(name: str) -> Tuple[str, List[str]]:
     raise KernelBuildError(f"unknown kernel library {name!r}")
 
 
+def _launcher_command(out: str) -> List[str]:
+    import torch
+
+    compiler = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    if not compiler:
+        raise KernelBuildError("no C++ compiler was found (looked at CXX and PATH for g++ and c++)")
+    base = os.path.dirname(torch.__file__)
+    include = [sysconfig.get_paths()["include"], os.path.join(base, "include"),
+               os.path.join(base, "include", "torch", "csrc", "api", "include")]
+    return [compiler, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"] + [f"-I{d}" for d in include] + [
+            os.path.join(CSRC, "launcher.cpp"), "-o", out, "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
+def _launcher_digest() -> str:
+    """Of the source and of what it is compiled against."""
+    import torch
+
+    h = hashlib.sha256()
+    with open(os.path.join(CSRC, "launcher.cpp"), "rb") as f:
+        h.update(f.read())
+    h.update(" ".join((torch.__version__, sys.version, _TAG) + tuple(_launcher_command("")[1:7])).encode())
+    return h.hexdigest()[:12]
+
+
 def _digest(source: str, flags: List[str]) -> str:
+    if source == "launcher.cpp":
+        return _launcher_digest()
     h = hashlib.sha256()
     for path in [os.path.join(CSRC, source)] + sorted(
             os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))):
@@ -136,7 +170,8 @@ def compile_library(name: str, verbose: bool = True) -> str:
     source, flags = _spec(name)
     out = library_path(name)
     tmp = out + f".tmp{os.getpid()}"
-    cmd = [find_nvcc()] + ARCH_FLAGS + BASE_FLAGS + flags + ["-o", tmp, os.path.join(CSRC, source)]
+    cmd = _launcher_command(tmp) if name == LAUNCHER else \
+        [find_nvcc()] + ARCH_FLAGS + BASE_FLAGS + flags + ["-o", tmp, os.path.join(CSRC, source)]
     start = time.time()
     if verbose:
         print(f"[fms_b200] compiling {source} {' '.join(flags)} for sm_100a ...", file=sys.stderr, flush=True)
@@ -151,7 +186,7 @@ def compile_library(name: str, verbose: bool = True) -> str:
     if proc.returncode != 0:
         if os.path.exists(tmp):
             os.remove(tmp)
-        raise KernelBuildError(f"nvcc failed on {source}:\n{' '.join(cmd)}\n{output}")
+        raise KernelBuildError(f"{os.path.basename(cmd[0])} failed on {source}:\n{' '.join(cmd)}\n{output}")
     os.replace(tmp, out)
     for stale in os.listdir(os.path.dirname(out)):  # earlier builds of this library, from other sources or flags
         if (stale.startswith(f"libfms_{name}{_TAG}_") and stale.endswith(".so") and stale != os.path.basename(out)
@@ -199,6 +234,22 @@ def load_library(name: str) -> ctypes.CDLL:
         return lib
 
 
+_launcher = None
+
+
+def load_launcher():
+    """The extension that calls the libraries' entries with tensors, compiled first if need be."""
+    global _launcher
+    with _lock:
+        if _launcher is None:
+            path = find_built(LAUNCHER) or compile_library(LAUNCHER)
+            loader = importlib.machinery.ExtensionFileLoader(LAUNCHER, path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(LAUNCHER, path, loader=loader))
+            loader.exec_module(module)
+            _launcher = module
+        return _launcher
+
+
 def loaded_libraries() -> Dict[str, ctypes.CDLL]:
     with _lock:
         return dict(_loaded)
@@ -220,4 +271,4 @@ def bounds_violations() -> List[str]:
 
 
 def all_library_names(head_dims=(16, 32, 48, 64, 128, 256)) -> List[str]:
-    return list(PLAIN_LIBRARIES) + [f"attention_hd{h}" for h in head_dims]
+    return list(PLAIN_LIBRARIES) + [LAUNCHER] + [f"attention_hd{h}" for h in head_dims]

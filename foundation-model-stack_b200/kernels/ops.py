@@ -27,10 +27,11 @@ from typing import Optional
 
 import torch
 
-from .build import load_library
+from .build import load_launcher, load_library
 
 F32, BF16 = 0, 1
-_P, _I, _F, _U64, _L = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_ulonglong, ctypes.c_long
+# kinds of parameters: a pointer (a tensor's, an address or None), whole numbers of 32 and 64 bits, a float
+_P, _I, _F, _U64, _L = "p", "i", "f", "i", "i"
 
 _SIGNATURES = {
     "fms_embed_rows": [_P, _I, _P, _P, _I, _I, _I, _F, _P, _P],
@@ -128,29 +129,28 @@ def _fn(library: str, name: str):
     f = _functions.get(key)
     if f is None:
         lib = load_library(library)
-        f = getattr(lib, name)
-        f.argtypes = _SIGNATURES[name]
-        f.restype = ctypes.c_int
-        _functions[key] = f = (f, lib)
+        address = ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
+        _functions[key] = f = (load_launcher().entry(address, "".join(_SIGNATURES[name]), KernelError), lib)
     return f
 
 
 def _call(library: str, name: str, *args):
+    """A library's entry.  Tensors stand for their data's address; one that is on the CPU or not contiguous raises."""
     global launches
-    f, lib = _fn(library, name)
+    f = _functions.get((library, name)) or _fn(library, name)
     launches += 1
-    rc = f(*args)
-    if rc != 0:
-        raise KernelError(f"{name}: {lib.fms_last_error().decode(errors='replace')}")
+    if f[0](*args) != 0:
+        raise KernelError(f"{name}: {f[1].fms_last_error().decode(errors='replace')}")
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)  # without a look at whether CUDA is initialised: a tensor is there
 
 
 def _stream() -> int:
     """The current stream's handle (the direct getter where torch has it: a step makes some hundred launches)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -178,29 +178,34 @@ _error_flags = {}
 def error_flag(device) -> torch.Tensor:
     """An int32 on the device that kernels set when they meet what the host should have prevented (a token
     id outside the vocabulary, a position without a cache block).  ``check_error_flag`` reads it."""
+    flag = _error_flags.get(device)
+    return _indexed(_error_flags, device, lambda d: torch.zeros(1, dtype=torch.int32, device=d)) if flag is None else flag
+
+
+def _indexed(table: dict, device, make):
+    """``table``'s entry of a device, which may come as a name or without an index; the keys are devices with one."""
     device = torch.device(device)
-    key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
-    if key not in _error_flags:
-        _error_flags[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _error_flags[key]
+    if device.index is None:
+        device = torch.device(device.type, torch.cuda.current_device())
+    if device not in table:
+        table[device] = make(device)
+    return table[device]
 
 
 _work_counters = {}
 WORK_COUNTERS = 4096
 
 
-def _work_counter(device) -> torch.Tensor:
-    """An int32 on the device that is 0 between launches: the persistent decode-attention kernel's warps draw
-    their units from it, and the kernel that merges the splits puts it back.  Every call hands out the next of
+def _work_counter(device) -> int:
+    """The address of an int32 on the device that is 0 between launches: the persistent decode-attention kernel's warps
+    draw their units from it, and the kernel that merges the splits puts it back.  Every call hands out the next of
     4,096, so that launches in flight at the same time (other streams, the launches inside captured graphs) do
     not share one."""
-    device = torch.device(device)
-    key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
-    if key not in _work_counters:
-        _work_counters[key] = [torch.zeros(WORK_COUNTERS, dtype=torch.int32, device=device), 0]
-    entry = _work_counters[key]
-    entry[1] = (entry[1] + 1) % WORK_COUNTERS
-    return entry[0][entry[1]:entry[1] + 1]
+    entry = _work_counters.get(device)
+    if entry is None:
+        entry = _indexed(_work_counters, device, lambda d: [torch.zeros(WORK_COUNTERS, dtype=torch.int32, device=d), 0])
+    entry[1] = at = (entry[1] + 1) % WORK_COUNTERS
+    return entry[0].data_ptr() + 4 * at
 
 
 def check_error_flag(device) -> None:
@@ -228,8 +233,8 @@ def embed(table: torch.Tensor, tokens: torch.Tensor, scale: float = 1.0) -> torc
     """Float32 rows of ``table`` at ``tokens``, times ``scale``: the start of the residual stream."""
     n, dim = tokens.shape[0], table.shape[1]
     out = torch.empty((n, dim), dtype=torch.float32, device=table.device)
-    _call("elementwise", "fms_embed_rows", _ptr(table), _code(table.dtype), _ptr(tokens), _ptr(out), n, dim,
-          table.shape[0], float(scale), _ptr(error_flag(table.device)), _stream())
+    _call("elementwise", "fms_embed_rows", table, _code(table.dtype), tokens, out, n, dim,
+          table.shape[0], float(scale), error_flag(table.device), _stream())
     return out
 
 
@@ -241,9 +246,9 @@ def embed_at(table: torch.Tensor, positions_table: torch.Tensor, batch, scale: f
         raise KernelError("embed_at: the table of positions has the token table's dtype and width")
     ids = getattr(batch, "position_ids", None)
     out = torch.empty((n, dim), dtype=torch.float32, device=table.device)
-    _call("elementwise", "fms_embed_rows_at", _ptr(table), _code(table.dtype), _ptr(batch.tokens), _ptr(out), n, dim,
-          table.shape[0], float(scale), _ptr(positions_table), _ptr(batch.positions if ids is None else ids),
-          positions_table.shape[0], _ptr(error_flag(table.device)), _stream())
+    _call("elementwise", "fms_embed_rows_at", table, _code(table.dtype), batch.tokens, out, n, dim,
+          table.shape[0], float(scale), positions_table, batch.positions if ids is None else ids,
+          positions_table.shape[0], error_flag(table.device), _stream())
     return out
 
 
@@ -257,10 +262,10 @@ def embed_pair_hash(table: torch.Tensor, pairs: torch.Tensor, batch, last_token:
         raise KernelError("embed_pair_hash: the pair table has the token table's dtype and buckets + 1 rows of its width; "
                           "the state is int32")
     out = torch.empty((n, dim), dtype=torch.float32, device=table.device)
-    _call("elementwise", "fms_embed_pair_hash", _ptr(table), _ptr(pairs), _code(table.dtype), _ptr(batch.tokens),
-          _ptr(batch.positions), _ptr(batch.token_seq), _ptr(batch.first_row), _ptr(batch.slots), _ptr(last_token),
-          _ptr(out), n, dim, table.shape[0], int(buckets), int(mul_prev), int(mul_cur), float(scale), 1,
-          batch.slots.shape[0], last_token.shape[0], _ptr(error_flag(table.device)), _stream())
+    _call("elementwise", "fms_embed_pair_hash", table, pairs, _code(table.dtype), batch.tokens,
+          batch.positions, batch.token_seq, batch.first_row, batch.slots, last_token,
+          out, n, dim, table.shape[0], int(buckets), int(mul_prev), int(mul_cur), float(scale), 1,
+          batch.slots.shape[0], last_token.shape[0], error_flag(table.device), _stream())
     return out
 
 
@@ -282,9 +287,9 @@ def normed_add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], po
     if len({v.dtype for v in vecs}) > 1:
         raise KernelError("normed_add_rmsnorm: the two gain vectors differ in dtype")
     out = torch.empty((n, dim), dtype=out_dtype, device=residual.device)
-    _call("elementwise", "fms_normed_add_rmsnorm", _ptr(residual), _ptr(delta), 0 if post is None else 1, _ptr(post_vec),
-          float(post_num), float(post_eps), _ptr(gain_vec), float(gain_num), float(eps),
-          _code(vecs[0].dtype) if vecs else F32, _ptr(out), _code(out_dtype), _ptr(rows), n, dim, residual.shape[0],
+    _call("elementwise", "fms_normed_add_rmsnorm", residual, delta, 0 if post is None else 1, post_vec,
+          float(post_num), float(post_eps), gain_vec, float(gain_num), float(eps),
+          _code(vecs[0].dtype) if vecs else F32, out, _code(out_dtype), rows, n, dim, residual.shape[0],
           _stream())
     return out
 
@@ -319,8 +324,8 @@ def normed_add_norm(residual: torch.Tensor, delta, post, out_norm, out_dtype: to
         if g is not None and (g.dtype != torch.float32 or g.shape[0] != dim):
             raise KernelError("normed_add_norm: gains are float32 vectors of the row's width")
     out = torch.empty((n, dim), dtype=out_dtype, device=residual.device) if want_out else None
-    _call("elementwise", "fms_normed_add_norm", _ptr(residual), *flat, int(post_mode), _ptr(post_gain), float(post_eps),
-          int(out_mode), _ptr(gain), _ptr(bias), float(eps), _ptr(out), _code(out_dtype), _ptr(rows), n, dim, residual.shape[0], _stream())
+    _call("elementwise", "fms_normed_add_norm", residual, *flat, int(post_mode), post_gain, float(post_eps),
+          int(out_mode), gain, bias, float(eps), out, _code(out_dtype), rows, n, dim, residual.shape[0], _stream())
     return out
 
 
@@ -335,8 +340,8 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], gain: tor
     if delta is not None and delta.dtype != out_dtype:
         raise KernelError(f"sublayer output is {delta.dtype}, compute dtype is {out_dtype}")
     out = torch.empty((n, dim), dtype=out_dtype, device=residual.device)
-    _call("elementwise", "fms_add_rmsnorm", _ptr(residual), _ptr(delta), _ptr(gain), _code(gain.dtype), float(eps),
-          _ptr(out), _code(out_dtype), _ptr(rows), n, dim, residual.shape[0], _stream())
+    _call("elementwise", "fms_add_rmsnorm", residual, delta, gain, _code(gain.dtype), float(eps),
+          out, _code(out_dtype), rows, n, dim, residual.shape[0], _stream())
     return out
 
 
@@ -352,8 +357,8 @@ def scaled_add_rmsnorm(residual: torch.Tensor, alpha: float, parts, gain: torch.
         raise KernelError("scaled_add_rmsnorm: one or two sublayer outputs of the stream's shape, in the compute dtype")
     (da, sa), (db, sb) = parts[0], (parts[1] if len(parts) > 1 else (None, 0.0))
     copy = None if out_dtype == torch.float32 else torch.empty((n, dim), dtype=out_dtype, device=residual.device)
-    _call("elementwise", "fms_scaled_add_rmsnorm", _ptr(residual), float(alpha), _ptr(da), float(sa), _ptr(db), float(sb),
-          _ptr(gain), _code(gain.dtype), float(eps), _ptr(copy), _code(out_dtype), n, dim, _stream())
+    _call("elementwise", "fms_scaled_add_rmsnorm", residual, float(alpha), da, float(sa), db, float(sb),
+          gain, _code(gain.dtype), float(eps), copy, _code(out_dtype), n, dim, _stream())
     return copy
 
 
@@ -377,9 +382,9 @@ def parts_group_rmsnorm(residual: torch.Tensor, parts, gains, eps: float, groups
     flat = []
     for i in range(4):
         flat += [_ptr(parts[i][0]), parts[i][1]] if i < len(parts) else [None, 0.0]
-    _call("elementwise", "fms_parts_group_rmsnorm", _ptr(residual), *flat, _ptr(gains[0]),
-          _ptr(gains[1]) if len(gains) > 1 else None, float(eps), int(groups), _ptr(outs[0]),
-          _ptr(outs[1]) if len(outs) > 1 else None, _code(out_dtype), _ptr(rows), n, dim, residual.shape[0], _stream())
+    _call("elementwise", "fms_parts_group_rmsnorm", residual, *flat, gains[0],
+          gains[1] if len(gains) > 1 else None, float(eps), int(groups), outs[0],
+          outs[1] if len(outs) > 1 else None, _code(out_dtype), rows, n, dim, residual.shape[0], _stream())
     return outs
 
 
@@ -406,8 +411,8 @@ def stream_mix_norm(streams, delta: Optional[torch.Tensor], on: Optional[torch.T
             streams.rows = torch.empty((n_all, n_streams, dim), dtype=torch.float32, device=start.device)
         dst = streams.rows
     out = torch.empty((n, dim), dtype=out_dtype, device=start.device)
-    _call("elementwise", "fms_stream_mix_norm", _ptr(src), src_streams, _ptr(dst), _ptr(delta), _ptr(on), _ptr(w_in), _ptr(gain),
-          float(eps), _ptr(out), _code(out_dtype), _ptr(rows), n, dim, n_streams, n_all, _stream())
+    _call("elementwise", "fms_stream_mix_norm", src, src_streams, dst, delta, on, w_in, gain,
+          float(eps), out, _code(out_dtype), rows, n, dim, n_streams, n_all, _stream())
     return out
 
 
@@ -416,7 +421,7 @@ def cast_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     if dtype == torch.float32:
         return x
     out = torch.empty(x.shape, dtype=dtype, device=x.device)
-    _call("elementwise", "fms_cast_rows", _ptr(x), _ptr(out), _code(dtype), x.numel(), _stream())
+    _call("elementwise", "fms_cast_rows", x, out, _code(dtype), x.numel(), _stream())
     return out
 
 
@@ -431,7 +436,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         x32 = x if x.dtype == torch.float32 else x.float()
         b32 = None if bias is None else (bias if bias.dtype == torch.float32 else bias.float())
         y = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
-        _call("gemm_f32", "fms_gemm_f32", _ptr(x32), _ptr(weight), _ptr(b32), _ptr(y), x.shape[0], weight.shape[0],
+        _call("gemm_f32", "fms_gemm_f32", x32, weight, b32, y, x.shape[0], weight.shape[0],
               weight.shape[1], _stream())
         return y if out_dtype == torch.float32 else y.to(out_dtype)
     if weight.dtype != torch.bfloat16 or x.dtype != torch.bfloat16:
@@ -439,13 +444,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if x.shape[0] <= SKINNY_ROWS and weight.shape[1] % 8 == 0 and (bias is None or bias.dtype == torch.bfloat16):
         # few rows (decode): the weight-streaming tensor-core kernel
         y = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
-        _call("gemm_bf16_skinny", "fms_linear_bf16_skinny", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), _code(out_dtype),
+        _call("gemm_bf16_skinny", "fms_linear_bf16_skinny", x, weight, bias, y, _code(out_dtype),
               x.shape[0], weight.shape[0], weight.shape[1], _stream())
         return y
     if _mid_fits(x, weight, bias):
         y = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
-        _call("gemm_bf16_mid", "fms_linear_bf16_mid", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), _code(out_dtype),
-              x.shape[0], weight.shape[0], weight.shape[1], _ptr(error_flag(x.device)), _stream())
+        _call("gemm_bf16_mid", "fms_linear_bf16_mid", x, weight, bias, y, _code(out_dtype),
+              x.shape[0], weight.shape[0], weight.shape[1], error_flag(x.device), _stream())
         return y
     if _tensor_core_fits(x, weight, bias):
         return linear_tensor_core(x, weight, bias, out_dtype)
@@ -461,11 +466,11 @@ def capped_logits(x: torch.Tensor, weight: torch.Tensor, scale: float, cap: floa
     product's epilogue, else a pass over the product's results."""
     if x.dtype == weight.dtype == torch.bfloat16 and x.shape[0] <= SKINNY_ROWS and weight.shape[1] % 8 == 0:
         y = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
-        _call("gemm_bf16_skinny", "fms_linear_cap_bf16_skinny", _ptr(x), _ptr(weight), _ptr(y), x.shape[0], weight.shape[0],
+        _call("gemm_bf16_skinny", "fms_linear_cap_bf16_skinny", x, weight, y, x.shape[0], weight.shape[0],
               weight.shape[1], float(scale), float(cap), _stream())
         return y
     y = linear(x, weight, None, torch.float32)
-    _call("elementwise", "fms_scale_cap", _ptr(y), float(scale), float(cap), y.numel(), _stream())
+    _call("elementwise", "fms_scale_cap", y, float(scale), float(cap), y.numel(), _stream())
     return y
 
 
@@ -521,8 +526,8 @@ def linear_tensor_core(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
     float32 out.  K must be a multiple of 8."""
     out_dtype = out_dtype or x.dtype
     y = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
-    _call("gemm_bf16_tc", "fms_gemm_bf16_tc", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), _code(out_dtype), x.shape[0],
-          weight.shape[0], weight.shape[1], _ptr(error_flag(x.device)), _stream())
+    _call("gemm_bf16_tc", "fms_gemm_bf16_tc", x, weight, bias, y, _code(out_dtype), x.shape[0],
+          weight.shape[0], weight.shape[1], error_flag(x.device), _stream())
     return y
 
 
@@ -531,8 +536,8 @@ def gated_linear_tensor_core(x: torch.Tensor, weight: torch.Tensor, bias: Option
     """act(x Wg^T) * (x Wu^T) in one tcgen05 kernel: gate and up rows share a tile, the epilogue multiplies."""
     hidden = weight.shape[0] // 2
     y = torch.empty((x.shape[0], hidden), dtype=torch.bfloat16, device=x.device)
-    _call("gemm_bf16_tc", "fms_glu_bf16_tc", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), x.shape[0], hidden,
-          weight.shape[1], int(activation), _ptr(error_flag(x.device)), _stream())
+    _call("gemm_bf16_tc", "fms_glu_bf16_tc", x, weight, bias, y, x.shape[0], hidden,
+          weight.shape[1], int(activation), error_flag(x.device), _stream())
     return y
 
 
@@ -548,14 +553,14 @@ def gated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
             and weight.shape[1] % 8 == 0 and (bias is None or bias.dtype == torch.bfloat16)):
         _ptr(x), _ptr(weight)
         y = torch.empty((x.shape[0], hidden), dtype=torch.bfloat16, device=x.device)
-        _call("gemm_bf16_skinny", "fms_glu_bf16_skinny", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), x.shape[0], hidden,
+        _call("gemm_bf16_skinny", "fms_glu_bf16_skinny", x, weight, bias, y, x.shape[0], hidden,
               weight.shape[1], int(activation), _stream())
         return y
     if _mid_fits(x, weight, bias, "glu"):
         _ptr(x), _ptr(weight)
         y = torch.empty((x.shape[0], hidden), dtype=torch.bfloat16, device=x.device)
-        _call("gemm_bf16_mid", "fms_glu_bf16_mid", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), x.shape[0], hidden,
-              weight.shape[1], int(activation), _ptr(error_flag(x.device)), _stream())
+        _call("gemm_bf16_mid", "fms_glu_bf16_mid", x, weight, bias, y, x.shape[0], hidden,
+              weight.shape[1], int(activation), error_flag(x.device), _stream())
         return y
     # the own kernel works on tiles of 256 rows: where the last one would be mostly padding, the library is ahead
     if (_tensor_core_fits(x, weight, bias, TENSOR_CORE_ROWS_GLU)
@@ -571,18 +576,18 @@ def activated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch
     own = x.dtype == weight.dtype == torch.bfloat16 and weight.shape[1] % 8 == 0 and (bias is None or bias.dtype == torch.bfloat16) \
         and activation <= 3
     if own and x.shape[0] <= SKINNY_ROWS:
-        y = torch.empty((x.shape[0], weight.shape[0]), dtype=x.dtype, device=x.device)
-        _call("gemm_bf16_skinny", "fms_linear_act_bf16_skinny", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), x.shape[0],
+        y = x.new_empty((x.shape[0], weight.shape[0]))
+        _call("gemm_bf16_skinny", "fms_linear_act_bf16_skinny", x, weight, bias, y, x.shape[0],
               weight.shape[0], weight.shape[1], int(activation), _stream())
         return y
     if (own and _tensor_core_fits(x, weight, bias, TENSOR_CORE_ROWS_GLU)
             and (x.shape[0] + 255) // 256 * 256 <= TENSOR_CORE_MAX_PADDING * x.shape[0]):
-        y = torch.empty((x.shape[0], weight.shape[0]), dtype=x.dtype, device=x.device)
-        _call("gemm_bf16_tc", "fms_linear_act_bf16_tc", _ptr(x), _ptr(weight), _ptr(bias), _ptr(y), x.shape[0], weight.shape[0],
-              weight.shape[1], int(activation), _ptr(error_flag(x.device)), _stream())
+        y = x.new_empty((x.shape[0], weight.shape[0]))
+        _call("gemm_bf16_tc", "fms_linear_act_bf16_tc", x, weight, bias, y, x.shape[0], weight.shape[0],
+              weight.shape[1], int(activation), error_flag(x.device), _stream())
         return y
     y = linear(x, weight, bias)
-    _call("elementwise", "fms_activation", _ptr(y), _code(y.dtype), int(activation), y.numel(), _stream())
+    _call("elementwise", "fms_activation", y, _code(y.dtype), int(activation), y.numel(), _stream())
     return y
 
 
@@ -590,8 +595,8 @@ def gated_activation(gate_up: torch.Tensor, activation: int) -> torch.Tensor:
     """act(gate) * up for rows [gate | up]."""
     n, two_f = gate_up.shape
     hidden = two_f // 2
-    out = torch.empty((n, hidden), dtype=gate_up.dtype, device=gate_up.device)
-    _call("elementwise", "fms_gated_activation", _ptr(gate_up), _ptr(out), _code(gate_up.dtype), n, hidden,
+    out = gate_up.new_empty((n, hidden))
+    _call("elementwise", "fms_gated_activation", gate_up, out, _code(gate_up.dtype), n, hidden,
           int(activation), _stream())
     return out
 
@@ -601,8 +606,8 @@ def token_gated_linear(x: torch.Tensor, weight: torch.Tensor, table: torch.Tenso
     """act(x weight^T) * table[tokens]: one kernel for a few bfloat16 rows, else the product and ``token_gate``."""
     if (x.dtype == weight.dtype == table.dtype == torch.bfloat16 and x.shape[0] <= SKINNY_ROWS and weight.shape[1] % 8 == 0
             and activation <= 3 and table.shape[1] == weight.shape[0]):
-        y = torch.empty((x.shape[0], weight.shape[0]), dtype=x.dtype, device=x.device)
-        _call("gemm_bf16_skinny", "fms_token_gate_bf16_skinny", _ptr(x), _ptr(weight), _ptr(table), _ptr(tokens), _ptr(y),
+        y = x.new_empty((x.shape[0], weight.shape[0]))
+        _call("gemm_bf16_skinny", "fms_token_gate_bf16_skinny", x, weight, table, tokens, y,
               x.shape[0], weight.shape[0], weight.shape[1], table.shape[0], int(activation), _stream())
         return y
     return token_gate(linear(x, weight), table, tokens, activation)
@@ -614,7 +619,7 @@ def token_gate(z: torch.Tensor, table: torch.Tensor, tokens: torch.Tensor, activ
     if table.dtype != z.dtype or table.shape[1] != dim:
         raise KernelError(f"token_gate: z {z.dtype} {tuple(z.shape)}, table {table.dtype} {tuple(table.shape)}")
     out = torch.empty_like(z)
-    _call("elementwise", "fms_token_gate", _ptr(z), _code(z.dtype), _ptr(table), _ptr(tokens), _ptr(out), n, dim, table.shape[0],
+    _call("elementwise", "fms_token_gate", z, _code(z.dtype), table, tokens, out, n, dim, table.shape[0],
           int(activation), _stream())
     return out
 
@@ -628,8 +633,8 @@ def joint_activation(o: torch.Tensor, proj: torch.Tensor, gate_col: int, ff_col:
     if proj.dtype != o.dtype or proj.shape[0] != n or o.shape[1] != nheads * pad \
             or proj.shape[1] < max(gate_col + nheads * vdim, ff_col + hidden * (2 if gated else 1) if hidden else 0):
         raise KernelError(f"joint_activation: o {o.dtype} {tuple(o.shape)}, proj {proj.dtype} {tuple(proj.shape)}")
-    out = torch.empty((n, nheads * vdim + hidden), dtype=o.dtype, device=o.device)
-    _call("elementwise", "fms_joint_activation", _ptr(o), _ptr(proj), proj.shape[1], int(gate_col), int(ff_col), _ptr(out),
+    out = o.new_empty((n, nheads * vdim + hidden))
+    _call("elementwise", "fms_joint_activation", o, proj, proj.shape[1], int(gate_col), int(ff_col), out,
           _code(o.dtype), n, nheads, vdim, pad, hidden, int(activation), 1 if gated else 0, _stream())
     return out
 
@@ -644,12 +649,12 @@ def rope_store(qkv: torch.Tensor, inv_freq: Optional[torch.Tensor], batch, view,
     n = qkv.shape[0]
     if view.keys.dtype != qkv.dtype:
         raise KernelError(f"cache is {view.keys.dtype}, activations are {qkv.dtype}")
-    q = torch.empty((n, nheads * head_dim), dtype=qkv.dtype, device=qkv.device)
-    _call("elementwise", "fms_rope_store", _ptr(qkv), _code(qkv.dtype), _ptr(q), _ptr(inv_freq), _ptr(batch.positions),
-          _ptr(getattr(batch, "position_ids", None)), _ptr(batch.token_seq), _ptr(batch.slots), _ptr(view.keys),
-          _ptr(view.values), _ptr(view.table),
+    q = qkv.new_empty((n, nheads * head_dim))
+    _call("elementwise", "fms_rope_store", qkv, _code(qkv.dtype), q, inv_freq, batch.positions,
+          getattr(batch, "position_ids", None), batch.token_seq, batch.slots, view.keys,
+          view.values, view.table,
           view.table.shape[1], view.block_tokens, n, nheads, kvheads, head_dim, 1 if writes_cache else 0,
-          _ptr(error_flag(qkv.device)), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _stream())
+          error_flag(qkv.device), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _stream())
     return q
 
 
@@ -666,8 +671,8 @@ def rotary_table(inv_freq: torch.Tensor, batch) -> torch.Tensor:
         return scratch[key]
     n, half = batch.positions.shape[0], inv_freq.shape[0]
     out = torch.empty((n, half, 2), dtype=torch.float32, device=inv_freq.device)
-    _call("elementwise", "fms_rotary_table", _ptr(inv_freq), _ptr(batch.positions), _ptr(getattr(batch, "position_ids", None)),
-          _ptr(out), n, half, _stream())
+    _call("elementwise", "fms_rotary_table", inv_freq, batch.positions, getattr(batch, "position_ids", None),
+          out, n, half, _stream())
     if scratch is not None:
         scratch[key] = out
     return out
@@ -683,22 +688,22 @@ def qkv_rope_store(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
             and weight.shape[1] % 8 == 0 and head_dim % 2 == 0 and (bias is None or bias.dtype == torch.bfloat16)
             and view.keys.dtype == torch.bfloat16 and weight.shape[0] == (nheads + 2 * kvheads) * head_dim):
         n = x.shape[0]
-        q = torch.empty((n, nheads * head_dim), dtype=x.dtype, device=x.device)
-        _call("gemm_bf16_skinny", "fms_qkv_rope_store_bf16_skinny", _ptr(x), _ptr(weight), _ptr(bias), _ptr(q),
-              _ptr(inv_freq), _ptr(batch.positions), _ptr(getattr(batch, "position_ids", None)), _ptr(batch.token_seq),
-              _ptr(batch.slots), _ptr(view.keys), _ptr(view.values), _ptr(view.table), view.table.shape[1],
+        q = x.new_empty((n, nheads * head_dim))
+        _call("gemm_bf16_skinny", "fms_qkv_rope_store_bf16_skinny", x, weight, bias, q,
+              inv_freq, batch.positions, getattr(batch, "position_ids", None), batch.token_seq,
+              batch.slots, view.keys, view.values, view.table, view.table.shape[1],
               view.block_tokens, n, weight.shape[1], nheads,
-              kvheads, head_dim, 1 if writes_cache else 0, _ptr(error_flag(x.device)), batch.slots.shape[0],
+              kvheads, head_dim, 1 if writes_cache else 0, error_flag(x.device), batch.slots.shape[0],
               view.table.shape[0], view.keys.shape[0], _stream())
         return q
     if (FUSE_QKV_ROPE and _mid_fits(x, weight, bias, "qkv") and head_dim % 2 == 0 and view.keys.dtype == torch.bfloat16
             and weight.shape[0] == (nheads + 2 * kvheads) * head_dim):
         n = x.shape[0]
-        q = torch.empty((n, nheads * head_dim), dtype=x.dtype, device=x.device)
-        _call("gemm_bf16_mid", "fms_qkv_rope_store_bf16_mid", _ptr(x), _ptr(weight), _ptr(bias), _ptr(q), _ptr(inv_freq),
-              _ptr(batch.positions), _ptr(getattr(batch, "position_ids", None)), _ptr(batch.token_seq), _ptr(batch.slots),
-              _ptr(view.keys), _ptr(view.values), _ptr(view.table), view.table.shape[1], view.block_tokens, n,
-              weight.shape[1], nheads, kvheads, head_dim, 1 if writes_cache else 0, _ptr(error_flag(x.device)),
+        q = x.new_empty((n, nheads * head_dim))
+        _call("gemm_bf16_mid", "fms_qkv_rope_store_bf16_mid", x, weight, bias, q, inv_freq,
+              batch.positions, getattr(batch, "position_ids", None), batch.token_seq, batch.slots,
+              view.keys, view.values, view.table, view.table.shape[1], view.block_tokens, n,
+              weight.shape[1], nheads, kvheads, head_dim, 1 if writes_cache else 0, error_flag(x.device),
               batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _stream())
         return q
     if (FUSE_QKV_ROPE and _tensor_core_fits(x, weight, bias, TENSOR_CORE_ROWS_QKV) and head_dim % 16 == 0
@@ -707,12 +712,12 @@ def qkv_rope_store(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
         # many tokens: the tcgen05 product with the rotation and the cache write in its epilogue; the angles' sines and
         # cosines come from a table that the step's first such layer makes for all layers with the same frequencies
         n = x.shape[0]
-        q = torch.empty((n, nheads * head_dim), dtype=x.dtype, device=x.device)
+        q = x.new_empty((n, nheads * head_dim))
         table = None if inv_freq is None else rotary_table(inv_freq, batch)
-        _call("gemm_bf16_tc", "fms_qkv_rope_store_bf16_tc", _ptr(x), _ptr(weight), _ptr(bias), _ptr(q), _ptr(table),
-              _ptr(batch.positions), _ptr(batch.token_seq), _ptr(batch.slots),
-              _ptr(view.keys), _ptr(view.values), _ptr(view.table), view.table.shape[1], view.block_tokens, n,
-              weight.shape[1], nheads, kvheads, head_dim, 1 if writes_cache else 0, _ptr(error_flag(x.device)),
+        _call("gemm_bf16_tc", "fms_qkv_rope_store_bf16_tc", x, weight, bias, q, table,
+              batch.positions, batch.token_seq, batch.slots,
+              view.keys, view.values, view.table, view.table.shape[1], view.block_tokens, n,
+              weight.shape[1], nheads, kvheads, head_dim, 1 if writes_cache else 0, error_flag(x.device),
               batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _stream())
         return q
     return rope_store(linear(x, weight, bias), inv_freq, batch, view, nheads, kvheads, head_dim, writes_cache)
@@ -768,17 +773,17 @@ def qk_prepare_store(proj: torch.Tensor, inv_freq: Optional[torch.Tensor], rot: 
     if view.keys.dtype != proj.dtype or view.keys.shape[-1] != pad:
         raise KernelError(f"cache is {view.keys.dtype} with heads of {view.keys.shape[-1]}, activations are {proj.dtype}, "
                           f"heads of {pad}")
-    q = None if q_in_place else torch.empty((n, nheads * pad), dtype=proj.dtype, device=proj.device)
+    q = None if q_in_place else proj.new_empty((n, nheads * pad))
     # many tokens: the angles' sines and cosines come from a table that all layers with the same frequencies share
     table = rotary_table(inv_freq, batch) if rot and n >= ROTARY_TABLE_ROWS and getattr(batch, "scratch", None) is not None else None
-    _call("elementwise", "fms_qk_prepare_store", _ptr(proj), _code(proj.dtype), proj.shape[1], _ptr(q), _ptr(inv_freq),
-          int(rot), float(rot_mult), 1 if qk_norm else 0, float(eps), _ptr(q_gain), _ptr(k_gain), 1 if norm_first else 0,
+    _call("elementwise", "fms_qk_prepare_store", proj, _code(proj.dtype), proj.shape[1], q, inv_freq,
+          int(rot), float(rot_mult), 1 if qk_norm else 0, float(eps), q_gain, k_gain, 1 if norm_first else 0,
           1 if halves else 0,
-          1 if values_are_keys else 0, _ptr(batch.positions), _ptr(getattr(batch, "position_ids", None)),
-          _ptr(batch.token_seq), _ptr(batch.slots), _ptr(view.keys), _ptr(view.values), _ptr(view.table),
+          1 if values_are_keys else 0, batch.positions, getattr(batch, "position_ids", None),
+          batch.token_seq, batch.slots, view.keys, view.values, view.table,
           view.table.shape[1], view.block_tokens, n, nheads, kvheads, dim, vdim, pad, 1 if writes_cache else 0,
-          _ptr(error_flag(proj.device)), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], first_ptr,
-          first_stride or 0, float(v_mix), _ptr(table), _stream())
+          error_flag(proj.device), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], first_ptr,
+          first_stride or 0, float(v_mix), table, _stream())
     return q
 
 
@@ -788,9 +793,9 @@ def sigmoid_gate(o: torch.Tensor, gate: Optional[torch.Tensor], gate_offset: int
     of ``pad`` values; ``gate`` is a matrix whose columns from ``gate_offset`` on hold the gates' logits (None: no
     gate, only the padding is dropped).  ``per_head``: one gate a head, sigmoid(gate[t, gate_offset + h])."""
     n = o.shape[0]
-    out = torch.empty((n, nheads * vdim), dtype=o.dtype, device=o.device)
+    out = o.new_empty((n, nheads * vdim))
     gate_ptr = None if gate is None else _ptr(gate) + gate_offset * gate.element_size()
-    _call("elementwise", "fms_sigmoid_gate", _ptr(o), gate_ptr, 0 if gate is None else gate.shape[1], _ptr(out),
+    _call("elementwise", "fms_sigmoid_gate", o, gate_ptr, 0 if gate is None else gate.shape[1], out,
           _code(o.dtype), n, nheads, vdim, pad, float(factor), 1 if per_head else 0, _stream())
     return out
 
@@ -814,35 +819,37 @@ def attention(q: torch.Tensor, batch, view, nheads: int, kvheads: int, head_dim:
         raise KernelError(f"attention: chunk {chunk}, window {window}, softcap {softcap}")
     if sink is not None and (sink.dtype != torch.float32 or sink.shape[0] != nheads):
         raise KernelError("attention: the sinks are float32, one per head")
-    out = torch.empty((q.shape[0], nheads * head_dim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((q.shape[0], nheads * head_dim))
     lib = _attention_library(head_dim)
     split, tile_rows = attention_constants(head_dim, q.dtype, nheads, kvheads)
-    common = (_ptr(q), _ptr(out), _code(q.dtype), _ptr(view.keys), _ptr(view.values), _ptr(view.table),
-              view.table.shape[1], view.block_tokens, _ptr(batch.slots), _ptr(batch.first_row), _ptr(batch.len_after))
+    common = (q, out, _code(q.dtype), view.keys, view.values, view.table,
+              view.table.shape[1], view.block_tokens, batch.slots, batch.first_row, batch.len_after)
     if batch.decode:
         n_splits = (batch.max_len_after + split - 1) // split
-        part_o = torch.empty((batch.n_seqs, nheads, n_splits, head_dim), dtype=torch.float32, device=q.device)
-        part_ml = torch.empty((batch.n_seqs, nheads, n_splits, 2), dtype=torch.float32, device=q.device)
+        # a split's results [head_dim] of all, then their maxima and sums [2]
+        parts = torch.empty((batch.n_seqs * nheads * n_splits * (head_dim + 2),), dtype=torch.float32, device=q.device)
+        part_o = parts.data_ptr()
+        part_ml = part_o + batch.n_seqs * nheads * n_splits * head_dim * 4
         # total_len (what the host knows of the sequences' lengths) chooses between the two bfloat16 decode kernels
-        tail = (_ptr(sink), int(chunk), float(softcap), _ptr(distance), q.shape[1]) if masked else \
-            (() if sink is None else (_ptr(sink),))
+        tail = (sink, int(chunk), float(softcap), distance, q.shape[1]) if masked else \
+            (() if sink is None else (sink,))
         _call(lib, "fms_attention_decode_masked" if masked else
               ("fms_attention_decode" if sink is None else "fms_attention_decode_sink"), *common, batch.n_seqs,
-              n_splits, _ptr(part_o), _ptr(part_ml), nheads,
+              n_splits, part_o, part_ml, nheads,
               kvheads, head_dim, float(scale), int(window), view.keys.shape[0], view.table.shape[0],
               int(getattr(batch, "total_len", 0)),
-              _ptr(_work_counter(q.device)), _ptr(error_flag(q.device)), *tail, _stream())
+              _work_counter(q.device), error_flag(q.device), *tail, _stream())
         if n_splits > 1 or q.dtype == torch.float32:
             global launches
             launches += 1  # the kernel that merges the splits
     else:
         tiles = batch.query_tiles(tile_rows)
-        tail = (_ptr(sink), int(chunk), float(softcap), _ptr(distance), q.shape[1]) if masked else \
-            (() if sink is None else (_ptr(sink),))
+        tail = (sink, int(chunk), float(softcap), distance, q.shape[1]) if masked else \
+            (() if sink is None else (sink,))
         _call(lib, "fms_attention_prefill_masked" if masked else
-              ("fms_attention_prefill" if sink is None else "fms_attention_prefill_sink"), *common, _ptr(tiles),
+              ("fms_attention_prefill" if sink is None else "fms_attention_prefill_sink"), *common, tiles,
               tiles.shape[0], nheads, kvheads, head_dim, float(scale), int(window), view.keys.shape[0],
-              view.table.shape[0], _ptr(error_flag(q.device)), *tail, _stream())
+              view.table.shape[0], error_flag(q.device), *tail, _stream())
     return out
 
 
@@ -860,8 +867,8 @@ def decode_advance(positions: torch.Tensor, lengths: torch.Tensor, offsets: Opti
     ``offsets`` (sequences that did not start at position 0) also position_ids[i] = positions[i] + offsets[i].
     With ``slots``: a row in ``spare_slot`` (one that only fills the step up to a captured size) restarts at
     position 0 every step."""
-    _call("elementwise", "fms_decode_advance", _ptr(positions), _ptr(lengths), _ptr(offsets), _ptr(position_ids),
-          _ptr(slots), int(spare_slot), positions.shape[0], _stream())
+    _call("elementwise", "fms_decode_advance", positions, lengths, offsets, position_ids,
+          slots, int(spare_slot), positions.shape[0], _stream())
 
 
 # ---- recurrence --------------------------------------------------------------------------------------
@@ -877,7 +884,7 @@ def mingru_scan(proj: torch.Tensor, state: torch.Tensor, batch, width: int, writ
     n = proj.shape[0]
     if proj.shape[1] != 3 * width or state.dtype != torch.float32 or state.shape[1] != width:
         raise KernelError("mingru_scan: proj is [tokens, 3 width], the state float32 [slots, width]")
-    y = torch.empty((n, width), dtype=proj.dtype, device=proj.device)
+    y = proj.new_empty((n, width))
     chunk_rows = first_chunk = ab = None
     n_chunks = 0
     if batch.max_new >= SCAN_CHUNKS_FROM:
@@ -886,9 +893,9 @@ def mingru_scan(proj: torch.Tensor, state: torch.Tensor, batch, width: int, writ
         chunk_rows, first_chunk = batch.row_chunks(_recurrent_chunk)
         n_chunks = chunk_rows.shape[0]
         ab = torch.empty((n_chunks, 2, width), dtype=torch.float32, device=proj.device)
-    _call("recurrent", "fms_mingru_scan", _ptr(proj), _code(proj.dtype), _ptr(state), _ptr(y), _ptr(batch.first_row),
-          _ptr(batch.slots), batch.n_seqs, width, state.shape[0], 1 if writes_state else 0, _ptr(chunk_rows),
-          _ptr(first_chunk), n_chunks, _ptr(ab), _stream())
+    _call("recurrent", "fms_mingru_scan", proj, _code(proj.dtype), state, y, batch.first_row,
+          batch.slots, batch.n_seqs, width, state.shape[0], 1 if writes_state else 0, chunk_rows,
+          first_chunk, n_chunks, ab, _stream())
     global launches
     launches += 2 if n_chunks else 0
     return y
@@ -907,8 +914,8 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
             or tuple(tail.shape[1:]) != (taps - 1, channels) or (bias is not None and bias.dtype != torch.float32):
         raise KernelError("causal_conv: weight [channels, taps], bias and tail [slots, taps - 1, channels] are float32")
     out = torch.empty((n, channels), dtype=torch.float32, device=x.device)
-    _call("state_scan", "fms_causal_conv", _ptr(x) + offset * x.element_size(), _code(x.dtype), x.shape[1], _ptr(weight),
-          _ptr(bias), _ptr(tail), _ptr(batch.token_seq), _ptr(batch.first_row), _ptr(batch.slots), _ptr(out), n,
+    _call("state_scan", "fms_causal_conv", _ptr(x) + offset * x.element_size(), _code(x.dtype), x.shape[1], weight,
+          bias, tail, batch.token_seq, batch.first_row, batch.slots, out, n,
           batch.n_seqs, channels, taps, 1 if activation else 0, 1 if writes_state else 0, tail.shape[0], _stream())
     global launches
     launches += 1 if writes_state and taps > 1 else 0
@@ -919,9 +926,9 @@ CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read ba
 # A scan under one decay a head goes run by run where the longest sequence of a step has CHUNK_SCAN_FROM tokens and, with heads
 # of 64 values, also a CHUNK_SCAN_SHARE-th of the step's: the walk takes a sequence's tokens one after the other, but a step
 # of many sequences fills the multiprocessors all the same.  Whole layers, walk / runs in us (gated with a normalizer, fixed decays,
-# state space with heads of 64): one prompt of 200 tokens 156 / 142, 127 / 136, 191 / 185; of 256 183 / 142, 141 / 137, 221 / 185;
-# of 2,048 1,623 / 635, 893 / 566, 1,457 / 863; eight of 2,048 tokens together, the longest 391, 697 / 651, 603 / 598, 858 / 859;
-# eight of 1,000 together, the longest 190, 361 / 314, 315 / 285, 455 / 486.
+# state space with heads of 64): one prompt of 200 tokens 157 / 135, 125 / 135, 191 / 170; of 256 181 / 132, 140 / 132, 220 / 170;
+# of 2,048 1,627 / 583, 886 / 519, 1,450 / 760; eight of 2,048 tokens together, the longest 391, 687 / 631, 603 / 587, 851 / 851;
+# eight of 1,000 together, the longest 190, 357 / 309, 307 / 280, 445 / 478.
 CHUNK_SCAN_FROM, CHUNK_SCAN_SHARE = 256, 5
 
 
@@ -958,9 +965,9 @@ def _chunk_scan(kind: int, q: int, k: int, v: int, row: int, plan, batch, state:
     factors, flags = new(per_pass, heads, 4, chunk), torch.empty((per_pass, heads), dtype=torch.int32, device=dev)
     norms = new(per_pass, heads, dim) if kind == 1 else None
     carry = new(2, heads, vdim, dim) if per_pass < n else None
-    _call("chunk_scan", "fms_chunk_scan", kind, q, k, v, row, _ptr(runs), _ptr(first_run), n, per_pass, _ptr(batch.slots), batch.n_seqs,
-          _ptr(decay), _ptr(gates), _ptr(norm_in), _ptr(norm_state), dt_raw, dt_dtype, dt_stride, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
-          _ptr(state), _ptr(carry), _ptr(scores), _ptr(factors), _ptr(totals), _ptr(states), _ptr(norms), _ptr(flags), _ptr(o), heads, key_heads, dim, vdim,
+    _call("chunk_scan", "fms_chunk_scan", kind, q, k, v, row, runs, first_run, n, per_pass, batch.slots, batch.n_seqs,
+          decay, gates, norm_in, norm_state, dt_raw, dt_dtype, dt_stride, dt_bias, a_log, d_skip,
+          state, carry, scores, factors, totals, states, norms, flags, o, heads, key_heads, dim, vdim,
           1 if writes_state else 0, state.shape[0], _stream())
     launches += 3 * ((n + per_pass - 1) // per_pass) - 1
 
@@ -983,9 +990,9 @@ def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bia
                     dt_raw=_ptr(proj) + dt_offset * proj.element_size(), dt_dtype=_code(proj.dtype), dt_stride=proj.shape[1],
                     dt_bias=dt_bias, a_log=a_log, d_skip=d_skip)
         return y
-    _call("state_scan", "fms_selective_scan", _ptr(xbc), _ptr(proj) + dt_offset * proj.element_size(), _code(proj.dtype),
-          proj.shape[1], _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(y), _ptr(batch.first_row),
-          _ptr(batch.slots), batch.n_seqs, heads, vdim, n_state, groups, 1 if writes_state else 0, state.shape[0],
+    _call("state_scan", "fms_selective_scan", xbc, _ptr(proj) + dt_offset * proj.element_size(), _code(proj.dtype),
+          proj.shape[1], dt_bias, a_log, d_skip, state, y, batch.first_row,
+          batch.slots, batch.n_seqs, heads, vdim, n_state, groups, 1 if writes_state else 0, state.shape[0],
           _stream())
     return y
 
@@ -1015,10 +1022,10 @@ def delta_rule_scan(qkv: torch.Tensor, proj: torch.Tensor, beta_offset: int, a_r
     o = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
     # decays [tokens, heads * dim], then betas [tokens, heads]
     scratch = torch.empty((n * heads * (dim + 1),), dtype=torch.float32, device=qkv.device)
-    _call("state_scan", "fms_delta_rule_scan", _ptr(qkv), _ptr(proj) + beta_offset * proj.element_size(),
-          _code(proj.dtype), proj.shape[1], a_ptr, a_stride, 1 if per_head else 0, _ptr(dt_bias), _ptr(a_log),
+    _call("state_scan", "fms_delta_rule_scan", qkv, _ptr(proj) + beta_offset * proj.element_size(),
+          _code(proj.dtype), proj.shape[1], a_ptr, a_stride, 1 if per_head else 0, dt_bias, a_log,
           scratch.data_ptr(),
-          scratch.data_ptr() + 4 * n * heads * dim, _ptr(state), _ptr(o), _ptr(batch.first_row), _ptr(batch.slots), n,
+          scratch.data_ptr() + 4 * n * heads * dim, state, o, batch.first_row, batch.slots, n,
           batch.n_seqs, heads, kvheads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
     global launches
     launches += 1  # the kernel that makes q, k, the decays and the betas ready
@@ -1050,24 +1057,24 @@ def gla_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: in
     if batch.max_new >= GLA_CHUNKS_FROM:
         lib = load_library("gated_linear")
         if _gla_chunk is None:
-            lib.fms_gla_record_floats.restype = _L
+            lib.fms_gla_record_floats.restype = ctypes.c_long
             _gla_chunk = int(lib.fms_gla_chunk_tokens())
         chunk_rows, first_chunk = batch.row_chunks(_gla_chunk)
         n_chunks = chunk_rows.shape[0]
         records = torch.empty((n_chunks * heads * int(lib.fms_gla_record_floats(dim, vdim)),), dtype=torch.float32, device=proj.device)
-        _call("gated_linear", "fms_gla_chunked", _ptr(proj), _code(proj.dtype), proj.shape[1], int(rank_offset), rank, _ptr(decay_weight),
-              _code(decay_weight.dtype), _ptr(decay_bias), float(tau), float(q_scale), _ptr(chunk_rows), _ptr(first_chunk), n_chunks,
-              _ptr(records), _ptr(state), _ptr(o), _ptr(batch.slots), n, batch.n_seqs, heads, dim, vdim, 1 if writes_state else 0,
-              state.shape[0], _ptr(error_flag(proj.device)), _stream())
+        _call("gated_linear", "fms_gla_chunked", proj, _code(proj.dtype), proj.shape[1], int(rank_offset), rank, decay_weight,
+              _code(decay_weight.dtype), decay_bias, float(tau), float(q_scale), chunk_rows, first_chunk, n_chunks,
+              records, state, o, batch.slots, n, batch.n_seqs, heads, dim, vdim, 1 if writes_state else 0,
+              state.shape[0], error_flag(proj.device), _stream())
         launches += 1
         return o
     qkv = torch.empty((n, cols), dtype=torch.float32, device=proj.device)
     decay = torch.empty((n, channels), dtype=torch.float32, device=proj.device)
-    _call("state_scan", "fms_gla_prepare", _ptr(proj), _code(proj.dtype), proj.shape[1], int(rank_offset), rank, _ptr(decay_weight),
-          _code(decay_weight.dtype), _ptr(decay_bias), float(tau), _ptr(decay), channels, _ptr(qkv), n, cols, channels,
+    _call("state_scan", "fms_gla_prepare", proj, _code(proj.dtype), proj.shape[1], int(rank_offset), rank, decay_weight,
+          _code(decay_weight.dtype), decay_bias, float(tau), decay, channels, qkv, n, cols, channels,
           float(q_scale), _stream())
-    _call("state_scan", "fms_decay_scan", _ptr(qkv), None, _code(proj.dtype), 0, None, 0.0, _ptr(decay), None, None, _ptr(state),
-          None, _ptr(o), _ptr(batch.first_row), _ptr(batch.slots), n, batch.n_seqs, heads, dim, vdim,
+    _call("state_scan", "fms_decay_scan", qkv, None, _code(proj.dtype), 0, None, 0.0, decay, None, None, state,
+          None, o, batch.first_row, batch.slots, n, batch.n_seqs, heads, dim, vdim,
           1 if writes_state else 0, state.shape[0], _stream())
     return o
 
@@ -1085,10 +1092,10 @@ def gla_read_out(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim
                 or proj.shape[1] < max(heads * (2 * dim + vdim), rank_offset + rank, gate_offset + heads * vdim) \
                 or decay_weight.shape[0] != heads * dim or decay_bias.dtype != torch.float32 or decay_bias.shape[0] != heads * dim:
             raise KernelError("gla_read_out: proj [tokens, q | k | v | ...], state float32 [slots, heads, vdim, dim], norm float32 [vdim]")
-        out = torch.empty((n, heads * vdim), dtype=proj.dtype, device=proj.device)
-        _call("gated_linear", "fms_gla_decode", _ptr(proj), _code(proj.dtype), proj.shape[1], int(rank_offset), rank, _ptr(decay_weight),
-              _code(decay_weight.dtype), _ptr(decay_bias), float(tau), float(q_scale), _ptr(state), _ptr(batch.slots), int(gate_offset),
-              _ptr(norm), float(eps), _ptr(out), n, heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
+        out = proj.new_empty((n, heads * vdim))
+        _call("gated_linear", "fms_gla_decode", proj, _code(proj.dtype), proj.shape[1], int(rank_offset), rank, decay_weight,
+              _code(decay_weight.dtype), decay_bias, float(tau), float(q_scale), state, batch.slots, int(gate_offset),
+              norm, float(eps), out, n, heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
         return out
     o = gla_scan(proj, state, batch, heads, dim, vdim, rank_offset, decay_weight, decay_bias, tau, q_scale, writes_state)
     return gated_group_rmsnorm(o, proj, gate_offset, GATE_SILU_AFTER, norm, eps, vdim, proj.dtype)
@@ -1128,7 +1135,7 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     if not gated and (decay.dtype != torch.float32 or decay.shape[0] != heads):
         raise KernelError("decay_scan: decays float32 [heads]")
     qkv = torch.empty((n, cols), dtype=torch.float32, device=proj.device)
-    _call("state_scan", "fms_linear_prepare", _ptr(proj), _code(proj.dtype), proj.shape[1], _ptr(qkv), n, cols, heads * dim,
+    _call("state_scan", "fms_linear_prepare", proj, _code(proj.dtype), proj.shape[1], qkv, n, cols, heads * dim,
           float(q_scale), int(activation), _stream())
     o = torch.empty((n, heads * vdim), dtype=torch.float32, device=proj.device)
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
@@ -1137,16 +1144,16 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     plan = _chunk_scan_runs(batch, dim, vdim, heads, heads) if not gated or vdim == 128 else None
     if plan is not None:
         if gated:
-            _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], _ptr(gate_bias), float(gate_cap),
-                  _ptr(norm_state), _ptr(norm_in), _ptr(gates), _ptr(batch.first_row), _ptr(batch.slots), n, batch.n_seqs, heads, dim,
+            _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias, float(gate_cap),
+                  norm_state, norm_in, gates, batch.first_row, batch.slots, n, batch.n_seqs, heads, dim,
                   1 if writes_state else 0, state.shape[0], _stream())
         q = _ptr(qkv)
         _chunk_scan(1 if gated else 0, q, q + heads * dim * 4, q + 2 * heads * dim * 4, cols, plan, batch, state, o, heads, heads, dim, vdim,
                     writes_state, decay=decay, gates=gates, norm_in=norm_in, norm_state=norm_state)
         return o
-    _call("state_scan", "fms_decay_scan", _ptr(qkv), gate_ptr, _code(proj.dtype), proj.shape[1], _ptr(gate_bias),
-          float(gate_cap), _ptr(gates), _ptr(norm_in), _ptr(decay), _ptr(state), _ptr(norm_state), _ptr(o), _ptr(batch.first_row),
-          _ptr(batch.slots), n, batch.n_seqs, heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
+    _call("state_scan", "fms_decay_scan", qkv, gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias,
+          float(gate_cap), gates, norm_in, decay, state, norm_state, o, batch.first_row,
+          batch.slots, n, batch.n_seqs, heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
     global launches
     launches += 1 if gated else 0  # the kernel that walks the gates
     return o
@@ -1169,9 +1176,9 @@ def gated_group_rmsnorm(x: torch.Tensor, gate: Optional[torch.Tensor], gate_offs
         raise KernelError(f"gated_group_rmsnorm: gate {gate.dtype}, compute dtype {out_dtype}")
     out = torch.empty((n, width), dtype=out_dtype, device=x.device)
     gate_ptr = None if gate is None else _ptr(gate) + gate_offset * gate.element_size()
-    _call("state_scan", "fms_gated_group_rmsnorm", _ptr(x), gate_ptr, _code(out_dtype), 0 if gate is None else gate.shape[1],
-          int(gate_mode) if gate is not None else GATE_NONE, _ptr(weight), weight.shape[0], float(eps), float(factor),
-          _ptr(out), n, width, int(group_size), _stream())
+    _call("state_scan", "fms_gated_group_rmsnorm", x, gate_ptr, _code(out_dtype), 0 if gate is None else gate.shape[1],
+          int(gate_mode) if gate is not None else GATE_NONE, weight, weight.shape[0], float(eps), float(factor),
+          out, n, width, int(group_size), _stream())
     return out
 
 
@@ -1199,10 +1206,10 @@ def grouped_linear(x: torch.Tensor, weight: torch.Tensor, groups: int, rows: int
             and _ptr(x) % 16 == 0 and groups <= 65535:
         # a decode step of few rows: the weight-streaming kernel, a block per group and run of its matrix's rows (8 rows, 32
         # groups of 512 x 96: 4.7 us, of 128 x 512: 3.5; 18 each with a warp a row of the matrix)
-        _call("gemm_bf16_skinny", "fms_strided_bf16_skinny", _ptr(x), _ptr(weight), _ptr(y), rows, groups, n_out, k, x_row_stride,
+        _call("gemm_bf16_skinny", "fms_strided_bf16_skinny", x, weight, y, rows, groups, n_out, k, x_row_stride,
               x_group_offset, y_row_stride, y_group_offset, _stream())
         return y
-    _call("grouped", "fms_grouped_linear", _ptr(x), _ptr(weight), _ptr(y), _code(x.dtype), None, None, None, groups, rows,
+    _call("grouped", "fms_grouped_linear", x, weight, y, _code(x.dtype), None, None, None, groups, rows,
           n_out, k, x_row_stride, x_group_offset, y_row_stride, y_group_offset, 0, 0.0, 0.0,
           1 if rows <= GROUPED_FEW_ROWS else 0, _stream())
     return y
@@ -1262,10 +1269,10 @@ def route(x: torch.Tensor, router: torch.Tensor, top: int, mode: int = ROUTE_SIG
     if x.dtype == router.dtype == torch.bfloat16 and n > ROUTE_FEW_ROWS and 8 * 4 * (2 * experts + groups) <= 48 * 1024:
         _ptr(x), _ptr(router)
         logits = torch.mm(x, router.t(), out_dtype=torch.float32)
-    _call("grouped", "fms_route", _ptr(x), _code(x.dtype), _ptr(router), _code(router.dtype), _ptr(r.expert),
-          _ptr(r.weight), _ptr(counts), _ptr(r.offsets), _ptr(r.tile_first), _ptr(r.row_of_pair), _ptr(r.group_of_row),
-          _ptr(r.rows), n, dim, experts, top, int(mode), _ptr(correction), float(route_scale), int(groups), int(keep),
-          _ptr(logits), router.shape[0], _ptr(bias), _ptr(r.side), _stream())
+    _call("grouped", "fms_route", x, _code(x.dtype), router, _code(router.dtype), r.expert,
+          r.weight, counts, r.offsets, r.tile_first, r.row_of_pair, r.group_of_row,
+          r.rows, n, dim, experts, top, int(mode), correction, float(route_scale), int(groups), int(keep),
+          logits, router.shape[0], bias, r.side, _stream())
     global launches
     launches += 2
     return r
@@ -1287,23 +1294,23 @@ def routed_linear(rows: torch.Tensor, weight: torch.Tensor, routing: Routing, gl
         _ptr(rows), _ptr(weight)
         y = torch.nn.functional.grouped_mm(rows, weight.transpose(1, 2), offs=routing.offsets[1:])
         if relu_squared and not glu:
-            _call("grouped", "fms_relu_squared", _ptr(y), _code(y.dtype), y.numel(), _stream())
+            _call("grouped", "fms_relu_squared", y, _code(y.dtype), y.numel(), _stream())
         if not glu:
             return y
         if silu:
             return gated_activation(y, 0)
-        out = torch.empty((n, n_out), dtype=rows.dtype, device=rows.device)
-        _call("grouped", "fms_gated_clamped", _ptr(y), _ptr(out), _code(y.dtype), n, n_out, float(limit), float(alpha),
+        out = rows.new_empty((n, n_out))
+        _call("grouped", "fms_gated_clamped", y, out, _code(y.dtype), n, n_out, float(limit), float(alpha),
               _stream())
         return out
-    y = torch.empty((n, n_out), dtype=rows.dtype, device=rows.device)
+    y = rows.new_empty((n, n_out))
     if rows.dtype == torch.bfloat16 and n <= SKINNY_ROWS * routing.top and k % 8 == 0:
         # up to eight tokens, so up to eight rows an expert: the weight-streaming kernel, a block per group and run of rows
-        _call("gemm_bf16_skinny", "fms_grouped_bf16_skinny", _ptr(rows), _ptr(weight), _ptr(y), _ptr(routing.offsets),
+        _call("gemm_bf16_skinny", "fms_grouped_bf16_skinny", rows, weight, y, routing.offsets,
               routing.experts, n_out, k, (3 if silu else 1) if glu else (2 if relu_squared else 0), float(limit), float(alpha), _stream())
         return y
-    _call("grouped", "fms_grouped_linear", _ptr(rows), _ptr(weight), _ptr(y), _code(rows.dtype), _ptr(routing.offsets),
-          _ptr(routing.tile_first), _ptr(routing.group_of_row), routing.experts, n, n_out, k, k, 0, n_out, 0,
+    _call("grouped", "fms_grouped_linear", rows, weight, y, _code(rows.dtype), routing.offsets,
+          routing.tile_first, routing.group_of_row, routing.experts, n, n_out, k, k, 0, n_out, 0,
           (3 if silu else 1) if glu else (2 if relu_squared else 0), float(limit), float(alpha), 1 if n <= GROUPED_FEW_ROWS else 0, _stream())
     return y
 
@@ -1315,10 +1322,10 @@ def route_gather(ys: torch.Tensor, routing: Routing, every: Optional[torch.Tenso
     if every is not None and (every.dtype != ys.dtype or tuple(every.shape) != (ys.shape[0] // routing.top, ys.shape[1])):
         raise KernelError(f"route_gather: rows {ys.dtype} {tuple(ys.shape)} of {routing.top} a token, beside {every.dtype} {tuple(every.shape)}")
     n = ys.shape[0] // routing.top
-    out = torch.empty((n, ys.shape[1]), dtype=ys.dtype, device=ys.device)
-    _call("grouped", "fms_route_gather", _ptr(ys), _code(ys.dtype), _ptr(routing.row_of_pair), _ptr(out), n, ys.shape[1],
-          routing.top, _ptr(routing.weight) if routing.weights_on_output else None, _ptr(every),
-          _ptr(routing.side) if every is not None else None, _stream())
+    out = ys.new_empty((n, ys.shape[1]))
+    _call("grouped", "fms_route_gather", ys, _code(ys.dtype), routing.row_of_pair, out, n, ys.shape[1],
+          routing.top, routing.weight if routing.weights_on_output else None, every,
+          routing.side if every is not None else None, _stream())
     return out
 
 
@@ -1343,12 +1350,12 @@ def latent_prepare(proj: torch.Tensor, q_full: torch.Tensor, c_gain: torch.Tenso
         raise KernelError("latent_prepare: the latent's matrix has the projection's dtype and rows, and rank + rot columns")
     if view.keys.dtype != proj.dtype or q_full.dtype != proj.dtype:
         raise KernelError(f"cache is {view.keys.dtype}, activations are {proj.dtype}")
-    _call("latent_attention", "fms_latent_prepare", _ptr(proj), _code(proj.dtype), proj.shape[1], _ptr(q_full),
-          q_full.shape[2], dim if own_space else rank, 1 if own_space else 0, _ptr(c_gain), _code(c_gain.dtype), float(eps), _ptr(inv_freq), int(rot_dims), _ptr(batch.positions),
-          _ptr(getattr(batch, "position_ids", None)), _ptr(batch.token_seq), _ptr(batch.slots), _ptr(view.keys),
-          _ptr(view.table), view.table.shape[1], view.block_tokens, proj.shape[0], heads, dim, rot, rank,
+    _call("latent_attention", "fms_latent_prepare", proj, _code(proj.dtype), proj.shape[1], q_full,
+          q_full.shape[2], dim if own_space else rank, 1 if own_space else 0, c_gain, _code(c_gain.dtype), float(eps), inv_freq, int(rot_dims), batch.positions,
+          getattr(batch, "position_ids", None), batch.token_seq, batch.slots, view.keys,
+          view.table, view.table.shape[1], view.block_tokens, proj.shape[0], heads, dim, rot, rank,
           1 if writes_cache else 0, batch.slots.shape[0], view.table.shape[0], view.keys.shape[0],
-          _ptr(error_flag(proj.device)), 1 if halves else 0, float(rot_mult), _ptr(kv), 0 if kv is None else kv.shape[1],
+          error_flag(proj.device), 1 if halves else 0, float(rot_mult), kv, 0 if kv is None else kv.shape[1],
           _stream())
 
 
@@ -1357,9 +1364,9 @@ def latent_query_norm(proj: torch.Tensor, offset: int, n: int, gain: torch.Tenso
     [n]: the query's latent on its way to the projection that makes the heads' queries of it."""
     if proj.shape[1] < offset + n or gain.shape[0] != n:
         raise KernelError("latent_query_norm: the columns lie inside the rows and the gain has their number")
-    out = torch.empty((proj.shape[0], n), dtype=proj.dtype, device=proj.device)
+    out = proj.new_empty((proj.shape[0], n))
     _call("latent_attention", "fms_latent_query_norm", _ptr(proj) + offset * proj.element_size(), _code(proj.dtype),
-          proj.shape[1], n, _ptr(gain), _code(gain.dtype), float(eps), _ptr(out), proj.shape[0], _stream())
+          proj.shape[1], n, gain, _code(gain.dtype), float(eps), out, proj.shape[0], _stream())
     return out
 
 
@@ -1399,11 +1406,11 @@ def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor
             or (sink is not None and sink.dtype != torch.float32) or (gate is not None and gate.dtype != q.dtype):
         raise KernelError(f"latent_attention_expanded: {heads} heads of {head_dim}, matrices {tuple(expand.shape)}, rows of {view.keys.shape[-1]}")
     start, first, base, rows = batch.key_rows(window)
-    cached = torch.empty((rows, width), dtype=q.dtype, device=q.device)
-    _call("latent_attention", "fms_latent_gather", _ptr(view.keys), width * q.element_size(), _ptr(view.table), view.table.shape[1],
-          view.block_tokens, _ptr(batch.slots), _ptr(start), _ptr(first), batch.n_seqs, _ptr(cached), rows, view.table.shape[0],
+    cached = q.new_empty((rows, width))
+    _call("latent_attention", "fms_latent_gather", view.keys, width * q.element_size(), view.table, view.table.shape[1],
+          view.block_tokens, batch.slots, start, first, batch.n_seqs, cached, rows, view.table.shape[0],
           view.keys.shape[0], _stream())
-    out = torch.empty((n, heads * head_dim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((n, heads * head_dim))
     lib = _attention_library(head_dim)
     tiles = batch.query_tiles(attention_constants(head_dim, q.dtype, 1, 1)[1])
     step = max(1, min(heads, LATENT_EXPANDED_BYTES // (rows * 2 * head_dim * q.element_size())))
@@ -1411,11 +1418,11 @@ def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor
         m = min(step, heads - h)
         kv = linear(cached, expand[h:h + m].view(m * 2 * head_dim, width))
         at = h * head_dim * q.element_size()
-        _call(lib, "fms_attention_prefill_rows", _ptr(q) + at, heads * head_dim, _ptr(out) + at, heads * head_dim, _ptr(kv),
-              _ptr(kv) + head_dim * kv.element_size(), kv.shape[1], 2 * head_dim, rows, _ptr(base), _ptr(batch.first_row),
-              _ptr(batch.len_after), _ptr(tiles), tiles.shape[0], m, head_dim, float(scale), int(window),
+        _call(lib, "fms_attention_prefill_rows", _ptr(q) + at, heads * head_dim, _ptr(out) + at, heads * head_dim, kv,
+              _ptr(kv) + head_dim * kv.element_size(), kv.shape[1], 2 * head_dim, rows, base, batch.first_row,
+              batch.len_after, tiles, tiles.shape[0], m, head_dim, float(scale), int(window),
               None if sink is None else _ptr(sink) + h * 4, None if gate is None else _ptr(gate) + (gate_offset + h) * gate.element_size(),
-              0 if gate is None else gate.shape[1], _ptr(error_flag(q.device)), _stream())
+              0 if gate is None else gate.shape[1], error_flag(q.device), _stream())
     return out
 
 
@@ -1428,7 +1435,7 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
     ``window`` > 0: the row at position p sees the keys p - window + 1 .. p only.  Returns [tokens, heads, rank]."""
     global _latent_split, launches
     n = q_full.shape[0]
-    out = torch.empty((n, heads, rank), dtype=q_full.dtype, device=q_full.device)
+    out = q_full.new_empty((n, heads, rank))
     if _latent_split is None:
         _latent_split = int(load_library("latent_attention").fms_latent_split_tokens())
     if (USE_LATENT_MMA and q_full.dtype == torch.bfloat16 and rank % 64 == 0 and rank <= 512
@@ -1444,8 +1451,9 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
                 split = LATENT_SHORT_SPLIT
             n_splits = max(1, (batch.max_len_after + split - 1) // split)
             if n_splits > 1:
-                part_o = torch.empty((n, heads, n_splits, rank), dtype=torch.float32, device=q_full.device)
-                part_ml = torch.empty((n, heads, n_splits, 2), dtype=torch.float32, device=q_full.device)
+                parts = torch.empty((n * heads * n_splits * (rank + 2),), dtype=torch.float32, device=q_full.device)
+                part_o = parts.data_ptr()  # [rank] of every split, then its maxima and sums [2]
+                part_ml = part_o + n * heads * n_splits * rank * 4
         else:
             heads_per_block = 1
             while heads_per_block < min(32, heads):
@@ -1453,12 +1461,12 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
         tile_tokens = 32 // heads_per_block
         tiles = batch.query_tiles(tile_tokens)
         gate_ptr = None if gate is None else _ptr(gate) + gate_offset * gate.element_size()
-        _call("latent_attention", "fms_latent_attention_prefill_bf16", _ptr(q_full), _ptr(out), _ptr(view.keys), gate_ptr,
-              0 if gate is None else gate.shape[1], _ptr(sink), _code(sink.dtype) if sink is not None else F32,
-              _ptr(view.table), view.table.shape[1], view.block_tokens, _ptr(batch.slots), _ptr(batch.first_row),
-              _ptr(batch.positions), _ptr(tiles), tiles.shape[0], tile_tokens, heads_per_block, heads, rank, rot,
-              float(scale), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _ptr(batch.token_seq), n_splits, split,
-              _ptr(part_o), _ptr(part_ml), int(window), _stream())
+        _call("latent_attention", "fms_latent_attention_prefill_bf16", q_full, out, view.keys, gate_ptr,
+              0 if gate is None else gate.shape[1], sink, _code(sink.dtype) if sink is not None else F32,
+              view.table, view.table.shape[1], view.block_tokens, batch.slots, batch.first_row,
+              batch.positions, tiles, tiles.shape[0], tile_tokens, heads_per_block, heads, rank, rot,
+              float(scale), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], batch.token_seq, n_splits, split,
+              part_o, part_ml, int(window), _stream())
         if n_splits > 1:
             launches += 1
         return out
@@ -1469,10 +1477,10 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
             part_o = torch.empty((n, heads, n_splits, rank), dtype=torch.float32, device=q_full.device)
             part_ml = torch.empty((n, heads, n_splits, 2), dtype=torch.float32, device=q_full.device)
     gate_ptr = None if gate is None else _ptr(gate) + gate_offset * gate.element_size()
-    _call("latent_attention", "fms_latent_attention", _ptr(q_full), _ptr(out), _code(q_full.dtype), _ptr(view.keys), gate_ptr,
-          0 if gate is None else gate.shape[1], _ptr(sink), _code(sink.dtype) if sink is not None else F32,
-          _ptr(view.table), view.table.shape[1], view.block_tokens, _ptr(batch.slots), _ptr(batch.token_seq),
-          _ptr(batch.positions), n, n_splits, _ptr(part_o), _ptr(part_ml), heads, rank, rot, float(scale),
+    _call("latent_attention", "fms_latent_attention", q_full, out, _code(q_full.dtype), view.keys, gate_ptr,
+          0 if gate is None else gate.shape[1], sink, _code(sink.dtype) if sink is not None else F32,
+          view.table, view.table.shape[1], view.block_tokens, batch.slots, batch.token_seq,
+          batch.positions, n, n_splits, part_o, part_ml, heads, rank, rot, float(scale),
           batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], int(window), _stream())
     if n_splits > 1:
         launches += 1
@@ -1485,7 +1493,7 @@ def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Te
     if logits.dtype != torch.float32:
         raise KernelError("logits are float32")
     out = out if out is not None else torch.empty((rows,), dtype=torch.int32, device=logits.device)
-    _call("sampling", "fms_argmax", _ptr(logits), _ptr(out), rows, vocab, _stream())
+    _call("sampling", "fms_argmax", logits, out, rows, vocab, _stream())
     return out
 
 
@@ -1495,6 +1503,6 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, seed: int, requ
     if logits.dtype != torch.float32:
         raise KernelError("logits are float32")
     out = out if out is not None else torch.empty((rows,), dtype=torch.int32, device=logits.device)
-    _call("sampling", "fms_sample", _ptr(logits), _ptr(out), rows, vocab, float(temperature), int(top_k),
-          int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(requests), int(step), _stream())
+    _call("sampling", "fms_sample", logits, out, rows, vocab, float(temperature), int(top_k),
+          int(seed) & 0xFFFFFFFFFFFFFFFF, requests, int(step), _stream())
     return out

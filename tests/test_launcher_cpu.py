@@ -1,0 +1,54 @@
+"""Arguments on their way from Python into a C entry (csrc/launcher.cpp): order, widths and what is refused."""
+import ctypes
+import itertools
+import subprocess
+
+import pytest
+import torch
+
+from fms_b200.kernels import build
+from fms_b200.kernels.ops import _SIGNATURES, KernelError
+
+C_TYPES = {"p": "void*", "i": "int", "l": "long", "f": "float"}
+
+
+def entry(tmp_path, kinds):
+    """An entry of these parameters that writes each, as a double, to the address in its first, and that address."""
+    source = tmp_path / "echo.c"
+    names = ", ".join(f"{C_TYPES[k]} a{i}" for i, k in enumerate(kinds))
+    body = "".join(f"  out[{i}] = (double){'(long)' if k == 'p' else ''}a{i};\n" for i, k in enumerate(kinds) if i)
+    source.write_text(f"int echo({names}) {{\n  double* out = (double*)a0;\n{body}  return 7;\n}}\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "echo.so"), str(source)], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "echo.so"))
+    address = ctypes.cast(lib.echo, ctypes.c_void_p).value
+    return build.load_launcher().entry(address, kinds.replace("l", "i"), KernelError), (ctypes.c_double * len(kinds))(), lib
+
+
+@pytest.mark.parametrize("kinds", ["p", "pi", "pf", "pifl", "piiiii", "piiiiii", "pfffffffi", "p" + "if" * 8, "pilfp" * 6 + "lliipp",
+                                   "p" + "i" * 45])
+def test_arguments_arrive_in_order(tmp_path, kinds):
+    f, out, lib = entry(tmp_path, kinds)
+    given = {"i": itertools.cycle((3, -5, 2 ** 31 - 1, True)), "l": itertools.cycle((-2 ** 40, 2 ** 45)),
+             "p": itertools.cycle((None, 4096)), "f": itertools.cycle((0.25, -3, 1e30))}
+    args = [ctypes.addressof(out)] + [next(given[k]) for k in kinds[1:]]
+    assert f(*args) == 7
+    single = lambda x: ctypes.c_float(x).value  # noqa: E731
+    assert list(out)[1:] == [single(a) if k == "f" else float(a or 0) for k, a in zip(kinds[1:], args[1:])]
+
+
+def test_what_an_entry_refuses(tmp_path):
+    f, out, lib = entry(tmp_path, "pif")
+    at = ctypes.addressof(out)
+    for args in ((at, 1), (at, 1, 1.0, 1), (at, 1.0, 1.0), (at, None, 1.0), (at, 1, None), (at, 1, "1"), (at, torch.zeros(1), 1.0)):
+        with pytest.raises(TypeError):
+            f(*args)
+    with pytest.raises(KernelError, match="on the CPU"):
+        f(torch.zeros(4), 1, 1.0)
+    for kinds in ("px", "p" * 47, "p" + "f" * 9):
+        with pytest.raises(ValueError):
+            build.load_launcher().entry(1, kinds, KernelError)
+
+
+def test_every_entry_fits():
+    for name, kinds in _SIGNATURES.items():
+        assert build.load_launcher().entry(1, "".join(kinds), KernelError), name
