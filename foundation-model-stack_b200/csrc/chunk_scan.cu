@@ -26,6 +26,14 @@
 // by max(|n . q|, e) + 1e-6.  KIND 2: a = exp(-exp(a_log) dt), b = dt = softplus(raw + bias), and o += d_skip v; key heads
 // are shared by groups of heads.
 //
+// KIND 3, the delta rule: S_t = a_t S_(t-1) + k_t u_t^T with u_t = beta_t (v_t - a_t S_(t-1)^T k_t).  Within a run the u hang
+// together by a lower triangle, (I + A) U = diag(beta) (V - diag(G) K S), A[t][s] = beta_t a_(s+1) .. a_t (k_t . k_s) for s < t:
+//
+//   chunk_solve    T' = (I + A)^-1 diag(beta) of every run and head, all at once
+//   delta_states   as chunk_states, with Y = V - diag(G) K S and U = T' Y first; U goes where o will be
+//
+// and chunk_outputs takes U for the values (b = 1).
+//
 // Sums are made of runs of 16 terms and products of decays in 64 bits, so that a state's error stays below the walk's (2,048
 // tokens under fixed decays: 1.1e-7 of its size against 2.6e-7; in chains of 128 and float32 products 5.5e-7) and an output's
 // beside it (9.5e-8 against 8.2e-8).  Measured alone: prompts of 1,062 and 638 tokens,
@@ -48,8 +56,10 @@ struct ChunkArgs {
   const int* runs;       // [runs, 2]: first row and end of every run
   const int* first_run;  // [n_seqs + 1]
   const int* slots;
-  const float* decay;    // KIND 0
-  const float* gates;    // KIND 1
+  long v_row;            // of v: row, or the stride of o where chunk_outputs reads U there
+  const float* decay;    // KIND 0: [heads]; KIND 3: [tokens, heads]
+  const float* gates;    // KIND 1; KIND 3: beta [tokens, heads]
+  float* solve;          // scratch, KIND 3: [runs of a pass, heads, C, C]: T', element [s][t]
   float* norm_in;        // KIND 1: [n_seqs, heads, dim], n before the step; carries n from pass to pass
   float* norm_state;     // KIND 1: [slots, heads, dim + 1]
   const void* dt_raw;    // KIND 2: column `head` of rows of dt_stride values
@@ -146,6 +156,7 @@ __device__ __forceinline__ float2 token_gates(const ChunkArgs& g, int t, int end
     const float* p = g.gates + ((size_t)t * g.heads + head) * 3;
     return make_float2(p[0], p[1]);
   }
+  if (KIND == 3) return make_float2(g.decay[(size_t)t * g.heads + head], 1.f);
   // in double, rounded once: a decay's error compounds over a sequence
   const size_t at = (size_t)t * g.dt_stride + head;
   const double x = (g.dt_is_bf16 ? (double)__bfloat162float(((const __nv_bfloat16*)g.dt_raw)[at]) : (double)((const float*)g.dt_raw)[at]) +
@@ -498,7 +509,7 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
   __syncthreads();  // the slices are free: the values go there
   for (int i = tid; i < C * (COLS / 4); i += 128) {
     const int t = i / (COLS / 4), c = (i % (COLS / 4)) * 4;
-    copy16(sm + t * CROW + c, g.v + (size_t)(row0 + min(t, rows - 1)) * g.row + (size_t)head0 * VDIM + c, t < rows);
+    copy16(sm + t * CROW + c, g.v + (size_t)(row0 + min(t, rows - 1)) * g.v_row + (size_t)head0 * VDIM + c, t < rows);
   }
   copies_commit();
   // G_t times what the state gives
@@ -554,6 +565,337 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
   }
 }
 
+// ---- the delta rule's triangles: a block a run and head -----------------------------------------------------------------
+// k . k^T as the scores (8 x 4 a thread), then the inverse of the 64 x 64 triangle by blocks of 16: the diagonal ones by substitution,
+// a thread a column; those below, diagonal by diagonal, T_ij = -T_ii sum_(j <= m < i) A_im T_mj.  A row takes no term of a later one.
+__global__ void __launch_bounds__(128) chunk_solve_kernel(ChunkArgs g) {
+  __shared__ __align__(16) float sm[2][C][SROW];  // slices of k, then T over them
+  __shared__ float A[C][C + 1], W[3][16][16], as[C], bt[C];
+  constexpr int TP = C + 1;
+  static_assert(C * TP <= 2 * C * SROW, "T lies where the slices were");
+  float* T = &sm[0][0][0];
+  pdl_wait();
+  const int local = blockIdx.x, run = g.run_lo + local, head = blockIdx.y, kh = head / (g.heads / g.key_heads), tid = threadIdx.x;
+  const int row0 = g.runs[2 * run], end = g.runs[2 * run + 1], rows = end - row0;
+  const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
+  auto issue = [&](int d0, int buf) {
+    for (int i = tid; i < C * (SLICE / 4); i += 128) {
+      const int t = i / (SLICE / 4), d = (i % (SLICE / 4)) * 4;
+      copy16(&sm[buf][t][d], k + (size_t)min(t, rows - 1) * g.row + d0 + d, t < rows);
+    }
+    copies_commit();
+  };
+  issue(0, 0);
+  if (tid < C) {
+    const size_t at = (size_t)(row0 + tid) * g.heads + head;
+    as[tid] = tid < rows ? g.decay[at] : 1.f;
+    bt[tid] = tid < rows ? g.gates[at] : 0.f;
+  }
+  const int ty = tid >> 4, tx = tid & 15;  // rows t = ty * 8 + i, columns s = tx + 16 j
+  float sum[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[i][j] = 0.f;
+#pragma unroll 1
+  for (int d0 = 0; d0 < DIM; d0 += SLICE) {
+    const int buf = (d0 / SLICE) & 1;
+    if (d0 + SLICE < DIM) {
+      issue(d0 + SLICE, buf ^ 1);
+      copies_wait<1>();
+    } else {
+      copies_wait<0>();
+    }
+    __syncthreads();
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll
+    for (int d = 0; d < SLICE; d += 4) {
+      float4 kx[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kx[j] = *reinterpret_cast<const float4*>(&sm[buf][tx + 16 * j][d]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 qx = *reinterpret_cast<const float4*>(&sm[buf][ty * 8 + i][d]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[i][j] = fmaf(qx.x, kx[j].x, acc[i][j]);
+          acc[i][j] = fmaf(qx.y, kx[j].y, acc[i][j]);
+          acc[i][j] = fmaf(qx.z, kx[j].z, acc[i][j]);
+          acc[i][j] = fmaf(qx.w, kx[j].w, acc[i][j]);
+        }
+      }
+      if ((d + 4) % PART == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            sum[i][j] += acc[i][j];
+            acc[i][j] = 0.f;
+          }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) A[ty * 8 + i][tx + 16 * j] = sum[i][j];
+  for (int i = tid; i < C * TP; i += 128) T[i] = 0.f;
+  __syncthreads();
+  if (tid < C) {  // a row a thread, s downwards
+    double e = bt[tid];
+    for (int s = tid - 1; s >= 0; --s) {
+      e *= as[s + 1];
+      A[tid][s] *= (float)e;
+    }
+  }
+  __syncthreads();
+  if (tid < C) {  // the diagonal blocks
+    const int base = tid & ~15, c = tid & 15;
+    float x[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      float y = t == c ? 1.f : 0.f;
+#pragma unroll
+      for (int s = 0; s < t; ++s)
+        if (s >= c) y = fmaf(-A[base + t][base + s], x[s], y);
+      x[t] = y;
+      T[(base + t) * TP + tid] = y;
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int far = 1; far < 4; ++far) {
+    const int items = (4 - far) * 256;
+    for (int e = tid; e < items; e += 128) {  // W_b = sum_m A_im T_mj for j = b, i = b + far
+      const int b = e >> 8, r = (e >> 4) & 15, c = e & 15, i0 = (b + far) * 16 + r, j0 = b * 16;
+      float y = 0.f;
+#pragma unroll 16
+      for (int m = 0; m < far * 16; ++m) y = fmaf(A[i0][j0 + m], T[(j0 + m) * TP + j0 + c], y);
+      W[b][r][c] = y;
+    }
+    __syncthreads();
+    for (int e = tid; e < items; e += 128) {
+      const int b = e >> 8, r = (e >> 4) & 15, c = e & 15, i0 = (b + far) * 16;
+      float y = 0.f;
+#pragma unroll
+      for (int m = 0; m < 16; ++m)
+        if (m <= r) y = fmaf(-T[(i0 + r) * TP + i0 + m], W[b][m][c], y);
+      T[(i0 + r) * TP + b * 16 + c] = y;
+    }
+    __syncthreads();
+  }
+  pdl_launch_dependents();
+  float* out = g.solve + ((size_t)local * g.heads + head) * C * C;
+  for (int i = tid; i < C * C; i += 128) {
+    const int s = i / C, t = i % C;
+    out[i] = s <= t ? T[t * TP + s] * bt[s] : 0.f;
+  }
+}
+
+// ---- the delta rule's states: 128 key channels x 16 value columns a block, 4 x 4 a thread ---------------------------------
+// As chunk_states, a sequence's runs in order, with U in front of every run's part of the state; three products in a row that wait
+// for one another, so narrow columns and more blocks.  Bound by what shared memory returns (half a word a multiply-add) and by the
+// three products' order: 4.6 us a run of 64 tokens, which the walk takes 28 us for (one sequence, 16 heads of 128: 149 us of
+// 2,048 tokens; scores 21, triangles 31, outputs 62; the walk 912).  From 64 bits: outputs 1.5e-7, states 1.6e-7 of their size
+// (the walk 1.5e-7, 2.3e-7).
+constexpr int DVT = 16, KROW = DIM + 4;
+constexpr size_t DELTA_SMEM = (size_t)(2 * C * KROW + 2 * C * DVT + C * TROW + DVT * KROW + C * DVT) * sizeof(float);
+
+__global__ void __launch_bounds__(128, 2) delta_states_kernel(ChunkArgs g) {
+  constexpr int VDIM = 128;
+  extern __shared__ __align__(16) float sm[];
+  float* kbuf = sm;                      // [2][C][KROW]
+  float* vbuf = kbuf + 2 * C * KROW;     // [2][C][DVT]: v, then Y in place
+  float* ts = vbuf + 2 * C * DVT;        // [C][TROW]: T', row s
+  float* st = ts + C * TROW;             // [DVT][KROW]: the state, a row a column
+  float* uw = st + DVT * KROW;           // [C][DVT]: U times the decays behind it
+  __shared__ float weight[C], upto[C];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int seq = blockIdx.y, tid = threadIdx.x;
+  const int lo = max(g.first_run[seq], g.run_lo), hi = min(g.first_run[seq + 1], g.run_hi);
+  if (lo >= hi) return;
+  const int slot = __ldcg(g.slots + seq);
+  if (!FMS_IN(slot, g.n_slots)) return;
+  const bool begins = lo == g.first_run[seq], ends = hi == g.first_run[seq + 1];
+  const int col0 = blockIdx.x * DVT, head = col0 / VDIM, kh = head / (g.heads / g.key_heads);
+  auto issue = [&](int run, int buf) {
+    const int row0 = g.runs[2 * run], rows = g.runs[2 * run + 1] - row0;
+    const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
+    const float* v = g.v + (size_t)row0 * g.row + col0;
+    for (int i = tid; i < C * (DIM / 4); i += 128) {
+      const int t = i / (DIM / 4), d = (i % (DIM / 4)) * 4;
+      copy16(kbuf + (buf * C + t) * KROW + d, k + (size_t)min(t, rows - 1) * g.row + d, t < rows);
+    }
+    for (int i = tid; i < C * (DVT / 4); i += 128) {
+      const int t = i / (DVT / 4), c = (i % (DVT / 4)) * 4;
+      copy16(vbuf + (buf * C + t) * DVT + c, v + (size_t)min(t, rows - 1) * g.row + c, t < rows);
+    }
+  };
+  auto issue_solve = [&](int run) {
+    const float* from = g.solve + ((size_t)(run - g.run_lo) * g.heads + head) * C * C;
+    for (int i = tid; i < C * (C / 4); i += 128) copy16(ts + i / (C / 4) * TROW + i % (C / 4) * 4, from + i * 4, true);
+  };
+  issue(lo, 0);
+  issue_solve(lo);
+  copies_commit();
+  const int td = (tid >> 2) * 4, tv = (tid & 3) * 4;   // of the state: channels td .. + 3, columns tv .. + 3
+  const int ky = tid >> 3, kx = tid & 7;               // of Y: tokens ky + 16 i, columns kx + 8 j
+  const int ut = (tid >> 3) * 4, uc = (tid & 7) * 2;   // of U: tokens ut .. + 3, columns uc, uc + 1
+  const size_t per_seq = (size_t)g.heads * VDIM * DIM;
+  const float* from = (begins ? g.state + (size_t)slot * per_seq : g.carry + (g.pass & 1) * per_seq) + (size_t)col0 * DIM;
+  float S[4][4];  // [channel][column]
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 x = *reinterpret_cast<const float4*>(from + (size_t)(tv + j) * DIM + td);
+    S[0][j] = x.x;
+    S[1][j] = x.y;
+    S[2][j] = x.z;
+    S[3][j] = x.w;
+  }
+#pragma unroll 1
+  for (int run = lo; run < hi; ++run) {
+    const int local = run - g.run_lo, buf = (run - lo) & 1;
+    const int row0 = g.runs[2 * run], rows = g.runs[2 * run + 1] - row0;
+    const float* ks = kbuf + buf * C * KROW;
+    float* vs = vbuf + buf * C * DVT;
+    const float total = g.totals[(size_t)local * g.heads + head];
+    if (tid < C) {
+      const float* f = g.factors + ((size_t)local * g.heads + head) * 4 * C + tid;
+      upto[tid] = f[2 * C];
+      weight[tid] = f[3 * C];
+    }
+    float* out = g.states + ((size_t)local * (g.heads * VDIM / COLS) + col0 / COLS) * DIM * COLS + col0 % COLS + tv;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)  // what is before the run goes out, and to where this block's threads read it
+      *reinterpret_cast<float4*>(out + (size_t)(td + i) * COLS) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(st + (tv + j) * KROW + td) = make_float4(S[0][j], S[1][j], S[2][j], S[3][j]);
+    copies_wait<0>();
+    __syncthreads();
+    if (run + 1 < hi) {
+      issue(run + 1, buf ^ 1);
+      copies_commit();
+    }
+    // Y = V - G (K S)
+    f32x2 even[4][2], odd[4][2];  // channels 0, 1 and 2, 3 of every four
+#pragma unroll
+    for (int i = 0; i < 4; ++i) even[i][0] = even[i][1] = odd[i][0] = odd[i][1] = 0;
+#pragma unroll 8
+    for (int d = 0; d < DIM; d += 4) {
+      ulonglong2 x[4], y[2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(ks + (ky + 16 * i) * KROW + d);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) y[j] = *reinterpret_cast<const ulonglong2*>(st + (kx + 8 * j) * KROW + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          even[i][j] = fma2(x[i].x, y[j].x, even[i][j]);
+          odd[i][j] = fma2(x[i].y, y[j].y, odd[i][j]);
+        }
+    }
+    int bad = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float a, b;
+        unpack2(add2(even[i][j], odd[i][j]), a, b);
+        float* y = vs + (ky + 16 * i) * DVT + kx + 8 * j;
+        const float x = fmaf(-upto[ky + 16 * i], a + b, *y);
+        *y = x;
+        bad |= !(fabsf(x) <= 3.4028235e38f);
+      }
+    bad = __syncthreads_or(bad);
+    // U = T' Y: rows up to the warp's last, later ones with zeros of T' (or, where a value is not finite, by selection)
+    float U[4][2], part[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) U[i][0] = U[i][1] = part[i][0] = part[i][1] = 0.f;
+    const int reach = (tid >> 5) * 16 + 16;
+#pragma unroll 1
+    for (int s0 = 0; s0 < reach; s0 += PART) {
+#pragma unroll
+      for (int s = s0; s < s0 + PART; ++s) {
+        const float4 x = *reinterpret_cast<const float4*>(ts + s * TROW + ut);
+        const float2 y = *reinterpret_cast<const float2*>(vs + s * DVT + uc);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (!bad || s <= ut + i) {
+            part[i][0] = fmaf(xs[i], y.x, part[i][0]);
+            part[i][1] = fmaf(xs[i], y.y, part[i][1]);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        U[i][0] += part[i][0];
+        U[i][1] += part[i][1];
+        part[i][0] = part[i][1] = 0.f;
+      }
+    }
+    bad = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = ut + i;
+      const float w = weight[t];
+      *reinterpret_cast<float2*>(uw + t * DVT + uc) = make_float2(U[i][0] * w, U[i][1] * w);
+      if (t < rows) *reinterpret_cast<float2*>(g.o + (size_t)(row0 + t) * g.heads * VDIM + col0 + uc) = make_float2(U[i][0], U[i][1]);
+      bad |= !(fabsf(U[i][0]) <= 3.4028235e38f && fabsf(U[i][1]) <= 3.4028235e38f);
+    }
+    if (__syncthreads_or(bad) && tid == 0) g.flags[(size_t)local * g.heads + head] = 1;
+    if (run + 1 < hi) {
+      issue_solve(run + 1);
+      copies_commit();
+    }
+    // S = total S + K^T (U times the decays behind it)
+    f32x2 acc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+#pragma unroll 8
+    for (int s = 0; s < C; ++s) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(ks + s * KROW + td);
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(uw + s * DVT + tv);
+      const f32x2 z0 = swapped(y.x), z1 = swapped(y.y);
+      acc[0][0] = fma2(x.x, y.x, acc[0][0]);
+      acc[0][1] = fma2(x.x, z0, acc[0][1]);
+      acc[0][2] = fma2(x.x, y.y, acc[0][2]);
+      acc[0][3] = fma2(x.x, z1, acc[0][3]);
+      acc[1][0] = fma2(x.y, y.x, acc[1][0]);
+      acc[1][1] = fma2(x.y, z0, acc[1][1]);
+      acc[1][2] = fma2(x.y, y.y, acc[1][2]);
+      acc[1][3] = fma2(x.y, z1, acc[1][3]);
+    }
+    float own[4][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        unpack2(acc[i][2 * j], own[2 * i][2 * j], own[2 * i + 1][2 * j + 1]);
+        unpack2(acc[i][2 * j + 1], own[2 * i][2 * j + 1], own[2 * i + 1][2 * j]);
+      }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) S[i][j] = fmaf(total, S[i][j], own[i][j]);
+    __syncthreads();  // the stage, the state's copy, U and the factors are free
+  }
+  if (!ends || g.write_state) {
+    float* to = (ends ? g.state + (size_t)slot * per_seq : g.carry + ((g.pass + 1) & 1) * per_seq) + (size_t)col0 * DIM;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<float4*>(to + (size_t)(tv + j) * DIM + td) = make_float4(S[0][j], S[1][j], S[2][j], S[3][j]);
+  }
+}
+
 template <int VDIM, int KIND, int VT>
 int launch_states(const ChunkArgs& g, cudaStream_t stream) {
   static bool configured = false;
@@ -574,6 +916,7 @@ int launch_passes(ChunkArgs g, int n_runs, int pass_runs, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(chunk_outputs_kernel<VDIM, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUT_SMEM<VDIM>);
+    if (KIND == 3 && e == cudaSuccess) e = cudaFuncSetAttribute(delta_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DELTA_SMEM);
     if (e != cudaSuccess) return fms_fail("chunk_scan: shared memory refused: %s", cudaGetErrorString(e));
     configured = true;
   }
@@ -583,8 +926,17 @@ int launch_passes(ChunkArgs g, int n_runs, int pass_runs, cudaStream_t stream) {
     g.run_hi = lo + pass_runs < n_runs ? lo + pass_runs : n_runs;
     const int n = g.run_hi - lo;
     fms_launch(chunk_scores_kernel<KIND>, dim3(n, g.key_heads), dim3(128), 0, stream, g);
-    if (columns_32(g, VDIM) ? launch_states<VDIM, KIND, 32>(g, stream) : launch_states<VDIM, KIND, 64>(g, stream)) return 1;
-    fms_launch(chunk_outputs_kernel<VDIM, KIND>, dim3(n, g.heads * VDIM / COLS), dim3(128), OUT_SMEM<VDIM>, stream, g);
+    if constexpr (KIND == 3) {
+      fms_launch(chunk_solve_kernel, dim3(n, g.heads), dim3(128), 0, stream, g);
+      fms_launch(delta_states_kernel, dim3(g.heads * VDIM / DVT, g.n_seqs), dim3(128), DELTA_SMEM, stream, g);
+      ChunkArgs u = g;
+      u.v = g.o;
+      u.v_row = (long)g.heads * VDIM;
+      fms_launch(chunk_outputs_kernel<VDIM, KIND>, dim3(n, g.heads * VDIM / COLS), dim3(128), OUT_SMEM<VDIM>, stream, u);
+    } else {
+      if (columns_32(g, VDIM) ? launch_states<VDIM, KIND, 32>(g, stream) : launch_states<VDIM, KIND, 64>(g, stream)) return 1;
+      fms_launch(chunk_outputs_kernel<VDIM, KIND>, dim3(n, g.heads * VDIM / COLS), dim3(128), OUT_SMEM<VDIM>, stream, g);
+    }
     if (fms_launch_status("chunk_scan")) return 1;
   }
   return 0;
@@ -606,21 +958,21 @@ FMS_API int fms_chunk_scan(int kind, const float* q, const float* k, const float
                            int n_runs, int pass_runs, const int* slots, int n_seqs, const float* decay, const float* gates,
                            float* norm_in, float* norm_state, const void* dt_raw, int dt_dtype, long dt_stride, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, float* carry, float* scores, float* factors,
-                           float* totals, float* states, float* norms, int* flags, float* o, int heads, int key_heads, int dim, int vdim,
+                           float* totals, float* states, float* norms, float* solve, int* flags, float* o, int heads, int key_heads, int dim, int vdim,
                            int write_state, int n_slots, cudaStream_t stream) {
   if (n_runs <= 0 || n_seqs <= 0) return 0;
-  if (heads <= 0 || key_heads <= 0 || heads % key_heads || !fms_chunk_scan_takes(dim, vdim, heads / key_heads) || (kind == 1 && vdim != 128))
+  if (heads <= 0 || key_heads <= 0 || heads % key_heads || !fms_chunk_scan_takes(dim, vdim, heads / key_heads) || ((kind == 1 || kind == 3) && vdim != 128))
     return fms_fail("chunk_scan: %d heads over %d, dim %d, vdim %d", heads, key_heads, dim, vdim);
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || row % 4 || !aligned16(state) || !aligned16(states) || (carry && !aligned16(carry)))
     return fms_fail("chunk_scan: rows of %ld values, or a pointer, not on 16 bytes", row);
   if (pass_runs <= 0 || (pass_runs < n_runs && carry == nullptr)) return fms_fail("chunk_scan: %d runs of %d a pass without a carry", pass_runs, n_runs);
   if (n_seqs > 65535 || heads > 65535) return fms_fail("chunk_scan: %d sequences, %d heads", n_seqs, heads);
   if (!scores || !factors || !states || !totals || !flags || (kind == 0 && !decay) || (kind == 1 && (!gates || !norm_in || !norm_state || !norms)) ||
-      (kind == 2 && (!dt_raw || !dt_bias || !a_log || !d_skip)))
+      (kind == 3 && (!decay || !gates || !solve)) || (kind == 2 && (!dt_raw || !dt_bias || !a_log || !d_skip)))
     return fms_fail("chunk_scan: kind %d without what it reads", kind);
   if (kind == 2 && dt_dtype != FMS_F32 && dt_dtype != FMS_BF16) return fms_fail("chunk_scan: dtype code %d", dt_dtype);
   ChunkArgs g = {};
-  g.q = q; g.k = k; g.v = v; g.row = row; g.runs = runs; g.first_run = first_run; g.slots = slots; g.decay = decay; g.gates = gates;
+  g.q = q; g.k = k; g.v = v; g.row = g.v_row = row; g.solve = solve; g.runs = runs; g.first_run = first_run; g.slots = slots; g.decay = decay; g.gates = gates;
   g.norm_in = norm_in; g.norm_state = norm_state; g.dt_raw = dt_raw; g.dt_bias = dt_bias; g.a_log = a_log; g.d_skip = d_skip;
   g.dt_stride = dt_stride; g.dt_is_bf16 = dt_dtype == FMS_BF16; g.state = state; g.carry = carry; g.scores = scores; g.factors = factors;
   g.states = states; g.norms = norms; g.totals = totals; g.flags = flags; g.o = o; g.heads = heads; g.key_heads = key_heads;
@@ -628,5 +980,6 @@ FMS_API int fms_chunk_scan(int kind, const float* q, const float* k, const float
   if (kind == 0) return vdim == 128 ? launch_passes<128, 0>(g, n_runs, pass_runs, stream) : launch_passes<64, 0>(g, n_runs, pass_runs, stream);
   if (kind == 1) return launch_passes<128, 1>(g, n_runs, pass_runs, stream);
   if (kind == 2) return vdim == 128 ? launch_passes<128, 2>(g, n_runs, pass_runs, stream) : launch_passes<64, 2>(g, n_runs, pass_runs, stream);
+  if (kind == 3) return launch_passes<128, 3>(g, n_runs, pass_runs, stream);
   return fms_fail("chunk_scan: kind %d", kind);
 }

@@ -460,7 +460,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const floa
 //   qkv [tokens, 2 kvheads * dim + heads * vdim] float32 (after the convolution): q | k | v;  q and k of every key head
 //   become unit vectors in place, x / sqrt(sum(x^2) + 1e-6), q also times dim^-1/2
 //   decay[t, h, n] = exp(-exp(a_log[h]) * softplus(a_raw[t, h, n] + dt_bias[h, n]));  beta[t, h] = sigmoid(beta_raw[t, h])
-//   `per_head`: one decay a head, exp(-exp(a_log[h]) * softplus(a_raw[t, h] + dt_bias[h])), written to all its channels
+//   `per_head`: one decay a head, exp(-exp(a_log[h]) * softplus(a_raw[t, h] + dt_bias[h])), written to all its channels (1) or
+//   as decay[t, h] (2)
 //   a_raw is walked by its row stride `a_stride`
 template <typename T>
 __global__ void delta_prepare_kernel(float* qkv, const T* a_raw, int a_stride, int per_head, const T* beta_raw,
@@ -485,7 +486,11 @@ __global__ void delta_prepare_kernel(float* qkv, const T* a_raw, int a_stride, i
       const size_t at = ((size_t)t * heads + h) * dim;
       if (per_head) {
         const float d = (float)exp(-A * softplus_d((double)to_f32(a_raw[(size_t)t * a_stride + h]) + (double)dt_bias[h]));
-        for (int n = lane; n < dim; n += 32) decay[at + n] = d;
+        if (per_head == 2) {
+          if (lane == 0) decay[(size_t)t * heads + h] = d;
+        } else {
+          for (int n = lane; n < dim; n += 32) decay[at + n] = d;
+        }
       } else {
         const T* ar = a_raw + (size_t)t * a_stride + (size_t)h * dim;
         for (int n = lane; n < dim; n += 32)
@@ -1180,6 +1185,19 @@ FMS_API int fms_selective_scan(const float* xbc, const void* dt_raw, int dtype, 
   FMS_SCAN_SHAPES(FMS_LAUNCH);
 #undef FMS_LAUNCH
   return fms_launch_status("selective_scan");
+}
+
+// What the delta rule with one decay a head reads, made ready for every token: qkv in place, decay and beta [tokens, heads]
+FMS_API int fms_delta_prepare(float* qkv, const void* beta_raw, int dtype, int beta_stride, const void* a_raw, int a_stride,
+                              const float* dt_bias, const float* a_log, float* decay, float* beta, int n_tokens, int heads, int kvheads,
+                              int dim, int vdim, cudaStream_t stream) {
+  if (n_tokens <= 0) return 0;
+  if (heads <= 0 || kvheads <= 0 || heads % kvheads || dim <= 0 || vdim <= 0)
+    return fms_fail("delta_prepare: %d heads over %d, dim %d, vdim %d", heads, kvheads, dim, vdim);
+  FMS_DISPATCH_DTYPE(dtype, T, fms_launch(delta_prepare_kernel<T>, dim3(n_tokens, (2 * kvheads + heads + 3) / 4), dim3(128), 0, stream, qkv, (const T*)a_raw,
+                                          a_stride, 2, (const T*)beta_raw, beta_stride, dt_bias, a_log, decay, beta, heads, kvheads, dim,
+                                          vdim));
+  return fms_launch_status("delta_prepare");
 }
 
 // decay [tokens, heads * dim] and beta [tokens, heads]: float32 scratch of the caller's.  a_raw: rows of a_stride

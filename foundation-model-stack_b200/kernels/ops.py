@@ -95,7 +95,8 @@ _SIGNATURES = {
     "fms_linear_prepare": [_P, _I, _I, _P, _I, _I, _I, _F, _I, _P],
     "fms_exp_gates": [_P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "fms_chunk_scan": [_I, _P, _P, _P, _L, _P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
-                       _I, _I, _I, _I, _I, _I, _P],
+                       _P, _I, _I, _I, _I, _I, _I, _P],
+    "fms_delta_prepare": [_P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fms_decay_scan": [_P, _P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_attention_prefill_sink": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
                                    _P],
@@ -932,16 +933,26 @@ CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read ba
 CHUNK_SCAN_FROM, CHUNK_SCAN_SHARE = 256, 5
 
 
-def chunk_scan_pays(batch, heads: int, vdim: int) -> bool:
+# The same for the delta rule, which has two more products a run.  Whole layers of 16 heads of 128, walk / runs in us: one prompt of
+# 130 tokens 102 / 121, of 200 141 / 131, of 2,048 1,106 / 453; 512 tokens of eight sequences, the longest 97, 175 / 205; 1,000 of
+# eight, the longest 190, 302 / 269; 2,048 of eight 581 / 457.
+DELTA_CHUNKS_FROM = 192
+
+
+def chunk_scan_pays(batch, heads: int, vdim: int, least: Optional[int] = None) -> bool:
     """Whether a step's scan goes run by run (``fms_chunk_scan``) or token by token."""
     longest = max(batch.num_new)
-    return longest >= CHUNK_SCAN_FROM and (vdim > 64 or CHUNK_SCAN_SHARE * longest >= sum(batch.num_new))
+    return longest >= (CHUNK_SCAN_FROM if least is None else least) and (vdim > 64 or CHUNK_SCAN_SHARE * longest >= sum(batch.num_new))
 
 
-def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int):
-    """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, decode steps and
-    short prompts (which go token by token), a capture that has not seen the batch before (the runs come from the host)."""
-    if batch.decode or not batch.num_new or not chunk_scan_pays(batch, heads, vdim):
+def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, rows: torch.Tensor, state: torch.Tensor,
+                     least: Optional[int] = None):
+    """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, rows or states
+    that do not lie on 16 bytes, decode steps and short prompts (which go token by token), a capture that has not seen the batch
+    before (the runs come from the host)."""
+    if batch.decode or not batch.num_new or not chunk_scan_pays(batch, heads, vdim, least):
+        return None
+    if (_ptr(rows) | _ptr(state)) & 15 or rows.shape[1] % 4 or batch.n_seqs > 65535:
         return None
     lib = load_library("chunk_scan")
     if not lib.fms_chunk_scan_takes(int(dim), int(vdim), heads // key_heads):
@@ -967,9 +978,9 @@ def _chunk_scan(kind: int, q: int, k: int, v: int, row: int, plan, batch, state:
     carry = new(2, heads, vdim, dim) if per_pass < n else None
     _call("chunk_scan", "fms_chunk_scan", kind, q, k, v, row, runs, first_run, n, per_pass, batch.slots, batch.n_seqs,
           decay, gates, norm_in, norm_state, dt_raw, dt_dtype, dt_stride, dt_bias, a_log, d_skip,
-          state, carry, scores, factors, totals, states, norms, flags, o, heads, key_heads, dim, vdim,
-          1 if writes_state else 0, state.shape[0], _stream())
-    launches += 3 * ((n + per_pass - 1) // per_pass) - 1
+          state, carry, scores, factors, totals, states, norms, new(per_pass, heads, chunk, chunk) if kind == 3 else None, flags, o,
+          heads, key_heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
+    launches += (4 if kind == 3 else 3) * ((n + per_pass - 1) // per_pass) - 1
 
 
 def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
@@ -983,7 +994,7 @@ def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bia
             or tuple(state.shape[1:]) != (heads, vdim, n_state):
         raise KernelError("selective_scan: xbc float32 [tokens, x | B | C], state float32 [slots, heads, vdim, state]")
     y = torch.empty((n, heads * vdim), dtype=torch.float32, device=xbc.device)
-    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups)
+    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups, xbc, state)
     if plan is not None:
         x, b = _ptr(xbc), _ptr(xbc) + heads * vdim * 4
         _chunk_scan(2, b + groups * n_state * 4, b, x, xbc.shape[1], plan, batch, state, y, heads, groups, n_state, vdim, writes_state,
@@ -1004,7 +1015,7 @@ def delta_rule_scan(qkv: torch.Tensor, proj: torch.Tensor, beta_offset: int, a_r
     [tokens, 2 kvheads * dim + heads * vdim] = [q | k | v]; beta = sigmoid(proj[:, beta_offset + head]);
     g = exp(-exp(a_log[head]) softplus(a_raw + dt_bias)), [heads * dim] a row; ``state`` float32 [slots, heads, vdim, dim].
     q and k of ``qkv`` are made unit vectors in place on the way.  Returns o float32 [tokens, heads * vdim].
-    ``decay_offset`` (with ``a_raw`` None): one decay a head instead of one a key channel,
+    ``decay_offset`` (with ``a_raw`` None): one decay a head instead of one a key channel (many tokens then go run by run),
     g = exp(-exp(a_log[head]) softplus(proj[:, decay_offset + head] + dt_bias[head])), dt_bias [heads]."""
     n = qkv.shape[0]
     per_head = decay_offset is not None
@@ -1020,6 +1031,15 @@ def delta_rule_scan(qkv: torch.Tensor, proj: torch.Tensor, beta_offset: int, a_r
             raise KernelError("delta_rule_scan: decays' logits [tokens, heads * dim] in the projection's dtype")
         a_ptr, a_stride = _ptr(a_raw), heads * dim
     o = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, kvheads, qkv, state, DELTA_CHUNKS_FROM) if per_head and vdim == 128 else None
+    if plan is not None:
+        decay, beta = (torch.empty((n, heads), dtype=torch.float32, device=qkv.device) for _ in range(2))
+        _call("state_scan", "fms_delta_prepare", qkv, _ptr(proj) + beta_offset * proj.element_size(), _code(proj.dtype), proj.shape[1],
+              a_ptr, a_stride, dt_bias, a_log, decay, beta, n, heads, kvheads, dim, vdim, _stream())
+        q = _ptr(qkv)
+        _chunk_scan(3, q, q + kvheads * dim * 4, q + 2 * kvheads * dim * 4, qkv.shape[1], plan, batch, state, o, heads, kvheads, dim,
+                    vdim, writes_state, decay=decay, gates=beta)
+        return o
     # decays [tokens, heads * dim], then betas [tokens, heads]
     scratch = torch.empty((n * heads * (dim + 1),), dtype=torch.float32, device=qkv.device)
     _call("state_scan", "fms_delta_rule_scan", qkv, _ptr(proj) + beta_offset * proj.element_size(),
@@ -1141,7 +1161,7 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
     norm_in = torch.empty((batch.n_seqs, heads, dim), dtype=torch.float32, device=proj.device) if gated else None
     gate_ptr = _ptr(proj) + gate_offset * proj.element_size() if gated else None
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads) if not gated or vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv, state) if not gated or vdim == 128 else None
     if plan is not None:
         if gated:
             _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias, float(gate_cap),

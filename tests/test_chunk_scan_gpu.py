@@ -5,7 +5,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-KINDS = ["fixed", "gated", "space"]
+KINDS = ["fixed", "gated", "space", "delta"]
 LENGTHS = [[64], [1, 65], [127, 3, 128], [200, 64, 129]]
 
 
@@ -30,6 +30,12 @@ def run(kind, batch, n, slots, vdim, seed, change=None, writes_state=True):
         if change:
             change(xbc)
         y = ops.selective_scan(xbc, proj, 0, r(heads) - 2.0, r(heads).abs(), r(heads), state, batch, heads, vdim, dim, 2, writes_state)
+        return y, [state]
+    if kind == "delta":  # two heads over one key head
+        qkv, proj = r(n, 2 * dim + heads * vdim), r(n, 2 * heads).bfloat16()
+        if change:
+            change(qkv)
+        y = ops.delta_rule_scan(qkv, proj, 0, None, r(heads) - 2.0, r(heads).abs(), state, batch, heads, 1, dim, vdim, writes_state, decay_offset=heads)
         return y, [state]
     proj = r(n, heads * (2 * dim + vdim) + 2 * heads)
     if change:
