@@ -856,24 +856,27 @@ __global__ void rope_store_kernel(const T* __restrict__ qkv, T* __restrict__ q_o
   dst[2 * i + 1] = from_f32<T>(x1);
 }
 
-// bfloat16, many tokens: one block per token, a thread per 16-byte piece (8 values = 4 pairs) of a head.  The
-// angle of a pair is the same for every head of the token: its sine and cosine are taken once, into shared memory.
+// Many tokens: one block per token, a thread per 16-byte piece (8 bfloat16 values = 4 pairs, 4 float32 = 2) of a head.
+// The angle of a pair is the same for every head of the token: its sine and cosine are taken once, into shared memory.
+// (float32, 1,100 tokens of 48 heads of 128: 11 us; a block a token and head, each with its own sines, 56.)
 constexpr int ROPE_VEC_MAX_PAIRS = 1024;  // head_dim / 2 that the table in shared memory holds
 
-__global__ void rope_store_vec_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ q_out,
+template <typename T>
+__global__ void rope_store_vec_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
                                       const float* __restrict__ inv_freq, const int* __restrict__ positions,
                                       const int* __restrict__ position_ids, const int* __restrict__ token_seq,
                                       const int* __restrict__ slots,
-                                      __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
+                                      T* __restrict__ k_cache, T* __restrict__ v_cache,
                                       const int* __restrict__ table, int table_stride, int block_tokens, int nheads,
                                       int kvheads, int head_dim, int write_cache, int* __restrict__ error_flag,
                                       int n_seqs, int table_rows, int pool_blocks) {
+  constexpr int PIECE = 16 / sizeof(T);  // values of a piece
   extern __shared__ float2 sincos_of_pair[];  // [head_dim / 2]: (sin, cos)
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
   const int pos = positions[t];
-  const int pieces = head_dim >> 3;
+  const int pieces = head_dim / PIECE;
   const int total = (nheads + 2 * kvheads) * pieces;
   const size_t width = (size_t)(nheads + 2 * kvheads) * head_dim;
   int blk = 0;
@@ -899,26 +902,32 @@ __global__ void rope_store_vec_kernel(const __nv_bfloat16* __restrict__ qkv, __n
   }
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int head = i / pieces, piece = i - head * pieces;
-    const uint4 v = *reinterpret_cast<const uint4*>(qkv + (size_t)t * width + (size_t)head * head_dim + piece * 8);
+    const uint4 v = *reinterpret_cast<const uint4*>(qkv + (size_t)t * width + (size_t)head * head_dim + piece * PIECE);
     uint32_t w[4] = {v.x, v.y, v.z, v.w};
     const bool is_v = head >= nheads + kvheads;
     if (!is_v && inv_freq != nullptr) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float x0 = __uint_as_float(w[k] << 16), x1 = __uint_as_float(w[k] & 0xffff0000u);
-        const float2 sc = sincos_of_pair[piece * 4 + k];
-        __nv_bfloat162 r = __floats2bfloat162_rn(sc.y * x0 - sc.x * x1, sc.x * x0 + sc.y * x1);
-        w[k] = *reinterpret_cast<uint32_t*>(&r);
+      for (int k = 0; k < PIECE / 2; ++k) {
+        const float2 sc = sincos_of_pair[piece * (PIECE / 2) + k];
+        if constexpr (PIECE == 8) {
+          const float x0 = __uint_as_float(w[k] << 16), x1 = __uint_as_float(w[k] & 0xffff0000u);
+          __nv_bfloat162 r = __floats2bfloat162_rn(sc.y * x0 - sc.x * x1, sc.x * x0 + sc.y * x1);
+          w[k] = *reinterpret_cast<uint32_t*>(&r);
+        } else {
+          const float x0 = __uint_as_float(w[2 * k]), x1 = __uint_as_float(w[2 * k + 1]);
+          w[2 * k] = __float_as_uint(sc.y * x0 - sc.x * x1);
+          w[2 * k + 1] = __float_as_uint(sc.x * x0 + sc.y * x1);
+        }
       }
     }
     const uint4 o = make_uint4(w[0], w[1], w[2], w[3]);
     if (head < nheads) {
-      *reinterpret_cast<uint4*>(q_out + ((size_t)t * nheads + head) * head_dim + piece * 8) = o;
+      *reinterpret_cast<uint4*>(q_out + ((size_t)t * nheads + head) * head_dim + piece * PIECE) = o;
     } else if (write_cache && blk >= 0) {
       const int kvh = is_v ? head - nheads - kvheads : head - nheads;
-      __nv_bfloat16* base = is_v ? v_cache : k_cache;
+      T* base = is_v ? v_cache : k_cache;
       *reinterpret_cast<uint4*>(base + (((size_t)blk * kvheads + kvh) * block_tokens + (pos % block_tokens)) * head_dim +
-                                piece * 8) = o;
+                                piece * PIECE) = o;
     }
   }
 }
@@ -931,14 +940,17 @@ FMS_API int fms_rope_store(const void* qkv, int dtype, void* q_out, const float*
   // n_seqs, table_rows, pool_blocks: extents of slots, of the table and of the cache, for the bounds-checked build (0: not known)
   if (n_tokens <= 0) return 0;
   if (head_dim <= 0 || head_dim % 2 || head_dim > 2048) return fms_fail("rope_store: head_dim %d", head_dim);
-  if (dtype == FMS_BF16 && head_dim % 8 == 0 && n_tokens >= 64 && head_dim / 2 <= ROPE_VEC_MAX_PAIRS) {
-    const int total = (nheads + 2 * kvheads) * (head_dim / 8);
+  const int piece = dtype == FMS_BF16 ? 8 : 4;
+  const uintptr_t places = (uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache;
+  if ((dtype == FMS_BF16 || (dtype == FMS_F32 && places % 16 == 0)) && head_dim % piece == 0 && n_tokens >= 64 &&
+      head_dim / 2 <= ROPE_VEC_MAX_PAIRS) {
+    const int total = (nheads + 2 * kvheads) * (head_dim / piece);
     const int threads = total >= 256 ? 256 : ((total + 31) / 32) * 32;
-    fms_launch(rope_store_vec_kernel, dim3(n_tokens), dim3(threads), (size_t)(head_dim / 2) * sizeof(float2), stream,
-               (const __nv_bfloat16*)qkv,
-               (__nv_bfloat16*)q_out, inv_freq, positions, position_ids, token_seq, slots, (__nv_bfloat16*)k_cache,
-               (__nv_bfloat16*)v_cache, table, table_stride, block_tokens, nheads, kvheads, head_dim, write_cache,
-               error_flag, n_seqs, table_rows, pool_blocks);
+    FMS_DISPATCH_DTYPE(dtype, T,
+                       fms_launch(rope_store_vec_kernel<T>, dim3(n_tokens), dim3(threads), (size_t)(head_dim / 2) * sizeof(float2), stream,
+                                  (const T*)qkv, (T*)q_out, inv_freq, positions, position_ids, token_seq, slots, (T*)k_cache, (T*)v_cache,
+                                  table, table_stride, block_tokens, nheads, kvheads, head_dim, write_cache, error_flag, n_seqs,
+                                  table_rows, pool_blocks));
     return fms_launch_status("rope_store");
   }
   dim3 grid(n_tokens, nheads + 2 * kvheads);
