@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
           gate += __bfloat162float(bias[row]);
           up += __bfloat162float(bias[hidden + row]);
         }
-        if (FMS_IN((size_t)m * hidden + row, (size_t)M * hidden)) y[(size_t)m * hidden + row] = from_f32<TOut>(extra.unit == UNIT_CLAMPED ? clamped_unit(gate, up, extra.cap, extra.scale) : activate(gate, act) * up);
+        if (FMS_IN((size_t)m * hidden + row, (size_t)M * hidden)) y[(size_t)m * hidden + row] = from_f32<TOut>(GROUPS == GROUPED && extra.unit == UNIT_CLAMPED ? clamped_unit(gate, up, extra.cap, extra.scale) : activate(gate, act) * up);
       }
     }
   } else if (MODE == QKV_ROPE) {
