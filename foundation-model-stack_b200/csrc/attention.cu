@@ -30,7 +30,7 @@ namespace {
 constexpr int HD = HEAD_DIM;
 constexpr int BLK = 64;           // tokens per cache block
 constexpr int SPLIT = 256;        // keys per decode split
-constexpr int GC = 8;             // query heads of one kv head handled by one decode block
+constexpr int GC_MOST = 8;        // query heads of one kv head handled by one decode block
 constexpr int TQ = 64;            // query rows per float32 prefill block
 
 template <typename T> struct Vec;  // 16-byte vectors
@@ -299,8 +299,12 @@ __global__ void __launch_bounds__(128, 2) attn_prefill_f32_kernel(AttnArgs a, co
 // decode: grid (sequences, kv heads * head chunks, splits), 128 threads.  One block handles up to GC
 // query heads of one kv head over one split of the keys and writes an unnormalised partial result
 // (m, l, o) per head; attn_combine_kernel merges the splits.
+// Bound by the trips to memory that wait for one another and by what shared memory returns (a word of the queries or of the
+// probabilities a multiply-add): eight loads of a thread are on their way at a time, and up to 4 heads a key head take a GC
+// of 4, which has half of that work of 8.  Measured (8 sequences, 9,520 cached keys together, 32 heads over 8 of 128):
+// 29 us; a GC of 8 for every model and a load at a time 74.
 // ---------------------------------------------------------------------------------------------------
-template <typename T>
+template <typename T, int GC>
 __global__ void __launch_bounds__(128) attn_decode_kernel(AttnArgs a, float* __restrict__ part_o,
                                                           float* __restrict__ part_ml, int n_splits) {
   constexpr int VN = Vec<T>::N;
@@ -361,13 +365,21 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnArgs a, float* __r
 #pragma unroll
       for (int g = 0; g < GC; ++g) dot[g] = 0.f;
       if (valid) {
-        for (int ch = half; ch < NCH; ch += 2) {
-          float kx[VN];
-          load_vec<T>(kbase + (size_t)key_of * HD + ch * VN, kx);
+        constexpr int AT_ONCE = 8;
+#pragma unroll 1
+        for (int c0 = half; c0 < NCH; c0 += 2 * AT_ONCE) {
+          float kx[AT_ONCE][VN];
 #pragma unroll
-          for (int g = 0; g < GC; ++g)
+          for (int k = 0; k < AT_ONCE; ++k)
+            if (c0 + 2 * k < NCH) load_vec<T>(kbase + (size_t)key_of * HD + (c0 + 2 * k) * VN, kx[k]);
 #pragma unroll
-            for (int e = 0; e < VN; ++e) dot[g] = fmaf(kx[e], qs[g][ch * VN + e], dot[g]);
+          for (int k = 0; k < AT_ONCE; ++k)
+            if (c0 + 2 * k < NCH) {
+#pragma unroll
+              for (int g = 0; g < GC; ++g)
+#pragma unroll
+                for (int e = 0; e < VN; ++e) dot[g] = fmaf(kx[k][e], qs[g][(c0 + 2 * k) * VN + e], dot[g]);
+            }
         }
       }
 #pragma unroll
@@ -413,16 +425,26 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnArgs a, float* __r
 #pragma unroll
         for (int e = 0; e < VN; ++e) acc[g][e] *= alpha;
       }
-      for (int key = rg; key < BLK; key += RP) {
-        const int kpos = kb * BLK + key;
-        if (kpos < k_lo || kpos >= k_hi) continue;
-        float vx[VN];
-        load_vec<T>(vbase + (size_t)key * HD + cv * VN, vx);
+      constexpr int AT_ONCE = 8;
+      const int key_lo = max(k_lo - kb * BLK, 0), key_hi = min(k_hi - kb * BLK, BLK);  // the block's keys that are seen
+#pragma unroll 1
+      for (int key0 = rg; key0 < key_hi; key0 += AT_ONCE * RP) {
+        float vx[AT_ONCE][VN];
 #pragma unroll
-        for (int g = 0; g < GC; ++g) {
-          const float p = ss[g][key];
+        for (int k = 0; k < AT_ONCE; ++k) {
+          const int key = key0 + k * RP;
+          if (key >= key_lo && key < key_hi) load_vec<T>(vbase + (size_t)key * HD + cv * VN, vx[k]);
+        }
 #pragma unroll
-          for (int e = 0; e < VN; ++e) acc[g][e] = fmaf(p, vx[e], acc[g][e]);
+        for (int k = 0; k < AT_ONCE; ++k) {
+          const int key = key0 + k * RP;
+          if (key < key_lo || key >= key_hi) continue;
+#pragma unroll
+          for (int g = 0; g < GC; ++g) {
+            const float p = ss[g][key];
+#pragma unroll
+            for (int e = 0; e < VN; ++e) acc[g][e] = fmaf(p, vx[k][e], acc[g][e]);
+          }
         }
       }
     }
@@ -601,9 +623,13 @@ int launch_decode(const char* what, const AttnArgs& a, int dtype, int n_seqs, in
   const int group = a.nheads / a.kvheads;
   if (a.nheads > 65535) return fms_fail("%s: %d heads", what, a.nheads);
   if (dtype == FMS_F32) {
-    const int chunks = (group + GC - 1) / GC;
-    fms_launch(attn_decode_kernel<float>, dim3(n_seqs, a.kvheads * chunks, n_splits), dim3(128), 0, stream, a, part_o,
-               part_ml, n_splits);
+    if (group <= 4) {
+      fms_launch(attn_decode_kernel<float, 4>, dim3(n_seqs, a.kvheads, n_splits), dim3(128), 0, stream, a, part_o, part_ml, n_splits);
+    } else {
+      const int chunks = (group + GC_MOST - 1) / GC_MOST;
+      fms_launch(attn_decode_kernel<float, GC_MOST>, dim3(n_seqs, a.kvheads * chunks, n_splits), dim3(128), 0, stream, a, part_o,
+                 part_ml, n_splits);
+    }
     fms_launch(attn_combine_kernel<float>, dim3(n_seqs, a.nheads), dim3(HD), 0, stream, a,
                (const float*)part_o, (const float*)part_ml, n_splits, (int*)nullptr, error_flag);
   } else if (dtype == FMS_BF16) {
@@ -669,9 +695,9 @@ int launch_prefill_tc(const char* what, const CUtensorMap& map_k, const CUtensor
                       int n_tiles, int* error_flag, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+    cudaError_t e = cudaSuccess;
+    for (auto kernel : {attn_prefill_tc_kernel<false, false>, attn_prefill_tc_kernel<true, false>, attn_prefill_tc_kernel<false, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
     if (e != cudaSuccess) return fms_fail("%s: shared memory of %zu bytes refused: %s", what, TC_SMEM, cudaGetErrorString(e));
     configured = true;
   }
@@ -679,8 +705,9 @@ int launch_prefill_tc(const char* what, const CUtensorMap& map_k, const CUtensor
   const int gh = tc_heads_per_block(group);
   const long blocks = (long)n_tiles * a.kvheads * ((group + gh - 1) / gh);
   if (blocks > 0x7fffffffL) return fms_fail("%s: %ld thread blocks", what, blocks);
-  fms_launch(a.distance ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>, dim3((unsigned)blocks), dim3(192), TC_SMEM, stream,
-             map_k, map_v, a, tiles, n_tiles, error_flag);
+  fms_launch(a.key_base ? attn_prefill_tc_kernel<false, true>
+                        : (a.distance ? attn_prefill_tc_kernel<true, false> : attn_prefill_tc_kernel<false, false>),
+             dim3((unsigned)blocks), dim3(192), TC_SMEM, stream, map_k, map_v, a, tiles, n_tiles, error_flag);
   return fms_launch_status(what);
 }
 #endif

@@ -50,8 +50,10 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __host__ __device__ inline int tc_heads_per_block(int group) { return group < TC_ROWS ? group : TC_ROWS; }
 __host__ __device__ inline int tc_positions_per_block(int group) { return TC_ROWS / tc_heads_per_block(group); }
 
-// DISTANCE: the kernel for calls with a distance term (the others have neither its table nor its registers)
-template <bool DISTANCE>
+// DISTANCE: the kernel for calls with a distance term (the others have neither its table nor its registers).  ROWS: keys and
+// values are rows of a matrix (AttnArgs::key_base); a kernel of its own, since the choice made in one cost calls over the
+// cache 0.6% (a layer of 2,048 tokens 204 instead of 203 us)
+template <bool DISTANCE, bool ROWS>
 __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                  const __grid_constant__ CUtensorMap map_v, AttnArgs a,
                                                                  const int* __restrict__ tiles, int n_tiles,
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
   const int n_new = a.first_row[seq + 1] - row_begin;
   const int len = a.len_after[seq];
   const int len_before = len - n_new;
-  const int slot = a.key_base ? 0 : a.slots[seq];
+  const int slot = ROWS ? 0 : a.slots[seq];
   const int pos_here = min(pp, n_new - r0);
   const int p_first = len_before + r0, p_last = p_first + pos_here - 1;
   const int kb_lo = first_visible(a, p_first) / BLK;
@@ -127,12 +129,12 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
     if (elect_one()) {
       for (int i = 0; i < nblocks && !*failed; ++i) {
         const int s = i % TC_STAGES;
-        const int blk = a.key_base ? 0 : block_of(a, slot, kb_lo + i);
+        const int blk = ROWS ? 0 : block_of(a, slot, kb_lo + i);
         unsigned char* kdst = kv + (size_t)s * 2 * TC_KV_TILE;
         unsigned char* vdst = kdst + TC_KV_TILE;
         // first row and column of the block in the [positions, HD] view of the cache, or in the matrix
-        const int row = a.key_base ? a.key_base[seq] + (kb_lo + i) * BLK : (max(blk, 0) * a.kvheads + kvh) * BLK;
-        const int col = a.key_base ? kvh * a.kv_cols : 0;
+        const int row = ROWS ? a.key_base[seq] + (kb_lo + i) * BLK : (max(blk, 0) * a.kvheads + kvh) * BLK;
+        const int col = ROWS ? kvh * a.kv_cols : 0;
         if (!wait_or_abort(&k_empty[s], ((i / TC_STAGES) & 1) ^ 1, failed)) break;
         mbar_arrive_expect_tx(&k_full[s], TC_KV_TILE);
 #pragma unroll
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
     bool ok = true;
     for (int i = 0; i < nblocks && ok; ++i) {
       const int kb = kb_lo + i, s = i % TC_STAGES;
-      const int blk = a.key_base ? 0 : block_of(a, slot, kb);  // asked for here: it is needed after the exponentials
+      const int blk = ROWS ? 0 : block_of(a, slot, kb);  // asked for here: it is needed after the exponentials
       if (tabled) {  // while the scores are on their way; distances of keys after a row count as 0 (they are masked)
         __syncwarp();
         float away[3];  // the distances of this lane's entries, at most 96 a head
@@ -322,11 +324,15 @@ __global__ void __launch_bounds__(192, 2) attn_prefill_tc_kernel(const __grid_co
       tc_fence_after();
       if (a.sink != nullptr && row_ok) l += exp2f(a.sink[kvh * group + g0 + gi] * LOG2E - (m_ref == -INFINITY ? 0.f : m_ref));
       float inv = l > 0.f ? 1.f / l : 0.f;
-      if (a.gate != nullptr && row_ok)
-        inv /= 1.f + __expf(-__bfloat162float(a.gate[(size_t)(row_begin + r0 + pi) * a.gate_stride + kvh * group + g0 + gi]));
-      __nv_bfloat16* o_row = (__nv_bfloat16*)a.out +
-                             (size_t)(row_begin + r0 + (row_ok ? pi : 0)) * (a.key_base ? a.out_stride : (long)a.nheads * HD) +
-                             (size_t)(kvh * group + g0 + (row_ok ? gi : 0)) * HD;
+      if (ROWS && a.gate != nullptr && row_ok)
+        inv *= 1.f / (1.f + expf(-__bfloat162float(a.gate[(size_t)(row_begin + r0 + pi) * a.gate_stride + kvh * group + g0 + gi])));
+      __nv_bfloat16* o_row;
+      if (ROWS)
+        o_row = (__nv_bfloat16*)a.out + (size_t)(row_begin + r0 + (row_ok ? pi : 0)) * a.out_stride +
+                (size_t)(kvh * group + g0 + (row_ok ? gi : 0)) * HD;
+      else
+        o_row = (__nv_bfloat16*)a.out +
+                ((size_t)(row_begin + r0 + (row_ok ? pi : 0)) * a.nheads + kvh * group + g0 + (row_ok ? gi : 0)) * HD;
 #pragma unroll
       for (int c0 = 0; c0 < HD; c0 += 32) {
         float o[32];
