@@ -945,14 +945,14 @@ def chunk_scan_pays(batch, heads: int, vdim: int, least: Optional[int] = None) -
     return longest >= (CHUNK_SCAN_FROM if least is None else least) and (vdim > 64 or CHUNK_SCAN_SHARE * longest >= sum(batch.num_new))
 
 
-def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, rows: torch.Tensor, state: torch.Tensor,
+def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, rows: torch.Tensor,
                      least: Optional[int] = None):
-    """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, rows or states
+    """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, rows
     that do not lie on 16 bytes, decode steps and short prompts (which go token by token), a capture that has not seen the batch
     before (the runs come from the host)."""
     if batch.decode or not batch.num_new or not chunk_scan_pays(batch, heads, vdim, least):
         return None
-    if (_ptr(rows) | _ptr(state)) & 15 or rows.shape[1] % 4 or batch.n_seqs > 65535:
+    if _ptr(rows) & 15 or rows.shape[1] % 4 or batch.n_seqs > 65535:
         return None
     lib = load_library("chunk_scan")
     if not lib.fms_chunk_scan_takes(int(dim), int(vdim), heads // key_heads):
@@ -994,7 +994,7 @@ def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bia
             or tuple(state.shape[1:]) != (heads, vdim, n_state):
         raise KernelError("selective_scan: xbc float32 [tokens, x | B | C], state float32 [slots, heads, vdim, state]")
     y = torch.empty((n, heads * vdim), dtype=torch.float32, device=xbc.device)
-    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups, xbc, state)
+    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups, xbc)
     if plan is not None:
         x, b = _ptr(xbc), _ptr(xbc) + heads * vdim * 4
         _chunk_scan(2, b + groups * n_state * 4, b, x, xbc.shape[1], plan, batch, state, y, heads, groups, n_state, vdim, writes_state,
@@ -1031,7 +1031,7 @@ def delta_rule_scan(qkv: torch.Tensor, proj: torch.Tensor, beta_offset: int, a_r
             raise KernelError("delta_rule_scan: decays' logits [tokens, heads * dim] in the projection's dtype")
         a_ptr, a_stride = _ptr(a_raw), heads * dim
     o = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, kvheads, qkv, state, DELTA_CHUNKS_FROM) if per_head and vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, kvheads, qkv, DELTA_CHUNKS_FROM) if per_head and vdim == 128 else None
     if plan is not None:
         decay, beta = (torch.empty((n, heads), dtype=torch.float32, device=qkv.device) for _ in range(2))
         _call("state_scan", "fms_delta_prepare", qkv, _ptr(proj) + beta_offset * proj.element_size(), _code(proj.dtype), proj.shape[1],
@@ -1161,7 +1161,7 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
     norm_in = torch.empty((batch.n_seqs, heads, dim), dtype=torch.float32, device=proj.device) if gated else None
     gate_ptr = _ptr(proj) + gate_offset * proj.element_size() if gated else None
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv, state) if not gated or vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv) if not gated or vdim == 128 else None
     if plan is not None:
         if gated:
             _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias, float(gate_cap),
