@@ -65,7 +65,9 @@ template <int CPT> __device__ __forceinline__ void load_channels(const __nv_bflo
 
 // A thread takes CPT consecutive channels of `groups` times CONV_TOKENS consecutive rows; TMAX bounds the taps (4 or MAX_TAPS), and
 // EXACT: the taps are TMAX.  Bound by the bytes of x and out.  Several groups of rows share the taps and the rows between them, and
-// where all rows lie inside one sequence, as nearly all do, nothing is looked up a token.
+// where all rows lie inside one sequence, as nearly all do, nothing is looked up a token.  Measured (2,048 rows of 10,240 channels in
+// bfloat16, 4 taps, 126 MB): 50 us, 2.5 TB/s; 97 with a look-up a token and the taps a variable; 109 with the rows in
+// registers picked by selects.
 template <typename T, int CPT, int TMAX, bool EXACT>
 __global__ void __launch_bounds__(CONV_THREADS) causal_conv_kernel(const T* x, int stride, const float* w, const float* bias,
                                                                    const float* tail, const int* token_seq,
@@ -170,7 +172,8 @@ __global__ void __launch_bounds__(CONV_THREADS) causal_conv_kernel(const T* x, i
 }
 
 // A decode step: one row a sequence.  The thread that makes a channel's value also leaves its tail, so that one kernel does what a
-// prompt's two do (the tail of a prompt is read by other blocks than the one that could write it).
+// prompt's two do (the tail of a prompt is read by other blocks than the one that could write it).  Bound by its launch: 3.7 us
+// for four sequences of 6,144 channels; the two 6.4.
 template <typename T, int CPT, int TMAX>
 __global__ void __launch_bounds__(CONV_THREADS) causal_conv_decode_kernel(const T* x, int stride, const float* w, const float* bias,
                                                                           float* tail, const int* token_seq, const int* slots, float* out,
@@ -637,7 +640,7 @@ __global__ void linear_prepare_kernel(const T* proj, int stride, float* out, int
 // where every block of the scan reads it (the scan's blocks do not all run at once, and one of them writes the new n
 // into norm_state).  A thread a token for the gates and the exponentials, as many tokens at a time as the block has threads, the
 // next ones on their way meanwhile; only the walk over the maxima, an addition and a comparison a token, is one thread's.  (With
-// a warp for all three, 1,700 tokens of two sequences took 67 us.)
+// a warp for all three, 1,700 tokens of two sequences took 67 us; so 19.)
 constexpr int GATE_THREADS = 256;
 
 template <typename T>
