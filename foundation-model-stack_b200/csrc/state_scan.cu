@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(CONV_THREADS) causal_conv_kernel(const T* x, i
 
 // A decode step: one row a sequence.  The thread that makes a channel's value also leaves its tail, so that one kernel does what a
 // prompt's two do (the tail of a prompt is read by other blocks than the one that could write it).  Bound by its launch: 3.7 us
-// for four sequences of 6,144 channels; the two 6.4.
+// for four sequences of 6,144 channels.
 template <typename T, int CPT, int TMAX>
 __global__ void __launch_bounds__(CONV_THREADS) causal_conv_decode_kernel(const T* x, int stride, const float* w, const float* bias,
                                                                           float* tail, const int* token_seq, const int* slots, float* out,

@@ -1225,7 +1225,7 @@ def grouped_linear(x: torch.Tensor, weight: torch.Tensor, groups: int, rows: int
     if x.dtype == torch.bfloat16 and rows <= SKINNY_ROWS and k % 8 == 0 and x_row_stride % 8 == 0 and x_group_offset % 8 == 0 \
             and (_ptr(x) | _ptr(weight)) % 16 == 0 and groups <= 65535:
         # a decode step of few rows: the weight-streaming kernel, a block per group and run of its matrix's rows (8 rows, 32
-        # groups of 512 x 96: 4.7 us, of 128 x 512: 3.5; 18 each with a warp a row of the matrix)
+        # groups of 512 x 96: 4.7 us, of 128 x 512: 3.5; the two 27 with a warp a row of the matrix)
         _call("gemm_bf16_skinny", "fms_strided_bf16_skinny", x, weight, y, rows, groups, n_out, k, x_row_stride,
               x_group_offset, y_row_stride, y_group_offset, _stream())
         return y
