@@ -72,7 +72,7 @@ static_assert(2 * BK * (BM + 4 + BN + 4) <= BM * BN, "operands");
 
 __global__ void __launch_bounds__(TILE_THREADS, 4)
     gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                         float* __restrict__ y, int M, int N, int K, int run_len, int ranks) {
+                         float* __restrict__ y, int M, int N, int K, int run_len, int ranks, int vec) {
   constexpr int THREADS = TILE_THREADS, LDX = BM + 4, LDW = BN + 4, NX = BM * 4 / THREADS, NW = BN * 4 / THREADS;
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;                 // [2][BK][LDX]
@@ -83,7 +83,6 @@ __global__ void __launch_bounds__(TILE_THREADS, 4)
   const int tiles_m = (M + BM - 1) / BM;
   const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
   const int tm = (warp / (BN / 64)) * (4 * TM) + (lane >> 3) * 4, tn = (warp % (BN / 64)) * 64 + (lane & 7) * 4;
-  const bool vec = (K % 4) == 0;
   const int k_begin = min(rank * run_len, K), k_end = min(k_begin + run_len, K);
 
   float4 px[NX], pw[NW];
@@ -231,7 +230,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4)
   cluster.sync();  // nobody leaves while its sums are still read
 }
 
-int launch_tiles(const float* x, const float* w, const float* bias, float* y, int M, int N, int K, cudaStream_t stream) {
+int launch_tiles(const float* x, const float* w, const float* bias, float* y, int M, int N, int K, int vec, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM);
@@ -240,7 +239,7 @@ int launch_tiles(const float* x, const float* w, const float* bias, float* y, in
   }
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   return launch_clusters(gemm_f32_tile_kernel, tiles, ranks_for(K), TILE_THREADS, TILE_SMEM, stream, x, w, bias, y, M, N, K,
-                         run_length(K), ranks_for(K));
+                         run_length(K), ranks_for(K), vec);
 }
 
 // ---- few rows (a decode step): a warp a run ---------------------------------------------------------------------------
@@ -377,8 +376,10 @@ FMS_API int fms_gemm_f32(const float* x, const float* w, const float* bias, floa
                          cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return fms_fail("gemm_f32: K %d", K);
+  // 16-byte loads only where every row starts on 16 bytes; else the tiles take one value at a time, in the same order
+  const bool vec = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
   // from 33 rows on the tiles of 64 rows are the faster ones (32 rows of 28,672 x 4,096: 251 against 330 us)
-  if (M <= FEW_MAX_ROWS && K % 4 == 0) {
+  if (M <= FEW_MAX_ROWS && vec) {
     if (M <= 1) return launch_few_rows<1, 32>(x, w, bias, y, M, N, K, stream);
     if (M <= 2) return launch_few_rows<2, 16>(x, w, bias, y, M, N, K, stream);
     if (M <= 4) return launch_few_rows<4, 16>(x, w, bias, y, M, N, K, stream);
@@ -386,5 +387,5 @@ FMS_API int fms_gemm_f32(const float* x, const float* w, const float* bias, floa
     if (M <= 16) return launch_few_rows<16, 8>(x, w, bias, y, M, N, K, stream);
     return launch_few_rows<32, 8>(x, w, bias, y, M, N, K, stream);
   }
-  return launch_tiles(x, w, bias, y, M, N, K, stream);
+  return launch_tiles(x, w, bias, y, M, N, K, vec, stream);
 }

@@ -50,6 +50,18 @@ def test_rotation_of_shifted_float32_rows(rows, hd):
     assert torch.equal(results[0][2], results[1][2])  # values are only moved
 
 
+@pytest.mark.parametrize("rows,n,k", [(1, 33, 132), (8, 96, 1024), (32, 31, 4), (33, 130, 260), (70, 129, 1056)])
+def test_float32_products_of_shifted_operands(rows, n, k):
+    """Few rows and many; x, the matrix or both four bytes off.  The sums run in the same order, so they are the same bits."""
+    from fms_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(rows)
+    x, w, b = torch.randn(rows, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda(), torch.randn(n, generator=g).cuda()
+    want = ops.linear(x, w, b)
+    for a, m in ((shifted(x), w), (x, shifted(w)), (shifted(x), shifted(w))):
+        assert torch.equal(ops.linear(a, m, shifted(b)), want)
+
+
 def test_scans_of_shifted_rows(monkeypatch):
     """The walk over tokens takes them; beside the runs that the same values on 16 bytes take, as in the test of the runs."""
     from fms_b200.kernels import ops
