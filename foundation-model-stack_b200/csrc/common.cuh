@@ -125,6 +125,10 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
+// Asks for a line to be brought into the second-level cache, where all writers' data meet: allowed before pdl_wait() for
+// any address, since nothing is read.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
 #include <stdlib.h>
 static inline bool fms_pdl_enabled() {
   static int enabled = -1;

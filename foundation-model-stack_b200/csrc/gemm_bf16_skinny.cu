@@ -178,10 +178,20 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
       for (int j = 0; j < NT; ++j) cp_async16(st + (WL + j) * THREADS, xp[j] + (kok ? k0 : 0), kok && xok[j], true);
     }
   };
+  if (GROUPS == STRIDED) {  // the matrices may be what the kernel in front makes: only asked into the second-level cache
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+      for (int t = 0; t < RT; ++t)
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h)
+          if (c == 0 && i < my_chunks) prefetch_l2(wp[t][h] + (warp + i * WARPS) * 32);
+    pdl_wait();
+  }
 #pragma unroll
   for (int i = 0; i < D; ++i) issue_w(i);  // weights: before the wait for the kernel that produces x
   cp_async_commit();
-  if (GROUPS != GROUPED) pdl_wait();
+  if (GROUPS == ALONE) pdl_wait();
 #pragma unroll
   for (int i = 0; i < D; ++i) issue_x(i);
   cp_async_commit();

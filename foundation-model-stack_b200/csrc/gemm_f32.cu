@@ -247,8 +247,7 @@ int launch_tiles(const float* x, const float* w, const float* bias, float* y, in
 // columns of y), each of its blocks is one warp with one run and a ring of its own: FEW_KT k of the 32 rows and of the
 // rows of x at a time by 16-byte asynchronous copies, no barrier but the cluster's at the end.  The lanes are G by XG: a
 // lane holds 32 / G rows of w and ROWS / XG rows of x, which share each other's reads (a row of w and eight of x a lane
-// read 36 words for 32 multiply-adds, two and four 24).  Rows are padded to 36 floats: no bank conflicts.  The first
-// copies of w are asked for before the kernel in front is waited for.  Measured (8 rows, w of 28,672 x 4,096 / 4,096 x
+// read 36 words for 32 multiply-adds, two and four 24).  Rows are padded to 36 floats: no bank conflicts.  Measured (8 rows, w of 28,672 x 4,096 / 4,096 x
 // 14,336, L2 flushed): 114 / 71 us (4.1 / 3.3 TB/s); all runs in one block of eight warps 131 / 72; one chain over K, where a
 // thread walks a row of w for two or four rows of x, as here before, 138 / 138.
 constexpr int FEW_MAX_ROWS = 32, FEW_WROWS = 32, FEW_KT = 32, FEW_STRIDE = FEW_KT + 4;
@@ -299,12 +298,16 @@ __global__ void __launch_bounds__(32) gemm_f32_few_rows_kernel(const float* __re
   for (int i = 0; i < XR; ++i)
 #pragma unroll
     for (int j = 0; j < R; ++j) acc[i][j] = 0.f;
+  // w may be what the kernel in front makes: before the wait it is only asked into the second-level cache
   for (int s = 0; s < STAGES - 1; ++s)
-    if (s < steps) issue_w(s);
+    if (s < steps) prefetch_l2(w + (size_t)min(n0 + lane, N - 1) * K + k_begin + s * FEW_KT);
   pdl_launch_dependents();
   pdl_wait();
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < steps) issue_x(s);
+    if (s < steps) {
+      issue_w(s);
+      issue_x(s);
+    }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
   for (int step = 0; step < steps; ++step) {

@@ -476,3 +476,22 @@ def test_a_product_a_group_of_few_rows(rows, groups, n_out, k):
     got = y[:, : groups * n_out].view(rows, groups, n_out).transpose(0, 1).double()
     bound = 2.0 ** -8 * want.abs() + (k + 8) * 2.0 ** -24 * torch.einsum("grk,gnk->grn", xs.abs(), w.double().abs())
     assert bool(((got - want).abs() <= bound).all()) and bool((y[:, groups * n_out:] == 7.0).all())
+
+
+def test_a_product_a_group_takes_matrices_that_the_product_before_it_made():
+    """The weight-streaming kernel over strided groups may start while the kernel in front still writes its matrices."""
+    from fms_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(3)
+    groups, n_out, k, rows = 16, 512, 512, 8
+    a, b, x = (torch.randn(*s, generator=g).to(torch.bfloat16).cuda() for s in ((8, 256), (groups * n_out * k // 8, 256), (rows, groups * k)))
+    y = torch.empty(rows, groups * n_out, dtype=torch.bfloat16).cuda()
+    made = lambda: ops.linear(a, b).view(groups, n_out, k)  # noqa: E731
+    product = lambda w: ops.grouped_linear(x, w, groups, rows, n_out, k, groups * k, k, y, groups * n_out, n_out)  # noqa: E731
+    w = made()
+    torch.cuda.synchronize()
+    want = product(w).clone()
+    for _ in range(20):
+        a.neg_()
+        want.neg_()
+        assert torch.equal(product(made()), want)

@@ -81,6 +81,22 @@ def test_gated_activation(ops, dtype, act):
     torch.testing.assert_close(got.float(), want, **tol(dtype))
 
 
+@pytest.mark.parametrize("m", [1, 8, 32])
+def test_a_float32_product_takes_a_matrix_that_the_product_before_it_made(ops, m):
+    """The few-rows kernel may start while the kernel in front still writes: it must not have read the matrix by then.
+    The same bits as after that kernel is over."""
+    g = torch.Generator().manual_seed(33)
+    a, b, x = (torch.randn(*s, generator=g).cuda() for s in ((2048, 1024), (1024, 1024), (m, 1024)))
+    w = ops.linear(a, b)
+    torch.cuda.synchronize()
+    want = ops.linear(x, w)
+    for _ in range(20):
+        a.mul_(-1.0)
+        got = ops.linear(x, ops.linear(a, b))
+        want.neg_()
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 331, 240), (5, 64, 17), (70, 130, 328), (129, 257, 1000)])
 @pytest.mark.parametrize("bias", [False, True])
 def test_linear_float32_is_true_float32(ops, m, n, k, bias):
