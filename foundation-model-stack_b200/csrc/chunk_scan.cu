@@ -34,18 +34,22 @@
 //
 // and chunk_outputs takes U for the values (b = 1).
 //
-// Sums are made of runs of 16 terms and products of decays in 64 bits, so that a state's error stays below the walk's (2,048
-// tokens under fixed decays: 1.1e-7 of its size against 2.6e-7; in chains of 128 and float32 products 5.5e-7) and an output's
-// beside it (9.5e-8 against 8.2e-8).  Measured alone: prompts of 1,062 and 638 tokens,
-// 32 heads of 128 with a normalizer, scores 31, states 94, outputs 99 us; one of 2,048, 128 heads of 64, 32, 166 and 179.
+// So that neither an output nor a state is further from 64 bits than the walk's: scores (and k . k) are summed in 64 bits and
+// rounded once, as products of decays are; an output's sums over channels and tokens are made of float32 runs of 16 terms that
+// 64 bits add up; u's of float32 runs of 16 terms.  A run's part of the state and of the normalizer is one float32 chain of its
+// 64 tokens.  Errors of outputs and of states as parts of the walk's (400 and 2,048 tokens): fixed decays 0.77 and 0.94, 0.46 and
+// 0.41; under a normalizer 0.88 and 0.83, 0.96 and 0.98; state space 0.95 and 0.96, 0.85 and 0.80; delta rule 0.97 and 0.86, 0.87 and
+// 0.77.  (With float32 sums throughout, outputs 1.05 to 1.15 of it and layers 7 to 10% faster: prompts of 1,062 and 638 tokens,
+// 32 heads of 128 with a normalizer, 498 instead of 550 us; one of 2,048, 128 heads of 64, 779 instead of 856.)
 #include "common.cuh"
 
 namespace {
 constexpr int C = 64;        // tokens of a run
 constexpr int COLS = 128;    // value columns of a block of outputs: one head of 128 values or two of 64
 constexpr int DIM = 128;     // key channels
-constexpr int PART = 16;     // terms that a sum takes together before they are added to the rest: a single chain loses more
-constexpr int SLICE = 32, SROW = SLICE + 4;  // of the scores: channels brought into shared memory at a time
+constexpr int PART = 16;     // terms of an output that float32 takes together before 64 bits add them to the rest
+constexpr int UPART = 16;    // terms of a delta rule's u that are taken together before they are added to the rest
+constexpr int SLICE = 16, SROW = SLICE + 2;  // of the scores: channels brought into shared memory at a time, rows padded by two
 constexpr int TROW = C + 4, CROW = COLS + 4; // rows of 64 tokens, of 128 columns, padded by four floats
 
 struct ChunkArgs {
@@ -165,25 +169,73 @@ __device__ __forceinline__ float2 token_gates(const ChunkArgs& g, int t, int end
   return make_float2((float)exp(-exp((double)g.a_log[head]) * dt), (float)dt);
 }
 
-// ---- scores: 64 x 64 a block, 8 x 4 a thread; the factors of the key head's heads, a warp a head ----------------------------
+// ---- products of 64 x 64 tokens of a run: sum[i][j] = x_t . y_s over all channels, t = tid / 16 * 8 + i, s = tid % 16 + 16 j ------
+// In 64 bits, rounded once: an output is a sum of few of them where decays are short, and with float32 sums of 16 terms (7e-8 of
+// a score's size, once rounded 2.5e-8) it was up to 20% further from 64 bits than the walk's.  Half the FMA pipe's rate, but a
+// twentieth of the scan's products.  A slice's values are widened on their way from registers to shared memory, the next slice's
+// loads are on their way meanwhile.  SAME: y is x.  sm: [2][SAME ? 1 : 2][C][SROW].
+template <bool SAME>
+__device__ __forceinline__ void run_products(const float* x, const float* y, long row, int rows, double* sm, double (&sum)[8][4]) {
+  constexpr int OPERANDS = SAME ? 1 : 2;
+  const int tid = threadIdx.x, t0 = tid >> 2, d0 = (tid & 3) * 4;  // of a slice: rows t0 and t0 + 32, channels d0 .. + 3
+  float4 next[OPERANDS][2];
+  auto fetch = [&](int d) {
+#pragma unroll
+    for (int o = 0; o < OPERANDS; ++o)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = t0 + 32 * h;
+        next[o][h] = t < rows ? *reinterpret_cast<const float4*>((o ? y : x) + (size_t)t * row + d + d0) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int o = 0; o < OPERANDS; ++o)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        double2* p = reinterpret_cast<double2*>(sm + ((buf * OPERANDS + o) * C + t0 + 32 * h) * SROW + d0);
+        p[0] = make_double2(next[o][h].x, next[o][h].y);
+        p[1] = make_double2(next[o][h].z, next[o][h].w);
+      }
+  };
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[i][j] = 0.0;
+  const int ty = tid >> 4, tx = tid & 15;
+  fetch(0);
+  put(0);
+  __syncthreads();
+#pragma unroll 1
+  for (int d = 0; d < DIM; d += SLICE) {
+    const int buf = (d / SLICE) & 1;
+    if (d + SLICE < DIM) fetch(d + SLICE);
+    const double* xs = sm + (buf * OPERANDS * C + ty * 8) * SROW;
+    const double* ys = sm + ((buf * OPERANDS + OPERANDS - 1) * C + tx) * SROW;
+#pragma unroll
+    for (int e = 0; e < SLICE; e += 2) {
+      double2 b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const double2*>(ys + 16 * j * SROW + e);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const double2 a = *reinterpret_cast<const double2*>(xs + i * SROW + e);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[i][j] = fma(a.y, b[j].y, fma(a.x, b[j].x, sum[i][j]));
+      }
+    }
+    if (d + SLICE < DIM) put(buf ^ 1);
+    __syncthreads();
+  }
+}
+
+// ---- scores: a block a run and key head; the factors of the key head's heads, a warp a head ----------------------------
 template <int KIND>
 __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
-  __shared__ __align__(16) float sm[2][2][C][SROW];
+  __shared__ __align__(16) double sm[2 * 2 * C * SROW];
   pdl_wait();
   const int run = g.run_lo + blockIdx.x, kh = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
   const int row0 = g.runs[2 * run], end = g.runs[2 * run + 1], rows = end - row0;
-  const float* q = g.q + (size_t)row0 * g.row + (size_t)kh * DIM;
-  const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
-  auto issue = [&](int d0, int buf) {
-    for (int i = tid; i < C * (SLICE / 4); i += 128) {
-      const int t = i / (SLICE / 4), d = (i % (SLICE / 4)) * 4;
-      const size_t at = (size_t)min(t, rows - 1) * g.row + d0 + d;
-      copy16(&sm[buf][0][t][d], q + at, t < rows);
-      copy16(&sm[buf][1][t][d], k + at, t < rows);
-    }
-    copies_commit();
-  };
-  issue(0, 0);
   const int shared = g.heads / g.key_heads;
   for (int head = kh * shared + (tid >> 5); head < (kh + 1) * shared; head += 4) {  // a lane two neighbouring tokens
     const float2 w0 = token_gates<KIND>(g, row0 + 2 * lane, end, head), w1 = token_gates<KIND>(g, row0 + 2 * lane + 1, end, head);
@@ -210,54 +262,8 @@ __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
     }
   }
   const int ty = tid >> 4, tx = tid & 15;  // tokens t = ty * 8 + i, s = tx + 16 j
-  float sum[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) sum[i][j] = 0.f;
-#pragma unroll 1
-  for (int d0 = 0; d0 < DIM; d0 += SLICE) {
-    const int buf = (d0 / SLICE) & 1;
-    if (d0 + SLICE < DIM) {
-      issue(d0 + SLICE, buf ^ 1);
-      copies_wait<1>();
-    } else {
-      copies_wait<0>();
-    }
-    __syncthreads();
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-#pragma unroll
-    for (int d = 0; d < SLICE; d += 4) {
-      float4 kx[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) kx[j] = *reinterpret_cast<const float4*>(&sm[buf][1][tx + 16 * j][d]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 qx = *reinterpret_cast<const float4*>(&sm[buf][0][ty * 8 + i][d]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(qx.x, kx[j].x, acc[i][j]);
-          acc[i][j] = fmaf(qx.y, kx[j].y, acc[i][j]);
-          acc[i][j] = fmaf(qx.z, kx[j].z, acc[i][j]);
-          acc[i][j] = fmaf(qx.w, kx[j].w, acc[i][j]);
-        }
-      }
-      if ((d + 4) % PART == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            sum[i][j] += acc[i][j];
-            acc[i][j] = 0.f;
-          }
-      }
-    }
-    __syncthreads();
-  }
+  double sum[8][4];
+  run_products<false>(g.q + (size_t)row0 * g.row + (size_t)kh * DIM, g.k + (size_t)row0 * g.row + (size_t)kh * DIM, g.row, rows, sm, sum);
   // only now: blocks of the states' kernel that come earlier gather on the multiprocessors that are free first, two together
   // where every one could have its own (a layer of two prompts, 1,062 and 638 tokens: 498 instead of 552 us)
   pdl_launch_dependents();
@@ -266,7 +272,8 @@ __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
   for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int i = 0; i < 8; i += 4)
-      *reinterpret_cast<float4*>(out + (tx + 16 * j) * C + ty * 8 + i) = make_float4(sum[i][j], sum[i + 1][j], sum[i + 2][j], sum[i + 3][j]);
+      *reinterpret_cast<float4*>(out + (tx + 16 * j) * C + ty * 8 + i) =
+          make_float4((float)sum[i][j], (float)sum[i + 1][j], (float)sum[i + 2][j], (float)sum[i + 3][j]);
 }
 
 // ---- the states before every run: 128 key channels x VT value columns a block, 8 x VT / 8 a thread ------------------------
@@ -392,6 +399,7 @@ __global__ void __launch_bounds__(128, 2) chunk_states_kernel(ChunkArgs g) {
 }
 
 // ---- outputs: 64 tokens x 128 value columns a block, 8 x 8 a thread ---------------------------------------------------
+// Bound by the FMA pipe and by registers: 64 sums in 64 bits beside 64 of a run of terms leave two blocks a multiprocessor.
 // First q against the state before the run, 16 channels at a time (q transposed on its way through registers, the state by
 // asynchronous copies), then the run's own tokens: P^T, a thread a token t walking s downwards.  A warp's 64 columns belong to one
 // head; it takes the tokens up to its last row, earlier rows with zeros of P (or, where a value is not finite, by selection).
@@ -402,7 +410,7 @@ static_assert(OSLICE == PART);
 static_assert(2 * OSLICE * (TROW + CROW) <= C * CROW, "the slices lie where the values go afterwards");
 
 template <int VDIM, int KIND>
-__global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
+__global__ void __launch_bounds__(128, 2) chunk_outputs_kernel(ChunkArgs g) {
   constexpr int HB = COLS / VDIM;
   extern __shared__ __align__(16) float sm[];
   float* qs = sm;                                 // [2][OSLICE][TROW], then the values [C][CROW] over both
@@ -452,7 +460,7 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
   }
   put_q(0);
   __syncthreads();
-  float p_sum = 0.f;
+  double p_sum = 0.0;
   if (tid < HB * C) {  // P^T[s][t] = b_s a_(s+1) .. a_t (q_t . k_s)
     const int h = tid / C, t = tid % C;
     const float* raw = g.scores + ((size_t)local * g.key_heads + kh) * C * C + t;
@@ -461,7 +469,7 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
 #pragma unroll 8
     for (int s = C - 1; s >= 0; --s) {
       const float x = raw[s * C];
-      const float w = s <= t ? x * (float)(e * bs[h][s]) : 0.f;
+      const float w = s <= t ? (float)(x * (e * bs[h][s])) : 0.f;
       if (s <= t) e *= as[h][s];
       p[s * TROW] = w;
       p_sum += w;
@@ -469,21 +477,29 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
   }
   const int tm = (warp >> 1) * 32 + (lane >> 3) * 4, tn = (warp & 1) * 64 + (lane & 7) * 4;
   const int my_head = (warp & 1) * 64 / VDIM;  // of the block's
-  f32x2 acc2[4][8], part[4][8];
+  f32x2 part[4][8];
+  double acc[8][8];
   auto add_part = [&]() {
+    float own[8][8];
+    outer_unpack<4>(part, own);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] += (double)own[i][j];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        acc2[i][j] = add2(acc2[i][j], part[i][j]);
-        part[i][j] = 0;
-      }
+      for (int j = 0; j < 8; ++j) part[i][j] = 0;
   };
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc2[i][j] = part[i][j] = 0;
-  float own_nq = 0.f;  // KIND 1, threads 0..63: q_t . n
+    for (int j = 0; j < 8; ++j) part[i][j] = 0;
+  double own_nq = 0.0;  // KIND 1, threads 0..63: q_t . n
   const float* n_before = KIND == 1 ? g.norms + ((size_t)local * g.heads + head0) * DIM : nullptr;
 #pragma unroll 1
   for (int d0 = 0; d0 < DIM; d0 += OSLICE) {
@@ -502,7 +518,7 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
     add_part();
     if (KIND == 1 && tid < C) {
 #pragma unroll
-      for (int d = 0; d < OSLICE; ++d) own_nq = fmaf(x[d * TROW + tid], n_before[d0 + d], own_nq);
+      for (int d = 0; d < OSLICE; ++d) own_nq = fma((double)x[d * TROW + tid], (double)n_before[d0 + d], own_nq);
     }
     if (more) put_q(buf ^ 1);
   }
@@ -514,18 +530,17 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
   copies_commit();
   // G_t times what the state gives
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float g0 = G[my_head][tm + (i >> 1) * 16 + (i & 1) * 2], g1 = G[my_head][tm + (i >> 1) * 16 + (i & 1) * 2 + 1];
+  for (int i = 0; i < 8; ++i) {
+    const double gt = G[my_head][tm + (i >> 2) * 16 + (i & 3)];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc2[i][j] = fma2(acc2[i][j], pack2(g0, g1), 0ull);
+    for (int j = 0; j < 8; ++j) acc[i][j] *= gt;
   }
-  if (KIND == 1 && tid < C) nq[tid] = fmaf(G[0][tid], own_nq, p_sum);  // n_t . q_t
+  if (KIND == 1 && tid < C) nq[tid] = (float)fma((double)G[0][tid], own_nq, p_sum);  // n_t . q_t
   const bool bad = g.flags[(size_t)local * g.heads + head0 + my_head] != 0;
   copies_wait<0>();
   __syncthreads();
   const float* p = Pt + my_head * C * TROW + tm;
   const int reach = (warp >> 1) * 32 + 32;
-  float acc[8][8];
   if (!bad) {
 #pragma unroll 1
     for (int s0 = 0; s0 < reach; s0 += PART) {
@@ -533,15 +548,14 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
       for (int s = s0; s < s0 + PART; ++s) outer_step<4, 16, 32>(p + s * TROW, sm + s * CROW + tn, part);
       add_part();
     }
-    outer_unpack<4>(acc2, acc);
   } else {
-    outer_unpack<4>(acc2, acc);
     for (int s = 0; s < reach; ++s)
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         if (s <= tm + (i & 3) + (i >> 2) * 16) {
+          const double w = p[s * TROW + (i & 3) + (i >> 2) * 16];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(p[s * TROW + (i & 3) + (i >> 2) * 16], sm[s * CROW + tn + (j & 3) + (j >> 2) * 32], acc[i][j]);
+          for (int j = 0; j < 8; ++j) acc[i][j] = fma(w, (double)sm[s * CROW + tn + (j & 3) + (j >> 2) * 32], acc[i][j]);
         }
   }
 #pragma unroll
@@ -554,7 +568,7 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
     float* out = g.o + (size_t)(row0 + t) * g.heads * VDIM + (size_t)head0 * VDIM + tn;
 #pragma unroll
     for (int j = 0; j < 8; j += 4) {
-      float4 x = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+      float4 x = make_float4((float)acc[i][j], (float)acc[i][j + 1], (float)acc[i][j + 2], (float)acc[i][j + 3]);
       if (KIND == 1) x = make_float4(x.x * scale, x.y * scale, x.z * scale, x.w * scale);
       if (KIND == 2) {
         const float4 v = *reinterpret_cast<const float4*>(sm + t * CROW + tn + (j >> 2) * 32);
@@ -566,91 +580,37 @@ __global__ void __launch_bounds__(128, 3) chunk_outputs_kernel(ChunkArgs g) {
 }
 
 // ---- the delta rule's triangles: a block a run and head -----------------------------------------------------------------
-// k . k^T as the scores (8 x 4 a thread), then the inverse of the 64 x 64 triangle by blocks of 16: the diagonal ones by substitution,
+// k . k^T as the scores, then the inverse of the 64 x 64 triangle by blocks of 16: the diagonal ones by substitution,
 // a thread a column; those below, diagonal by diagonal, T_ij = -T_ii sum_(j <= m < i) A_im T_mj.  A row takes no term of a later one.
 __global__ void __launch_bounds__(128) chunk_solve_kernel(ChunkArgs g) {
-  __shared__ __align__(16) float sm[2][C][SROW];  // slices of k, then T over them
+  __shared__ __align__(16) double sm[2 * C * SROW];  // slices of k, then T over them
   __shared__ float A[C][C + 1], W[3][16][16], as[C], bt[C];
   constexpr int TP = C + 1;
-  static_assert(C * TP <= 2 * C * SROW, "T lies where the slices were");
-  float* T = &sm[0][0][0];
+  static_assert(C * TP <= 2 * 2 * C * SROW, "T lies where the slices were");
+  float* T = reinterpret_cast<float*>(sm);
   pdl_wait();
   const int local = blockIdx.x, run = g.run_lo + local, head = blockIdx.y, kh = head / (g.heads / g.key_heads), tid = threadIdx.x;
   const int row0 = g.runs[2 * run], end = g.runs[2 * run + 1], rows = end - row0;
-  const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
-  auto issue = [&](int d0, int buf) {
-    for (int i = tid; i < C * (SLICE / 4); i += 128) {
-      const int t = i / (SLICE / 4), d = (i % (SLICE / 4)) * 4;
-      copy16(&sm[buf][t][d], k + (size_t)min(t, rows - 1) * g.row + d0 + d, t < rows);
-    }
-    copies_commit();
-  };
-  issue(0, 0);
   if (tid < C) {
     const size_t at = (size_t)(row0 + tid) * g.heads + head;
     as[tid] = tid < rows ? g.decay[at] : 1.f;
     bt[tid] = tid < rows ? g.gates[at] : 0.f;
   }
   const int ty = tid >> 4, tx = tid & 15;  // rows t = ty * 8 + i, columns s = tx + 16 j
-  float sum[8][4];
+  double sum[8][4];
+  const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
+  run_products<true>(k, k, g.row, rows, sm, sum);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sum[i][j] = 0.f;
-#pragma unroll 1
-  for (int d0 = 0; d0 < DIM; d0 += SLICE) {
-    const int buf = (d0 / SLICE) & 1;
-    if (d0 + SLICE < DIM) {
-      issue(d0 + SLICE, buf ^ 1);
-      copies_wait<1>();
-    } else {
-      copies_wait<0>();
-    }
-    __syncthreads();
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-#pragma unroll
-    for (int d = 0; d < SLICE; d += 4) {
-      float4 kx[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) kx[j] = *reinterpret_cast<const float4*>(&sm[buf][tx + 16 * j][d]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 qx = *reinterpret_cast<const float4*>(&sm[buf][ty * 8 + i][d]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(qx.x, kx[j].x, acc[i][j]);
-          acc[i][j] = fmaf(qx.y, kx[j].y, acc[i][j]);
-          acc[i][j] = fmaf(qx.z, kx[j].z, acc[i][j]);
-          acc[i][j] = fmaf(qx.w, kx[j].w, acc[i][j]);
-        }
-      }
-      if ((d + 4) % PART == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            sum[i][j] += acc[i][j];
-            acc[i][j] = 0.f;
-          }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) A[ty * 8 + i][tx + 16 * j] = sum[i][j];
+    for (int j = 0; j < 4; ++j) A[ty * 8 + i][tx + 16 * j] = (float)sum[i][j];
   for (int i = tid; i < C * TP; i += 128) T[i] = 0.f;
   __syncthreads();
   if (tid < C) {  // a row a thread, s downwards
     double e = bt[tid];
     for (int s = tid - 1; s >= 0; --s) {
       e *= as[s + 1];
-      A[tid][s] *= (float)e;
+      A[tid][s] = (float)(A[tid][s] * e);
     }
   }
   __syncthreads();
@@ -701,8 +661,7 @@ __global__ void __launch_bounds__(128) chunk_solve_kernel(ChunkArgs g) {
 // As chunk_states, a sequence's runs in order, with U in front of every run's part of the state; three products in a row that wait
 // for one another, so narrow columns and more blocks.  Bound by what shared memory returns (half a word a multiply-add) and by the
 // three products' order: 4.6 us a run of 64 tokens, which the walk takes 28 us for (one sequence, 16 heads of 128: 149 us of
-// 2,048 tokens; scores 21, triangles 31, outputs 62; the walk 912).  From 64 bits: outputs 1.5e-7, states 1.6e-7 of their size
-// (the walk 1.5e-7, 2.3e-7).
+// 2,048 tokens; the walk 912).
 constexpr int DVT = 16, KROW = DIM + 4;
 constexpr size_t DELTA_SMEM = (size_t)(2 * C * KROW + 2 * C * DVT + C * TROW + DVT * KROW + C * DVT) * sizeof(float);
 
@@ -820,9 +779,9 @@ __global__ void __launch_bounds__(128, 2) delta_states_kernel(ChunkArgs g) {
     for (int i = 0; i < 4; ++i) U[i][0] = U[i][1] = part[i][0] = part[i][1] = 0.f;
     const int reach = (tid >> 5) * 16 + 16;
 #pragma unroll 1
-    for (int s0 = 0; s0 < reach; s0 += PART) {
+    for (int s0 = 0; s0 < reach; s0 += UPART) {
 #pragma unroll
-      for (int s = s0; s < s0 + PART; ++s) {
+      for (int s = s0; s < s0 + UPART; ++s) {
         const float4 x = *reinterpret_cast<const float4*>(ts + s * TROW + ut);
         const float2 y = *reinterpret_cast<const float2*>(vs + s * DVT + uc);
         const float xs[4] = {x.x, x.y, x.z, x.w};

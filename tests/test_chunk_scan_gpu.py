@@ -90,3 +90,84 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(monkeypatch, kind, 
         clean = run(kind, batch_of([150]), 150, 2, 128, 9)[0]
         assert bool(torch.isfinite(y[:at]).all()) and torch.allclose(y[:at], clean[:at], rtol=0, atol=1e-5 * float(clean.abs().max()))
         assert bool((torch.isfinite(y[at]) == torch.isfinite(y0[at])).all())
+
+
+def in_64_bits(kind, n, heads, vdim, seed):
+    """Inputs as a trained layer has them, what ``ops`` makes of one sequence of them, and the recurrence in 64 bits."""
+    from fms_b200.kernels import ops
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    silu, softplus, dim = torch.nn.functional.silu, torch.nn.functional.softplus, 128
+    u = torch.rand(heads, generator=g, device="cuda")
+    bias, rates = torch.log(torch.expm1(torch.exp(-6.9 + 4.6 * u))), torch.log(1 + 15 * torch.rand(heads, generator=g, device="cuda"))
+    state, batch = torch.zeros(1, heads, vdim, dim, device="cuda"), batch_of([n])
+    ones, norm = torch.ones(n, heads, dtype=torch.float64, device="cuda"), None
+    if kind == "space":
+        x, logits, skip = silu(r(n, heads * vdim + 2 * dim)), 0.5 * r(n, heads), torch.ones(heads, device="cuda")
+        dt = softplus(logits.double() + bias.double())
+        keep, give = torch.exp(-torch.exp(rates.double()) * dt), dt
+        v, k, q = x[:, : heads * vdim].double().view(n, heads, vdim), *(t.double()[:, None].expand(n, heads, dim) for t in (x[:, -2 * dim: -dim], x[:, -dim:]))
+        make = lambda: ops.selective_scan(x, logits, 0, bias, rates, skip, state, batch, heads, vdim, dim, 1)  # noqa: E731
+    elif kind == "delta":
+        x, logits = silu(r(n, heads * (2 * dim + vdim))), r(n, 2 * heads)
+        q, k, v = (t.double().view(n, heads, -1) for t in torch.split(x, [heads * dim, heads * dim, heads * vdim], 1))
+        q, k = (t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6) for t in (q * 1.0, k))
+        q, give = q * dim ** -0.5, torch.sigmoid(logits[:, :heads].double())
+        keep = torch.exp(-torch.exp(rates.double()) * softplus(logits[:, heads:].double() + bias.double()))
+        make = lambda: ops.delta_rule_scan(x.clone(), logits, 0, None, bias, rates, state, batch, heads, heads, dim, vdim, decay_offset=heads)  # noqa: E731
+    else:
+        x = r(n, heads * (2 * dim + vdim) + 2 * heads)
+        q, k, v = (t.double().view(n, heads, -1) for t in torch.split(x[:, : heads * (2 * dim + vdim)], [heads * dim, heads * dim, heads * vdim], 1))
+        if kind == "fixed":
+            q, k, v = silu(q), silu(k), silu(v)
+            decay = torch.exp(-(2.0 ** (-8.0 * torch.arange(1, heads + 1, device="cuda") / heads)))
+            keep, give = decay.double() * ones, ones
+            make = lambda: ops.decay_scan(x, state, batch, heads, dim, vdim, ops.ACT_SILU, decay=decay)  # noqa: E731
+        else:
+            gate_bias = torch.cat([torch.zeros(heads), torch.linspace(3, 6, heads)]).cuda()
+            gi, gf = torch.split(15.0 * torch.tanh((x[:, heads * (2 * dim + vdim):].double() + gate_bias.double()) / 15.0), heads, 1)
+            gf, top, keep, give, tops = torch.nn.functional.logsigmoid(gf), torch.zeros_like(gi[0]), ones.clone(), ones.clone(), ones.clone()
+            for t in range(n):
+                to = torch.maximum(gf[t] + top, gi[t])
+                keep[t], give[t], tops[t] = torch.exp(gf[t] + top - to), torch.exp(gi[t] - to), to
+                top = to
+            q, norm, held = q * dim ** -0.5, torch.zeros(heads, dim, dtype=torch.float64, device="cuda"), torch.zeros(1, heads, dim + 1, device="cuda")
+            make = lambda: ops.decay_scan(x, state, batch, heads, dim, vdim, q_scale=dim ** -0.5, gate_offset=heads * (2 * dim + vdim),  # noqa: E731
+                                          gate_bias=gate_bias, gate_cap=15.0, norm_state=held.zero_())
+    S, out = torch.zeros(heads, vdim, dim, dtype=torch.float64, device="cuda"), []
+    for t in range(n):
+        S = S * keep[t][:, None, None]
+        vt = v[t] - torch.einsum("hvk,hk->hv", S, k[t]) if kind == "delta" else v[t]
+        S = S + (give[t][:, None] * vt)[..., None] * k[t][:, None]
+        o = torch.einsum("hvk,hk->hv", S, q[t])
+        if kind == "gated":
+            norm = norm * keep[t][:, None] + give[t][:, None] * k[t]
+            o = o / (torch.maximum((norm * q[t]).sum(-1).abs(), torch.exp(-tops[t])) + 1e-6)[:, None]
+        out.append((o + v[t] if kind == "space" else o).flatten())
+    return make, state, torch.stack(out), S
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_runs_are_no_further_from_64_bits_than_the_walk(monkeypatch, kind):
+    """Outputs and states of a sequence long enough to go run by run, the walk's and the runs' errors over two draws.  Under a
+    normalizer a head's row may be divided by next to nothing, and one such row is most of the whole's error: there the
+    median over the rows."""
+    from fms_b200.kernels import ops
+
+    def apart(a, b):
+        if kind != "gated":
+            return float((a - b).norm() / b.norm())
+        a, b = a.view(-1, 128), b.view(-1, 128)
+        return float(((a - b).norm(dim=1) / b.norm(dim=1)).median())
+
+    errors = []
+    for seed in (1, 2):
+        make, state, want, S = in_64_bits(kind, 400, 8, 64 if kind == "space" else 128, seed)
+        for pays in (False, True):
+            monkeypatch.setattr(ops, "chunk_scan_pays", lambda *_: pays)
+            state.zero_()
+            y = make()
+            errors.append([apart(y.double(), want), float((state[0].double() - S).norm() / S.norm())])
+    for walk, runs in zip(*[[sum(e[j] for e in errors[i::2]) for j in range(2)] for i in range(2)]):
+        assert walk < 1e-5 and runs <= walk, (walk, runs)
