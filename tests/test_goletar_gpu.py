@@ -495,3 +495,35 @@ def test_a_product_a_group_takes_matrices_that_the_product_before_it_made():
         a.neg_()
         want.neg_()
         assert torch.equal(product(made()), want)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_in_the_heads_own_space_rounds_values_that_are_alike_once(hd):
+    """A few keys whose values are nearly the same: the probabilities are rounded to bfloat16, and unless they are summed as
+    rounded, every row is off by what their roundings come to.  Against the same keys and values in 64 bits, no further off
+    than rounding the result to bfloat16 alone, but for a twentieth."""
+    from fms_b200.cache import Cache, KVRequest
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    heads, width, n = 32, 72, 12
+    g = torch.Generator().manual_seed(hd)
+    cache = Cache([KVRequest(1, width, 0, planes=1)], 64, 64, torch.bfloat16, "cuda", max_slots=1)
+    slots = cache.begin(1)
+    batch = Batch.from_lists(slots, cache.prepare(slots, [n]), [[0] * n], [[]], "cuda")
+    view = cache.layer_view(0)
+    rows = torch.randn(n, width, generator=g)
+    rows[:, 0] = 1.0
+    rows = rows.to(torch.bfloat16).cuda()
+    view.keys[int(view.table[slots[0], 0]), 0, :n] = rows
+    expand = torch.randn(heads, 2 * hd, width, generator=g) * 0.3
+    expand[:, hd:] *= 0.03
+    expand[:, hd:, 0] = 1.5
+    expand = expand.to(torch.bfloat16).cuda()
+    q = torch.randn(n, heads, hd, generator=g).to(torch.bfloat16).cuda()
+    got = ops.latent_attention_expanded(q, batch, view, expand, None, heads, hd, hd ** -0.5).view(n, heads, hd).double()
+    k, v = ops.linear(rows, expand.view(-1, width)).view(n, heads, 2, hd).double().unbind(2)
+    scores = torch.einsum("ihd,jhd->hij", q.double(), k) * hd ** -0.5
+    scores = scores.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.einsum("hij,jhd->ihd", torch.softmax(scores, -1), v)
+    assert float((got - want).norm()) <= 1.05 * float((want.to(torch.bfloat16).double() - want).norm())
