@@ -89,6 +89,13 @@ PyObject* entry_call(PyObject* callable, PyObject* const* args, size_t nargsf, P
       whole[w++] = 0;
     } else if (kind == 'p' && THPVariable_Check(a)) {
       if (!address(self, a, &whole[w++])) return nullptr;
+    } else if (kind == 'i' && PyIndex_Check(a)) {  // numpy's whole numbers and the like, as ctypes takes them
+      PyObject* index = PyNumber_Index(a);
+      if (!index) return nullptr;
+      const u64 x = PyLong_AsUnsignedLongLongMask(index);
+      Py_DECREF(index);
+      if (x == ~0ull && PyErr_Occurred()) return nullptr;
+      whole[w++] = x;
     } else {
       return PyErr_Format(PyExc_TypeError, "argument %zd: '%s' where a %s is taken", i + 1, Py_TYPE(a)->tp_name,
                           kind == 'p' ? "tensor, an address or None" : "whole number");

@@ -3,6 +3,7 @@ import ctypes
 import itertools
 import subprocess
 
+import numpy
 import pytest
 import torch
 
@@ -34,6 +35,26 @@ def test_arguments_arrive_in_order(tmp_path, kinds):
     assert f(*args) == 7
     single = lambda x: ctypes.c_float(x).value  # noqa: E731
     assert list(out)[1:] == [single(a) if k == "f" else float(a or 0) for k, a in zip(kinds[1:], args[1:])]
+
+
+class Indexed:
+    def __index__(self):
+        return -9
+
+
+def test_whole_numbers_that_are_no_python_int(tmp_path):
+    """Whatever has an ``__index__`` is a whole number, as for ctypes; an address is an int, a tensor or None."""
+    f, out, lib = entry(tmp_path, "pilf")
+    at = ctypes.addressof(out)
+    for a, b in ((numpy.int64(-3), numpy.int64(2 ** 40)), (numpy.uint8(5), numpy.int32(-1)), (Indexed(), torch.tensor(7)), (True, Indexed())):
+        assert f(at, a, b, numpy.float32(0.5)) == 7
+        assert list(out)[1:] == [float(a.__index__()), float(b.__index__()), 0.5]
+    for bad in (numpy.float32(1.0), numpy.bool_(True), torch.zeros(1), torch.zeros(2, dtype=torch.int32)):
+        with pytest.raises(TypeError):
+            f(at, bad, 1, 1.0)
+    for bad in (numpy.int64(at), Indexed()):
+        with pytest.raises(TypeError):
+            f(bad, 1, 1, 1.0)
 
 
 def test_what_an_entry_refuses(tmp_path):
