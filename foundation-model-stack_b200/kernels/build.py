@@ -16,6 +16,7 @@ import hashlib
 import importlib.machinery
 import importlib.util
 import os
+import shlex
 import shutil
 import subprocess
 import sys
@@ -113,28 +114,33 @@ def _spec(name: str) -> Tuple[str, List[str]]:
     raise KernelBuildError(f"unknown kernel library {name!r}")
 
 
+def _launcher_flags() -> List[str]:
+    import torch
+
+    return ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+
+
 def _launcher_command(out: str) -> List[str]:
     import torch
 
-    compiler = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    compiler = shlex.split(os.environ.get("CXX", "")) or [c for c in (shutil.which("g++") or shutil.which("c++"),) if c]
     if not compiler:
         raise KernelBuildError("no C++ compiler was found (looked at CXX and PATH for g++ and c++)")
     base = os.path.dirname(torch.__file__)
     include = [sysconfig.get_paths()["include"], os.path.join(base, "include"),
                os.path.join(base, "include", "torch", "csrc", "api", "include")]
-    return [compiler, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"] + [f"-I{d}" for d in include] + [
-            os.path.join(CSRC, "launcher.cpp"), "-o", out, "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    return compiler + _launcher_flags() + [f"-I{d}" for d in include] + [
+        os.path.join(CSRC, "launcher.cpp"), "-o", out, "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
 
 
 def _launcher_digest() -> str:
-    """Of the source and of what it is compiled against."""
+    """Of the source and of what it is compiled against; a machine that has it compiled needs no compiler."""
     import torch
 
     h = hashlib.sha256()
     with open(os.path.join(CSRC, "launcher.cpp"), "rb") as f:
         h.update(f.read())
-    h.update(" ".join((torch.__version__, sys.version, _TAG) + tuple(_launcher_command("")[1:7])).encode())
+    h.update(" ".join([torch.__version__, sys.version, _TAG] + _launcher_flags()).encode())
     return h.hexdigest()[:12]
 
 

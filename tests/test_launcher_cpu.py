@@ -73,3 +73,13 @@ def test_what_an_entry_refuses(tmp_path):
 def test_every_entry_fits():
     for name, kinds in _SIGNATURES.items():
         assert build.load_launcher().entry(1, "".join(kinds), KernelError), name
+
+
+def test_a_machine_without_a_compiler_takes_what_is_built(monkeypatch):
+    build.load_launcher()
+    built = build.find_built(build.LAUNCHER)
+    monkeypatch.delenv("CXX", raising=False)
+    monkeypatch.setattr(build.shutil, "which", lambda *_: None)
+    assert built is not None and build.find_built(build.LAUNCHER) == built
+    with pytest.raises(build.KernelBuildError, match="no C"):
+        build.compile_library(build.LAUNCHER)
