@@ -113,7 +113,7 @@ class Engine:
         """Compiles, side by side, the kernel libraries this model's parts name and that are not built yet."""
         from ..kernels import build
 
-        names = list(dict.fromkeys(self.decoder.kernel_libraries(self.decoder.dtype)))
+        names = [build.LAUNCHER] + list(dict.fromkeys(self.decoder.kernel_libraries(self.decoder.dtype)))
         if sampling:
             names.append("sampling")
         build.compile_many(names)

@@ -170,7 +170,7 @@ class GatedDeltaRule(Part):
         return self.dense.forward(self.heads_out(x, batch, cache_view, writes_cache))
 
     def kernel_libraries(self, dtype):
-        return super().kernel_libraries(dtype) + ["state_scan"]
+        return super().kernel_libraries(dtype) + ["state_scan"] + (["chunk_scan"] if self.per_head else [])
 
 
 class ParallelMixers(Part):

@@ -83,3 +83,23 @@ def test_a_machine_without_a_compiler_takes_what_is_built(monkeypatch):
     assert built is not None and build.find_built(build.LAUNCHER) == built
     with pytest.raises(build.KernelBuildError, match="no C"):
         build.compile_library(build.LAUNCHER)
+
+
+@pytest.mark.parametrize("decay", ["head", "channel"])
+def test_an_engine_compiles_what_its_first_prompt_will_launch(monkeypatch, decay):
+    """The launcher, and the runs' kernels where a layer's prompts may go run by run: not in the middle of a request."""
+    import types
+
+    import fms_b200.parts.state_space  # noqa: F401
+    from fms_b200.config.specs import MixerSpec
+    from fms_b200.engine.step import Engine
+    from fms_b200.parts.registry import build_mixer
+
+    asked = []
+    monkeypatch.setattr(build, "compile_many", lambda names, *_: asked.extend(names))
+    options = (("vdim", 128), ("conv", 4), ("eps", 1e-5), ("decay", decay), ("decay_rank", 8), ("gate_rank", 8))
+    part = build_mixer(MixerSpec("gated_delta_rule", dim=64, nheads=2, kvheads=1, head_dim=128, options=options))
+    decoder = types.SimpleNamespace(kernel_libraries=part.kernel_libraries, dtype=torch.bfloat16)
+    Engine._compile_what_this_model_needs(types.SimpleNamespace(decoder=decoder), True)
+    assert {build.LAUNCHER, "state_scan", "sampling"} <= set(asked)
+    assert ("chunk_scan" in asked) == (decay == "head")
