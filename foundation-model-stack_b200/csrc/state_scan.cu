@@ -251,6 +251,10 @@ __global__ void conv_tail_kernel(const T* x, int stride, float* tail, const int*
 // same order whatever VP is, whatever else is in the batch and however the prompt was cut.  The tokens' vectors
 // come through shared memory CH tokens at a time by cp.async into two stages: the next chunk is on its way while this
 // one is walked.  Rows of shared memory are padded to PARTS * NP values with zeros, so the inner loops need no bounds.
+// by_runs [sequences + 1], or null: where each sequence's runs start in the list of those that have gone run by run
+// (csrc/chunk_scan.cu); a sequence that has some is left alone here.
+__device__ __forceinline__ bool went_by_runs(const int* by_runs, int seq) { return by_runs != nullptr && by_runs[seq] < by_runs[seq + 1]; }
+
 constexpr int SCAN_THREADS = 128;  // PARTS threads share a group of value columns; a block has 128 / PARTS groups
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
@@ -360,7 +364,7 @@ template <int NP, int VP, int PARTS>
 __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const float* xbc, const void* dt_raw, int dt_is_bf16,
                                                              int dt_stride, const float* dt_bias, const float* a_log,
                                                              const float* d_skip, float* state, float* y,
-                                                             const int* first_row, const int* slots, int heads, int vdim,
+                                                             const int* first_row, const int* by_runs, const int* slots, int heads, int vdim,
                                                              int n_state, int groups, int write_state, int n_slots,
                                                              int vec_bc, int vec_x) {
   constexpr int GROUPS = SCAN_THREADS / PARTS, NPAD = RowLayout<NP, PARTS>::ROW, RUN = RowLayout<NP, PARTS>::RUN, VB = GROUPS * VP;
@@ -372,6 +376,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const floa
   const int slot = __ldcg(slots + seq);
   if (!FMS_IN(slot, n_slots)) return;
   const int lo = first_row[seq], hi = first_row[seq + 1];
+  if (went_by_runs(by_runs, seq)) return;
   const int inner = heads * vdim, row_w = inner + 2 * groups * n_state;
   const int group = head / (heads / groups);
   constexpr int STAGE = CH * (2 * NPAD + VB);
@@ -463,13 +468,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const floa
 //   qkv [tokens, 2 kvheads * dim + heads * vdim] float32 (after the convolution): q | k | v;  q and k of every key head
 //   become unit vectors in place, x / sqrt(sum(x^2) + 1e-6), q also times dim^-1/2
 //   decay[t, h, n] = exp(-exp(a_log[h]) * softplus(a_raw[t, h, n] + dt_bias[h, n]));  beta[t, h] = sigmoid(beta_raw[t, h])
-//   `per_head`: one decay a head, exp(-exp(a_log[h]) * softplus(a_raw[t, h] + dt_bias[h])), written to all its channels (1) or
-//   as decay[t, h] (2)
+//   `per_head`: one decay a head, exp(-exp(a_log[h]) * softplus(a_raw[t, h] + dt_bias[h])), written to all its channels and,
+//   where it is not null, to head_decay[t, h]; decay may then be null
 //   a_raw is walked by its row stride `a_stride`
 template <typename T>
 __global__ void delta_prepare_kernel(float* qkv, const T* a_raw, int a_stride, int per_head, const T* beta_raw,
-                                     int beta_stride, const float* dt_bias, const float* a_log, float* decay, float* beta,
-                                     int heads, int kvheads, int dim, int vdim) {
+                                     int beta_stride, const float* dt_bias, const float* a_log, float* decay, float* head_decay,
+                                     float* beta, int heads, int kvheads, int dim, int vdim) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x & 31;
@@ -489,11 +494,9 @@ __global__ void delta_prepare_kernel(float* qkv, const T* a_raw, int a_stride, i
       const size_t at = ((size_t)t * heads + h) * dim;
       if (per_head) {
         const float d = (float)exp(-A * softplus_d((double)to_f32(a_raw[(size_t)t * a_stride + h]) + (double)dt_bias[h]));
-        if (per_head == 2) {
-          if (lane == 0) decay[(size_t)t * heads + h] = d;
-        } else {
+        if (head_decay != nullptr && lane == 0) head_decay[(size_t)t * heads + h] = d;
+        if (decay != nullptr)
           for (int n = lane; n < dim; n += 32) decay[at + n] = d;
-        }
       } else {
         const T* ar = a_raw + (size_t)t * a_stride + (size_t)h * dim;
         for (int n = lane; n < dim; n += 32)
@@ -507,7 +510,7 @@ __global__ void delta_prepare_kernel(float* qkv, const T* a_raw, int a_stride, i
 // qkv as delta_prepare_kernel left it; decay [tokens, heads * dim], beta [tokens, heads]; o [tokens, heads * vdim]
 template <int NP, int VP, int PARTS>
 __global__ void __launch_bounds__(SCAN_THREADS) delta_rule_scan_kernel(const float* qkv, const float* decay, const float* beta,
-                                                              float* state, float* o, const int* first_row,
+                                                              float* state, float* o, const int* first_row, const int* by_runs,
                                                               const int* slots, int heads, int kvheads, int dim, int vdim,
                                                               int write_state, int n_slots, int vec_qk, int vec_g,
                                                               int vec_v) {
@@ -520,6 +523,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_rule_scan_kernel(const flo
   const int slot = __ldcg(slots + seq);
   if (!FMS_IN(slot, n_slots)) return;
   const int lo = first_row[seq], hi = first_row[seq + 1];
+  if (went_by_runs(by_runs, seq)) return;
   const int kvh = head / (heads / kvheads);
   const int row_w = 2 * kvheads * dim + heads * vdim;
   constexpr int STAGE = CH * (3 * NPAD + VB + 1);
@@ -788,8 +792,8 @@ __global__ void __launch_bounds__(GLA_THREADS) gla_prepare_kernel(const T* proj,
 template <int NP, int VP, int PARTS, int KIND>
 __global__ void __launch_bounds__(SCAN_THREADS) decay_scan_kernel(const float* qkv, const float* gates, const float* decay,
                                                                   float* state, const float* norm_in, float* norm_state,
-                                                                  float* o, const int* first_row, const int* slots,
-                                                                  int heads, int dim, int vdim, int write_state,
+                                                                  float* o, const int* first_row, const int* by_runs,
+                                                                  const int* slots, int heads, int dim, int vdim, int write_state,
                                                                   int n_slots, int vec_qk, int vec_v, int vec_g) {
   constexpr bool GATED = KIND == 1, CHANNEL = KIND == 2;
   constexpr int GROUPS = SCAN_THREADS / PARTS, NPAD = RowLayout<NP, PARTS>::ROW, RUN = RowLayout<NP, PARTS>::RUN, VB = GROUPS * VP;
@@ -801,6 +805,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) decay_scan_kernel(const float* q
   const int slot = __ldcg(slots + seq);
   if (!FMS_IN(slot, n_slots)) return;
   const int lo = first_row[seq], hi = first_row[seq + 1];
+  if (went_by_runs(by_runs, seq)) return;
   const int row_w = 2 * heads * dim + heads * vdim;
   constexpr int STAGE = CH * ((CHANNEL ? 3 : 2) * NPAD + VB + 4);
   const int cols = min(VB, vdim - v0);
@@ -1164,7 +1169,7 @@ static bool rows_allow_16(const void* base, long offset, long stride, int count)
   } while (0)
 
 FMS_API int fms_selective_scan(const float* xbc, const void* dt_raw, int dtype, int dt_stride, const float* dt_bias,
-                               const float* a_log, const float* d_skip, float* state, float* y, const int* first_row,
+                               const float* a_log, const float* d_skip, float* state, float* y, const int* first_row, const int* by_runs,
                                const int* slots, int n_seqs, int heads, int vdim, int n_state, int groups,
                                int write_state, int n_slots, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
@@ -1182,7 +1187,7 @@ FMS_API int fms_selective_scan(const float* xbc, const void* dt_raw, int dtype, 
     const size_t smem = ((size_t)2 * CH * (2 * RowLayout<NP, PARTS>::ROW + SCAN_THREADS / PARTS * VP) + 2 * CH) * sizeof(float); \
     cudaFuncSetAttribute(selective_scan_kernel<NP, VP, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
     fms_launch(selective_scan_kernel<NP, VP, PARTS>, grid, block, smem, stream, xbc, dt_raw, dtype == FMS_BF16 ? 1 : 0, dt_stride, \
-               dt_bias, a_log, d_skip, state, y, first_row, slots, heads, vdim, n_state, groups, write_state, n_slots,   \
+               dt_bias, a_log, d_skip, state, y, first_row, by_runs, slots, heads, vdim, n_state, groups, write_state, n_slots,   \
                vec_bc, vec_x);                                                                                           \
   } while (0)
   FMS_SCAN_SHAPES(FMS_LAUNCH);
@@ -1190,31 +1195,34 @@ FMS_API int fms_selective_scan(const float* xbc, const void* dt_raw, int dtype, 
   return fms_launch_status("selective_scan");
 }
 
-// What the delta rule with one decay a head reads, made ready for every token: qkv in place, decay and beta [tokens, heads]
+// What the delta rule with one decay a head reads, made ready for every token: qkv in place, decay [tokens, heads * dim] (or null),
+// head_decay and beta [tokens, heads]
 FMS_API int fms_delta_prepare(float* qkv, const void* beta_raw, int dtype, int beta_stride, const void* a_raw, int a_stride,
-                              const float* dt_bias, const float* a_log, float* decay, float* beta, int n_tokens, int heads, int kvheads,
-                              int dim, int vdim, cudaStream_t stream) {
+                              const float* dt_bias, const float* a_log, float* decay, float* head_decay, float* beta, int n_tokens,
+                              int heads, int kvheads, int dim, int vdim, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (heads <= 0 || kvheads <= 0 || heads % kvheads || dim <= 0 || vdim <= 0)
     return fms_fail("delta_prepare: %d heads over %d, dim %d, vdim %d", heads, kvheads, dim, vdim);
   FMS_DISPATCH_DTYPE(dtype, T, fms_launch(delta_prepare_kernel<T>, dim3(n_tokens, (2 * kvheads + heads + 3) / 4), dim3(128), 0, stream, qkv, (const T*)a_raw,
-                                          a_stride, 2, (const T*)beta_raw, beta_stride, dt_bias, a_log, decay, beta, heads, kvheads, dim,
-                                          vdim));
+                                          a_stride, 1, (const T*)beta_raw, beta_stride, dt_bias, a_log, decay, head_decay, beta, heads,
+                                          kvheads, dim, vdim));
   return fms_launch_status("delta_prepare");
 }
 
 // decay [tokens, heads * dim] and beta [tokens, heads]: float32 scratch of the caller's.  a_raw: rows of a_stride
-// values, of which the first heads * dim (per_head: the first heads) are the decays' logits
+// values, of which the first heads * dim (per_head: the first heads) are the decays' logits.  by_runs: see went_by_runs; with it
+// qkv, decay and beta are as fms_delta_prepare has left them.
 FMS_API int fms_delta_rule_scan(float* qkv, const void* beta_raw, int dtype, int beta_stride, const void* a_raw,
                                 int a_stride, int per_head, const float* dt_bias, const float* a_log, float* decay, float* beta, float* state, float* o,
-                                const int* first_row, const int* slots, int n_tokens, int n_seqs, int heads, int kvheads,
+                                const int* first_row, const int* by_runs, const int* slots, int n_tokens, int n_seqs, int heads, int kvheads,
                                 int dim, int vdim, int write_state, int n_slots, cudaStream_t stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return 0;
   if (heads <= 0 || kvheads <= 0 || heads % kvheads || dim <= 0 || dim > 256 || vdim <= 0)
     return fms_fail("delta_rule_scan: %d heads over %d, dim %d (up to 256), vdim %d", heads, kvheads, dim, vdim);
-  FMS_DISPATCH_DTYPE(dtype, T, fms_launch(delta_prepare_kernel<T>, dim3(n_tokens, (2 * kvheads + heads + 3) / 4), dim3(128), 0, stream, qkv, (const T*)a_raw,
-                                          a_stride, per_head, (const T*)beta_raw, beta_stride, dt_bias, a_log, decay, beta, heads, kvheads, dim,
-                                          vdim));
+  if (by_runs == nullptr)
+    FMS_DISPATCH_DTYPE(dtype, T, fms_launch(delta_prepare_kernel<T>, dim3(n_tokens, (2 * kvheads + heads + 3) / 4), dim3(128), 0, stream, qkv,
+                                            (const T*)a_raw, a_stride, per_head, (const T*)beta_raw, beta_stride, dt_bias, a_log, decay,
+                                            (float*)nullptr, beta, heads, kvheads, dim, vdim));
   const ScanShape shape = scan_shape(n_seqs, heads, vdim, dim);
   const int vb = SCAN_THREADS / shape.parts * shape.vp;  // value columns of a block
   const long row_w = 2L * kvheads * dim + (long)heads * vdim;
@@ -1227,7 +1235,7 @@ FMS_API int fms_delta_rule_scan(float* qkv, const void* beta_raw, int dtype, int
     const size_t smem = ((size_t)2 * CH * (3 * RowLayout<NP, PARTS>::ROW + SCAN_THREADS / PARTS * VP + 1)) * sizeof(float); \
     cudaFuncSetAttribute(delta_rule_scan_kernel<NP, VP, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     fms_launch(delta_rule_scan_kernel<NP, VP, PARTS>, grid, block, smem, stream, (const float*)qkv, (const float*)decay, \
-               (const float*)beta, state, o, first_row, slots, heads, kvheads, dim, vdim, write_state, n_slots, vec_qk,  \
+               (const float*)beta, state, o, first_row, by_runs, slots, heads, kvheads, dim, vdim, write_state, n_slots, vec_qk,  \
                vec_g, vec_v);                                                                                            \
   } while (0)
   FMS_SCAN_SHAPES(FMS_LAUNCH);
@@ -1291,10 +1299,11 @@ FMS_API int fms_exp_gates(const void* gate_raw, int dtype, int gate_stride, cons
 // gate_stride values, bias [2 heads], cap): exponential gates, with normalizer and running maximum in norm_state
 // [slots, heads, dim + 1]; gates [tokens, heads, 3] and norm_in [sequences, heads, dim] are float32 scratch of the
 // caller's.  With gates but no gate_raw: one decay a token and key channel, gates [tokens, heads * dim].  Else: decay [heads].
+// by_runs: see went_by_runs; with it gates and norm_in are as fms_exp_gates has left them.
 FMS_API int fms_decay_scan(const float* qkv, const void* gate_raw, int dtype, int gate_stride, const float* gate_bias,
                            float cap, float* gates, float* norm_in, const float* decay, float* state, float* norm_state, float* o,
-                           const int* first_row, const int* slots, int n_tokens, int n_seqs, int heads, int dim, int vdim,
-                           int write_state, int n_slots, cudaStream_t stream) {
+                           const int* first_row, const int* by_runs, const int* slots, int n_tokens, int n_seqs, int heads, int dim,
+                           int vdim, int write_state, int n_slots, cudaStream_t stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return 0;
   if (heads <= 0 || dim <= 0 || dim > 256 || vdim <= 0)
     return fms_fail("decay_scan: %d heads, dim %d (up to 256), vdim %d", heads, dim, vdim);
@@ -1303,7 +1312,7 @@ FMS_API int fms_decay_scan(const float* qkv, const void* gate_raw, int dtype, in
   const bool channel = !gated && gates != nullptr;
   if (!gated && !channel && !decay) return fms_fail("decay_scan: neither gates nor decays");
   const long row_w = 2L * heads * dim + (long)heads * vdim;
-  if (gated) {
+  if (gated && by_runs == nullptr) {
     if (fms_exp_gates(gate_raw, dtype, gate_stride, gate_bias, cap, norm_state, norm_in, gates, first_row, slots, n_tokens, n_seqs, heads,
                       dim, write_state, n_slots, stream))
       return 1;
@@ -1322,7 +1331,8 @@ FMS_API int fms_decay_scan(const float* qkv, const void* gate_raw, int dtype, in
     const size_t smem = ((size_t)2 * CH * ((KIND == 2 ? 3 : 2) * RowLayout<NP, PARTS>::ROW + SCAN_THREADS / PARTS * VP + 4)) * sizeof(float); \
     cudaFuncSetAttribute(decay_scan_kernel<NP, VP, PARTS, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     fms_launch(decay_scan_kernel<NP, VP, PARTS, KIND>, grid, block, smem, stream, qkv, (const float*)gates, decay, state, \
-               (const float*)norm_in, norm_state, o, first_row, slots, heads, dim, vdim, write_state, n_slots, vec_qk, vec_v, vec_g); \
+               (const float*)norm_in, norm_state, o, first_row, by_runs, slots, heads, dim, vdim, write_state, n_slots, vec_qk, vec_v, \
+               vec_g);                                                                                                     \
   } while (0)
 #define FMS_LAUNCH_F(NP, VP, PARTS) FMS_LAUNCH_G(NP, VP, PARTS, 0)
 #define FMS_LAUNCH_T(NP, VP, PARTS) FMS_LAUNCH_G(NP, VP, PARTS, 1)

@@ -84,21 +84,27 @@ class Batch:
         b.len_before_host = list(len_before)
         return b
 
-    def row_chunks(self, chunk: int):
+    def row_chunks(self, chunk: int, chosen: Optional[Sequence[bool]] = None):
         """(chunk_rows [chunks, 2] int32: first row and end of every run of up to ``chunk`` rows of one sequence;
         first_chunk [n_seqs + 1] int32: where each sequence's runs start in that list), for kernels that walk a
-        sequence's rows run by run."""
-        key = ("chunks", chunk)
+        sequence's rows run by run.  ``chosen``: whether a sequence has runs at all (default: every one)."""
+        key = self.row_chunks_key(chunk, chosen)
         if key not in self._tiles:
             rows, first, base = [], [0], 0
-            for n in self.num_new:
-                for r in range(0, n, chunk):
-                    rows.append((base + r, base + min(n, r + chunk)))
+            for i, n in enumerate(self.num_new):
+                if chosen is None or chosen[i]:
+                    for r in range(0, n, chunk):
+                        rows.append((base + r, base + min(n, r + chunk)))
                 first.append(len(rows))
                 base += n
             packed = torch.tensor([v for p in rows for v in p] + first, dtype=torch.int32).to(self.tokens.device)
             self._tiles[key] = (packed[: 2 * len(rows)].view(-1, 2), packed[2 * len(rows):])
         return self._tiles[key]
+
+    @staticmethod
+    def row_chunks_key(chunk: int, chosen: Optional[Sequence[bool]] = None):
+        """Where ``row_chunks`` keeps what it makes."""
+        return ("chunks", chunk) if chosen is None or all(chosen) else ("chunks", chunk, tuple(chosen))
 
     def key_rows(self, window: int):
         """(start, first, base: int32 [n_seqs + 1], [n_seqs], [n_seqs]; rows): the keys that a step of several tokens sees,

@@ -96,8 +96,8 @@ _SIGNATURES = {
     "fms_exp_gates": [_P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "fms_chunk_scan": [_I, _P, _P, _P, _L, _P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
                        _P, _I, _I, _I, _I, _I, _I, _P],
-    "fms_delta_prepare": [_P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "fms_decay_scan": [_P, _P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "fms_delta_prepare": [_P, _P, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "fms_decay_scan": [_P, _P, _I, _I, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_attention_prefill_sink": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
                                    _P],
     "fms_attention_prefill_masked": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
@@ -107,8 +107,8 @@ _SIGNATURES = {
     "fms_attention_decode_sink": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I, _I, _I, _L,
                                   _P, _P, _P, _P],
     "fms_causal_conv": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
-    "fms_selective_scan": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
-    "fms_delta_rule_scan": [_P, _P, _I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+    "fms_selective_scan": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "fms_delta_rule_scan": [_P, _P, _I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_gated_group_rmsnorm": [_P, _P, _I, _I, _I, _P, _I, _F, _F, _P, _I, _I, _I, _P],
     "fms_argmax": [_P, _P, _I, _I, _P],
     "fms_sample": [_P, _P, _I, _I, _F, _I, _U64, _P, _I, _P],
@@ -924,33 +924,36 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
 
 
 CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
-# A scan under one decay a head goes run by run where the longest sequence of a step has CHUNK_SCAN_FROM tokens and, with heads
-# of 64 values, also a CHUNK_SCAN_SHARE-th of the step's: the walk takes a sequence's tokens one after the other, but a step
-# of many sequences fills the multiprocessors all the same.  Whole layers, walk / runs in us (gated with a normalizer, fixed decays,
-# state space with heads of 64): one prompt of 200 tokens 157 / 135, 125 / 135, 191 / 170; of 256 181 / 132, 140 / 132, 220 / 170;
-# of 2,048 1,627 / 583, 886 / 519, 1,450 / 760; eight of 2,048 tokens together, the longest 391, 687 / 631, 603 / 587, 851 / 851;
-# eight of 1,000 together, the longest 190, 357 / 309, 307 / 280, 445 / 478.
-CHUNK_SCAN_FROM, CHUNK_SCAN_SHARE = 256, 5
+# A sequence goes run by run through a scan under one decay a head from CHUNK_SCAN_FROM tokens of a step on, and through the delta
+# rule with one decay a head, which has two more products a run, from DELTA_CHUNKS_FROM on: its own tokens decide, so that
+# its results do not depend on what else is in the step.  Whole layers of one prompt, walk / runs in us (gated with a normalizer,
+# fixed decays, state space with heads of 64; delta rule of 16 heads of 128): 130 tokens - , - , - , 102 / 121; 200: 157 / 135,
+# 125 / 135, 191 / 170, 141 / 131; 256: 181 / 132, 140 / 132, 220 / 170, - ; 2,048: 1,627 / 583, 886 / 519, 1,450 / 760, 1,106 / 453.
+CHUNK_SCAN_FROM, DELTA_CHUNKS_FROM = 256, 192
 
 
-# The same for the delta rule, which has two more products a run.  Whole layers of 16 heads of 128, walk / runs in us: one prompt of
-# 130 tokens 102 / 121, of 200 141 / 131, of 2,048 1,106 / 453; 512 tokens of eight sequences, the longest 97, 175 / 205; 1,000 of
-# eight, the longest 190, 302 / 269; 2,048 of eight 581 / 457.
-DELTA_CHUNKS_FROM = 192
+def chunk_scan_pays(n: int, least: Optional[int] = None) -> bool:
+    """Whether a sequence's ``n`` tokens of a step go run by run (``fms_chunk_scan``) or token by token."""
+    return n >= (CHUNK_SCAN_FROM if least is None else least)
 
 
-def chunk_scan_pays(batch, heads: int, vdim: int, least: Optional[int] = None) -> bool:
-    """Whether a step's scan goes run by run (``fms_chunk_scan``) or token by token."""
-    longest = max(batch.num_new)
-    return longest >= (CHUNK_SCAN_FROM if least is None else least) and (vdim > 64 or CHUNK_SCAN_SHARE * longest >= sum(batch.num_new))
+class _Runs:
+    """The sequences of a step that go run by run."""
+
+    def __init__(self, rows: torch.Tensor, first: torch.Tensor, whole: bool) -> None:
+        self.rows, self.first = rows, first  # as ``Batch.row_chunks``
+        self.whole = whole  # every sequence of the step is among them
 
 
 def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, rows: torch.Tensor,
-                     least: Optional[int] = None):
-    """The step's rows as runs for ``fms_chunk_scan``, or None where it does not take them: other head sizes, rows
+                     least: Optional[int] = None) -> Optional[_Runs]:
+    """The step's rows as runs for ``fms_chunk_scan``, or None where it takes none of them: other head sizes, rows
     that do not lie on 16 bytes, decode steps and short prompts (which go token by token), a capture that has not seen the batch
     before (the runs come from the host)."""
-    if batch.decode or not batch.num_new or not chunk_scan_pays(batch, heads, vdim, least):
+    if batch.decode or not batch.num_new:
+        return None
+    chosen = [chunk_scan_pays(n, least) for n in batch.num_new]
+    if not any(chosen):
         return None
     if _ptr(rows) & 15 or rows.shape[1] % 4 or batch.n_seqs > 65535:
         return None
@@ -958,17 +961,17 @@ def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, row
     if not lib.fms_chunk_scan_takes(int(dim), int(vdim), heads // key_heads):
         return None
     chunk = int(lib.fms_chunk_scan_tokens())
-    if ("chunks", chunk) not in batch._tiles and torch.cuda.is_current_stream_capturing():
+    if batch.row_chunks_key(chunk, chosen) not in batch._tiles and torch.cuda.is_current_stream_capturing():
         return None
-    return batch.row_chunks(chunk)
+    return _Runs(*batch.row_chunks(chunk, chosen), all(chosen))
 
 
-def _chunk_scan(kind: int, q: int, k: int, v: int, row: int, plan, batch, state: torch.Tensor, o: torch.Tensor, heads: int,
+def _chunk_scan(kind: int, q: int, k: int, v: int, row: int, plan: _Runs, batch, state: torch.Tensor, o: torch.Tensor, heads: int,
                 key_heads: int, dim: int, vdim: int, writes_state: bool, decay=None, gates=None, norm_in=None, norm_state=None,
                 dt_raw: Optional[int] = None, dt_dtype: int = F32, dt_stride: int = 0, dt_bias=None, a_log=None, d_skip=None) -> None:
     """``fms_chunk_scan`` with its scratch; q, k, v, dt_raw: addresses."""
     global launches
-    runs, first_run = plan
+    runs, first_run = plan.rows, plan.first
     n, chunk, dev = runs.shape[0], 64, state.device
     per_pass = max(1, min(n, CHUNK_STATE_BYTES // (heads * vdim * dim * 4)))
     new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)  # noqa: E731
@@ -1000,9 +1003,10 @@ def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bia
         _chunk_scan(2, b + groups * n_state * 4, b, x, xbc.shape[1], plan, batch, state, y, heads, groups, n_state, vdim, writes_state,
                     dt_raw=_ptr(proj) + dt_offset * proj.element_size(), dt_dtype=_code(proj.dtype), dt_stride=proj.shape[1],
                     dt_bias=dt_bias, a_log=a_log, d_skip=d_skip)
-        return y
+        if plan.whole:
+            return y
     _call("state_scan", "fms_selective_scan", xbc, _ptr(proj) + dt_offset * proj.element_size(), _code(proj.dtype),
-          proj.shape[1], dt_bias, a_log, d_skip, state, y, batch.first_row,
+          proj.shape[1], dt_bias, a_log, d_skip, state, y, batch.first_row, None if plan is None else plan.first,
           batch.slots, batch.n_seqs, heads, vdim, n_state, groups, 1 if writes_state else 0, state.shape[0],
           _stream())
     return y
@@ -1032,23 +1036,26 @@ def delta_rule_scan(qkv: torch.Tensor, proj: torch.Tensor, beta_offset: int, a_r
         a_ptr, a_stride = _ptr(a_raw), heads * dim
     o = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
     plan = _chunk_scan_runs(batch, dim, vdim, heads, kvheads, qkv, DELTA_CHUNKS_FROM) if per_head and vdim == 128 else None
+    # decays [tokens, heads * dim] where a sequence walks, then betas and, where one goes run by run, decays [tokens, heads]
+    walks = plan is None or not plan.whole
+    scratch = torch.empty((n * heads * ((dim if walks else 0) + (1 if plan is None else 2)),), dtype=torch.float32, device=qkv.device)
+    channels = scratch.data_ptr() if walks else None
+    beta = scratch.data_ptr() + (4 * n * heads * dim if walks else 0)
     if plan is not None:
-        decay, beta = (torch.empty((n, heads), dtype=torch.float32, device=qkv.device) for _ in range(2))
+        decay = beta + 4 * n * heads
         _call("state_scan", "fms_delta_prepare", qkv, _ptr(proj) + beta_offset * proj.element_size(), _code(proj.dtype), proj.shape[1],
-              a_ptr, a_stride, dt_bias, a_log, decay, beta, n, heads, kvheads, dim, vdim, _stream())
+              a_ptr, a_stride, dt_bias, a_log, channels, decay, beta, n, heads, kvheads, dim, vdim, _stream())
         q = _ptr(qkv)
         _chunk_scan(3, q, q + kvheads * dim * 4, q + 2 * kvheads * dim * 4, qkv.shape[1], plan, batch, state, o, heads, kvheads, dim,
                     vdim, writes_state, decay=decay, gates=beta)
-        return o
-    # decays [tokens, heads * dim], then betas [tokens, heads]
-    scratch = torch.empty((n * heads * (dim + 1),), dtype=torch.float32, device=qkv.device)
+        if not walks:
+            return o
     _call("state_scan", "fms_delta_rule_scan", qkv, _ptr(proj) + beta_offset * proj.element_size(),
-          _code(proj.dtype), proj.shape[1], a_ptr, a_stride, 1 if per_head else 0, dt_bias, a_log,
-          scratch.data_ptr(),
-          scratch.data_ptr() + 4 * n * heads * dim, state, o, batch.first_row, batch.slots, n,
+          _code(proj.dtype), proj.shape[1], a_ptr, a_stride, 1 if per_head else 0, dt_bias, a_log, channels, beta, state, o,
+          batch.first_row, None if plan is None else plan.first, batch.slots, n,
           batch.n_seqs, heads, kvheads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
     global launches
-    launches += 1  # the kernel that makes q, k, the decays and the betas ready
+    launches += 1 if plan is None else 0  # the kernel that makes q, k, the decays and the betas ready
     return o
 
 
@@ -1094,7 +1101,7 @@ def gla_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: in
           _code(decay_weight.dtype), decay_bias, float(tau), decay, channels, qkv, n, cols, channels,
           float(q_scale), _stream())
     _call("state_scan", "fms_decay_scan", qkv, None, _code(proj.dtype), 0, None, 0.0, decay, None, None, state,
-          None, o, batch.first_row, batch.slots, n, batch.n_seqs, heads, dim, vdim,
+          None, o, batch.first_row, None, batch.slots, n, batch.n_seqs, heads, dim, vdim,
           1 if writes_state else 0, state.shape[0], _stream())
     return o
 
@@ -1170,12 +1177,13 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
         q = _ptr(qkv)
         _chunk_scan(1 if gated else 0, q, q + heads * dim * 4, q + 2 * heads * dim * 4, cols, plan, batch, state, o, heads, heads, dim, vdim,
                     writes_state, decay=decay, gates=gates, norm_in=norm_in, norm_state=norm_state)
-        return o
+        if plan.whole:
+            return o
     _call("state_scan", "fms_decay_scan", qkv, gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias,
-          float(gate_cap), gates, norm_in, decay, state, norm_state, o, batch.first_row,
+          float(gate_cap), gates, norm_in, decay, state, norm_state, o, batch.first_row, None if plan is None else plan.first,
           batch.slots, n, batch.n_seqs, heads, dim, vdim, 1 if writes_state else 0, state.shape[0], _stream())
     global launches
-    launches += 1 if gated else 0  # the kernel that walks the gates
+    launches += 1 if gated and plan is None else 0  # the kernel that walks the gates
     return o
 
 

@@ -171,3 +171,44 @@ def test_runs_are_no_further_from_64_bits_than_the_walk(monkeypatch, kind):
             errors.append([apart(y.double(), want), float((state[0].double() - S).norm() / S.norm())])
     for walk, runs in zip(*[[sum(e[j] for e in errors[i::2]) for j in range(2)] for i in range(2)]):
         assert walk < 1e-5 and runs <= walk, (walk, runs)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("vdim", [128, 64])
+def test_a_sequence_comes_out_alike_alone_and_among_others(kind, vdim):
+    """Sequences below and above the number of tokens from which they go run by run, together and each alone: the same bits."""
+    from fms_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(4)
+    lengths, dim, heads = [100, 300, 1, 255, 256], 128, 4
+    r = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    n = sum(lengths)
+    key_heads = 2 if kind == "space" else heads
+    rows = r(n, heads * vdim + 2 * key_heads * dim + (2 * heads if kind in ("fixed", "gated") else 0)) * 0.3
+    logits, bias, rates, skip = r(n, 2 * heads), r(heads) - 2.0, r(heads).abs(), r(heads)
+    start = r(len(lengths), heads, vdim, dim)
+    norms, gate_bias = r(len(lengths), heads, dim + 1), torch.cat([r(heads), r(heads) + 4.0])
+    decay = torch.tensor([0.999, 0.9, 0.5, 0.97]).cuda()
+
+    def scan(which):
+        x = torch.cat([rows[sum(lengths[:i]): sum(lengths[: i + 1])] for i in which])
+        z = torch.cat([logits[sum(lengths[:i]): sum(lengths[: i + 1])] for i in which])
+        batch = batch_of([lengths[i] for i in which])
+        state, norm = start[which[::-1]].clone(), norms[which[::-1]].clone()  # the slots are in the other order
+        if kind == "space":
+            y = ops.selective_scan(x, z, 0, bias, rates, skip, state, batch, heads, vdim, dim, key_heads)
+        elif kind == "delta":
+            y = ops.delta_rule_scan(x, z, 0, None, bias, rates, state, batch, heads, heads, dim, vdim, decay_offset=heads)
+        elif kind == "fixed":
+            y = ops.decay_scan(x, state, batch, heads, dim, vdim, ops.ACT_SILU, decay=decay)
+        else:
+            y = ops.decay_scan(x, state, batch, heads, dim, vdim, q_scale=dim ** -0.5, gate_offset=heads * (2 * dim + vdim),
+                               gate_bias=gate_bias, gate_cap=15.0, norm_state=norm)
+        return [(t, state[len(which) - 1 - j], norm[len(which) - 1 - j]) for j, t in enumerate(torch.split(y, [lengths[i] for i in which]))]
+
+    together = scan(list(range(len(lengths))))
+    for i in range(len(lengths)):
+        for a, b in zip(scan([i])[0], together[i]):
+            assert torch.equal(a, b)
+    for a, b in zip(scan([0, 2, 3]), (together[0], together[2], together[3])):  # none goes run by run
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
