@@ -804,6 +804,11 @@ FMS_API int fms_joint_activation(const void* o, const void* proj, int stride, in
 //   rotated q -> q_out[t]; rotated k and v -> the cache block of the token's slot and position
 // grid (token, head), one thread per pair.
 // ---------------------------------------------------------------------------------------------------
+// A pair turned; the roundings are spelled out, so that a row comes out alike in every kernel here, however many rows a step has
+__device__ __forceinline__ float2 turned(float sine, float cosine, float x0, float x1) {
+  return make_float2(__fmaf_rn(cosine, x0, -__fmul_rn(sine, x1)), __fmaf_rn(sine, x0, __fmul_rn(cosine, x1)));
+}
+
 template <typename T>
 __global__ void rope_store_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* __restrict__ inv_freq,
                                   const int* __restrict__ positions, const int* __restrict__ position_ids,
@@ -827,10 +832,9 @@ __global__ void rope_store_kernel(const T* __restrict__ qkv, T* __restrict__ q_o
     const float angle = (float)(position_ids ? position_ids[t] : pos) * inv_freq[i];
     float s, c;
     sincosf(angle, &s, &c);
-    const float r0 = c * x0 - s * x1;
-    const float r1 = s * x0 + c * x1;
-    x0 = r0;
-    x1 = r1;
+    const float2 r = turned(s, c, x0, x1);
+    x0 = r.x;
+    x1 = r.y;
   }
   if (head < nheads) {
     T* dst = q_out + (size_t)t * nheads * head_dim + (size_t)head * head_dim;
@@ -911,12 +915,13 @@ __global__ void rope_store_vec_kernel(const T* __restrict__ qkv, T* __restrict__
         const float2 sc = sincos_of_pair[piece * (PIECE / 2) + k];
         if constexpr (PIECE == 8) {
           const float x0 = __uint_as_float(w[k] << 16), x1 = __uint_as_float(w[k] & 0xffff0000u);
-          __nv_bfloat162 r = __floats2bfloat162_rn(sc.y * x0 - sc.x * x1, sc.x * x0 + sc.y * x1);
+          const float2 y = turned(sc.x, sc.y, x0, x1);
+          __nv_bfloat162 r = __floats2bfloat162_rn(y.x, y.y);
           w[k] = *reinterpret_cast<uint32_t*>(&r);
         } else {
-          const float x0 = __uint_as_float(w[2 * k]), x1 = __uint_as_float(w[2 * k + 1]);
-          w[2 * k] = __float_as_uint(sc.y * x0 - sc.x * x1);
-          w[2 * k + 1] = __float_as_uint(sc.x * x0 + sc.y * x1);
+          const float2 y = turned(sc.x, sc.y, __uint_as_float(w[2 * k]), __uint_as_float(w[2 * k + 1]));
+          w[2 * k] = __float_as_uint(y.x);
+          w[2 * k + 1] = __float_as_uint(y.y);
         }
       }
     }

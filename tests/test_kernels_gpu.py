@@ -463,6 +463,23 @@ def test_attention(ops, dtype, nheads, kvheads, hd, lens_before, num_new, window
     torch.testing.assert_close(got.float(), want.float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hd", [128, 48])
+def test_rotation_of_a_row_does_not_depend_on_how_many_rows_a_step_has(ops, dtype, hd):
+    """64 rows and more go through the vector kernel, fewer through the other: the same bits."""
+    g = torch.Generator().manual_seed(64)
+    inv = 1.0 / (10000.0 ** (torch.arange(0, hd, 2).float() / hd))
+    qkv = torch.randn(300, (5 + 2 * 2) * hd, generator=g).to(dtype).cuda()
+    outs = []
+    for n in (300, 63):
+        cache, view, batch = make_cache_case(dtype, 5, 2, hd, [1000], [n], 30, 0)
+        q = ops.rope_store(qkv[:n].contiguous(), inv.cuda(), batch, view, 5, 2, hd)
+        blocks = view.table[int(batch.slots[0]), 1000 // 64: (1000 + 63) // 64 + 1].long()
+        kept = torch.stack([t[blocks].transpose(1, 2).flatten(0, 1)[1000 % 64: 1000 % 64 + 63] for t in (view.keys, view.values)])
+        outs.append((q[:63], kept))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("nheads,kvheads,hd,window", [(4, 2, 128, 0), (3, 1, 48, 70), (2, 2, 256, 0), (5, 1, 16, 0)])
 @pytest.mark.parametrize("num_new", [[2, 15], [16, 17], [63, 64], [65, 130]])
 def test_prefill_attention_float32_at_the_edges_of_its_tiles(ops, nheads, kvheads, hd, window, num_new):
