@@ -943,7 +943,8 @@ __global__ void __launch_bounds__(TPU == 32 ? 128 : TPU) gated_group_rmsnorm_onc
                                                                                          int gate_mode, const float* weight,
                                                                                          int weight_period, float eps, float factor,
                                                                                          T* out, int n_tokens, int width, int gs) {
-  __shared__ float scratch[33];
+  constexpr bool AS_A_WARP = TPU == 256 && NI == 1;
+  __shared__ float scratch[AS_A_WARP ? 256 : 33];
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x % TPU;
@@ -968,15 +969,25 @@ __global__ void __launch_bounds__(TPU == 32 ? 128 : TPU) gated_group_rmsnorm_onc
   }
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < NI; ++i)
+  for (int i = 0; i < NI; ++i) {
+    float four = 0.f;  // a sum of its own for every four values: a block of one four a thread then adds in the warp's order
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       if (gate_mode == 1) v[i][k] *= z[i][k] * sigmoid_f(z[i][k]);
-      ss = fmaf(v[i][k], v[i][k], ss);
+      four = fmaf(v[i][k], v[i][k], four);
     }
+    ss += four;
+  }
   float total;
   if constexpr (TPU == 32) total = warp_sum(ss);
-  else total = block_sum(ss, scratch);
+  else if constexpr (AS_A_WARP) {
+    scratch[lane] = ss;
+    __syncthreads();
+    float sum = scratch[lane & 31];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) sum += scratch[i * 32 + (lane & 31)];
+    total = warp_sum(sum);
+  } else total = block_sum(ss, scratch);
   const float inv = 1.f / sqrtf(total / (float)gs + eps);
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
@@ -1368,7 +1379,8 @@ FMS_API int fms_gated_group_rmsnorm(const float* x, const void* gate, int dtype,
                                           factor, (T*)out, n_tokens, width, group_size))
   const bool once = four && weight_period % 4 == 0 && (uintptr_t)weight % 16 == 0 && group_size <= 4096;
   if (once) {
-    // a warp a group, except where few long groups would leave most of the multiprocessors without one
+    // a warp a group, except where few long groups would leave most of the multiprocessors without one; how many there are must
+    // not show in a row, so groups of 257 to 1,024 values are summed in the same order by a warp and by a block
     if (group_size <= 128) FMS_NORM_ONCE(32, 1, (units + 3) / 4, 128);
     else if (group_size <= 256) FMS_NORM_ONCE(32, 2, (units + 3) / 4, 128);
     else if (group_size <= 1024 && units >= 8 * 148) FMS_NORM_ONCE(32, 8, (units + 3) / 4, 128);

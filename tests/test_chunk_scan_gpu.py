@@ -212,3 +212,25 @@ def test_a_sequence_comes_out_alike_alone_and_among_others(kind, vdim):
             assert torch.equal(a, b)
     for a, b in zip(scan([0, 2, 3]), (together[0], together[2], together[3])):  # none goes run by run
         assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("group", [128, 132, 260, 512, 1000, 1024, 1028])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_row_is_normed_alike_alone_and_among_many(group, dtype):
+    """Few long groups take a block each, many a warp each: the same bits."""
+    from fms_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(group)
+    x, gate, w = (torch.randn(*s, generator=g).cuda() for s in ((700, 2 * group), (700, 2 * group), (2 * group,)))
+    gate = gate.to(dtype)
+    for mode in (ops.GATE_SILU_BEFORE, ops.GATE_SIGMOID_AFTER):
+        norm = lambda n: ops.gated_group_rmsnorm(x[:n].contiguous(), gate[:n].contiguous(), 0, mode, w, 1e-5, group, dtype)  # noqa: E731
+        many = norm(700)
+        assert torch.equal(norm(3), many[:3])
+        y = x[:3].double() * torch.nn.functional.silu(gate[:3].double()) if mode == ops.GATE_SILU_BEFORE else x[:3].double()
+        y = y.view(3, 2, group)
+        y = (y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)).flatten(1) * w.double()
+        if mode == ops.GATE_SIGMOID_AFTER:
+            y = y * torch.sigmoid(gate[:3].double())
+        eps = 2.0 ** -8 if dtype == torch.bfloat16 else 16 * 2.0 ** -24
+        assert float((many[:3].double() - y).abs().max()) <= eps * float(y.abs().max())
