@@ -59,6 +59,7 @@ struct RowArgs {
   const int* offsets;          // [groups + 1]
   float scale, cap;
   long x_row = 0, x_group = 0, y_row = 0, y_group = 0;  // STRIDED: values from row to row and from group to group
+  long y_values = 0;  // STRIDED: extent of y, for the bounds-checked build (0: not known)
 };
 enum Groups { ALONE = 0, GROUPED = 1, STRIDED = 2 };
 
@@ -319,8 +320,9 @@ __global__ void __launch_bounds__(THREADS) linear_skinny_kernel(const __nv_bfloa
           v *= extra.scale;
           if (extra.cap > 0.f) v = extra.cap * tanhf(v / extra.cap);
         }
-        if (GROUPS == STRIDED) y[(size_t)m * extra.y_row + row] = from_f32<TOut>(v);
-        else if (FMS_IN((size_t)m * N + row, (size_t)M * N)) y[(size_t)m * N + row] = from_f32<TOut>(v);
+        if (GROUPS == STRIDED) {
+          if (FMS_IN(blockIdx.y * extra.y_group + (long)m * extra.y_row + row, extra.y_values)) y[(size_t)m * extra.y_row + row] = from_f32<TOut>(v);
+        } else if (FMS_IN((size_t)m * N + row, (size_t)M * N)) y[(size_t)m * N + row] = from_f32<TOut>(v);
       }
     }
   }
@@ -419,14 +421,14 @@ FMS_API int fms_grouped_bf16_skinny(const void* x, const void* w, void* y, const
 }
 
 // A product a group for up to 8 rows: y[r, g * y_group + :N] = x[r, g * x_group + :K] w[g]^T, w [groups, N, K]; rows of x
-// x_row values apart and of y y_row.
+// x_row values apart and of y y_row.  y_values: how many y has (0: not known).
 FMS_API int fms_strided_bf16_skinny(const void* x, const void* w, void* y, int M, int groups, int N, int K, long x_row, long x_group,
-                                    long y_row, long y_group, cudaStream_t stream) {
+                                    long y_row, long y_group, long y_values, cudaStream_t stream) {
   if (M <= 0 || groups <= 0 || N <= 0) return 0;
   if (M > 8 || groups > 65535 || K <= 0 || K % 8 || x_row % 8 || x_group % 8 || (uintptr_t)x % 16)
     return fms_fail("strided_bf16_skinny: %d rows, %d groups, K %d, rows %ld and groups %ld values apart", M, groups, K, x_row, x_group);
   RowArgs extra{nullptr, nullptr, 0, UNIT_NONE, nullptr, 1.f, 0.f};
-  extra.x_row = x_row; extra.x_group = x_group; extra.y_row = y_row; extra.y_group = y_group;
+  extra.x_row = x_row; extra.x_group = x_group; extra.y_row = y_row; extra.y_group = y_group; extra.y_values = y_values;
   // short rows of w: 32 of them a block, so that a block has something to read
   if (K <= 256 && N >= 64) return launch_typed<1, 2, ROWS16, __nv_bfloat16, STRIDED>(x, w, nullptr, y, M, N, K, 0, 0, stream, RopeArgs{}, extra, groups);
   return launch_typed<1, 1, ROWS16, __nv_bfloat16, STRIDED>(x, w, nullptr, y, M, N, K, 0, 0, stream, RopeArgs{}, extra, groups);

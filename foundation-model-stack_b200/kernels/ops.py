@@ -47,7 +47,7 @@ _SIGNATURES = {
     "fms_linear_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     "fms_token_gate_bf16_skinny": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fms_grouped_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _F, _F, _P],
-    "fms_strided_bf16_skinny": [_P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _L, _P],
+    "fms_strided_bf16_skinny": [_P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _L, _L, _P],
     "fms_linear_act_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     "fms_linear_cap_bf16_skinny": [_P, _P, _P, _I, _I, _I, _F, _F, _P],
     "fms_glu_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
@@ -1235,7 +1235,7 @@ def grouped_linear(x: torch.Tensor, weight: torch.Tensor, groups: int, rows: int
         # a decode step of few rows: the weight-streaming kernel, a block per group and run of its matrix's rows (8 rows, 32
         # groups of 512 x 96: 4.7 us, of 128 x 512: 3.5; the two 27 with a warp a row of the matrix)
         _call("gemm_bf16_skinny", "fms_strided_bf16_skinny", x, weight, y, rows, groups, n_out, k, x_row_stride,
-              x_group_offset, y_row_stride, y_group_offset, _stream())
+              x_group_offset, y_row_stride, y_group_offset, y.numel(), _stream())
         return y
     _call("grouped", "fms_grouped_linear", x, weight, y, _code(x.dtype), None, None, None, groups, rows,
           n_out, k, x_row_stride, x_group_offset, y_row_stride, y_group_offset, 0, 0.0, 0.0,

@@ -47,6 +47,23 @@ ops.check_error_flag("cuda")                              # the record was clear
 print("recorded and skipped")
 '''
 
+RECORDS_A_STORE = r'''
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+from fms_b200.kernels import build, ops
+assert build.DEBUG_BOUNDS
+groups, n, k, rows = 3, 64, 64, 2
+storage = torch.zeros(rows * groups * n, dtype=torch.bfloat16, device="cuda")  # three groups are really there
+x, w = (torch.ones(*s, dtype=torch.bfloat16, device="cuda") for s in ((rows, groups * k), (groups, n, k)))
+ops.grouped_linear(x, w, groups, rows, n, k, groups * k, k, storage[: groups * n + 2 * n], groups * n, n)  # one row and two groups are declared
+torch.cuda.synchronize()
+text = " ".join(build.bounds_violations())
+assert "gemm_bf16_skinny: 64 accesses" in text and "extent 320" in text, text
+assert float(storage[:320].float().sum()) == 320 * k and float(storage[320:].float().abs().sum()) == 0.0
+assert build.bounds_violations() == []
+print("recorded and skipped")
+'''
+
 GENERATES = r'''
 import sys, tempfile, torch
 sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[1] + "/tests")
@@ -73,6 +90,12 @@ print("generated")
 
 def _run(code):
     return subprocess.run([sys.executable, "-c", code, ROOT], env=ENV, capture_output=True, text=True, timeout=1500)
+
+
+@pytest.mark.expects_a_recorded_index
+def test_a_store_outside_a_product_a_groups_result_is_recorded_and_skipped():
+    r = _run(RECORDS_A_STORE)
+    assert r.returncode == 0 and "recorded and skipped" in r.stdout, r.stdout + r.stderr
 
 
 @pytest.mark.expects_a_recorded_index
