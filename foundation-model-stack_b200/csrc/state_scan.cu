@@ -1070,14 +1070,15 @@ FMS_API int fms_scan_chunk_tokens() { return CH; }
 
 FMS_API int fms_causal_conv(const void* x, int dtype, int stride, const float* w, const float* bias, float* tail,
                             const int* token_seq, const int* first_row, const int* slots, float* out, int n_tokens,
-                            int n_seqs, int channels, int taps, int act, int write_state, int n_slots,
-                            cudaStream_t stream) {
+                            int n_seqs, int channels, int taps, int act, int write_state, int n_slots, int decode,
+                            cudaStream_t stream) {  // decode: every sequence brings exactly one row
   if (n_tokens <= 0) return 0;
+  if (decode && n_tokens != n_seqs) return fms_fail("causal_conv: a decode step of %d rows for %d sequences", n_tokens, n_seqs);
   if (taps < 1 || taps > MAX_TAPS) return fms_fail("causal_conv: %d taps (1..%d)", taps, MAX_TAPS);
   const size_t item = dtype == FMS_BF16 ? 2 : 4;
   const bool four = channels % 4 == 0 && stride % 4 == 0 && (uintptr_t)x % (4 * item) == 0 && (uintptr_t)out % 16 == 0;
   const unsigned across = (channels / (four ? 4 : 1) + CONV_THREADS - 1) / CONV_THREADS;
-  if (n_tokens == n_seqs && n_tokens <= 65535) {  // every sequence brings at least one row, so each brings one
+  if (decode && n_tokens <= 65535) {
     const bool four_tail = four && (uintptr_t)tail % 16 == 0;
     const dim3 grid((channels / (four_tail ? 4 : 1) + CONV_THREADS - 1) / CONV_THREADS, n_tokens);
 #define FMS_CONV(CPT, TMAX)                                                                                                        \

@@ -106,7 +106,7 @@ _SIGNATURES = {
                                     _P, _P, _P, _I, _F, _P, _L, _P],
     "fms_attention_decode_sink": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I, _I, _I, _L,
                                   _P, _P, _P, _P],
-    "fms_causal_conv": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "fms_causal_conv": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_selective_scan": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_delta_rule_scan": [_P, _P, _I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "fms_gated_group_rmsnorm": [_P, _P, _I, _I, _I, _P, _I, _F, _F, _P, _I, _I, _I, _P],
@@ -915,11 +915,13 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
             or tuple(tail.shape[1:]) != (taps - 1, channels) or (bias is not None and bias.dtype != torch.float32):
         raise KernelError("causal_conv: weight [channels, taps], bias and tail [slots, taps - 1, channels] are float32")
     out = torch.empty((n, channels), dtype=torch.float32, device=x.device)
+    decode = batch.decode and n == batch.n_seqs and n <= 65535  # as many rows as sequences alone may be two of one and none of another
     _call("state_scan", "fms_causal_conv", _ptr(x) + offset * x.element_size(), _code(x.dtype), x.shape[1], weight,
           bias, tail, batch.token_seq, batch.first_row, batch.slots, out, n,
-          batch.n_seqs, channels, taps, 1 if activation else 0, 1 if writes_state else 0, tail.shape[0], _stream())
+          batch.n_seqs, channels, taps, 1 if activation else 0, 1 if writes_state else 0, tail.shape[0],
+          1 if decode else 0, _stream())
     global launches
-    launches += 1 if writes_state and taps > 1 else 0
+    launches += 1 if writes_state and taps > 1 and not decode else 0  # the tails' kernel (a decode step's does both)
     return out
 
 

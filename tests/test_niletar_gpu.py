@@ -140,6 +140,32 @@ def test_norm_after_the_sum(dtype, dim):
             assert torch.equal(copy.cpu(), r.cpu().to(dt))
 
 
+@pytest.mark.parametrize("counts", [[2, 0], [0, 2], [1, 0], [1, 0, 2], [1, 1], [3, 0, 0, 1]])
+def test_causal_convolution_of_steps_with_sequences_that_bring_nothing(counts):
+    """As many rows as sequences do not make a decode step.  Every sequence against itself in a step of its own, which is a step
+    of one or more rows of one sequence; the kernels launched are counted."""
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(len(counts))
+    channels, taps, n = 40, 4, sum(counts)
+    x, w, b = (torch.randn(*s, generator=g).cuda() for s in ((n, channels), (channels, taps), (channels,)))
+    tails = torch.randn(len(counts), taps - 1, channels, generator=g).cuda()
+    batch_of = lambda slots, some: Batch.from_lists(slots, [5] * len(some), [[0] * c for c in some], [[]] * len(some), "cuda")  # noqa: E731
+    left, before = tails.clone(), ops.launches
+    y = ops.causal_conv(x, 0, channels, w, b, left, batch_of(list(range(len(counts))), counts))
+    assert ops.launches - before == (1 if counts == [1, 1] else 2)
+    at = 0
+    for i, c in enumerate(counts):
+        if c:
+            alone = tails.clone()
+            assert torch.equal(ops.causal_conv(x[at: at + c].contiguous(), 0, channels, w, b, alone, batch_of([i], [c])), y[at: at + c])
+            assert torch.equal(alone[i], left[i])
+        else:
+            assert torch.equal(tails[i], left[i])
+        at += c
+
+
 @pytest.mark.parametrize("dtype", ["fp32", "bf16"])
 @pytest.mark.parametrize("taps", [1, 2, 4, 7])
 def test_causal_convolution_with_tails(dtype, taps):
