@@ -35,20 +35,19 @@
 // and chunk_outputs takes U for the values (b = 1).
 //
 // So that neither an output nor a state is further from 64 bits than the walk's: scores (and k . k) are summed in 64 bits and
-// rounded once, as products of decays are; an output's sums over channels and tokens are made of float32 runs of 16 terms that
-// 64 bits add up; u's of float32 runs of 16 terms.  A run's part of the state and of the normalizer is one float32 chain of its
-// 64 tokens.  Errors of outputs and of states as parts of the walk's (400 and 2,048 tokens): fixed decays 0.77 and 0.94, 0.46 and
-// 0.41; under a normalizer 0.88 and 0.83, 0.96 and 0.98; state space 0.95 and 0.96, 0.85 and 0.80; delta rule 0.97 and 0.86, 0.87 and
-// 0.77.  (With float32 sums throughout, outputs 1.05 to 1.15 of it and layers 7 to 10% faster: prompts of 1,062 and 638 tokens,
-// 32 heads of 128 with a normalizer, 498 instead of 550 us; one of 2,048, 128 heads of 64, 779 instead of 856.)
+// rounded once, as products of decays are; the other sums of an output and of a u are made of float32 runs of 16 terms, which
+// under fixed decays 64 bits add up.  A run's part of the state and of the normalizer is one float32 chain of its 64 tokens.
+// Errors of outputs and of states as parts of the walk's (400 and 2,048 tokens): fixed decays 0.77 and 0.94, 0.46 and 0.41; under a
+// normalizer 0.88 and 0.83, 0.96 and 0.98; state space 0.98 and 0.99, 0.85 and 0.80; delta rule 0.99 and 0.90, 0.87 and 0.77.  (With
+// float32 sums throughout outputs were at 1.05 to 1.15 of it, and a layer of 2,048 tokens under fixed decays took 531 us instead of
+// 590, prompts of 1,062 and 638 tokens with a normalizer 503 instead of 516.)
 #include "common.cuh"
 
 namespace {
 constexpr int C = 64;        // tokens of a run
 constexpr int COLS = 128;    // value columns of a block of outputs: one head of 128 values or two of 64
 constexpr int DIM = 128;     // key channels
-constexpr int PART = 16;     // terms of an output that float32 takes together before 64 bits add them to the rest
-constexpr int UPART = 16;    // terms of a delta rule's u that are taken together before they are added to the rest
+constexpr int PART = 16;     // terms that a sum takes together before they are added to the rest: a single chain loses more
 constexpr int SLICE = 16, SROW = SLICE + 2;  // of the scores: channels brought into shared memory at a time, rows padded by two
 constexpr int TROW = C + 4, CROW = COLS + 4; // rows of 64 tokens, of 128 columns, padded by four floats
 
@@ -404,13 +403,77 @@ __global__ void __launch_bounds__(128, 2) chunk_states_kernel(ChunkArgs g) {
 // asynchronous copies), then the run's own tokens: P^T, a thread a token t walking s downwards.  A warp's 64 columns belong to one
 // head; it takes the tokens up to its last row, earlier rows with zeros of P (or, where a value is not finite, by selection).
 constexpr int OSLICE = 16;  // channels brought into shared memory at a time
+// whether 64 bits add up the float32 runs of terms: where float32 would leave outputs further from 64 bits than the walk's
+template <int KIND> constexpr bool WIDE = KIND == 0;
 template <int VDIM>
 constexpr size_t OUT_SMEM = (size_t)(C * CROW + COLS / VDIM * C * TROW) * sizeof(float);
 static_assert(OSLICE == PART);
 static_assert(2 * OSLICE * (TROW + CROW) <= C * CROW, "the slices lie where the values go afterwards");
 
+// A thread's 8 x 8 sums of runs of terms, in float32 pairs as outer_step leaves them, or in 64 bits
+template <bool IN_64_BITS> struct RunSums {
+  f32x2 sum[4][8];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[i][j] = 0;
+  }
+  __device__ __forceinline__ void add(f32x2 (&part)[4][8]) {  // and part is cleared
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        sum[i][j] = add2(sum[i][j], part[i][j]);
+        part[i][j] = 0;
+      }
+  }
+  __device__ __forceinline__ void scale(const float* of_row) {  // row i's factor at (i & 3) + (i >> 2) * 16
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* f = of_row + (i >> 1) * 16 + (i & 1) * 2;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[i][j] = fma2(sum[i][j], pack2(f[0], f[1]), 0ull);
+    }
+  }
+  __device__ __forceinline__ void get(float (&out)[8][8]) const { outer_unpack<4>(sum, out); }
+};
+template <> struct RunSums<true> {
+  double sum[8][8];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[i][j] = 0.0;
+  }
+  __device__ __forceinline__ void add(f32x2 (&part)[4][8]) {
+    float own[8][8];
+    outer_unpack<4>(part, own);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[i][j] += (double)own[i][j];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) part[i][j] = 0;
+  }
+  __device__ __forceinline__ void scale(const float* of_row) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[i][j] *= (double)of_row[(i & 3) + (i >> 2) * 16];
+  }
+  __device__ __forceinline__ void get(float (&out)[8][8]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) out[i][j] = (float)sum[i][j];
+  }
+};
+
 template <int VDIM, int KIND>
-__global__ void __launch_bounds__(128, 2) chunk_outputs_kernel(ChunkArgs g) {
+__global__ void __launch_bounds__(128, WIDE<KIND> ? 2 : 3) chunk_outputs_kernel(ChunkArgs g) {
   constexpr int HB = COLS / VDIM;
   extern __shared__ __align__(16) float sm[];
   float* qs = sm;                                 // [2][OSLICE][TROW], then the values [C][CROW] over both
@@ -478,23 +541,8 @@ __global__ void __launch_bounds__(128, 2) chunk_outputs_kernel(ChunkArgs g) {
   const int tm = (warp >> 1) * 32 + (lane >> 3) * 4, tn = (warp & 1) * 64 + (lane & 7) * 4;
   const int my_head = (warp & 1) * 64 / VDIM;  // of the block's
   f32x2 part[4][8];
-  double acc[8][8];
-  auto add_part = [&]() {
-    float own[8][8];
-    outer_unpack<4>(part, own);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] += (double)own[i][j];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) part[i][j] = 0;
-  };
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+  RunSums<WIDE<KIND>> sums;
+  sums.clear();
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -515,7 +563,7 @@ __global__ void __launch_bounds__(128, 2) chunk_outputs_kernel(ChunkArgs g) {
     const float* y = ss + buf * OSLICE * CROW;
 #pragma unroll
     for (int d = 0; d < OSLICE; ++d) outer_step<4, 16, 32>(x + d * TROW + tm, y + d * CROW + tn, part);
-    add_part();
+    sums.add(part);
     if (KIND == 1 && tid < C) {
 #pragma unroll
       for (int d = 0; d < OSLICE; ++d) own_nq = fma((double)x[d * TROW + tid], (double)n_before[d0 + d], own_nq);
@@ -528,34 +576,30 @@ __global__ void __launch_bounds__(128, 2) chunk_outputs_kernel(ChunkArgs g) {
     copy16(sm + t * CROW + c, g.v + (size_t)(row0 + min(t, rows - 1)) * g.v_row + (size_t)head0 * VDIM + c, t < rows);
   }
   copies_commit();
-  // G_t times what the state gives
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const double gt = G[my_head][tm + (i >> 2) * 16 + (i & 3)];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] *= gt;
-  }
+  sums.scale(G[my_head] + tm);  // G_t times what the state gives
   if (KIND == 1 && tid < C) nq[tid] = (float)fma((double)G[0][tid], own_nq, p_sum);  // n_t . q_t
   const bool bad = g.flags[(size_t)local * g.heads + head0 + my_head] != 0;
   copies_wait<0>();
   __syncthreads();
   const float* p = Pt + my_head * C * TROW + tm;
   const int reach = (warp >> 1) * 32 + 32;
+  float acc[8][8];
   if (!bad) {
 #pragma unroll 1
     for (int s0 = 0; s0 < reach; s0 += PART) {
 #pragma unroll 8
       for (int s = s0; s < s0 + PART; ++s) outer_step<4, 16, 32>(p + s * TROW, sm + s * CROW + tn, part);
-      add_part();
+      sums.add(part);
     }
+    sums.get(acc);
   } else {
+    sums.get(acc);
     for (int s = 0; s < reach; ++s)
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         if (s <= tm + (i & 3) + (i >> 2) * 16) {
-          const double w = p[s * TROW + (i & 3) + (i >> 2) * 16];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fma(w, (double)sm[s * CROW + tn + (j & 3) + (j >> 2) * 32], acc[i][j]);
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(p[s * TROW + (i & 3) + (i >> 2) * 16], sm[s * CROW + tn + (j & 3) + (j >> 2) * 32], acc[i][j]);
         }
   }
 #pragma unroll
@@ -568,7 +612,7 @@ __global__ void __launch_bounds__(128, 2) chunk_outputs_kernel(ChunkArgs g) {
     float* out = g.o + (size_t)(row0 + t) * g.heads * VDIM + (size_t)head0 * VDIM + tn;
 #pragma unroll
     for (int j = 0; j < 8; j += 4) {
-      float4 x = make_float4((float)acc[i][j], (float)acc[i][j + 1], (float)acc[i][j + 2], (float)acc[i][j + 3]);
+      float4 x = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
       if (KIND == 1) x = make_float4(x.x * scale, x.y * scale, x.z * scale, x.w * scale);
       if (KIND == 2) {
         const float4 v = *reinterpret_cast<const float4*>(sm + t * CROW + tn + (j >> 2) * 32);
@@ -779,9 +823,9 @@ __global__ void __launch_bounds__(128, 2) delta_states_kernel(ChunkArgs g) {
     for (int i = 0; i < 4; ++i) U[i][0] = U[i][1] = part[i][0] = part[i][1] = 0.f;
     const int reach = (tid >> 5) * 16 + 16;
 #pragma unroll 1
-    for (int s0 = 0; s0 < reach; s0 += UPART) {
+    for (int s0 = 0; s0 < reach; s0 += PART) {
 #pragma unroll
-      for (int s = s0; s < s0 + UPART; ++s) {
+      for (int s = s0; s < s0 + PART; ++s) {
         const float4 x = *reinterpret_cast<const float4*>(ts + s * TROW + ut);
         const float2 y = *reinterpret_cast<const float2*>(vs + s * DVT + uc);
         const float xs[4] = {x.x, x.y, x.z, x.w};
