@@ -501,12 +501,13 @@ def test_a_product_a_group_takes_matrices_that_the_product_before_it_made():
 def test_attention_in_the_heads_own_space_rounds_values_that_are_alike_once(hd):
     """A few keys whose values are nearly the same: the probabilities are rounded to bfloat16, and unless they are summed as
     rounded, every row is off by what their roundings come to.  Against the same keys and values in 64 bits, no further off
-    than rounding the result to bfloat16 alone, but for a twentieth."""
+    than rounding the result to bfloat16 alone, but for 3% (unless they are summed as rounded 11%: for two to four keys the
+    probabilities' roundings come to half of the result's)."""
     from fms_b200.cache import Cache, KVRequest
     from fms_b200.engine.batch import Batch
     from fms_b200.kernels import ops
 
-    heads, width, n = 32, 72, 12
+    heads, width, n = 128, 72, 4
     g = torch.Generator().manual_seed(hd)
     cache = Cache([KVRequest(1, width, 0, planes=1)], 64, 64, torch.bfloat16, "cuda", max_slots=1)
     slots = cache.begin(1)
@@ -518,7 +519,7 @@ def test_attention_in_the_heads_own_space_rounds_values_that_are_alike_once(hd):
     view.keys[int(view.table[slots[0], 0]), 0, :n] = rows
     expand = torch.randn(heads, 2 * hd, width, generator=g) * 0.3
     expand[:, hd:] *= 0.03
-    expand[:, hd:, 0] = 1.5
+    expand[:, hd:, 0] = 1.9
     expand = expand.to(torch.bfloat16).cuda()
     q = torch.randn(n, heads, hd, generator=g).to(torch.bfloat16).cuda()
     got = ops.latent_attention_expanded(q, batch, view, expand, None, heads, hd, hd ** -0.5).view(n, heads, hd).double()
@@ -526,4 +527,4 @@ def test_attention_in_the_heads_own_space_rounds_values_that_are_alike_once(hd):
     scores = torch.einsum("ihd,jhd->hij", q.double(), k) * hd ** -0.5
     scores = scores.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
     want = torch.einsum("hij,jhd->ihd", torch.softmax(scores, -1), v)
-    assert float((got - want).norm()) <= 1.05 * float((want.to(torch.bfloat16).double() - want).norm())
+    assert float((got - want).norm()) <= 1.03 * float((want.to(torch.bfloat16).double() - want).norm())
