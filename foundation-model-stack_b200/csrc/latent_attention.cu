@@ -25,7 +25,7 @@ __device__ __forceinline__ int ld_fresh(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_fresh(const float* p) { return __ldcg(p); }
 
 namespace {
-constexpr int SPLIT = 256;  // keys of one split of a decode step
+constexpr int SPLIT = 256;  // keys of one split of a decode step: fixed, so a sequence's sums depend on its length only
 constexpr int KT = 32;      // keys brought into shared memory at a time
 constexpr int HG = 8;       // heads a block takes
 constexpr int THREADS = 256;
@@ -207,8 +207,11 @@ struct LatentArgs {
   int table_stride, block_tokens, heads, rank, rot, n_splits, n_seqs, n_slots, n_blocks;
   float scale;
   int window;  // > 0: the row at position p sees the keys p - window + 1 .. p only
-  int split;  // keys of a split: a multiple of 32
+  int split, short_split, short_up_to;  // keys of a split, a multiple of 32: short_split for a row at a position before short_up_to
 };
+
+// A row's own place decides, so that its sums do not depend on what else is in the step.
+__device__ __forceinline__ int split_of(const LatentArgs& a, int pos) { return pos < a.short_up_to ? a.short_split : a.split; }
 
 // One block per (row, split of keys, group of HG heads).  Keys come KT at a time into shared memory as float32; a warp
 // takes the scores of one head (a lane a key), then 32 threads a head take the sums over the keys for rank / 32
@@ -344,8 +347,8 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(LatentArgs a) {
   __shared__ float factor;
   const int t = blockIdx.x, h = blockIdx.y;
   const int pos = ld_fresh(a.positions + t);
-  const int used = min(a.n_splits, pos / a.split + 1);
-  const int s_lo = a.window > 0 ? min(max(0, pos - a.window + 1) / a.split, used - 1) : 0;  // splits before the window hold nothing
+  const int split = split_of(a, pos), used = min(a.n_splits, pos / split + 1);
+  const int s_lo = a.window > 0 ? min(max(0, pos - a.window + 1) / split, used - 1) : 0;  // splits before the window hold nothing
   const size_t at = ((size_t)t * a.heads + h) * a.n_splits;
   const bool held = used - s_lo <= HELD;
   float m = a.sink ? to_f32(((const TS*)a.sink)[h]) : -INFINITY;
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(LatentArgs a) {
 // flash-attention kernel) and the sum; (C) warp w adds P . c for 16 rows and a quarter of the latent's columns
 // (rank / 4, its share of the accumulator in registers), c being read as it lies in the key tile.
 // With n_splits > 1 (a decode step: tq = 1, the block's rows are one token's heads) block z takes the keys of split z
-// (a.split keys) and leaves its unnormed sums, maximum and sum for latent_combine_kernel.
+// (split_of keys) and leaves its unnormed sums, maximum and sum for latent_combine_kernel.
 constexpr int MR = 32, MK = 32;
 
 __device__ __forceinline__ void lat_mma(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -452,8 +455,9 @@ __global__ void __launch_bounds__(256) latent_prefill_mma_kernel(LatentArgs a, c
   const int last_pos = ld_fresh(a.positions + first + ntok - 1);
   const int first_pos = ld_fresh(a.positions + first);
   const int seen = a.window > 0 ? max(0, first_pos - a.window + 1) : 0;  // the first key that any row of the tile sees
-  const int kt_lo = max(a.n_splits > 1 ? split * (a.split / MK) : 0, seen / MK);
-  const int n_kt = a.n_splits > 1 ? min(last_pos / MK + 1, (split + 1) * (a.split / MK)) : last_pos / MK + 1;
+  const int tiles_of_split = split_of(a, last_pos) / MK;
+  const int kt_lo = max(a.n_splits > 1 ? split * tiles_of_split : 0, seen / MK);
+  const int n_kt = a.n_splits > 1 ? min(last_pos / MK + 1, (split + 1) * tiles_of_split) : last_pos / MK + 1;
   if (kt_lo >= n_kt) return;  // a split beyond the sequence or before the window: the merge does not look at it
   if (tid < MR) {
     const int tok = tid / hb, hh = tid - tok * hb;
@@ -706,7 +710,7 @@ FMS_API int fms_latent_attention(const void* q, void* out, int dtype, const void
   a.table_stride = table_stride; a.block_tokens = block_tokens; a.heads = heads; a.rank = rank; a.rot = rot;
   a.n_splits = n_splits; a.n_seqs = n_seqs; a.n_slots = n_slots; a.n_blocks = n_blocks; a.scale = scale;
   a.window = window > 0 ? window : 0;
-  a.split = SPLIT;
+  a.split = SPLIT; a.short_split = 0; a.short_up_to = 0;
   FMS_DISPATCH_DTYPE(dtype, T, FMS_DISPATCH_DTYPE(sink ? sink_dtype : dtype, TS, return launch_attention<T, TS>(a, n_tokens, stream)));
   return 0;
 }
@@ -720,9 +724,10 @@ FMS_API int fms_latent_attention_prefill_bf16(const void* q, void* out, const vo
                                               const int* positions, const int* tiles, int n_tiles, int tile_tokens,
                                               int heads_per_block, int heads, int rank, int rot, float scale, int n_seqs,
                                               int n_slots, int n_blocks, const int* token_seq, int n_splits, int split_tokens,
-                                              float* part_o, float* part_ml, int window, cudaStream_t stream) {
+                                              int short_split_tokens, int short_up_to, float* part_o, float* part_ml, int window, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
-  if (n_splits > 1 && (split_tokens <= 0 || split_tokens % MK)) return fms_fail("latent_attention_prefill: splits of %d keys", split_tokens);
+  if (n_splits > 1 && (split_tokens <= 0 || split_tokens % MK || (short_up_to > 0 && (short_split_tokens <= 0 || short_split_tokens % MK))))
+    return fms_fail("latent_attention_prefill: splits of %d keys, %d up to %d", split_tokens, short_split_tokens, short_up_to);
   if (n_splits < 1 || (n_splits > 1 && (tile_tokens != 1 || part_o == nullptr || part_ml == nullptr || token_seq == nullptr)))
     return fms_fail("latent_attention_prefill: %d splits need one token a tile and scratch", n_splits);
   const int width = rank + rot;
@@ -734,7 +739,7 @@ FMS_API int fms_latent_attention_prefill_bf16(const void* q, void* out, const vo
   a.table_stride = table_stride; a.block_tokens = block_tokens; a.heads = heads; a.rank = rank; a.rot = rot;
   a.n_splits = n_splits; a.n_seqs = n_seqs; a.n_slots = n_slots; a.n_blocks = n_blocks; a.scale = scale;
   a.window = window > 0 ? window : 0;
-  a.split = split_tokens;
+  a.split = split_tokens; a.short_split = short_split_tokens; a.short_up_to = short_up_to;
   const int rowb = width * 2 + 16;
   const size_t smem = (size_t)(MR + 2 * MK) * rowb + MR * (MK + 1) * 4 + MR * (MK * 2 + 16) + MR * 16;
   dim3 grid(n_tiles, (heads + heads_per_block - 1) / heads_per_block, n_splits);

@@ -71,7 +71,7 @@ _SIGNATURES = {
     "fms_relu_squared": [_P, _I, _L, _P],
     "fms_gated_clamped": [_P, _P, _I, _I, _I, _F, _F, _P],
     "fms_latent_attention_prefill_bf16": [_P, _P, _P, _P, _L, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
-                                          _F, _I, _I, _I, _P, _I, _I, _P, _P, _I, _P],
+                                          _F, _I, _I, _I, _P, _I, _I, _I, _I, _P, _P, _I, _P],
     "fms_latent_gather": [_P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _I, _I, _I, _P],
     "fms_attention_prefill_rows": [_P, _L, _P, _L, _P, _P, _L, _I, _L, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P, _L, _P, _P],
     "fms_latent_prepare": [_P, _I, _I, _P, _I, _I, _I, _P, _I, _F, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
@@ -1362,7 +1362,10 @@ def route_gather(ys: torch.Tensor, routing: Routing, every: Optional[torch.Tenso
 
 # ---- attention over cached latents -------------------------------------------------------------------
 _latent_split = None
-LATENT_SHORT_SPLIT = 64  # keys of a split of the tensor-core kernel in a decode step of few sequences
+# Keys of a split of the tensor-core kernel in a decode step: LATENT_SHORT_SPLIT for a row that sees up to LATENT_SHORT_UP_TO,
+# else 256.  A block walks its split's keys one tile after the other (0.15 us a key), so short splits end sooner; long rows have
+# blocks enough, and each split costs its partial result.  8 sequences of 1,024 keys: 35 us in splits of 256, 19 of 64.
+LATENT_SHORT_SPLIT, LATENT_SHORT_UP_TO = 64, 2048
 USE_LATENT_MMA = os.environ.get("FMS_B200_LATENT_MMA", "1") != "0"  # 0: a prompt's rows through the float32 kernel too
 
 
@@ -1476,15 +1479,11 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
         n_splits, part_o, part_ml, split = 1, None, None, _latent_split
         if batch.decode:
             heads_per_block = 32
-            # a block walks its split's keys one tile after the other (0.15 us a key): where the splits would leave
-            # multiprocessors without a block, splits of 64 keys instead of 256 (8 x 1,024 keys: 35 -> 19 us)
-            if n * ((batch.max_len_after + split - 1) // split) * ((heads + 31) // 32) < 148:
-                split = LATENT_SHORT_SPLIT
-            n_splits = max(1, (batch.max_len_after + split - 1) // split)
-            if n_splits > 1:
-                parts = torch.empty((n * heads * n_splits * (rank + 2),), dtype=torch.float32, device=q_full.device)
-                part_o = parts.data_ptr()  # [rank] of every split, then its maxima and sums [2]
-                part_ml = part_o + n * heads * n_splits * rank * 4
+            # two at least: the merge rounds its results its own way, and the longest row must not decide for the others
+            n_splits = max(2, -(-min(batch.max_len_after, LATENT_SHORT_UP_TO) // LATENT_SHORT_SPLIT), -(-batch.max_len_after // split))
+            parts = torch.empty((n * heads * n_splits * (rank + 2),), dtype=torch.float32, device=q_full.device)
+            part_o = parts.data_ptr()  # [rank] of every split, then its maxima and sums [2]
+            part_ml = part_o + n * heads * n_splits * rank * 4
         else:
             heads_per_block = 1
             while heads_per_block < min(32, heads):
@@ -1497,7 +1496,7 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
               view.table, view.table.shape[1], view.block_tokens, batch.slots, batch.first_row,
               batch.positions, tiles, tiles.shape[0], tile_tokens, heads_per_block, heads, rank, rot,
               float(scale), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], batch.token_seq, n_splits, split,
-              part_o, part_ml, int(window), _stream())
+              LATENT_SHORT_SPLIT, LATENT_SHORT_UP_TO, part_o, part_ml, int(window), _stream())
         if n_splits > 1:
             launches += 1
         return out

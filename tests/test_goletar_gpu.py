@@ -528,3 +528,41 @@ def test_attention_in_the_heads_own_space_rounds_values_that_are_alike_once(hd):
     scores = scores.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
     want = torch.einsum("hij,jhd->ihd", torch.softmax(scores, -1), v)
     assert float((got - want).norm()) <= 1.03 * float((want.to(torch.bfloat16).double() - want).norm())
+
+
+@pytest.mark.parametrize("window", [0, 300])
+@pytest.mark.parametrize("sink", [True, False])
+def test_latent_decode_of_a_row_does_not_depend_on_the_others(window, sink):
+    """Rows whose splits are 64 keys and rows whose splits are 256, below and at the edges of one split, alone and together, and
+    among so many others that the step has blocks enough: the same bits; against the float32 kernel within bfloat16's rounding
+    of probabilities and results."""
+    from fms_b200.cache import Cache, KVRequest
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    heads, rank, rot = 32, 128, 32
+    lengths = [1, 5, 64, 65, 256, 700, 2047, 2048, 2049, 3000] + [900] * 40
+    g = torch.Generator().manual_seed(7)
+    cache = Cache([KVRequest(1, rank + rot, 0, planes=1)], sum((n + 63) // 64 * 64 for n in lengths), 4096, torch.bfloat16, "cuda", max_slots=len(lengths))
+    slots = cache.begin(len(lengths))
+    cache.prepare(slots, lengths)
+    view = cache.layer_view(0)
+    view.keys.copy_(torch.randn(view.keys.shape, generator=g))
+    q = torch.randn(len(lengths), heads, rank + rot, generator=g).to(torch.bfloat16).cuda()
+    gate = torch.randn(len(lengths), heads, generator=g).to(torch.bfloat16).cuda()
+    sinks = torch.randn(heads, generator=g).cuda() if sink else None
+
+    def decode(which):
+        batch = Batch.from_lists([slots[i] for i in which], [lengths[i] - 1 for i in which], [[0]] * len(which), [[]] * len(which), "cuda")
+        return ops.latent_attention(q[which].contiguous(), batch, view, gate[which].contiguous(), 0, sinks, heads, rank, rot, 0.1, window=window)
+
+    together = decode(list(range(len(lengths))))
+    for i in range(11):
+        assert torch.equal(decode([i])[0], together[i])
+    assert torch.equal(decode([0, 1, 2, 3]), together[:4]) and torch.equal(decode([9, 4, 7]), together[[9, 4, 7]])
+    before, ops.USE_LATENT_MMA = ops.USE_LATENT_MMA, False
+    try:
+        want = decode(list(range(len(lengths)))).double()
+    finally:
+        ops.USE_LATENT_MMA = before
+    assert float((together.double() - want).norm()) <= 2.0 ** -7 * float(want.norm())
