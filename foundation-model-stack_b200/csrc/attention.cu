@@ -727,6 +727,15 @@ FMS_API int fms_attn_prefill_tile_positions(int dtype, int nheads, int kvheads) 
   return TQ;
 }
 
+// Positions of one sequence that a block of fms_attention_prefill_rows takes; 0 where that entry has no kernel (other head sizes, or
+// FMS_B200_ATTN_TC=0)
+FMS_API int fms_attn_rows_tile_positions() {
+#if FMS_ATTENTION_TC
+  if (prefill_on_tcgen05()) return tc_positions_per_block(1);
+#endif
+  return 0;
+}
+
 static int attention_prefill(const void* q, void* out, int dtype, const void* keys, const void* values,
                              const int* table, int table_stride, int block_tokens, const int* slots,
                              const int* first_row, const int* len_after, const int* tiles, int n_tiles,
@@ -797,6 +806,7 @@ FMS_API int fms_attention_prefill_rows(const void* q, long q_stride, void* out, 
                                        cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
 #if FMS_ATTENTION_TC
+  if (!prefill_on_tcgen05()) return fms_fail("attention_prefill_rows: the tcgen05 kernel is switched off");
   if (check_args("attention_prefill_rows", nheads, nheads, head_dim, BLK)) return 1;
   if (check_mask("attention_prefill_rows", window, 0, 0.f)) return 1;
   if (check_queries(q, FMS_BF16, q_stride, nheads)) return 1;

@@ -1415,10 +1415,21 @@ LATENT_EXPANDED_BYTES = 512 << 20
 LATENT_WALK_NS, LATENT_PAIR_NS, LATENT_KEY_NS = 160.0, 0.02, 0.44
 
 
-def latent_prefers_expanded(batch, window: int, heads: int) -> bool:
+_rows_tiles = {}
+
+
+def _rows_tile(head_dim: int) -> int:
+    """Positions of a tile of the prefill kernel over rows of a matrix; 0: there is none for this head size, or it is switched off."""
+    if head_dim not in _rows_tiles:
+        _rows_tiles[head_dim] = int(load_library(_attention_library(head_dim)).fms_attn_rows_tile_positions())
+    return _rows_tiles[head_dim]
+
+
+def latent_prefers_expanded(batch, window: int, heads: int, head_dim: int) -> bool:
     """Whether a step's rows attend over keys and values made of the cached latents (``latent_attention_expanded``) rather
-    than in the latent's space: unless so few queries share a key that its making does not pay."""
-    if batch.decode or getattr(batch, "len_before_host", None) is None:
+    than in the latent's space: unless so few queries share a key that its making does not pay, or the tensor-core kernels of
+    either form are switched off (FMS_B200_LATENT_MMA, FMS_B200_ATTN_TC)."""
+    if batch.decode or getattr(batch, "len_before_host", None) is None or not USE_LATENT_MMA or not _rows_tile(head_dim):
         return False
     pairs = keys = longest = 0
     for before, n in zip(batch.len_before_host, batch.num_new):
@@ -1446,7 +1457,9 @@ def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor
           view.keys.shape[0], _stream())
     out = q.new_empty((n, heads * head_dim))
     lib = _attention_library(head_dim)
-    tiles = batch.query_tiles(attention_constants(head_dim, q.dtype, 1, 1)[1])
+    if not _rows_tile(head_dim):
+        raise KernelError(f"latent_attention_expanded: no tcgen05 prefill kernel for heads of {head_dim}, or it is switched off")
+    tiles = batch.query_tiles(_rows_tile(head_dim))
     step = max(1, min(heads, LATENT_EXPANDED_BYTES // (rows * 2 * head_dim * q.element_size())))
     for h in range(0, heads, step):
         m = min(step, heads - h)

@@ -120,7 +120,7 @@ class LatentAttention(Part):
     def forward(self, x, batch, cache_view, writes_cache: bool = True):
         n, width = x.shape[0], self.rank + self.rot
         proj = self.in_proj.forward(x)
-        expanded = self._expand is not None and ops.latent_prefers_expanded(batch, self.window, self.heads)
+        expanded = self._expand is not None and ops.latent_prefers_expanded(batch, self.window, self.heads, self.vdim)
         q_full = torch.empty((n, self.heads, self.vdim if expanded else width), dtype=proj.dtype, device=proj.device)
         kv, queries = None, proj
         if self.q_rank:

@@ -1,7 +1,9 @@
 """Arguments on their way from Python into a C entry (csrc/launcher.cpp): order, widths and what is refused."""
 import ctypes
 import itertools
+import os
 import subprocess
+import sys
 
 import numpy
 import pytest
@@ -10,6 +12,7 @@ import torch
 from fms_b200.kernels import build
 from fms_b200.kernels.ops import _SIGNATURES, KernelError
 
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 C_TYPES = {"p": "void*", "i": "int", "l": "long", "f": "float"}
 
 
@@ -103,3 +106,14 @@ def test_an_engine_compiles_what_its_first_prompt_will_launch(monkeypatch, decay
     Engine._compile_what_this_model_needs(types.SimpleNamespace(decoder=decoder), True)
     assert {build.LAUNCHER, "state_scan", "sampling"} <= set(asked)
     assert ("chunk_scan" in asked) == (decay == "head")
+
+
+@pytest.mark.parametrize("switch,expanded", [({}, True), ({"FMS_B200_LATENT_MMA": "0"}, False), ({"FMS_B200_ATTN_TC": "0"}, False)])
+def test_the_switches_of_the_tensor_core_kernels_reach_latent_prompts(switch, expanded):
+    """Each, in a process of its own: a prompt's latent attention does not take the form that the switched-off kernel makes."""
+    code = ("import torch; from fms_b200.kernels import ops; from fms_b200.engine.batch import Batch; "
+            "b = Batch.from_lists([0], [0], [[0] * 500], [[]], 'cpu'); "
+            "print(ops.latent_prefers_expanded(b, 0, 32, 128), ops.latent_prefers_expanded(b, 0, 32, 48))")
+    env = {**os.environ, **switch}
+    out = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, check=True)
+    assert out.stdout.split() == [str(expanded), "False"]
