@@ -106,29 +106,36 @@ class Batch:
         """Where ``row_chunks`` keeps what it makes."""
         return ("chunks", chunk) if chosen is None or all(chosen) else ("chunks", chunk, tuple(chosen))
 
-    def key_rows(self, window: int):
+    def key_rows(self, window: int, members: Optional[Sequence[int]] = None):
         """(start, first, base: int32 [n_seqs + 1], [n_seqs], [n_seqs]; rows): the keys that a step of several tokens sees,
         laid one sequence behind the other.  Sequence i's are the rows start[i] .. start[i + 1] and begin at its position
         first[i] (0, or with a window the first of the cache block that holds the earliest key seen); its position p is row
-        base[i] + p."""
-        key = ("keys", window)
+        base[i] + p.  ``members``: the sequences that have rows (default: every one)."""
+        key = ("keys", window, self._of(members))
         if key not in self._tiles:
             start, first = [0], []
-            for before, n in zip(self.len_before_host, self.num_new):
+            for i, (before, n) in enumerate(zip(self.len_before_host, self.num_new)):
                 first.append(max(0, before - window + 1) // 64 * 64 if window > 0 else 0)
-                start.append(start[-1] + before + n - first[-1])
+                start.append(start[-1] + (before + n - first[-1] if members is None or i in members else 0))
             base = [a - b for a, b in zip(start, first)]
             packed = torch.tensor(start + first + base, dtype=torch.int32).to(self.tokens.device)
             s = len(first)
             self._tiles[key] = (packed[: s + 1], packed[s + 1: 2 * s + 1], packed[2 * s + 1:], start[-1])
         return self._tiles[key]
 
-    def query_tiles(self, tile_rows: int) -> torch.Tensor:
+    def query_tiles(self, tile_rows: int, members: Optional[Sequence[int]] = None) -> torch.Tensor:
         """[tiles, 2] int32: (sequence index, first row of the tile within the sequence's new tokens), for
-        kernels that give each thread block ``tile_rows`` rows of one sequence."""
-        if tile_rows not in self._tiles:
+        kernels that give each thread block ``tile_rows`` rows of one sequence.  ``members``: the sequences that have
+        tiles (default: every one)."""
+        key = (tile_rows, self._of(members))
+        if key not in self._tiles:
             t = []
             for i, n in enumerate(self.num_new):
-                t.extend((i, r) for r in range(0, n, tile_rows))
-            self._tiles[tile_rows] = torch.tensor(t, dtype=torch.int32).to(self.tokens.device)
-        return self._tiles[tile_rows]
+                if members is None or i in members:
+                    t.extend((i, r) for r in range(0, n, tile_rows))
+            self._tiles[key] = torch.tensor(t, dtype=torch.int32).to(self.tokens.device)
+        return self._tiles[key]
+
+    def _of(self, members: Optional[Sequence[int]]):
+        """Part of a key: the sequences that something is made for, None for all of them."""
+        return None if members is None or len(members) == self.n_seqs else tuple(members)

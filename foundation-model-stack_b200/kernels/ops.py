@@ -1406,13 +1406,14 @@ def latent_query_norm(proj: torch.Tensor, offset: int, n: int, gain: torch.Tenso
 
 # Bytes of keys and values that ``latent_attention_expanded`` makes at a time (heads are taken a few at a time beyond it)
 LATENT_EXPANDED_BYTES = 512 << 20
-# Nanoseconds that decide between the two forms of a prompt's latent attention.  In the latent's space a block walks a
-# sequence's keys at LATENT_WALK_NS a key, and a (query, key) pair of a head takes LATENT_PAIR_NS where all multiprocessors
-# are busy; making a key and a value of a head and attending over them takes LATENT_KEY_NS.  Measured with heads of 96 + 32
-# over a latent of 512, 32 heads, whole layers, latent's space / heads' space in us: a prompt of 64 tokens 45 / 41, of 256
-# 88 / 53, two of 2,048 together 873 / 209; 16 tokens onto 1,024 cached ones 244 / 68, onto 8,000 1,356 / 220; 64 tokens of
-# four sequences onto 1,000 each 211 / 106, of eight onto 1,000 each 219 / 138.
-LATENT_WALK_NS, LATENT_PAIR_NS, LATENT_KEY_NS = 160.0, 0.02, 0.44
+# What decides between the two forms of a prompt's latent attention, a sequence at a time and by its own tokens, so that its results
+# do not depend on what else is in the step.  In the latent's space a (query, key) pair of a head takes LATENT_PAIR ns a value of
+# its two products where all multiprocessors are busy; making a key and a value of a head takes LATENT_MAKE ns a multiply-add, once
+# for all queries: with heads of 96 + 32 over a latent of 512 0.02 and 0.44 ns, so that making them pays from 23 tokens on, whatever is
+# cached.  (A sequence alone gains sooner: a block walks its keys at 160 ns a key.  But the more sequences, the less that counts: 16 of
+# 2 tokens onto 1,000 cached ones each would take half as long again.)  Whole layers, latent's space / heads' space in us: a
+# prompt of 64 tokens 45 / 41, of 256 88 / 53, two of 2,048 together 873 / 209; 64 tokens onto 8,000 cached ones 1,400 / 260.
+LATENT_PAIR, LATENT_MAKE = 0.02 / (2 * 512 + 32), 0.44 / (128 * (512 + 32))
 
 
 _rows_tiles = {}
@@ -1425,41 +1426,45 @@ def _rows_tile(head_dim: int) -> int:
     return _rows_tiles[head_dim]
 
 
-def latent_prefers_expanded(batch, window: int, heads: int, head_dim: int) -> bool:
-    """Whether a step's rows attend over keys and values made of the cached latents (``latent_attention_expanded``) rather
-    than in the latent's space: unless so few queries share a key that its making does not pay, or the tensor-core kernels of
-    either form are switched off (FMS_B200_LATENT_MMA, FMS_B200_ATTN_TC)."""
-    if batch.decode or getattr(batch, "len_before_host", None) is None or not USE_LATENT_MMA or not _rows_tile(head_dim):
+def latent_prefers_expanded(batch, n: int, head_dim: int, rank: int, rot: int) -> bool:
+    """Whether a sequence that brings ``n`` tokens attends over keys and values made of the cached latents
+    (``latent_attention_expanded``) rather than in the latent's space: unless so few queries share a key that its making does
+    not pay, or the tensor-core kernels of either form are switched off (FMS_B200_LATENT_MMA, FMS_B200_ATTN_TC)."""
+    if batch.decode or not USE_LATENT_MMA or not _rows_tile(head_dim):
         return False
-    pairs = keys = longest = 0
-    for before, n in zip(batch.len_before_host, batch.num_new):
-        seen = min(before + n, window + n) if window > 0 else before + n
-        keys, longest = keys + seen, max(longest, seen)
-        pairs += n * min(before + (n + 1) // 2, seen)
-    return max(longest * LATENT_WALK_NS, pairs * heads * LATENT_PAIR_NS) > keys * heads * LATENT_KEY_NS
+    return n * LATENT_PAIR * (2 * rank + rot) > LATENT_MAKE * head_dim * (rank + rot)
+
+
+def latent_expanded_members(batch, head_dim: int, rank: int, rot: int):
+    """The sequences of a step that ``latent_prefers_expanded`` sends into the heads' own space (none of a batch whose lengths the
+    host does not know)."""
+    if batch.decode or getattr(batch, "len_before_host", None) is None:
+        return []
+    return [i for i, n in enumerate(batch.num_new) if n > 0 and latent_prefers_expanded(batch, n, head_dim, rank, rot)]
 
 
 def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor, sink: Optional[torch.Tensor], heads: int,
                               head_dim: int, scale: float, window: int = 0, gate: Optional[torch.Tensor] = None,
-                              gate_offset: int = 0) -> torch.Tensor:
+                              gate_offset: int = 0, members=None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The same attention in the heads' own space, for steps of many tokens: the cached rows [c | kr] that the step sees
     are gathered, every head's keys and values made of them in one product, and the tcgen05 prefill kernel runs over those.
     ``q`` [tokens, heads, head_dim]; ``expand`` [heads, 2 * head_dim, rank + rot]: head h's matrix that makes [key | value] of
-    a cached row; ``sink`` float32 or None; ``gate`` as in ``latent_attention``.  Returns [tokens, heads * head_dim]."""
+    a cached row; ``sink`` float32 or None; ``gate`` as in ``latent_attention``; ``members``: the sequences whose rows are made
+    (default: all), the others' rows of ``out`` being left as they are.  Returns [tokens, heads * head_dim]."""
     n, width = q.shape[0], expand.shape[2]
     if tuple(expand.shape[:2]) != (heads, 2 * head_dim) or view.keys.shape[-1] != width or q.dtype != torch.bfloat16 \
             or (sink is not None and sink.dtype != torch.float32) or (gate is not None and gate.dtype != q.dtype):
         raise KernelError(f"latent_attention_expanded: {heads} heads of {head_dim}, matrices {tuple(expand.shape)}, rows of {view.keys.shape[-1]}")
-    start, first, base, rows = batch.key_rows(window)
+    start, first, base, rows = batch.key_rows(window, members)
     cached = q.new_empty((rows, width))
     _call("latent_attention", "fms_latent_gather", view.keys, width * q.element_size(), view.table, view.table.shape[1],
           view.block_tokens, batch.slots, start, first, batch.n_seqs, cached, rows, view.table.shape[0],
           view.keys.shape[0], _stream())
-    out = q.new_empty((n, heads * head_dim))
+    out = q.new_empty((n, heads * head_dim)) if out is None else out
     lib = _attention_library(head_dim)
     if not _rows_tile(head_dim):
         raise KernelError(f"latent_attention_expanded: no tcgen05 prefill kernel for heads of {head_dim}, or it is switched off")
-    tiles = batch.query_tiles(_rows_tile(head_dim))
+    tiles = batch.query_tiles(_rows_tile(head_dim), members)
     step = max(1, min(heads, LATENT_EXPANDED_BYTES // (rows * 2 * head_dim * q.element_size())))
     for h in range(0, heads, step):
         m = min(step, heads - h)
@@ -1475,11 +1480,12 @@ def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor
 
 def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Tensor], gate_offset: int,
                      sink: Optional[torch.Tensor], heads: int, rank: int, rot: int, scale: float,
-                     window: int = 0) -> torch.Tensor:
+                     window: int = 0, members=None) -> torch.Tensor:
     """Causal softmax attention of the step's rows over the cached latent rows [c | kr] (which already hold the step's
     own), with a per-head sink in the denominator and a per-head sigmoid gate on the result.  ``gate``: the matrix
     whose column ``gate_offset + h`` holds head h's gate logit of each row (None: no gate); ``sink`` None: no sink;
-    ``window`` > 0: the row at position p sees the keys p - window + 1 .. p only.  Returns [tokens, heads, rank]."""
+    ``window`` > 0: the row at position p sees the keys p - window + 1 .. p only.  ``members``: the sequences whose rows are
+    wanted (default: all; the others' rows may hold anything).  Returns [tokens, heads, rank]."""
     global _latent_split, launches
     n = q_full.shape[0]
     out = q_full.new_empty((n, heads, rank))
@@ -1502,7 +1508,7 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
             while heads_per_block < min(32, heads):
                 heads_per_block *= 2
         tile_tokens = 32 // heads_per_block
-        tiles = batch.query_tiles(tile_tokens)
+        tiles = batch.query_tiles(tile_tokens, members)
         gate_ptr = None if gate is None else _ptr(gate) + gate_offset * gate.element_size()
         _call("latent_attention", "fms_latent_attention_prefill_bf16", q_full, out, view.keys, gate_ptr,
               0 if gate is None else gate.shape[1], sink, _code(sink.dtype) if sink is not None else F32,

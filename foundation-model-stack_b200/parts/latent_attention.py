@@ -16,8 +16,8 @@ q_h . Wuk,h c = (Wuk,h^T q_h) . c, so the query is taken into the latent's space
 ``uk`` transposed once at load time), attention runs over the latent rows as they lie, and the head's result, a
 weighted sum of latents, goes through Wuv,h afterwards.  [Wq; Wdkv; Wg] is one fused projection.
 
-A step of many tokens of a bfloat16 model whose heads' keys and values are equally long (64 or 128 values) goes the other
-way where that is the shorter one (``ops.latent_prefers_expanded``): every head's keys and values are made of the cached rows
+A sequence that brings many tokens to a bfloat16 model whose heads' keys and values are equally long (64 or 128 values) goes the
+other way where that is the shorter one (``ops.latent_prefers_expanded``): every head's keys and values are made of the cached rows
 in one product (``_expand``: [Wuk,h 0; 0 1; Wuv,h 0] takes a row [c | kr] to [k_h | v_h]), and attention runs over those.
 
 Options of the ``MixerSpec``: ``rot`` (rotated values per head), ``vdim``, ``rank``, ``rot_dims``; ``head_dim`` is the
@@ -120,30 +120,39 @@ class LatentAttention(Part):
     def forward(self, x, batch, cache_view, writes_cache: bool = True):
         n, width = x.shape[0], self.rank + self.rot
         proj = self.in_proj.forward(x)
-        expanded = self._expand is not None and ops.latent_prefers_expanded(batch, self.window, self.heads, self.vdim)
-        q_full = torch.empty((n, self.heads, self.vdim if expanded else width), dtype=proj.dtype, device=proj.device)
         kv, queries = None, proj
         if self.q_rank:
             kv = proj
             queries = self.q_up.forward(ops.latent_query_norm(proj, width, self.q_rank, self.tensor("q_norm"), self.eps))
-        ops.latent_prepare(queries, q_full, self.tensor("latent_norm"), self.eps, self._inv_freq, self.rot_dims, batch,
-                           cache_view, self.heads, self.dim, self.rot, self.rank, writes_cache, halves=self.halves,
-                           rot_mult=self.rot_mult, kv=kv, own_space=expanded)
-        if expanded:
-            o = ops.latent_attention_expanded(q_full, batch, cache_view, self._expand, self._sink, self.heads, self.vdim, self.scale,
-                                              self.window, proj if self.has_gate else None, self.gate_col)
-            return self.dense.forward(o)
-        if self.dim:
-            ops.grouped_linear(queries, self._uk_t, self.heads, n, self.rank, self.dim, queries.shape[1], self.dim + self.rot,
-                               q_full, self.heads * width, width)
-        else:
-            q_full[:, :, : self.rank].zero_()
-        latent = ops.latent_attention(q_full, batch, cache_view, proj if self.has_gate else None, self.gate_col,
-                                      self.tensor("sink") if self.has_sink else None, self.heads, self.rank, self.rot,
-                                      self.scale, window=self.window)
-        o = torch.empty((n, self.heads * self.vdim), dtype=proj.dtype, device=proj.device)
-        ops.grouped_linear(latent, self._uv, self.heads, n, self.vdim, self.rank, self.heads * self.rank, self.rank, o,
-                           self.heads * self.vdim, self.vdim)
+
+        def prepared(own_space, writes):
+            q = torch.empty((n, self.heads, self.vdim if own_space else width), dtype=proj.dtype, device=proj.device)
+            ops.latent_prepare(queries, q, self.tensor("latent_norm"), self.eps, self._inv_freq, self.rot_dims, batch,
+                               cache_view, self.heads, self.dim, self.rot, self.rank, writes, halves=self.halves,
+                               rot_mult=self.rot_mult, kv=kv, own_space=own_space)
+            return q
+
+        # the sequences whose rows attend in the heads' own space; the others' do in the latent's
+        own = [] if self._expand is None else ops.latent_expanded_members(batch, self.vdim, self.rank, self.rot)
+        o = None
+        if len(own) < batch.n_seqs:
+            q_full = prepared(False, writes_cache)
+            if self.dim:
+                ops.grouped_linear(queries, self._uk_t, self.heads, n, self.rank, self.dim, queries.shape[1], self.dim + self.rot,
+                                   q_full, self.heads * width, width)
+            else:
+                q_full[:, :, : self.rank].zero_()
+            latent = ops.latent_attention(q_full, batch, cache_view, proj if self.has_gate else None, self.gate_col,
+                                          self.tensor("sink") if self.has_sink else None, self.heads, self.rank, self.rot,
+                                          self.scale, window=self.window,
+                                          members=[i for i in range(batch.n_seqs) if i not in own] if own else None)
+            o = torch.empty((n, self.heads * self.vdim), dtype=proj.dtype, device=proj.device)
+            ops.grouped_linear(latent, self._uv, self.heads, n, self.vdim, self.rank, self.heads * self.rank, self.rank, o,
+                               self.heads * self.vdim, self.vdim)
+        if own:
+            o = ops.latent_attention_expanded(prepared(True, writes_cache and o is None), batch, cache_view, self._expand, self._sink,
+                                              self.heads, self.vdim, self.scale, self.window, proj if self.has_gate else None,
+                                              self.gate_col, members=own, out=o)
         return self.dense.forward(o)
 
     def kernel_libraries(self, dtype):

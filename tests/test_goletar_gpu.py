@@ -566,3 +566,47 @@ def test_latent_decode_of_a_row_does_not_depend_on_the_others(window, sink):
     finally:
         ops.USE_LATENT_MMA = before
     assert float((together.double() - want).norm()) <= 2.0 ** -7 * float(want.norm())
+
+
+@pytest.mark.parametrize("window", [0, 70])
+def test_each_sequence_of_a_step_takes_the_form_of_latent_attention_that_its_own_tokens_choose(window):
+    """Long and short portions in one step, onto what is cached, some in the heads' own space and some in the latent's: against the
+    formulas, and the rows that attention makes of a sequence beside the same sequence's alone.  (The products around it choose
+    their kernels by the rows of a step, so alone and together agree within bfloat16's roundings.)"""
+    from fms_b200.cache import Cache
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    heads, dim, rot, vdim, rank = 3, 96, 32, 128, 64
+    m = gm.latent(heads, dim, rot, vdim, rank, 300.0, None, rot_dims=32)["mixer"]
+    g = torch.Generator().manual_seed(11)
+    w = latent_tensors(g, 40, m)
+    mixer = latent_mixer(m, 40, w, 1e-5, torch.bfloat16)
+    mixer.window = window
+    least = next(n for n in range(1, 200) if ops.latent_prefers_expanded(Batch.from_lists([0], [0], [[0] * 2], [[]], "cpu"), n, vdim, rank, rot))
+    assert 2 < least < 100
+    portions = [[80, least - 1], [150, 1], [40, least], [0, 200], [129, 2]]
+    xs = [torch.randn(sum(p), 40, generator=g).to(torch.bfloat16) for p in portions]
+
+    def steps(which):
+        cache = Cache([mixer.cache_request()], 64 * 5 * len(which), 512, torch.bfloat16, "cuda")
+        slots, out = cache.begin(len(which)), None
+        for step in range(2):
+            live = [j for j, i in enumerate(which) if portions[i][step]]
+            counts = [portions[which[j]][step] for j in live]
+            lens = cache.prepare([slots[j] for j in live], counts)
+            batch = Batch.from_lists([slots[j] for j in live], lens, [[0] * c for c in counts], [[] for _ in live], "cuda")
+            if step and len(which) > 1:
+                assert ops.latent_expanded_members(batch, vdim, rank, rot) == [2, 3]
+            rows = torch.cat([xs[which[j]][lens[k]: lens[k] + counts[k]] for k, j in enumerate(live)]).cuda()
+            out = mixer.forward(rows, batch, cache.layer_view(0))
+            cache.commit([slots[j] for j in live], counts)
+        return torch.split(out, [portions[i][1] for i in which])
+
+    together = steps([0, 1, 2, 3, 4])
+    d = {k: v.double() for k, v in w.items()}
+    for i, got in enumerate(together):
+        if not window:
+            want, _ = pg.latent_attention(xs[i].double(), m, 1e-5, d["q"], d["dkv"], d["norm"], d["uk"], d["uv"], d["sink"], d["g"], d["o"])
+            close(got, want[portions[i][0]:], "bf16")
+        close(got, steps([i])[0].double().cpu(), "bf16")
