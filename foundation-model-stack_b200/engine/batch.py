@@ -106,6 +106,23 @@ class Batch:
         """Where ``row_chunks`` keeps what it makes."""
         return ("chunks", chunk) if chosen is None or all(chosen) else ("chunks", chunk, tuple(chosen))
 
+    def rows_seen(self, i: int, window: int) -> int:
+        """How many rows ``key_rows`` lays out for sequence i."""
+        before = self.len_before_host[i]
+        return before + self.num_new[i] - (max(0, before - window + 1) // 64 * 64 if window > 0 else 0)
+
+    def key_passes(self, window: int, most: int, members: Optional[Sequence[int]] = None) -> List[List[int]]:
+        """The sequences (default: all) in runs that see at most ``most`` rows together; one that sees more is a run of its own."""
+        passes, rows = [], 0
+        for i in (range(self.n_seqs) if members is None else members):
+            seen = self.rows_seen(i, window)
+            if not passes or rows + seen > most:
+                passes.append([])
+                rows = 0
+            passes[-1].append(i)
+            rows += seen
+        return passes
+
     def key_rows(self, window: int, members: Optional[Sequence[int]] = None):
         """(start, first, base: int32 [n_seqs + 1], [n_seqs], [n_seqs]; rows): the keys that a step of several tokens sees,
         laid one sequence behind the other.  Sequence i's are the rows start[i] .. start[i + 1] and begin at its position
@@ -115,8 +132,9 @@ class Batch:
         if key not in self._tiles:
             start, first = [0], []
             for i, (before, n) in enumerate(zip(self.len_before_host, self.num_new)):
-                first.append(max(0, before - window + 1) // 64 * 64 if window > 0 else 0)
-                start.append(start[-1] + (before + n - first[-1] if members is None or i in members else 0))
+                seen = self.rows_seen(i, window)
+                first.append(before + n - seen)
+                start.append(start[-1] + (seen if members is None or i in members else 0))
             base = [a - b for a, b in zip(start, first)]
             packed = torch.tensor(start + first + base, dtype=torch.int32).to(self.tokens.device)
             s = len(first)

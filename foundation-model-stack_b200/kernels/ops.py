@@ -1404,8 +1404,10 @@ def latent_query_norm(proj: torch.Tensor, offset: int, n: int, gain: torch.Tenso
     return out
 
 
-# Bytes of keys and values that ``latent_attention_expanded`` makes at a time (heads are taken a few at a time beyond it)
-LATENT_EXPANDED_BYTES = 512 << 20
+# Bytes that ``latent_attention_expanded`` takes at a time for gathered rows and the keys and values made of them: sequences, and
+# then heads, are taken a few at a time beyond it, and a sequence whose rows with one head's keys and values are more than that stays
+# in the latent's space.  (There a prompt of 2,048 tokens takes 138 MB for the queries and results of 32 heads over a latent of 512.)
+LATENT_EXPANDED_BYTES = 128 << 20
 # What decides between the two forms of a prompt's latent attention, a sequence at a time and by its own tokens, so that its results
 # do not depend on what else is in the step.  In the latent's space a (query, key) pair of a head takes LATENT_PAIR ns a value of
 # its two products where all multiprocessors are busy; making a key and a value of a head takes LATENT_MAKE ns a multiply-add, once
@@ -1426,21 +1428,23 @@ def _rows_tile(head_dim: int) -> int:
     return _rows_tiles[head_dim]
 
 
-def latent_prefers_expanded(batch, n: int, head_dim: int, rank: int, rot: int) -> bool:
-    """Whether a sequence that brings ``n`` tokens attends over keys and values made of the cached latents
+def latent_prefers_expanded(batch, n: int, seen: int, head_dim: int, rank: int, rot: int) -> bool:
+    """Whether a sequence that brings ``n`` tokens, which see ``seen`` cached rows, attends over keys and values made of the cached latents
     (``latent_attention_expanded``) rather than in the latent's space: unless so few queries share a key that its making does
-    not pay, or the tensor-core kernels of either form are switched off (FMS_B200_LATENT_MMA, FMS_B200_ATTN_TC)."""
-    if batch.decode or not USE_LATENT_MMA or not _rows_tile(head_dim):
+    not pay, its rows are too many (LATENT_EXPANDED_BYTES), or the tensor-core kernels of either form are switched off
+    (FMS_B200_LATENT_MMA, FMS_B200_ATTN_TC)."""
+    if batch.decode or not USE_LATENT_MMA or not _rows_tile(head_dim) or seen * (rank + rot + 2 * head_dim) * 2 > LATENT_EXPANDED_BYTES:
         return False
     return n * LATENT_PAIR * (2 * rank + rot) > LATENT_MAKE * head_dim * (rank + rot)
 
 
-def latent_expanded_members(batch, head_dim: int, rank: int, rot: int):
+def latent_expanded_members(batch, window: int, head_dim: int, rank: int, rot: int):
     """The sequences of a step that ``latent_prefers_expanded`` sends into the heads' own space (none of a batch whose lengths the
     host does not know)."""
     if batch.decode or getattr(batch, "len_before_host", None) is None:
         return []
-    return [i for i, n in enumerate(batch.num_new) if n > 0 and latent_prefers_expanded(batch, n, head_dim, rank, rot)]
+    return [i for i, n in enumerate(batch.num_new) if n > 0 and
+            latent_prefers_expanded(batch, n, batch.rows_seen(i, window), head_dim, rank, rot)]
 
 
 def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor, sink: Optional[torch.Tensor], heads: int,
@@ -1455,26 +1459,30 @@ def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor
     if tuple(expand.shape[:2]) != (heads, 2 * head_dim) or view.keys.shape[-1] != width or q.dtype != torch.bfloat16 \
             or (sink is not None and sink.dtype != torch.float32) or (gate is not None and gate.dtype != q.dtype):
         raise KernelError(f"latent_attention_expanded: {heads} heads of {head_dim}, matrices {tuple(expand.shape)}, rows of {view.keys.shape[-1]}")
-    start, first, base, rows = batch.key_rows(window, members)
-    cached = q.new_empty((rows, width))
-    _call("latent_attention", "fms_latent_gather", view.keys, width * q.element_size(), view.table, view.table.shape[1],
-          view.block_tokens, batch.slots, start, first, batch.n_seqs, cached, rows, view.table.shape[0],
-          view.keys.shape[0], _stream())
-    out = q.new_empty((n, heads * head_dim)) if out is None else out
-    lib = _attention_library(head_dim)
     if not _rows_tile(head_dim):
         raise KernelError(f"latent_attention_expanded: no tcgen05 prefill kernel for heads of {head_dim}, or it is switched off")
-    tiles = batch.query_tiles(_rows_tile(head_dim), members)
-    step = max(1, min(heads, LATENT_EXPANDED_BYTES // (rows * 2 * head_dim * q.element_size())))
-    for h in range(0, heads, step):
-        m = min(step, heads - h)
-        kv = linear(cached, expand[h:h + m].view(m * 2 * head_dim, width))
-        at = h * head_dim * q.element_size()
-        _call(lib, "fms_attention_prefill_rows", _ptr(q) + at, heads * head_dim, _ptr(out) + at, heads * head_dim, kv,
-              _ptr(kv) + head_dim * kv.element_size(), kv.shape[1], 2 * head_dim, rows, base, batch.first_row,
-              batch.len_after, tiles, tiles.shape[0], m, head_dim, float(scale), int(window),
-              None if sink is None else _ptr(sink) + h * 4, None if gate is None else _ptr(gate) + (gate_offset + h) * gate.element_size(),
-              0 if gate is None else gate.shape[1], error_flag(q.device), _stream())
+    out = q.new_empty((n, heads * head_dim)) if out is None else out
+    size, lib = q.element_size(), _attention_library(head_dim)
+    gate_ptr = None if gate is None else _ptr(gate) + gate_offset * gate.element_size()
+    for some in batch.key_passes(window, LATENT_EXPANDED_BYTES // ((width + 2 * head_dim) * size), members):
+        start, first, base, rows = batch.key_rows(window, some)
+        tiles = batch.query_tiles(_rows_tile(head_dim), some)
+        cached = q.new_empty((rows, width))
+        _call("latent_attention", "fms_latent_gather", view.keys, width * size, view.table, view.table.shape[1],
+              view.block_tokens, batch.slots, start, first, batch.n_seqs, cached, rows, view.table.shape[0],
+              view.keys.shape[0], _stream())
+        step = max(1, min(heads, (LATENT_EXPANDED_BYTES - rows * width * size) // (rows * 2 * head_dim * size)))
+        for h in range(0, heads, step):
+            m = min(step, heads - h)
+            kv = linear(cached, expand[h:h + m].view(m * 2 * head_dim, width))
+            at = h * head_dim * size
+            _call(lib, "fms_attention_prefill_rows", _ptr(q) + at, heads * head_dim, _ptr(out) + at, heads * head_dim, kv,
+                  _ptr(kv) + head_dim * size, kv.shape[1], 2 * head_dim, rows, base, batch.first_row,
+                  batch.len_after, tiles, tiles.shape[0], m, head_dim, float(scale), int(window),
+                  None if sink is None else _ptr(sink) + h * 4, None if gate is None else gate_ptr + h * gate.element_size(),
+                  0 if gate is None else gate.shape[1], error_flag(q.device), _stream())
+            del kv  # before the next ones are made
+        del cached
     return out
 
 

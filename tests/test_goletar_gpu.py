@@ -583,7 +583,7 @@ def test_each_sequence_of_a_step_takes_the_form_of_latent_attention_that_its_own
     w = latent_tensors(g, 40, m)
     mixer = latent_mixer(m, 40, w, 1e-5, torch.bfloat16)
     mixer.window = window
-    least = next(n for n in range(1, 200) if ops.latent_prefers_expanded(Batch.from_lists([0], [0], [[0] * 2], [[]], "cpu"), n, vdim, rank, rot))
+    least = next(n for n in range(1, 200) if ops.latent_prefers_expanded(Batch.from_lists([0], [0], [[0] * 2], [[]], "cpu"), n, n, vdim, rank, rot))
     assert 2 < least < 100
     portions = [[80, least - 1], [150, 1], [40, least], [0, 200], [129, 2]]
     xs = [torch.randn(sum(p), 40, generator=g).to(torch.bfloat16) for p in portions]
@@ -597,7 +597,7 @@ def test_each_sequence_of_a_step_takes_the_form_of_latent_attention_that_its_own
             lens = cache.prepare([slots[j] for j in live], counts)
             batch = Batch.from_lists([slots[j] for j in live], lens, [[0] * c for c in counts], [[] for _ in live], "cuda")
             if step and len(which) > 1:
-                assert ops.latent_expanded_members(batch, vdim, rank, rot) == [2, 3]
+                assert ops.latent_expanded_members(batch, window, vdim, rank, rot) == [2, 3]
             rows = torch.cat([xs[which[j]][lens[k]: lens[k] + counts[k]] for k, j in enumerate(live)]).cuda()
             out = mixer.forward(rows, batch, cache.layer_view(0))
             cache.commit([slots[j] for j in live], counts)
@@ -610,3 +610,39 @@ def test_each_sequence_of_a_step_takes_the_form_of_latent_attention_that_its_own
             want, _ = pg.latent_attention(xs[i].double(), m, 1e-5, d["q"], d["dkv"], d["norm"], d["uk"], d["uv"], d["sink"], d["g"], d["o"])
             close(got, want[portions[i][0]:], "bf16")
         close(got, steps([i])[0].double().cpu(), "bf16")
+
+
+@pytest.mark.parametrize("window", [0, 70])
+def test_scratch_of_attention_in_the_heads_own_space_is_bounded(monkeypatch, window):
+    """Sequences that do not fit together are gathered a few at a time, heads likewise, with the same results as all at once; a
+    sequence that does not fit with one head stays in the latent's space; and no more is held at a time than the limit."""
+    from fms_b200.cache import Cache, KVRequest
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    heads, hd, rank, rot = 8, 64, 64, 32
+    width, lens, new = rank + rot, [300, 40, 0, 700, 129], [70, 64, 65, 130, 1]
+    g = torch.Generator().manual_seed(13)
+    cache = Cache([KVRequest(1, width, 0, planes=1)], 64 * 30, 1024, torch.bfloat16, "cuda", max_slots=5)
+    slots = cache.begin(5)
+    cache.prepare(slots, [a + b for a, b in zip(lens, new)])
+    batch = Batch.from_lists(slots, lens, [[0] * n for n in new], [[]] * 5, "cuda")
+    view = cache.layer_view(0)
+    view.keys.copy_(torch.randn(view.keys.shape, generator=g))
+    q = torch.randn(sum(new), heads, hd, generator=g).to(torch.bfloat16).cuda()
+    expand = (torch.randn(heads, 2 * hd, width, generator=g) * 0.2).to(torch.bfloat16).cuda()
+    row = 2 * (width + 2 * hd)
+    monkeypatch.setattr(ops, "linear", lambda x, w, *_: x @ w.T)  # one kernel however many rows and columns there are
+    make = lambda: ops.latent_attention_expanded(q, batch, view, expand, None, heads, hd, 0.1, window)  # noqa: E731
+    whole = make()
+    torch.cuda.synchronize()
+    for limit in (400 * row, 900 * row):
+        monkeypatch.setattr(ops, "LATENT_EXPANDED_BYTES", limit)
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        got = make()
+        longest = max(batch.rows_seen(i, window) for i in range(5)) * row
+        assert torch.cuda.max_memory_allocated() - before <= max(limit, longest) + got.numel() * 2 + 64 * 1024
+        assert float((got.double() - whole.double()).norm()) <= 2.0 ** -8 * float(whole.double().norm())
+        fits = ops.latent_expanded_members(batch, window, hd, rank, rot)
+        assert fits == [i for i in range(4) if batch.rows_seen(i, window) * row <= limit]

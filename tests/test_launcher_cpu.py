@@ -113,7 +113,7 @@ def test_the_switches_of_the_tensor_core_kernels_reach_latent_prompts(switch, ex
     """Each, in a process of its own: a prompt's latent attention does not take the form that the switched-off kernel makes."""
     code = ("import torch; from fms_b200.kernels import ops; from fms_b200.engine.batch import Batch; "
             "b = Batch.from_lists([0], [0], [[0] * 500], [[]], 'cpu'); "
-            "print(*(bool(ops.latent_expanded_members(b, h, 512, 32)) for h in (128, 48)))")
+            "print(*(bool(ops.latent_expanded_members(b, 0, h, 512, 32)) for h in (128, 48)))")
     env = {**os.environ, **switch}
     out = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, check=True)
     assert out.stdout.split() == [str(expanded), "False"]
