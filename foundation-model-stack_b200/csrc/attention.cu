@@ -248,6 +248,28 @@ __device__ __forceinline__ void prefill_f32_tile(const AttnArgs& a, float* smem,
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
+    // A value that is not finite must not reach the rows that do not see its key, not even times zero: in a block that some
+    // row does not see whole, such values are looked for (a part in a hundred of the block's work), and keys then selected.
+    if (kb * BLK + BLK - 1 > p_first || kb * BLK < first_visible(a, p_last)) {
+      int bad = 0;
+      for (int i = tid; i < BLK * (HD / 4); i += 128) {
+        const float4 x = *reinterpret_cast<const float4*>(vs + 4 * i);
+        bad |= !(fabsf(x.x) <= 3.4028235e38f && fabsf(x.y) <= 3.4028235e38f && fabsf(x.z) <= 3.4028235e38f && fabsf(x.w) <= 3.4028235e38f);
+      }
+      if (__syncthreads_or(bad)) {
+#pragma unroll 1
+        for (int key = 0; key < BLK; ++key)
+#pragma unroll
+          for (int i = 0; i < RPT; ++i) {
+            const int r = ty + 8 * i, kpos = kb * BLK + key, my_pos = p_first + r;
+            if (r >= rows_here || kpos > my_pos || kpos < first_visible(a, my_pos)) continue;
+            const float p = ps[r * PSTRIDE + key];
+#pragma unroll
+            for (int c = 0; c < HD / 16; ++c) acc[i][c] = fmaf(p, vs[key * HD + tx + 16 * c], acc[i][c]);
+          }
+        continue;
+      }
+    }
 #pragma unroll 1
     for (int key = 0; key < BLK; key += 4) {
       float4 p[RPT];

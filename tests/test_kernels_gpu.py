@@ -497,6 +497,30 @@ def test_prefill_attention_float32_at_the_edges_of_its_tiles(ops, nheads, kvhead
     assert torch.equal(ops.attention(wide, batch, view, nheads, kvheads, hd, scale, window), got)
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("what", [0, 1])
+@pytest.mark.parametrize("num_new,window", [(200, 0), (200, 70), (12, 0), (64, 5)])
+def test_prefill_attention_float32_keeps_a_value_that_is_not_finite_to_the_rows_that_see_it(ops, num_new, window, what, value):
+    """One value of one token's key or value is not finite: the rows before it, and with a window those it has left, come out as
+    they do without it; rows that see it show it."""
+    nheads, kvheads, hd, before = 2, 1, 48, 37
+    cache, view, batch = make_cache_case(torch.float32, nheads, kvheads, hd, [before], [num_new], 9, window)
+    g = torch.Generator().manual_seed(21)
+    qkv = torch.randn(num_new, (nheads + 2 * kvheads) * hd, generator=g).cuda()
+    q = ops.rope_store(qkv, None, batch, view, nheads, kvheads, hd)
+    clean = ops.attention(q, batch, view, nheads, kvheads, hd, 0.2, window)
+    assert bool(torch.isfinite(clean).all())
+    at = num_new * 3 // 5
+    qkv[at, (nheads + what * kvheads) * hd + 3] = value
+    ops.rope_store(qkv, None, batch, view, nheads, kvheads, hd)
+    got = ops.attention(q, batch, view, nheads, kvheads, hd, 0.2, window)
+    sees = torch.zeros(num_new, dtype=torch.bool)
+    sees[at: at + window if window else num_new] = True
+    assert torch.equal(got[~sees.cuda()], clean[~sees.cuda()])
+    if what == 1:
+        assert not bool(torch.isfinite(got.view(num_new, nheads, hd)[sees.cuda()][..., 3]).any())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_finds_one_far_key(ops, dtype):
     """One key among hundreds is scaled so that it takes nearly all the weight: its value must come out,
