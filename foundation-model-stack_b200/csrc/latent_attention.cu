@@ -49,6 +49,8 @@ __device__ __forceinline__ void rotate_run(const T* src, T* dst, int i, int half
   }
 }
 
+constexpr int MOST_TURNS = 4096;  // pairs whose sines and cosines shared memory holds; further ones are taken where they are needed
+
 template <typename T, typename TG>
 __global__ void __launch_bounds__(128) latent_prepare_kernel(
     const T* __restrict__ proj, int proj_width, T* __restrict__ q_out, int q_width, int q_rot, int q_copy,
@@ -57,7 +59,7 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(
     T* __restrict__ cache, const int* __restrict__ table, int table_stride, int block_tokens, int heads, int dim, int rot,
     int rank, int write_cache, int n_seqs, int n_slots, int n_blocks, int* __restrict__ error_flag, int halves,
     float rot_mult, const T* __restrict__ kv, int kv_width) {
-  extern __shared__ float2 turns[];  // [rot_dims / 2]: sine, cosine
+  extern __shared__ float2 turns[];  // [min(rot_dims / 2, MOST_TURNS)]: sine, cosine
   __shared__ float scratch[33];
   pdl_launch_dependents();
   pdl_wait();
@@ -67,17 +69,18 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(
   const float position = (float)(position_ids ? ld_fresh(position_ids + t) : ld_fresh(positions + t));
   const int width = rank + rot;
   const int half = rot_dims / 2, units = rot - half;  // of a run: its pairs, and the values behind them one by one
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+  auto turn = [&](int i) {
     float sn, cs;
     sincosf(position * inv_freq[i], &sn, &cs);
-    turns[i] = make_float2(sn * rot_mult, cs * rot_mult);
-  }
+    return make_float2(sn * rot_mult, cs * rot_mult);
+  };
+  auto turn_of = [&](int u) { return u >= half ? make_float2(0.f, 0.f) : (u < MOST_TURNS ? turns[u] : turn(u)); };
+  for (int i = threadIdx.x; i < min(half, MOST_TURNS); i += blockDim.x) turns[i] = turn(i);
   __syncthreads();
   // the rotated part of every head's query
   for (int i = threadIdx.x; i < heads * units; i += blockDim.x) {
     const int h = i / units, u = i - h * units;
-    rotate_run(row + (size_t)h * (dim + rot) + dim, q_out + ((size_t)t * heads + h) * q_width + q_rot, u, half, halves, rot,
-               u < half ? turns[u] : make_float2(0.f, 0.f));
+    rotate_run(row + (size_t)h * (dim + rot) + dim, q_out + ((size_t)t * heads + h) * q_width + q_rot, u, half, halves, rot, turn_of(u));
   }
   if (q_copy) {
     constexpr int V = 16 / sizeof(T);
@@ -118,7 +121,7 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(
   const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
   for (int d = threadIdx.x; d < rank; d += blockDim.x) dst[d] = from_f32<T>(to_f32(c[d]) * inv * to_f32(c_gain[d]));
   for (int i = threadIdx.x; i < units; i += blockDim.x)
-    rotate_run(c + rank, dst + rank, i, half, halves, rot, i < half ? turns[i] : make_float2(0.f, 0.f));
+    rotate_run(c + rank, dst + rank, i, half, halves, rot, turn_of(i));
 }
 
 // The cached rows of a step's sequences one behind the other: row r of `out` is position first[s] + r - start[s] of
@@ -670,12 +673,13 @@ FMS_API int fms_latent_prepare(const void* proj, int dtype, int proj_width, void
                                int rot, int rank, int write_cache, int n_seqs, int n_slots, int n_blocks, int* error_flag,
                                int halves, float rot_mult, const void* kv, int kv_width, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  if (heads <= 0 || dim < 0 || rot < 0 || rank <= 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) || rot_dims > 8192 ||
+  if (heads <= 0 || dim < 0 || rot < 0 || rank <= 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) ||
       q_rot < (q_copy ? dim : 0) || q_width < q_rot + rot)
     return fms_fail("latent_prepare: heads %d, dim %d, rot %d (%d rotated), rank %d, rows of %d with the rotated part at %d", heads, dim,
                     rot, rot_dims, rank, q_width, q_rot);
   FMS_DISPATCH_DTYPE(dtype, T, FMS_DISPATCH_DTYPE(gain_dtype, TG,
-                     fms_launch(latent_prepare_kernel<T, TG>, dim3(n_tokens), dim3(128), rot_dims / 2 * sizeof(float2), stream,
+                     fms_launch(latent_prepare_kernel<T, TG>, dim3(n_tokens), dim3(128),
+                                (rot_dims / 2 < MOST_TURNS ? rot_dims / 2 : MOST_TURNS) * sizeof(float2), stream,
                                 (const T*)proj, proj_width, (T*)q_out, q_width, q_rot, q_copy, (const TG*)c_gain, eps, inv_freq,
                                 rot_dims, positions, position_ids, token_seq, slots, (T*)cache, table, table_stride, block_tokens,
                                 heads, dim, rot, rank, write_cache, n_seqs, n_slots, n_blocks, error_flag, halves, rot_mult,

@@ -1378,14 +1378,15 @@ def latent_prepare(proj: torch.Tensor, q_full: torch.Tensor, c_gain: torch.Tenso
     (queries that come from a projection of their own; ``proj`` then holds the query heads only).  ``halves``: value i
     of a rotated run turns with value i + rot_dims / 2 instead of its neighbour; ``rot_mult`` multiplies sines and cosines.
     ``own_space``: ``q_full`` is [tokens, heads, dim + rot] and takes every head's whole query, its rot part turned."""
-    if tuple(q_full.shape) != (proj.shape[0], heads, (dim if own_space else rank) + rot):
+    q_width = (dim if own_space else rank) + rot
+    if q_full.numel() != proj.shape[0] * heads * q_width:
         raise KernelError(f"latent_prepare: queries {tuple(q_full.shape)} for {heads} heads of {dim} + {rot}, rank {rank}")
     if kv is not None and (kv.dtype != proj.dtype or kv.shape[0] != proj.shape[0] or kv.shape[1] < rank + rot):
         raise KernelError("latent_prepare: the latent's matrix has the projection's dtype and rows, and rank + rot columns")
     if view.keys.dtype != proj.dtype or q_full.dtype != proj.dtype:
         raise KernelError(f"cache is {view.keys.dtype}, activations are {proj.dtype}")
     _call("latent_attention", "fms_latent_prepare", proj, _code(proj.dtype), proj.shape[1], q_full,
-          q_full.shape[2], dim if own_space else rank, 1 if own_space else 0, c_gain, _code(c_gain.dtype), float(eps), inv_freq, int(rot_dims), batch.positions,
+          q_width, dim if own_space else rank, 1 if own_space else 0, c_gain, _code(c_gain.dtype), float(eps), inv_freq, int(rot_dims), batch.positions,
           getattr(batch, "position_ids", None), batch.token_seq, batch.slots, view.keys,
           view.table, view.table.shape[1], view.block_tokens, proj.shape[0], heads, dim, rot, rank,
           1 if writes_cache else 0, batch.slots.shape[0], view.table.shape[0], view.keys.shape[0],

@@ -646,3 +646,28 @@ def test_scratch_of_attention_in_the_heads_own_space_is_bounded(monkeypatch, win
         assert float((got.double() - whole.double()).norm()) <= 2.0 ** -8 * float(whole.double().norm())
         fits = ops.latent_expanded_members(batch, window, hd, rank, rot)
         assert fits == [i for i in range(4) if batch.rows_seen(i, window) * row <= limit]
+
+
+@pytest.mark.parametrize("halves", [False, True])
+def test_latent_rotation_of_more_pairs_than_shared_memory_holds(halves):
+    """Sizes that were taken before sines and cosines went through shared memory, and queries as a matrix; rotations in 64 bits of
+    the float32 angles."""
+    from fms_b200.cache import Cache, KVRequest
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    heads, dim, rot, rank, n = 1, 2, 8200, 8, 3
+    g = torch.Generator().manual_seed(2)
+    cache = Cache([KVRequest(1, rank + rot, 0, planes=1)], 64, 64, torch.float32, "cuda", max_slots=1)
+    slots = cache.begin(1)
+    batch = Batch.from_lists(slots, cache.prepare(slots, [n]), [[0] * n], [[]], "cuda")
+    proj = torch.randn(n, heads * (dim + rot) + rank + rot, generator=g)
+    freq = torch.rand(rot // 2, generator=g)
+    q = torch.zeros(n, heads * (rank + rot), device="cuda")
+    ops.latent_prepare(proj.cuda(), q, torch.ones(rank, device="cuda"), 1e-5, freq.cuda(), rot, batch, cache.layer_view(0), heads, dim, rot, rank, halves=halves)
+    angle = (torch.arange(n).float()[:, None] * freq).double()
+    for got, x in ((q[:, rank:], proj[:, dim: dim + rot]), (cache.layer_view(0).keys[int(cache.groups[0].table_host[slots[0], 0]), 0, :n, rank:], proj[:, dim + rot + rank:])):
+        a, b = (x[:, : rot // 2], x[:, rot // 2:]) if halves else (x[:, 0::2], x[:, 1::2])
+        a, b = a.double() * torch.cos(angle) - b.double() * torch.sin(angle), b.double() * torch.cos(angle) + a.double() * torch.sin(angle)
+        want = torch.cat([a, b], 1) if halves else torch.stack([a, b], -1).flatten(1)
+        assert float((got.double().cpu() - want).abs().max()) <= 8 * 2.0 ** -23 * float(want.abs().max())
