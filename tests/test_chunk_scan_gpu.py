@@ -6,7 +6,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 KINDS = ["fixed", "gated", "space", "delta"]
-LENGTHS = [[64], [1, 65], [127, 3, 128], [200, 64, 129]]
+TAKEN = [(kind, 128) for kind in KINDS] + [("space", 64)]  # what the runs' kernels take; the others walk with 64 values
+LENGTHS = [[64], [1, 65], [127, 3, 128], [200, 64, 129], [330, 5]]  # the last: one sequence over three passes and more
 
 
 def batch_of(lengths):
@@ -23,7 +24,7 @@ def run(kind, batch, n, slots, vdim, seed, change=None, writes_state=True):
 
     g = torch.Generator().manual_seed(seed)
     r = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
-    dim, heads = 128, 4 if kind == "space" else 2
+    dim, heads = 128, heads_of(kind)
     state = r(slots, heads, vdim, dim)
     if kind == "space":
         xbc, proj = r(n, heads * vdim + 2 * 2 * dim) * 0.3, r(n, heads).bfloat16()
@@ -49,28 +50,41 @@ def run(kind, batch, n, slots, vdim, seed, change=None, writes_state=True):
     return y, [state, norm]
 
 
+def heads_of(kind):
+    return 4 if kind == "space" else 2
+
+
 def both(monkeypatch, *args, **kw):
+    """(by runs, walked); that each went the way it was sent is looked at."""
     from fms_b200.kernels import ops
 
+    calls, entry = [], ops._call
+    monkeypatch.setattr(ops, "_call", lambda library, name, *a: (calls.append((name, a)), entry(library, name, *a))[1])
     monkeypatch.setattr(ops, "chunk_scan_pays", lambda *_: False)
     want = run(*args, **kw)
+    assert "fms_chunk_scan" not in [name for name, _ in calls]
+    calls.clear()
     monkeypatch.setattr(ops, "chunk_scan_pays", lambda *_: True)
-    return run(*args, **kw), want
+    got = run(*args, **kw)
+    names = [name for name, _ in calls]
+    assert names.count("fms_chunk_scan") == 1 and not {"fms_decay_scan", "fms_selective_scan", "fms_delta_rule_scan"} & set(names)
+    monkeypatch.setattr(ops, "_call", entry)
+    return got, want, next(a for name, a in calls if name == "fms_chunk_scan")
 
 
-@pytest.mark.parametrize("kind", KINDS)
-@pytest.mark.parametrize("vdim", [128, 64])
+@pytest.mark.parametrize("kind,vdim", TAKEN)
 @pytest.mark.parametrize("lengths", LENGTHS)
 @pytest.mark.parametrize("pass_runs", [1, 2, 1000])
 def test_runs_equal_the_walk_over_tokens(monkeypatch, kind, vdim, lengths, pass_runs):
-    """Remainders of runs, sequences cut by a pass, states that are not zero before the step.  Both sides are sums of the
+    """Remainders of runs, sequences cut by one pass and by several, states that are not zero before the step.  Both sides are sums of the
     same up to 200 terms in float32, in another order: a few units of 2^-24 of the largest partial sums."""
     from fms_b200.kernels import ops
 
-    monkeypatch.setattr(ops, "CHUNK_STATE_BYTES", pass_runs * 4 * vdim * 128 * 4)
-    batch = batch_of(lengths)
+    monkeypatch.setattr(ops, "CHUNK_STATE_BYTES", pass_runs * heads_of(kind) * vdim * 128 * 4)
+    batch, runs = batch_of(lengths), sum((n + 63) // 64 for n in lengths)
     for writes in (True, False):
-        (y, left), (y0, left0) = both(monkeypatch, kind, batch, sum(lengths), len(lengths) + 1, vdim, 7, writes_state=writes)
+        (y, left), (y0, left0), sent = both(monkeypatch, kind, batch, sum(lengths), len(lengths) + 1, vdim, 7, writes_state=writes)
+        assert sent[7:9] == (runs, min(pass_runs, runs))  # runs of the step and of a pass
         for a, b in zip([y] + left, [y0] + left0):
             assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
             assert float((a - b).norm()) <= 2e-6 * float(b.norm())
@@ -86,7 +100,7 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(monkeypatch, kind, 
         def change(m):
             m[at, column] = value
 
-        (y, _), (y0, _) = both(monkeypatch, kind, batch_of([150]), 150, 2, 128, 9, change=change)
+        (y, _), (y0, _), _ = both(monkeypatch, kind, batch_of([150]), 150, 2, 128, 9, change=change)
         clean = run(kind, batch_of([150]), 150, 2, 128, 9)[0]
         assert bool(torch.isfinite(y[:at]).all()) and torch.allclose(y[:at], clean[:at], rtol=0, atol=1e-5 * float(clean.abs().max()))
         assert bool((torch.isfinite(y[at]) == torch.isfinite(y0[at])).all())
