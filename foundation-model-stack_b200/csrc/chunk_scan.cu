@@ -964,7 +964,7 @@ FMS_API int fms_chunk_scan(int kind, const float* q, const float* k, const float
                            float* totals, float* states, float* norms, float* solve, int* flags, float* o, int heads, int key_heads, int dim, int vdim,
                            int write_state, int n_slots, cudaStream_t stream) {
   if (n_runs <= 0 || n_seqs <= 0) return 0;
-  if (heads <= 0 || key_heads <= 0 || heads % key_heads || !fms_chunk_scan_takes(dim, vdim, heads / key_heads) || ((kind == 1 || kind == 3) && vdim != 128))
+  if (heads <= 0 || key_heads <= 0 || heads % key_heads || !fms_chunk_scan_takes(dim, vdim, heads / key_heads) || (kind != 2 && vdim != 128))
     return fms_fail("chunk_scan: %d heads over %d, dim %d, vdim %d", heads, key_heads, dim, vdim);
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || row % 4 || !aligned16(state) || !aligned16(states) || (carry && !aligned16(carry)))
     return fms_fail("chunk_scan: rows of %ld values, or a pointer, not on 16 bytes", row);
@@ -980,7 +980,7 @@ FMS_API int fms_chunk_scan(int kind, const float* q, const float* k, const float
   g.dt_stride = dt_stride; g.dt_is_bf16 = dt_dtype == FMS_BF16; g.state = state; g.carry = carry; g.scores = scores; g.factors = factors;
   g.states = states; g.norms = norms; g.totals = totals; g.flags = flags; g.o = o; g.heads = heads; g.key_heads = key_heads;
   g.n_seqs = n_seqs; g.n_slots = n_slots; g.write_state = write_state;
-  if (kind == 0) return vdim == 128 ? launch_passes<128, 0>(g, n_runs, pass_runs, stream) : launch_passes<64, 0>(g, n_runs, pass_runs, stream);
+  if (kind == 0) return launch_passes<128, 0>(g, n_runs, pass_runs, stream);
   if (kind == 1) return launch_passes<128, 1>(g, n_runs, pass_runs, stream);
   if (kind == 2) return vdim == 128 ? launch_passes<128, 2>(g, n_runs, pass_runs, stream) : launch_passes<64, 2>(g, n_runs, pass_runs, stream);
   if (kind == 3) return launch_passes<128, 3>(g, n_runs, pass_runs, stream);

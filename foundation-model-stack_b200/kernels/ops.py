@@ -1170,7 +1170,7 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
     norm_in = torch.empty((batch.n_seqs, heads, dim), dtype=torch.float32, device=proj.device) if gated else None
     gate_ptr = _ptr(proj) + gate_offset * proj.element_size() if gated else None
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv) if not gated or vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv) if vdim == 128 else None
     if plan is not None:
         if gated:
             _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias, float(gate_cap),
