@@ -926,12 +926,16 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
 
 
 CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
-# A sequence goes run by run through a scan under one decay a head from CHUNK_SCAN_FROM tokens of a step on, and through the delta
-# rule with one decay a head, which has two more products a run, from DELTA_CHUNKS_FROM on: its own tokens decide, so that
-# its results do not depend on what else is in the step.  Whole layers of one prompt, walk / runs in us (gated with a normalizer,
-# fixed decays, state space with heads of 64; delta rule of 16 heads of 128): 130 tokens - , - , - , 102 / 121; 200: 157 / 135,
-# 125 / 135, 191 / 170, 141 / 131; 256: 181 / 132, 140 / 132, 220 / 170, - ; 2,048: 1,627 / 583, 886 / 519, 1,450 / 760, 1,106 / 453.
-CHUNK_SCAN_FROM, DELTA_CHUNKS_FROM = 256, 192
+# A sequence goes run by run through a scan under one decay a head from CHUNK_SCAN_FROM tokens of a step on, under exponential
+# gates (a token's walk there has a normalizer too) from GATED_CHUNKS_FROM, through the delta rule with one decay a head (two more
+# products a run) from DELTA_CHUNKS_FROM: its own tokens decide, so that its results do not depend on what else is in the step.
+# Whole layers, all walk / all by runs / by this rule in us: one prompt of 130 tokens gated 115 / 123, fixed decays 96 / 123, state space
+# with heads of 64 142 / 161, delta rule of 16 heads of 128 103 / 120; of 200 156 / 143, 124 / 136, 191 / 177, 141 / 158; of 256 183 / 144,
+# 140 / 138, 221 / 177, 166 / 160; of 2,048 1,327 / 613, 890 / 580, 1,452 / 779, 1,109 / 480; four of 2,048 together, all by runs, 913 / 657,
+# 695 / 636, 962 / 854, 867 / 465.  The walk takes a sequence's tokens one after the other, but many sequences fill the multiprocessors
+# all the same, and a step that mixes both pays for both: eight of 131 to 392 tokens, fixed decays 601 / 660 / 614, state space 858 / 879 /
+# 895.
+CHUNK_SCAN_FROM, GATED_CHUNKS_FROM, DELTA_CHUNKS_FROM = 256, 160, 256
 
 
 def chunk_scan_pays(n: int, least: Optional[int] = None) -> bool:
@@ -1170,7 +1174,7 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
     norm_in = torch.empty((batch.n_seqs, heads, dim), dtype=torch.float32, device=proj.device) if gated else None
     gate_ptr = _ptr(proj) + gate_offset * proj.element_size() if gated else None
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv) if vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv, GATED_CHUNKS_FROM if gated else None) if vdim == 128 else None
     if plan is not None:
         if gated:
             _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias, float(gate_cap),
