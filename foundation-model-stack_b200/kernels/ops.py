@@ -1366,10 +1366,11 @@ def route_gather(ys: torch.Tensor, routing: Routing, every: Optional[torch.Tenso
 
 # ---- attention over cached latents -------------------------------------------------------------------
 _latent_split = None
-# Keys of a split of the tensor-core kernel in a decode step: LATENT_SHORT_SPLIT for a row that sees up to LATENT_SHORT_UP_TO,
-# else 256.  A block walks its split's keys one tile after the other (0.15 us a key), so short splits end sooner; long rows have
-# blocks enough, and each split costs its partial result.  8 sequences of 1,024 keys: 35 us in splits of 256, 19 of 64.
-LATENT_SHORT_SPLIT, LATENT_SHORT_UP_TO = 64, 2048
+# Keys of a split of the tensor-core kernel in a decode step: LATENT_SHORT_SPLIT for a row that sees up to LATENT_SHORT_UP_TO, in steps
+# of more than LATENT_FEW_ROWS rows up to LATENT_SHORT_UP_TO_MANY, else 256.  A block walks its split's keys one tile after the other
+# (0.15 us a key), so short splits end sooner, but each costs its partial result.  Whole layers, splits of 256 / of 64 in us: 8
+# rows of 1,000 keys 111 / 62, 32 186 / 168, 64 109 / 131, 128 164 / 203; 64 of 250 85 / 72.
+LATENT_SHORT_SPLIT, LATENT_SHORT_UP_TO, LATENT_SHORT_UP_TO_MANY, LATENT_FEW_ROWS = 64, 2048, 512, 32
 USE_LATENT_MMA = os.environ.get("FMS_B200_LATENT_MMA", "1") != "0"  # 0: a prompt's rows through the float32 kernel too
 
 
@@ -1413,14 +1414,16 @@ def latent_query_norm(proj: torch.Tensor, offset: int, n: int, gain: torch.Tenso
 # then heads, are taken a few at a time beyond it, and a sequence whose rows with one head's keys and values are more than that stays
 # in the latent's space.  (There a prompt of 2,048 tokens takes 138 MB for the queries and results of 32 heads over a latent of 512.)
 LATENT_EXPANDED_BYTES = 128 << 20
-# What decides between the two forms of a prompt's latent attention, a sequence at a time and by its own tokens, so that its results
-# do not depend on what else is in the step.  In the latent's space a (query, key) pair of a head takes LATENT_PAIR ns a value of
-# its two products where all multiprocessors are busy; making a key and a value of a head takes LATENT_MAKE ns a multiply-add, once
-# for all queries: with heads of 96 + 32 over a latent of 512 0.02 and 0.44 ns, so that making them pays from 23 tokens on, whatever is
-# cached.  (A sequence alone gains sooner: a block walks its keys at 160 ns a key.  But the more sequences, the less that counts: 16 of
-# 2 tokens onto 1,000 cached ones each would take half as long again.)  Whole layers, latent's space / heads' space in us: a
-# prompt of 64 tokens 45 / 41, of 256 88 / 53, two of 2,048 together 873 / 209; 64 tokens onto 8,000 cached ones 1,400 / 260.
-LATENT_PAIR, LATENT_MAKE = 0.02 / (2 * 512 + 32), 0.44 / (128 * (512 + 32))
+# What decides between the two forms of a prompt's latent attention, a sequence at a time: its own tokens and whether the step has more
+# than LATENT_FEW_SEQS sequences, not what the others bring.  In the latent's space a block walks a sequence's keys at LATENT_WALK ns a
+# value of a key's two products, and a (query, key) pair of a head takes LATENT_PAIR ns a value where all multiprocessors are busy;
+# making a key and a value of a head takes LATENT_MAKE ns a multiply-add, once for all queries: with heads of 96 + 32 over a latent of
+# 512 160, 0.02 and 0.44 ns.  So up to 8 sequences of 32 heads are made sooner than one is walked, and of more sequences those that bring
+# 23 tokens or more (32 sequences of 8 tokens onto 1,000 cached ones each would take three times as long).  Whole layers, latent's space /
+# heads' space in us: a prompt of 40 tokens 51 / 46, 16 tokens onto 1,024 cached ones 252 / 70, two prompts of 2,048 together
+# 852 / 183, 64 tokens of eight sequences onto 8,192 230 / 146, 256 of eight 310 / 152.
+LATENT_WALK, LATENT_PAIR, LATENT_MAKE = 160.0 / (2 * 512 + 32), 0.02 / (2 * 512 + 32), 0.44 / (128 * (512 + 32))
+LATENT_FEW_SEQS = 8
 
 
 _rows_tiles = {}
@@ -1433,23 +1436,26 @@ def _rows_tile(head_dim: int) -> int:
     return _rows_tiles[head_dim]
 
 
-def latent_prefers_expanded(batch, n: int, seen: int, head_dim: int, rank: int, rot: int) -> bool:
-    """Whether a sequence that brings ``n`` tokens, which see ``seen`` cached rows, attends over keys and values made of the cached latents
-    (``latent_attention_expanded``) rather than in the latent's space: unless so few queries share a key that its making does
-    not pay, its rows are too many (LATENT_EXPANDED_BYTES), or the tensor-core kernels of either form are switched off
-    (FMS_B200_LATENT_MMA, FMS_B200_ATTN_TC)."""
+def latent_prefers_expanded(batch, n: int, seen: int, heads: int, head_dim: int, rank: int, rot: int) -> bool:
+    """Whether a sequence that brings ``n`` tokens, which see ``seen`` cached rows, attends over keys and values made of the
+    cached latents (``latent_attention_expanded``) rather than in the latent's space: unless their making does not pay, its rows are
+    too many (LATENT_EXPANDED_BYTES), or the tensor-core kernels of either form are switched off (FMS_B200_LATENT_MMA,
+    FMS_B200_ATTN_TC)."""
     if batch.decode or not USE_LATENT_MMA or not _rows_tile(head_dim) or seen * (rank + rot + 2 * head_dim) * 2 > LATENT_EXPANDED_BYTES:
         return False
-    return n * LATENT_PAIR * (2 * rank + rot) > LATENT_MAKE * head_dim * (rank + rot)
+    make, values = LATENT_MAKE * head_dim * (rank + rot), 2 * rank + rot
+    if batch.n_seqs <= LATENT_FEW_SEQS and LATENT_FEW_SEQS * heads * make < LATENT_WALK * values:
+        return True
+    return n * LATENT_PAIR * values > make
 
 
-def latent_expanded_members(batch, window: int, head_dim: int, rank: int, rot: int):
+def latent_expanded_members(batch, window: int, heads: int, head_dim: int, rank: int, rot: int):
     """The sequences of a step that ``latent_prefers_expanded`` sends into the heads' own space (none of a batch whose lengths the
     host does not know)."""
     if batch.decode or getattr(batch, "len_before_host", None) is None:
         return []
     return [i for i, n in enumerate(batch.num_new) if n > 0 and
-            latent_prefers_expanded(batch, n, batch.rows_seen(i, window), head_dim, rank, rot)]
+            latent_prefers_expanded(batch, n, batch.rows_seen(i, window), heads, head_dim, rank, rot)]
 
 
 def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor, sink: Optional[torch.Tensor], heads: int,
@@ -1508,11 +1514,12 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
             and (rank + rot) % 32 == 0 and (gate is None or gate.dtype == torch.bfloat16)):
         # both products on the tensor cores, 32 rows a block: a prompt's rows as tokens x heads over all their keys; a
         # decode step's as one token's heads over one split of the keys, merged afterwards
-        n_splits, part_o, part_ml, split = 1, None, None, _latent_split
+        n_splits, part_o, part_ml, split, short = 1, None, None, _latent_split, 0
         if batch.decode:
             heads_per_block = 32
             # two at least: the merge rounds its results its own way, and the longest row must not decide for the others
-            n_splits = max(2, -(-min(batch.max_len_after, LATENT_SHORT_UP_TO) // LATENT_SHORT_SPLIT), -(-batch.max_len_after // split))
+            short = LATENT_SHORT_UP_TO if n <= LATENT_FEW_ROWS else LATENT_SHORT_UP_TO_MANY
+            n_splits = max(2, -(-min(batch.max_len_after, short) // LATENT_SHORT_SPLIT), -(-batch.max_len_after // split))
             parts = torch.empty((n * heads * n_splits * (rank + 2),), dtype=torch.float32, device=q_full.device)
             part_o = parts.data_ptr()  # [rank] of every split, then its maxima and sums [2]
             part_ml = part_o + n * heads * n_splits * rank * 4
@@ -1528,7 +1535,7 @@ def latent_attention(q_full: torch.Tensor, batch, view, gate: Optional[torch.Ten
               view.table, view.table.shape[1], view.block_tokens, batch.slots, batch.first_row,
               batch.positions, tiles, tiles.shape[0], tile_tokens, heads_per_block, heads, rank, rot,
               float(scale), batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], batch.token_seq, n_splits, split,
-              LATENT_SHORT_SPLIT, LATENT_SHORT_UP_TO, part_o, part_ml, int(window), _stream())
+              LATENT_SHORT_SPLIT, short, part_o, part_ml, int(window), _stream())
         if n_splits > 1:
             launches += 1
         return out

@@ -133,7 +133,7 @@ class LatentAttention(Part):
             return q
 
         # the sequences whose rows attend in the heads' own space; the others' do in the latent's
-        own = [] if self._expand is None else ops.latent_expanded_members(batch, self.window, self.vdim, self.rank, self.rot)
+        own = [] if self._expand is None else ops.latent_expanded_members(batch, self.window, self.heads, self.vdim, self.rank, self.rot)
         o = None
         if len(own) < batch.n_seqs:
             q_full = prepared(False, writes_cache)

@@ -533,15 +533,15 @@ def test_attention_in_the_heads_own_space_rounds_values_that_are_alike_once(hd):
 @pytest.mark.parametrize("window", [0, 300])
 @pytest.mark.parametrize("sink", [True, False])
 def test_latent_decode_of_a_row_does_not_depend_on_the_others(window, sink):
-    """Rows whose splits are 64 keys and rows whose splits are 256, below and at the edges of one split, alone and together, and
-    among so many others that the step has blocks enough: the same bits; against the float32 kernel within bfloat16's rounding
+    """Rows whose splits are 64 keys and rows whose splits are 256, below and at the edges of one split, alone and together, in
+    steps of few rows and in steps of many: the same bits in each; against the float32 kernel within bfloat16's rounding
     of probabilities and results."""
     from fms_b200.cache import Cache, KVRequest
     from fms_b200.engine.batch import Batch
     from fms_b200.kernels import ops
 
     heads, rank, rot = 32, 128, 32
-    lengths = [1, 5, 64, 65, 256, 700, 2047, 2048, 2049, 3000] + [900] * 40
+    lengths = [1, 5, 64, 65, 256, 512, 513, 700, 2047, 2048, 2049, 3000] + [900] * 40
     g = torch.Generator().manual_seed(7)
     cache = Cache([KVRequest(1, rank + rot, 0, planes=1)], sum((n + 63) // 64 * 64 for n in lengths), 4096, torch.bfloat16, "cuda", max_slots=len(lengths))
     slots = cache.begin(len(lengths))
@@ -556,10 +556,12 @@ def test_latent_decode_of_a_row_does_not_depend_on_the_others(window, sink):
         batch = Batch.from_lists([slots[i] for i in which], [lengths[i] - 1 for i in which], [[0]] * len(which), [[]] * len(which), "cuda")
         return ops.latent_attention(q[which].contiguous(), batch, view, gate[which].contiguous(), 0, sinks, heads, rank, rot, 0.1, window=window)
 
-    together = decode(list(range(len(lengths))))
-    for i in range(11):
+    together = decode(list(range(32)))
+    for i in range(13):
         assert torch.equal(decode([i])[0], together[i])
-    assert torch.equal(decode([0, 1, 2, 3]), together[:4]) and torch.equal(decode([9, 4, 7]), together[[9, 4, 7]])
+    assert torch.equal(decode([0, 1, 2, 3]), together[:4]) and torch.equal(decode([11, 4, 7]), together[[11, 4, 7]])
+    together = decode(list(range(len(lengths))))  # more than 32 rows
+    assert torch.equal(decode(list(range(33))), together[:33]) and torch.equal(decode(list(range(40, 4, -1))), together[list(range(40, 4, -1))])
     before, ops.USE_LATENT_MMA = ops.USE_LATENT_MMA, False
     try:
         want = decode(list(range(len(lengths)))).double()
@@ -583,9 +585,10 @@ def test_each_sequence_of_a_step_takes_the_form_of_latent_attention_that_its_own
     w = latent_tensors(g, 40, m)
     mixer = latent_mixer(m, 40, w, 1e-5, torch.bfloat16)
     mixer.window = window
-    least = next(n for n in range(1, 200) if ops.latent_prefers_expanded(Batch.from_lists([0], [0], [[0] * 2], [[]], "cpu"), n, n, vdim, rank, rot))
+    many = Batch.from_lists(list(range(10)), [0] * 10, [[0] * 2] * 10, [[]] * 10, "cpu")
+    least = next(n for n in range(1, 200) if ops.latent_prefers_expanded(many, n, n, heads, vdim, rank, rot))
     assert 2 < least < 100
-    portions = [[80, least - 1], [150, 1], [40, least], [0, 200], [129, 2]]
+    portions = [[80, least - 1], [150, 1], [40, least], [0, 200], [129, 2]] * 2
     xs = [torch.randn(sum(p), 40, generator=g).to(torch.bfloat16) for p in portions]
 
     def steps(which):
@@ -593,19 +596,21 @@ def test_each_sequence_of_a_step_takes_the_form_of_latent_attention_that_its_own
         slots, out = cache.begin(len(which)), None
         for step in range(2):
             live = [j for j, i in enumerate(which) if portions[i][step]]
+            if not live:
+                continue
             counts = [portions[which[j]][step] for j in live]
             lens = cache.prepare([slots[j] for j in live], counts)
             batch = Batch.from_lists([slots[j] for j in live], lens, [[0] * c for c in counts], [[] for _ in live], "cuda")
             if step and len(which) > 1:
-                assert ops.latent_expanded_members(batch, window, vdim, rank, rot) == [2, 3]
+                assert ops.latent_expanded_members(batch, window, heads, vdim, rank, rot) == [2, 3, 7, 8]
             rows = torch.cat([xs[which[j]][lens[k]: lens[k] + counts[k]] for k, j in enumerate(live)]).cuda()
             out = mixer.forward(rows, batch, cache.layer_view(0))
             cache.commit([slots[j] for j in live], counts)
         return torch.split(out, [portions[i][1] for i in which])
 
-    together = steps([0, 1, 2, 3, 4])
+    together = steps(list(range(10)))
     d = {k: v.double() for k, v in w.items()}
-    for i, got in enumerate(together):
+    for i, got in enumerate(together[:5]):
         if not window:
             want, _ = pg.latent_attention(xs[i].double(), m, 1e-5, d["q"], d["dkv"], d["norm"], d["uk"], d["uv"], d["sink"], d["g"], d["o"])
             close(got, want[portions[i][0]:], "bf16")
@@ -644,8 +649,8 @@ def test_scratch_of_attention_in_the_heads_own_space_is_bounded(monkeypatch, win
         longest = max(batch.rows_seen(i, window) for i in range(5)) * row
         assert torch.cuda.max_memory_allocated() - before <= max(limit, longest) + got.numel() * 2 + 64 * 1024
         assert float((got.double() - whole.double()).norm()) <= 2.0 ** -8 * float(whole.double().norm())
-        fits = ops.latent_expanded_members(batch, window, hd, rank, rot)
-        assert fits == [i for i in range(4) if batch.rows_seen(i, window) * row <= limit]
+        fits = ops.latent_expanded_members(batch, window, heads, hd, rank, rot)
+        assert fits == [i for i in range(5) if batch.rows_seen(i, window) * row <= limit]
 
 
 @pytest.mark.parametrize("halves", [False, True])

@@ -113,7 +113,24 @@ def test_the_switches_of_the_tensor_core_kernels_reach_latent_prompts(switch, ex
     """Each, in a process of its own: a prompt's latent attention does not take the form that the switched-off kernel makes."""
     code = ("import torch; from fms_b200.kernels import ops; from fms_b200.engine.batch import Batch; "
             "b = Batch.from_lists([0], [0], [[0] * 500], [[]], 'cpu'); "
-            "print(*(bool(ops.latent_expanded_members(b, 0, h, 512, 32)) for h in (128, 48)))")
+            "print(*(bool(ops.latent_expanded_members(b, 0, 32, h, 512, 32)) for h in (128, 48)))")
     env = {**os.environ, **switch}
     out = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, check=True)
     assert out.stdout.split() == [str(expanded), "False"]
+
+
+def test_the_form_of_a_sequences_latent_attention_does_not_depend_on_what_the_others_bring():
+    """Heads of 128 over a latent of 512: in steps of up to eight sequences every one is made keys and values, in larger ones those of
+    23 tokens or more, whatever is cached and whatever the others bring."""
+    from fms_b200.engine.batch import Batch
+    from fms_b200.kernels import ops
+
+    def members(new, before=0, heads=32):
+        return ops.latent_expanded_members(Batch.from_lists(list(range(len(new))), [before] * len(new), [[0] * n for n in new], [[]] * len(new), "cpu"),
+                                           0, heads, 128, 512, 32)
+
+    assert members([2] * 8, 8000) == members([1, 2, 500, 1, 1, 1, 1, 1]) == list(range(8))
+    for others in (2, 22, 500):
+        assert [i for i in members([others] * 9 + [23, 22, 1, 600], 1000) if i > 8] == [9, 12]
+    assert members([2, 40] * 4, heads=64) == [1, 3, 5, 7]  # eight sequences of 64 heads would not be made sooner than one is walked
+    assert members([40], before=200000) == [] and members([1] * 4) == []
