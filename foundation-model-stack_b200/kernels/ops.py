@@ -1412,8 +1412,9 @@ def latent_query_norm(proj: torch.Tensor, offset: int, n: int, gain: torch.Tenso
 
 # Bytes that ``latent_attention_expanded`` takes at a time for gathered rows and the keys and values made of them: sequences, and
 # then heads, are taken a few at a time beyond it, and a sequence whose rows with one head's keys and values are more than that stays
-# in the latent's space.  (There a prompt of 2,048 tokens takes 138 MB for the queries and results of 32 heads over a latent of 512.)
-LATENT_EXPANDED_BYTES = 128 << 20
+# in the latent's space.  Room for 8,192 rows of 32 heads of 128 at once (in two passes eight sequences of 8 tokens onto 1,024 cached
+# ones each took 178 instead of 146 us a layer); in the latent's space a prompt of 2,500 tokens takes as much for its queries and results.
+LATENT_EXPANDED_BYTES = 160 << 20
 # What decides between the two forms of a prompt's latent attention, a sequence at a time: its own tokens and whether the step has more
 # than LATENT_FEW_SEQS sequences, not what the others bring.  In the latent's space a block walks a sequence's keys at LATENT_WALK ns a
 # value of a key's two products, and a (query, key) pair of a head takes LATENT_PAIR ns a value where all multiprocessors are busy;
@@ -1483,6 +1484,7 @@ def latent_attention_expanded(q: torch.Tensor, batch, view, expand: torch.Tensor
               view.block_tokens, batch.slots, start, first, batch.n_seqs, cached, rows, view.table.shape[0],
               view.keys.shape[0], _stream())
         step = max(1, min(heads, (LATENT_EXPANDED_BYTES - rows * width * size) // (rows * 2 * head_dim * size)))
+        step = -(-heads // -(-heads // step))  # as many heads in the last pass as in the others, or nearly
         for h in range(0, heads, step):
             m = min(step, heads - h)
             kv = linear(cached, expand[h:h + m].view(m * 2 * head_dim, width))
