@@ -168,11 +168,14 @@ __device__ __forceinline__ float2 token_gates(const ChunkArgs& g, int t, int end
   return make_float2((float)exp(-exp((double)g.a_log[head]) * dt), (float)dt);
 }
 
-// ---- products of 64 x 64 tokens of a run: sum[i][j] = x_t . y_s over all channels, t = tid / 16 * 8 + i, s = tid % 16 + 16 j ------
+// ---- products of 64 x 64 tokens of a run: sum[i][j] = x_t . y_s over all channels, t = product_row(i), s = tid % 16 + 16 j ------
+// Only blocks of 16 x 16 that hold an s <= t are made (20 of every thread's 32 products), the others are left at zero.
 // In 64 bits, rounded once: an output is a sum of few of them where decays are short, and with float32 sums of 16 terms (7e-8 of
 // a score's size, once rounded 2.5e-8) it was up to 20% further from 64 bits than the walk's.  Half the FMA pipe's rate, but a
 // twentieth of the scan's products.  A slice's values are widened on their way from registers to shared memory, the next slice's
 // loads are on their way meanwhile.  SAME: y is x.  sm: [2][SAME ? 1 : 2][C][SROW].
+__device__ __forceinline__ int product_row(int i) { return 2 * (threadIdx.x >> 4) + (i & 1) + 16 * (i >> 1); }
+
 template <bool SAME>
 __device__ __forceinline__ void run_products(const float* x, const float* y, long row, int rows, double* sm, double (&sum)[8][4]) {
   constexpr int OPERANDS = SAME ? 1 : 2;
@@ -209,7 +212,7 @@ __device__ __forceinline__ void run_products(const float* x, const float* y, lon
   for (int d = 0; d < DIM; d += SLICE) {
     const int buf = (d / SLICE) & 1;
     if (d + SLICE < DIM) fetch(d + SLICE);
-    const double* xs = sm + (buf * OPERANDS * C + ty * 8) * SROW;
+    const double* xs = sm + (buf * OPERANDS * C + 2 * ty) * SROW;
     const double* ys = sm + ((buf * OPERANDS + OPERANDS - 1) * C + tx) * SROW;
 #pragma unroll
     for (int e = 0; e < SLICE; e += 2) {
@@ -218,9 +221,9 @@ __device__ __forceinline__ void run_products(const float* x, const float* y, lon
       for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const double2*>(ys + 16 * j * SROW + e);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const double2 a = *reinterpret_cast<const double2*>(xs + i * SROW + e);
+        const double2 a = *reinterpret_cast<const double2*>(xs + ((i & 1) + 16 * (i >> 1)) * SROW + e);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sum[i][j] = fma(a.y, b[j].y, fma(a.x, b[j].x, sum[i][j]));
+        for (int j = 0; j <= (i >> 1); ++j) sum[i][j] = fma(a.y, b[j].y, fma(a.x, b[j].x, sum[i][j]));
       }
     }
     if (d + SLICE < DIM) put(buf ^ 1);
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
       g.flags[(size_t)blockIdx.x * g.heads + head] = 0;
     }
   }
-  const int ty = tid >> 4, tx = tid & 15;  // tokens t = ty * 8 + i, s = tx + 16 j
+  const int tx = tid & 15;  // tokens t = product_row(i), s = tx + 16 j
   double sum[8][4];
   run_products<false>(g.q + (size_t)row0 * g.row + (size_t)kh * DIM, g.k + (size_t)row0 * g.row + (size_t)kh * DIM, g.row, rows, sm, sum);
   // only now: blocks of the states' kernel that come earlier gather on the multiprocessors that are free first, two together
@@ -268,11 +271,10 @@ __global__ void __launch_bounds__(128) chunk_scores_kernel(ChunkArgs g) {
   pdl_launch_dependents();
   float* out = g.scores + ((size_t)blockIdx.x * g.key_heads + kh) * C * C;
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+  for (int i = 0; i < 8; i += 2)
 #pragma unroll
-    for (int i = 0; i < 8; i += 4)
-      *reinterpret_cast<float4*>(out + (tx + 16 * j) * C + ty * 8 + i) =
-          make_float4((float)sum[i][j], (float)sum[i + 1][j], (float)sum[i + 2][j], (float)sum[i + 3][j]);
+    for (int j = 0; j <= (i >> 1); ++j)  // what lies above is not read
+      *reinterpret_cast<float2*>(out + (tx + 16 * j) * C + product_row(i)) = make_float2((float)sum[i][j], (float)sum[i + 1][j]);
 }
 
 // ---- the states before every run: 128 key channels x VT value columns a block, 8 x VT / 8 a thread ------------------------
@@ -640,14 +642,14 @@ __global__ void __launch_bounds__(128) chunk_solve_kernel(ChunkArgs g) {
     as[tid] = tid < rows ? g.decay[at] : 1.f;
     bt[tid] = tid < rows ? g.gates[at] : 0.f;
   }
-  const int ty = tid >> 4, tx = tid & 15;  // rows t = ty * 8 + i, columns s = tx + 16 j
+  const int tx = tid & 15;  // rows t = product_row(i), columns s = tx + 16 j
   double sum[8][4];
   const float* k = g.k + (size_t)row0 * g.row + (size_t)kh * DIM;
   run_products<true>(k, k, g.row, rows, sm, sum);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) A[ty * 8 + i][tx + 16 * j] = (float)sum[i][j];
+    for (int j = 0; j < 4; ++j) A[product_row(i)][tx + 16 * j] = (float)sum[i][j];
   for (int i = tid; i < C * TP; i += 128) T[i] = 0.f;
   __syncthreads();
   if (tid < C) {  // a row a thread, s downwards

@@ -926,21 +926,20 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
 
 
 CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
-# A sequence goes run by run through a scan under one decay a head from CHUNK_SCAN_FROM tokens of a step on, under exponential
-# gates (a token's walk there has a normalizer too) from GATED_CHUNKS_FROM, through the delta rule with one decay a head (two more
-# products a run) from DELTA_CHUNKS_FROM: its own tokens decide, so that its results do not depend on what else is in the step.
-# Whole layers, all walk / all by runs / by this rule in us: one prompt of 130 tokens gated 115 / 123, fixed decays 96 / 123, state space
-# with heads of 64 142 / 161, delta rule of 16 heads of 128 103 / 120; of 200 156 / 143, 124 / 136, 191 / 177, 141 / 158; of 256 183 / 144,
-# 140 / 138, 221 / 177, 166 / 160; of 2,048 1,327 / 613, 890 / 580, 1,452 / 779, 1,109 / 480; four of 2,048 together, all by runs, 913 / 657,
-# 695 / 636, 962 / 854, 867 / 465.  The walk takes a sequence's tokens one after the other, but many sequences fill the multiprocessors
-# all the same, and a step that mixes both pays for both: eight of 131 to 392 tokens, fixed decays 601 / 660 / 614, state space 858 / 879 /
-# 895.
-CHUNK_SCAN_FROM, GATED_CHUNKS_FROM, DELTA_CHUNKS_FROM = 256, 160, 256
+# A sequence goes run by run through a scan under one decay a head from so many tokens of a step on: its own tokens decide, so that
+# its results do not depend on what else is in the step.  Whole layers, all walk / all by runs in us, under exponential gates with a
+# normalizer, fixed decays, state space with heads of 64, delta rule of 16 heads of 128: one prompt of 200 tokens 156 / 140, 125 / 137,
+# 192 / 178, 140 / 160; of 256 183 / 142, 140 / 140, 219 / 179, 165 / 158; of 512 329 / 201, 240 / 183, 389 / 245, 295 / 199; of 2,048
+# 1,327 / 607, 891 / 574, 1,455 / 782, 1,110 / 462; eight of 131 to 392 693 / 673, 598 / 652, 868 / 891, 566 / 468.  The walk takes a sequence's
+# tokens one after the other, but many sequences fill the multiprocessors all the same, and a step that mixes both forms pays for both
+# (eight of 131 to 392, those of 256 and more by runs: fixed decays 613, state space 902): so the lines lie where a mixed step seldom
+# takes longer than its walk, for the kinds whose runs gain least highest.
+CHUNK_SCAN_FROM = {"gated": 256, "fixed": 512, "space": 384, "delta": 256}
 
 
-def chunk_scan_pays(n: int, least: Optional[int] = None) -> bool:
+def chunk_scan_pays(n: int, kind: str) -> bool:
     """Whether a sequence's ``n`` tokens of a step go run by run (``fms_chunk_scan``) or token by token."""
-    return n >= (CHUNK_SCAN_FROM if least is None else least)
+    return n >= CHUNK_SCAN_FROM[kind]
 
 
 class _Runs:
@@ -951,14 +950,13 @@ class _Runs:
         self.whole = whole  # every sequence of the step is among them
 
 
-def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, rows: torch.Tensor,
-                     least: Optional[int] = None) -> Optional[_Runs]:
+def _chunk_scan_runs(batch, dim: int, vdim: int, heads: int, key_heads: int, rows: torch.Tensor, kind: str) -> Optional[_Runs]:
     """The step's rows as runs for ``fms_chunk_scan``, or None where it takes none of them: other head sizes, rows
     that do not lie on 16 bytes, decode steps and short prompts (which go token by token), a capture that has not seen the batch
     before (the runs come from the host)."""
     if batch.decode or not batch.num_new:
         return None
-    chosen = [chunk_scan_pays(n, least) for n in batch.num_new]
+    chosen = [chunk_scan_pays(n, kind) for n in batch.num_new]
     if not any(chosen):
         return None
     if _ptr(rows) & 15 or rows.shape[1] % 4 or batch.n_seqs > 65535:
@@ -1003,7 +1001,7 @@ def selective_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_bia
             or tuple(state.shape[1:]) != (heads, vdim, n_state):
         raise KernelError("selective_scan: xbc float32 [tokens, x | B | C], state float32 [slots, heads, vdim, state]")
     y = torch.empty((n, heads * vdim), dtype=torch.float32, device=xbc.device)
-    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups, xbc)
+    plan = _chunk_scan_runs(batch, n_state, vdim, heads, groups, xbc, "space")
     if plan is not None:
         x, b = _ptr(xbc), _ptr(xbc) + heads * vdim * 4
         _chunk_scan(2, b + groups * n_state * 4, b, x, xbc.shape[1], plan, batch, state, y, heads, groups, n_state, vdim, writes_state,
@@ -1041,7 +1039,7 @@ def delta_rule_scan(qkv: torch.Tensor, proj: torch.Tensor, beta_offset: int, a_r
             raise KernelError("delta_rule_scan: decays' logits [tokens, heads * dim] in the projection's dtype")
         a_ptr, a_stride = _ptr(a_raw), heads * dim
     o = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, kvheads, qkv, DELTA_CHUNKS_FROM) if per_head and vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, kvheads, qkv, "delta") if per_head and vdim == 128 else None
     # decays [tokens, heads * dim] where a sequence walks, then betas and, where one goes run by run, decays [tokens, heads]
     walks = plan is None or not plan.whole
     scratch = torch.empty((n * heads * ((dim if walks else 0) + (1 if plan is None else 2)),), dtype=torch.float32, device=qkv.device)
@@ -1174,7 +1172,7 @@ def decay_scan(proj: torch.Tensor, state: torch.Tensor, batch, heads: int, dim: 
     gates = torch.empty((n, heads, 3), dtype=torch.float32, device=proj.device) if gated else None
     norm_in = torch.empty((batch.n_seqs, heads, dim), dtype=torch.float32, device=proj.device) if gated else None
     gate_ptr = _ptr(proj) + gate_offset * proj.element_size() if gated else None
-    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv, GATED_CHUNKS_FROM if gated else None) if vdim == 128 else None
+    plan = _chunk_scan_runs(batch, dim, vdim, heads, heads, qkv, "gated" if gated else "fixed") if vdim == 128 else None
     if plan is not None:
         if gated:
             _call("state_scan", "fms_exp_gates", gate_ptr, _code(proj.dtype), proj.shape[1], gate_bias, float(gate_cap),
