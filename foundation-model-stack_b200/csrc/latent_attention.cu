@@ -49,9 +49,11 @@ __device__ __forceinline__ void rotate_run(const T* src, T* dst, int i, int half
   }
 }
 
-constexpr int MOST_TURNS = 4096;  // pairs whose sines and cosines shared memory holds; further ones are taken where they are needed
+// Pairs whose sines and cosines shared memory holds; with MORE, a kernel of its own (sines in the loop over the heads' pairs cost the
+// usual one half as much again), further ones are taken where they are needed.
+constexpr int MOST_TURNS = 4096;
 
-template <typename T, typename TG>
+template <typename T, typename TG, bool MORE>
 __global__ void __launch_bounds__(128) latent_prepare_kernel(
     const T* __restrict__ proj, int proj_width, T* __restrict__ q_out, int q_width, int q_rot, int q_copy,
     const TG* __restrict__ c_gain, float eps, const float* __restrict__ inv_freq, int rot_dims, const int* __restrict__ positions,
@@ -74,8 +76,12 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(
     sincosf(position * inv_freq[i], &sn, &cs);
     return make_float2(sn * rot_mult, cs * rot_mult);
   };
-  auto turn_of = [&](int u) { return u >= half ? make_float2(0.f, 0.f) : (u < MOST_TURNS ? turns[u] : turn(u)); };
-  for (int i = threadIdx.x; i < min(half, MOST_TURNS); i += blockDim.x) turns[i] = turn(i);
+  auto turn_of = [&](int u) {
+    if (u >= half) return make_float2(0.f, 0.f);
+    if (MORE && u >= MOST_TURNS) return turn(u);
+    return turns[u];
+  };
+  for (int i = threadIdx.x; i < (MORE ? MOST_TURNS : half); i += blockDim.x) turns[i] = turn(i);
   __syncthreads();
   // the rotated part of every head's query
   for (int i = threadIdx.x; i < heads * units; i += blockDim.x) {
@@ -677,13 +683,17 @@ FMS_API int fms_latent_prepare(const void* proj, int dtype, int proj_width, void
       q_rot < (q_copy ? dim : 0) || q_width < q_rot + rot)
     return fms_fail("latent_prepare: heads %d, dim %d, rot %d (%d rotated), rank %d, rows of %d with the rotated part at %d", heads, dim,
                     rot, rot_dims, rank, q_width, q_rot);
-  FMS_DISPATCH_DTYPE(dtype, T, FMS_DISPATCH_DTYPE(gain_dtype, TG,
-                     fms_launch(latent_prepare_kernel<T, TG>, dim3(n_tokens), dim3(128),
-                                (rot_dims / 2 < MOST_TURNS ? rot_dims / 2 : MOST_TURNS) * sizeof(float2), stream,
-                                (const T*)proj, proj_width, (T*)q_out, q_width, q_rot, q_copy, (const TG*)c_gain, eps, inv_freq,
-                                rot_dims, positions, position_ids, token_seq, slots, (T*)cache, table, table_stride, block_tokens,
-                                heads, dim, rot, rank, write_cache, n_seqs, n_slots, n_blocks, error_flag, halves, rot_mult,
-                                (const T*)kv, kv_width)));
+  const int held = rot_dims / 2 < MOST_TURNS ? rot_dims / 2 : MOST_TURNS;
+#define FMS_PREPARE(MORE)                                                                                                       \
+  FMS_DISPATCH_DTYPE(dtype, T, FMS_DISPATCH_DTYPE(gain_dtype, TG,                                                                \
+                     fms_launch(latent_prepare_kernel<T, TG, MORE>, dim3(n_tokens), dim3(128), held * sizeof(float2), stream,    \
+                                (const T*)proj, proj_width, (T*)q_out, q_width, q_rot, q_copy, (const TG*)c_gain, eps, inv_freq, \
+                                rot_dims, positions, position_ids, token_seq, slots, (T*)cache, table, table_stride, block_tokens, \
+                                heads, dim, rot, rank, write_cache, n_seqs, n_slots, n_blocks, error_flag, halves, rot_mult,     \
+                                (const T*)kv, kv_width)))
+  if (held < rot_dims / 2) FMS_PREPARE(true);
+  else FMS_PREPARE(false);
+#undef FMS_PREPARE
   return fms_launch_status("latent_prepare");
 }
 
