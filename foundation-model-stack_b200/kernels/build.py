@@ -40,6 +40,7 @@ if DEBUG_BOUNDS:
 PLAIN_LIBRARIES = {
     "elementwise": ("elementwise.cu", []),
     "gemm_f32": ("gemm_f32.cu", []),
+    "gemm_f32_tc": ("gemm_f32_tc.cu", []),
     "gemm_bf16_skinny": ("gemm_bf16_skinny.cu", []),
     "gemm_bf16_mid": ("gemm_bf16_mid.cu", []),
     "gemm_bf16_tc": ("gemm_bf16_tc.cu", []),

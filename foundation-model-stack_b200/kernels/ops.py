@@ -4,7 +4,8 @@ Tensors are torch tensors on a CUDA device (torch is used for memory and for the
 product only); every function launches on torch's current stream.  There is no CPU implementation and
 no fallback: a tensor on another device, a missing compiler or a failed build raises.
 
-Matrix products: float32 runs ``gemm_f32`` (FFMA, no tensor-core mode).  bfloat16 runs the weight-streaming
+Matrix products: float32 runs ``gemm_f32`` (FFMA, no tensor-core mode) and, for a prompt's rows times a large matrix, ``gemm_f32_tc``
+(the tensor cores over operands split into three bfloat16 parts, which lose nothing).  bfloat16 runs the weight-streaming
 ``mma.sync`` kernel up to 8 rows (decode of few sequences) and otherwise the library product (cuBLAS through
 ``torch.nn.functional.linear``), as the reference does for every linear layer (fms/modules/linear.py:119-156) —
 except the gated feed-forward product, which from ``TENSOR_CORE_ROWS_GLU`` (512) rows on, where its tiles of 256
@@ -22,6 +23,7 @@ products and the fused projection up to 256 rows (clusters of blocks share a til
 from __future__ import annotations
 
 import ctypes
+import itertools
 import os
 from typing import Optional
 
@@ -44,6 +46,7 @@ _SIGNATURES = {
     "fms_decode_advance": [_P, _P, _P, _P, _P, _I, _I, _P],
     "fms_rotary_table": [_P, _P, _P, _P, _I, _I, _P],
     "fms_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _P],
+    "fms_gemm_f32_tc": [_P, _P, _P, _P, _P, _L, _I, _I, _I, _P, _P],
     "fms_linear_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
     "fms_token_gate_bf16_skinny": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fms_grouped_bf16_skinny": [_P, _P, _P, _P, _I, _I, _I, _I, _F, _F, _P],
@@ -427,18 +430,64 @@ def cast_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 
 
 # ---- linear ------------------------------------------------------------------------------------------
+# Tokens of a sequence from which the float32 products of its rows go to the tensor cores (gemm_f32_tc.cu: operands in three bfloat16
+# parts), where the matrix is large enough.  The sequence's own tokens decide, and what a row gets there does not depend on the other
+# rows, so that a sequence's results do not depend on what else is in the step.  CUDA cores / tensor cores in us, by rows: w of 28,672 x
+# 4,096 17 240 / 153, 64 335 / 175, 256 1,260 / 345; 4,096 x 14,336 17 120 / 81, 256 700 / 157; 4,096 x 4,096 16 33 / 34, 17 43 / 34;
+# 2,048 x 2,048 17 18 / 22, 33 37 / 22; 1,024 x 1,024 32 14 / 17, 33 18 / 17, 256 26 / 20.
+F32_SPLIT_SIZE, F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_SMALL = 12 << 20, 17, 33
+F32_SPLIT_BYTES = 256 << 20  # of scratch that a product takes at a time for the parts of its rows (2,816 rows of 14,336 values)
+
+
+def f32_split_tokens(weight: torch.Tensor) -> int:
+    """Tokens from which a sequence's rows go to the tensor cores; 0: never."""
+    n, k = weight.shape
+    if min(n, k) < 1024:
+        return 0
+    return F32_SPLIT_TOKENS if n * k >= F32_SPLIT_SIZE else F32_SPLIT_TOKENS_SMALL
+
+
+def _linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], sequences) -> torch.Tensor:
+    m, (n, k) = x.shape[0], weight.shape
+    if hasattr(sequences, "num_new"):
+        sequences = None if sequences.decode else sequences.num_new or None
+    y = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    least = f32_split_tokens(weight) if sequences is not None and m >= F32_SPLIT_TOKENS else 0
+    if not least or max(sequences) < least or sum(sequences) != m:
+        _call("gemm_f32", "fms_gemm_f32", x, weight, bias, y, m, n, k, _stream())
+        return y
+    at = 0
+    for many, rows in itertools.groupby(sequences, lambda tokens: tokens >= least):  # runs of rows that go the same way
+        count = sum(rows)
+        if not count:
+            continue
+        if not many:
+            _call("gemm_f32", "fms_gemm_f32", x[at:at + count], weight, bias, y[at:at + count], count, n, k, _stream())
+            at += count
+            continue
+        size = (k + 63) // 64 * 64 * 6 + 1  # of a row of x in its parts
+        step = max(256, F32_SPLIT_BYTES // size // 256 * 256)
+        scratch = torch.empty((min(count, step) * size,), dtype=torch.uint8, device=x.device)
+        for first in range(at, at + count, step):
+            some = min(step, at + count - first)
+            _call("gemm_f32_tc", "fms_gemm_f32_tc", x[first:first + some], weight, bias, y[first:first + some], scratch, scratch.numel(),
+                  some, n, k, error_flag(x.device), _stream())
+        at += count
+    return y
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
-           out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """x [rows, in] times weight [out, in] transposed (+ bias).  ``out_dtype`` defaults to x's dtype."""
+           out_dtype: Optional[torch.dtype] = None, sequences=None) -> torch.Tensor:
+    """x [rows, in] times weight [out, in] transposed (+ bias).  ``out_dtype`` defaults to x's dtype.  ``sequences``: the rows'
+    ``Batch`` or how many rows each sequence has, one behind the other (a large float32 product chooses its kernel by it); None:
+    every row stands alone."""
     out_dtype = out_dtype or x.dtype
     _ptr(x), _ptr(weight)
     if weight.dtype == torch.float32:
         # true float32: also taken by a float32-stored matrix inside a bfloat16 model
         x32 = x if x.dtype == torch.float32 else x.float()
         b32 = None if bias is None else (bias if bias.dtype == torch.float32 else bias.float())
-        y = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
-        _call("gemm_f32", "fms_gemm_f32", x32, weight, b32, y, x.shape[0], weight.shape[0],
-              weight.shape[1], _stream())
+        y = _linear_f32(x32, weight, b32, sequences)
         return y if out_dtype == torch.float32 else y.to(out_dtype)
     if weight.dtype != torch.bfloat16 or x.dtype != torch.bfloat16:
         raise KernelError(f"linear: x {x.dtype}, weight {weight.dtype}")
@@ -546,7 +595,8 @@ SKINNY_ROWS = 8  # rows up to which the weight-streaming kernels are used (more 
 
 
 # ---- feed-forward ------------------------------------------------------------------------------------
-def gated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], activation: int) -> torch.Tensor:
+def gated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], activation: int,
+                 sequences=None) -> torch.Tensor:
     """act(x Wg^T) * (x Wu^T) for weight = [Wg; Wu]: one kernel for few bfloat16 rows, else the product
     followed by ``gated_activation``."""
     hidden = weight.shape[0] // 2
@@ -567,10 +617,11 @@ def gated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
     if (_tensor_core_fits(x, weight, bias, TENSOR_CORE_ROWS_GLU)
             and (x.shape[0] + 255) // 256 * 256 <= TENSOR_CORE_MAX_PADDING * x.shape[0]):
         return gated_linear_tensor_core(x, weight, bias, activation)
-    return gated_activation(linear(x, weight, bias), activation)
+    return gated_activation(linear(x, weight, bias, None, sequences), activation)
 
 
-def activated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], activation: int) -> torch.Tensor:
+def activated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], activation: int,
+                     sequences=None) -> torch.Tensor:
     """act(x weight^T + bias): the first product of an ungated feed-forward.  A few bfloat16 rows: the weight-streaming kernel
     with the activation in its epilogue; many, where its tiles fit (as for the gated product): the tcgen05 kernel with
     the activation in its epilogue; else the product and then the activation in place."""
@@ -587,7 +638,7 @@ def activated_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch
         _call("gemm_bf16_tc", "fms_linear_act_bf16_tc", x, weight, bias, y, x.shape[0], weight.shape[0],
               weight.shape[1], int(activation), error_flag(x.device), _stream())
         return y
-    y = linear(x, weight, bias)
+    y = linear(x, weight, bias, None, sequences)
     _call("elementwise", "fms_activation", y, _code(y.dtype), int(activation), y.numel(), _stream())
     return y
 
@@ -721,7 +772,7 @@ def qkv_rope_store(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
               weight.shape[1], nheads, kvheads, head_dim, 1 if writes_cache else 0, error_flag(x.device),
               batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _stream())
         return q
-    return rope_store(linear(x, weight, bias), inv_freq, batch, view, nheads, kvheads, head_dim, writes_cache)
+    return rope_store(linear(x, weight, bias, *((None, batch) if weight.dtype == torch.float32 and f32_split_tokens(weight) else ())), inv_freq, batch, view, nheads, kvheads, head_dim, writes_cache)
 
 
 def _attention_library(head_dim: int) -> str:

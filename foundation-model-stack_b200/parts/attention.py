@@ -62,7 +62,7 @@ class MultiHeadAttention(Part):
         # the position part applies the projection, encodes q and k and writes k and v into the cache
         q = self.position.project(x, self.qkv, batch, cache_view, self.nheads, self.kvheads, self.head_dim, writes_cache)
         o = ops.attention(q, batch, cache_view, self.nheads, self.kvheads, self.head_dim, self.scale, self.window)
-        return self.dense.forward(o)
+        return self.dense.forward(o, sequences=batch)
 
     def kernel_libraries(self, dtype):
         return (super().kernel_libraries(dtype) + self.position.kernel_libraries(dtype)
@@ -230,7 +230,7 @@ class SinkAttention(Part):
 
     def heads_out(self, x, batch, cache_view, writes_cache: bool = True):
         """The gated heads' results [tokens, nheads * vdim], before the output projection."""
-        proj = self.in_proj.forward(x)
+        proj = self.in_proj.forward(x, sequences=batch)
         o = self.attend(proj, batch, cache_view, writes_cache)
         if not self.has_gate and self.pad == self.vdim and self.out_factor == 1.0:
             return o  # no gate, no padding to drop, no factor: the heads' results as attention left them
@@ -238,7 +238,7 @@ class SinkAttention(Part):
                                 self.out_factor, self.gate_per_head)
 
     def forward(self, x, batch, cache_view, writes_cache: bool = True):
-        return self.dense.forward(self.heads_out(x, batch, cache_view, writes_cache))
+        return self.dense.forward(self.heads_out(x, batch, cache_view, writes_cache), sequences=batch)
 
     def kernel_libraries(self, dtype):
         return super().kernel_libraries(dtype) + ["elementwise", f"attention_hd{self.pad}"]

@@ -39,6 +39,7 @@ from __future__ import annotations
 
 from ..config.specs import BlockSpec
 from .base import Part
+from .feedforward import feed_forward_of
 from ..kernels import ops
 from .linear import Linear
 from .norm import NormedDelta, StreamCopy
@@ -63,7 +64,7 @@ class PreNormBlock(Part):
         h = self.mixer_norm.apply(residual, pending, dtype)
         a = self.mixer.forward(h, batch, cache_view, writes_cache)
         h = self.feed_forward_norm.apply(residual, a, dtype)
-        return self.feed_forward.forward(h)
+        return feed_forward_of(self.feed_forward, h, batch)
 
 
 class SandwichBlock(Part):
@@ -92,7 +93,7 @@ class SandwichBlock(Part):
         if self.feed_forward is None:
             return pending
         h = self.feed_forward_norm.apply(residual, pending, dtype)
-        return NormedDelta(self.feed_forward.forward(h), self.feed_forward_post_norm)
+        return NormedDelta(feed_forward_of(self.feed_forward, h, batch), self.feed_forward_post_norm)
 
 
 class ScaledParts:
@@ -139,7 +140,7 @@ class PostNormBlock(Part):
         parts = a.parts if isinstance(a, ScaledParts) else [(a, 1.0)]
         h = self.mixer_norm.apply_after_sum(residual, self.alpha, parts, dtype)
         if self.feed_forward is not None:
-            h = self.feed_forward_norm.apply_after_sum(residual, self.alpha, [(self.feed_forward.forward(h), 1.0)], dtype)
+            h = self.feed_forward_norm.apply_after_sum(residual, self.alpha, [(feed_forward_of(self.feed_forward, h, batch), 1.0)], dtype)
         return StreamCopy(h)
 
     def kernel_libraries(self, dtype):
@@ -181,7 +182,7 @@ class OutputNormBlock(Part):
         if self.feed_forward is None:
             return NormedDelta(a, self.mixer_norm)
         h = self.mixer_norm.add(residual, a, dtype)
-        return NormedDelta(self.feed_forward.forward(h), self.feed_forward_norm)
+        return NormedDelta(feed_forward_of(self.feed_forward, h, batch), self.feed_forward_norm)
 
     def kernel_libraries(self, dtype):
         return super().kernel_libraries(dtype) + ["elementwise"]
@@ -219,7 +220,7 @@ class ParallelResidualBlock(Part):
         h1, h2 = self.mixer_norm.apply_pair(residual, pending, self.feed_forward_norm, dtype)
         a = self.mixer.forward(h1, batch, cache_view, writes_cache)
         parts = list(a.parts) if isinstance(a, ScaledParts) else [(a, 1.0)]
-        return ScaledParts(parts + [(self.feed_forward.forward(h2), 1.0)])
+        return ScaledParts(parts + [(feed_forward_of(self.feed_forward, h2, batch), 1.0)])
 
     def kernel_libraries(self, dtype):
         return super().kernel_libraries(dtype) + ["elementwise"]
@@ -309,7 +310,7 @@ class HyperConnectedBlock(Part):
         if self.feed_forward is None:
             return pending
         h = self.feed_forward_norm.apply_mixed(residual, pending, self.feed_forward_connection.w_in, dtype)
-        return StreamMix(self.feed_forward.forward(h), self.feed_forward_connection)
+        return StreamMix(feed_forward_of(self.feed_forward, h, batch), self.feed_forward_connection)
 
     def kernel_libraries(self, dtype):
         return super().kernel_libraries(dtype) + ["elementwise"]

@@ -6,6 +6,8 @@ one matrix, gate first (fms/modules/feedforward.py:227-240 for the sizes, :288-2
 Interface of a feed-forward (what a block calls):
 
     forward(x) -> y          x, y: [tokens, dim] in the compute dtype
+    forward(x, sequences)    where ``takes_sequences`` is set: with the step's ``Batch``, or how many rows each sequence has (None:
+                             every row stands alone; left out: all rows are one sequence's): large float32 products choose by it
 
 A feed-forward with routing implements the same call and keeps router and experts inside.
 
@@ -29,6 +31,14 @@ ACTIVATIONS = {"silu": 0, "swish": 0, "gelu": 1, "gelu-tanh": 2, "gelu_pytorch_t
 UNGATED_ACTIVATIONS = dict(ACTIVATIONS, relu_squared=4)
 
 
+ONE_SEQUENCE = object()
+
+
+def feed_forward_of(part, x, batch):
+    """A feed-forward's call in a step: the rows ``x`` are those of ``batch``."""
+    return part.forward(x, batch) if getattr(part, "takes_sequences", False) else part.forward(x)
+
+
 class GatedLinearUnit(Part):
     def __init__(self, spec: FeedForwardSpec) -> None:
         super().__init__()
@@ -40,9 +50,13 @@ class GatedLinearUnit(Part):
         self.gate_up = self.add("wg1_fused", Linear(spec.dim, 2 * spec.hidden, spec.bias))
         self.down = self.add("w2", Linear(spec.hidden, spec.dim, spec.bias))
 
-    def forward(self, x):
-        h = ops.gated_linear(x, self.gate_up.tensor("weight"), self.gate_up.tensor("bias"), self.activation)
-        return self.down.forward(h)
+    takes_sequences = True
+
+    def forward(self, x, sequences=ONE_SEQUENCE):
+        sequences = [x.shape[0]] if sequences is ONE_SEQUENCE else sequences
+        further = (sequences,) if self.gate_up.by_sequence() else ()
+        h = ops.gated_linear(x, self.gate_up.tensor("weight"), self.gate_up.tensor("bias"), self.activation, *further)
+        return self.down.forward(h, sequences=sequences)
 
     def kernel_libraries(self, dtype):
         return super().kernel_libraries(dtype) + ["elementwise"]
@@ -58,8 +72,13 @@ class PlainUnit(Part):
         self.up = self.add("w1", Linear(spec.dim, spec.hidden, spec.bias))
         self.down = self.add("w2", Linear(spec.hidden, spec.dim, spec.bias))
 
-    def forward(self, x):
-        return self.down.forward(ops.activated_linear(x, self.up.tensor("weight"), self.up.tensor("bias"), self.activation))
+    takes_sequences = True
+
+    def forward(self, x, sequences=ONE_SEQUENCE):
+        sequences = [x.shape[0]] if sequences is ONE_SEQUENCE else sequences
+        further = (sequences,) if self.up.by_sequence() else ()
+        h = ops.activated_linear(x, self.up.tensor("weight"), self.up.tensor("bias"), self.activation, *further)
+        return self.down.forward(h, sequences=sequences)
 
     def kernel_libraries(self, dtype):
         return super().kernel_libraries(dtype) + ["elementwise"]
