@@ -579,7 +579,10 @@ __global__ void __launch_bounds__(128, WIDE<KIND> ? 2 : 3) chunk_outputs_kernel(
   }
   copies_commit();
   sums.scale(G[my_head] + tm);  // G_t times what the state gives
-  if (KIND == 1 && tid < C) nq[tid] = (float)fma((double)G[0][tid], own_nq, p_sum);  // n_t . q_t
+  if (KIND == 1 && tid < C) {  // of n_t . q_t, what divides the row; here, since a load between the row's stores would wait for each
+    const float least = tid < rows ? g.gates[((size_t)(row0 + tid) * g.heads + head0) * 3 + 2] : 1.f;
+    nq[tid] = 1.f / (fmaxf(fabsf((float)fma((double)G[0][tid], own_nq, p_sum)), least) + 1e-6f);
+  }
   const bool bad = g.flags[(size_t)local * g.heads + head0 + my_head] != 0;
   copies_wait<0>();
   __syncthreads();
@@ -604,13 +607,13 @@ __global__ void __launch_bounds__(128, WIDE<KIND> ? 2 : 3) chunk_outputs_kernel(
           for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(p[s * TROW + (i & 3) + (i >> 2) * 16], sm[s * CROW + tn + (j & 3) + (j >> 2) * 32], acc[i][j]);
         }
   }
+  const float skip = KIND == 2 ? g.d_skip[head0 + my_head] : 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int t = tm + (i & 3) + (i >> 2) * 16;
     if (t >= rows) continue;
-    float scale = 1.f, skip = 0.f;
-    if (KIND == 1) scale = 1.f / (fmaxf(fabsf(nq[t]), g.gates[((size_t)(row0 + t) * g.heads + head0) * 3 + 2]) + 1e-6f);
-    if (KIND == 2) skip = g.d_skip[head0 + my_head];
+    float scale = 1.f;
+    if (KIND == 1) scale = nq[t];
     float* out = g.o + (size_t)(row0 + t) * g.heads * VDIM + (size_t)head0 * VDIM + tn;
 #pragma unroll
     for (int j = 0; j < 8; j += 4) {
@@ -913,8 +916,10 @@ int launch_states(const ChunkArgs& g, cudaStream_t stream) {
   return 0;
 }
 
-// a block walks a sequence's runs one by one: 32 columns a block where 64 would leave multiprocessors without one
-bool columns_32(const ChunkArgs& g, int vdim) { return (long)g.n_seqs * g.heads * vdim / 64 < 128; }
+// A block walks a sequence's runs one by one: 32 columns a block where 64 would give most multiprocessors no second block, whose
+// instructions fill the gaps of the first's (two prompts of 32 heads, 128 blocks of 64 or 256 of 32: 94 -> 78 us of 1,700 tokens;
+// one of 128 heads of 64 values: 167 -> 161 of 2,048).
+bool columns_32(const ChunkArgs& g, int vdim) { return (long)g.n_seqs * g.heads * vdim / 64 <= 148; }
 
 template <int VDIM, int KIND>
 int launch_passes(ChunkArgs g, int n_runs, int pass_runs, cudaStream_t stream) {
