@@ -561,6 +561,8 @@ __global__ void attn_combine_kernel(AttnArgs a, const float* __restrict__ part_o
 #if HEAD_DIM == 64 || HEAD_DIM == 128
 #define FMS_ATTENTION_TC 1
 #include "attention_tc.cuh"
+#include "split_f32.cuh"
+#include "attention_f32_tc.cuh"
 #include "attention_stream.cuh"
 #else
 #define FMS_ATTENTION_TC 0
@@ -815,6 +817,44 @@ FMS_API int fms_attention_prefill(const void* q, void* out, int dtype, const voi
   return attention_prefill(q, out, dtype, keys, values, table, table_stride, block_tokens, slots, first_row, len_after,
                            tiles, n_tiles, nheads, kvheads, head_dim, scale, window, pool_blocks, table_rows, error_flag,
                            nullptr, stream);
+}
+
+// Whether fms_attention_prefill_f32_split takes this many heads (of the library's size).
+FMS_API int fms_attn_f32_split_takes(int nheads, int kvheads) {
+#if FMS_ATTENTION_TC
+  if (prefill_on_tcgen05()) return kvheads > 0 && nheads % kvheads == 0 && nheads / kvheads % 2 == 0 ? 1 : 0;
+#endif
+  return 0;
+}
+
+// float32 prefill attention on the tensor cores, without a cap and without a distance term; the rest as fms_attention_prefill_masked.
+FMS_API int fms_attention_prefill_f32_split(const void* q, void* out, const void* keys, const void* values, const int* table, int table_stride,
+                                            int block_tokens, const int* slots, const int* first_row, const int* len_after, const int* tiles,
+                                            int n_tiles, int nheads, int kvheads, int head_dim, float scale, int window, int pool_blocks,
+                                            int table_rows, int* error_flag, const float* sink, int chunk, long q_stride, cudaStream_t stream) {
+  if (n_tiles <= 0) return 0;
+#if FMS_ATTENTION_TC
+  if (check_args("attention_prefill_f32_split", nheads, kvheads, head_dim, block_tokens)) return 1;
+  if (check_mask("attention_prefill_f32_split", window, chunk, 0.f)) return 1;
+  if (!fms_attn_f32_split_takes(nheads, kvheads)) return fms_fail("attention_prefill_f32_split: %d heads over %d", nheads, kvheads);
+  AttnArgs a{q, out, keys, values, table, table_stride, slots, first_row, len_after, nheads, kvheads, scale, window,
+             table_rows, pool_blocks, sink, chunk, 0.f, nullptr, q_stride > 0 ? q_stride : (long)nheads * HD};
+  if (check_queries(q, FMS_F32, a.q_stride, nheads)) return 1;
+  if (((uintptr_t)out | (uintptr_t)keys | (uintptr_t)values) & 15) return fms_fail("attention_prefill_f32_split: operands must be 16-byte aligned");
+  if (!(scale > 0.f)) return fms_fail("attention_prefill_f32_split: the scale of the scores is %g; it must be positive", (double)scale);
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FT_SMEM);
+    if (e != cudaSuccess) return fms_fail("attention_prefill_f32_split: shared memory of %zu bytes refused: %s", FT_SMEM, cudaGetErrorString(e));
+    configured = true;
+  }
+  const long blocks = (long)n_tiles * (nheads / 2);
+  if (blocks > 0x7fffffffL) return fms_fail("attention_prefill_f32_split: %ld thread blocks", blocks);
+  fms_launch(attn_prefill_f32_tc_kernel, dim3((unsigned)blocks), dim3(FT_THREADS), FT_SMEM, stream, a, tiles, n_tiles, error_flag);
+  return fms_launch_status("attention_prefill_f32_split");
+#else
+  return fms_fail("attention_prefill_f32_split: head size %d has no tcgen05 kernel", HD);
+#endif
 }
 
 // Prefill attention with a key and a value head for every query head, over keys and values that lie in the rows of a matrix

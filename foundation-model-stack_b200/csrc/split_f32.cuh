@@ -1,0 +1,49 @@
+// float32 values as sums of three bfloat16 values, for products on the tensor cores that lose nothing of the operands (nearest, nearest
+// of the rest, the rest: 8 bits of mantissa each).  Included inside the anonymous namespace of the kernels that use it.
+#pragma once
+
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {  // nearest bfloat16 of a in the low half, of b in the high half
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+// the larger magnitude of either half (its sign means nothing), or not a number
+__device__ __forceinline__ uint32_t most2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// v - the two bfloat16 of h, side by side
+__device__ __forceinline__ float2 rest2(float2 v, uint32_t h) {
+  unsigned long long r, a, b, c;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(a) : "f"(v.x), "f"(v.y));
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(b) : "r"(h << 16), "r"(h & 0xffff0000u));
+  asm("mov.b64 %0, {%1, %1};\n" : "=l"(c) : "f"(-1.f));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(b), "l"(c), "l"(a));
+  float2 o;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(o.x), "=f"(o.y) : "l"(r));
+  return o;
+}
+// eight values of consecutive k as three times 16 bytes; most: the largest magnitudes so far
+__device__ __forceinline__ void split8(const float* v, uint4* hi, uint4* mid, uint4* lo, uint32_t& most) {
+  uint32_t h[4], m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    h[i] = bf16_pair(v[2 * i], v[2 * i + 1]);
+    const float2 r = rest2(make_float2(v[2 * i], v[2 * i + 1]), h[i]);
+    m[i] = bf16_pair(r.x, r.y);
+    const float2 t = rest2(r, m[i]);
+    l[i] = bf16_pair(t.x, t.y);
+  }
+  most = most2(most2(most, h[0]), most2(most2(h[1], h[2]), h[3]));
+  *hi = make_uint4(h[0], h[1], h[2], h[3]);
+  *mid = make_uint4(m[0], m[1], m[2], m[3]);
+  *lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+// What a row holds, from its largest magnitudes: bit 0 something beyond 2^100 or no number, bit 1 something but zeros, bit 2 something
+// from 2^-64 on.  Kinds of the parts of a row are or-ed; a row is split unless bit 0 is set, or bit 1 without bit 2.
+__device__ __forceinline__ unsigned kind_of(uint32_t most) {
+  const uint32_t a = most & 0x7fffu, b = (most >> 16) & 0x7fffu, m = a > b ? a : b;  // order of magnitudes is order of bits; NaN above all
+  return (m > (227u << 7) ? 1u : 0u) | (m ? 2u : 0u) | (m >= (63u << 7) ? 4u : 0u);
+}
+__device__ __forceinline__ bool stays_whole(unsigned kind) { return (kind & 1u) || (kind & 6u) == 2u; }

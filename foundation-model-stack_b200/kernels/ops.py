@@ -115,6 +115,7 @@ _SIGNATURES = {
     "fms_gated_group_rmsnorm": [_P, _P, _I, _I, _I, _P, _I, _F, _F, _P, _I, _I, _I, _P],
     "fms_argmax": [_P, _P, _I, _I, _P],
     "fms_sample": [_P, _P, _I, _I, _F, _I, _U64, _P, _I, _P],
+    "fms_attention_prefill_f32_split": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _L, _P],
     "fms_attention_prefill": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P],
     "fms_attention_decode": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I, _I, _I, _L, _P, _P,
                              _P],
@@ -852,6 +853,20 @@ def sigmoid_gate(o: torch.Tensor, gate: Optional[torch.Tensor], gate_offset: int
     return out
 
 
+# Tokens of a sequence from which its float32 prefill attention goes to the tensor cores (attention_f32_tc.cuh); its own tokens decide.
+# CUDA cores / tensor cores in us, 32 heads of 128 over 8: 16 tokens onto 1,000 cached ones 97 / 119 (tiles of up to 16 rows take a
+# shorter walk there), 17 onto 1,000 236 / 119, 17 alone 29 / 27, 128 alone 39 / 29, three prompts of 1,100 tokens together 207 / 95.
+F32_SPLIT_ATTENTION_TOKENS = 17
+_f32_split_takes = {}
+
+
+def _f32_split_attention(head_dim: int, nheads: int, kvheads: int) -> bool:
+    key = (head_dim, nheads, kvheads)
+    if key not in _f32_split_takes:
+        _f32_split_takes[key] = bool(load_library(_attention_library(head_dim)).fms_attn_f32_split_takes(nheads, kvheads))
+    return _f32_split_takes[key]
+
+
 def attention(q: torch.Tensor, batch, view, nheads: int, kvheads: int, head_dim: int, scale: float,
               window: int, sink: Optional[torch.Tensor] = None, chunk: int = 0, softcap: float = 0.0,
               distance: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -895,7 +910,18 @@ def attention(q: torch.Tensor, batch, view, nheads: int, kvheads: int, head_dim:
             global launches
             launches += 1  # the kernel that merges the splits
     else:
-        tiles = batch.query_tiles(tile_rows)
+        members = None
+        if q.dtype == torch.float32 and not softcap and distance is None and _f32_split_attention(head_dim, nheads, kvheads):
+            long = [i for i, n in enumerate(batch.num_new) if n >= F32_SPLIT_ATTENTION_TOKENS]
+            if long:
+                tiles = batch.query_tiles(tile_rows, long)
+                _call(lib, "fms_attention_prefill_f32_split", q, out, view.keys, view.values, view.table, view.table.shape[1], view.block_tokens,
+                      batch.slots, batch.first_row, batch.len_after, tiles, tiles.shape[0], nheads, kvheads, head_dim, float(scale), int(window),
+                      view.keys.shape[0], view.table.shape[0], error_flag(q.device), sink, int(chunk), q.shape[1], _stream())
+                if len(long) == batch.n_seqs:
+                    return out
+                members = [i for i, n in enumerate(batch.num_new) if 0 < n < F32_SPLIT_ATTENTION_TOKENS]
+        tiles = batch.query_tiles(tile_rows, members)
         tail = (sink, int(chunk), float(softcap), distance, q.shape[1]) if masked else \
             (() if sink is None else (sink,))
         _call(lib, "fms_attention_prefill_masked" if masked else

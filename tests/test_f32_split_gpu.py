@@ -74,3 +74,94 @@ def test_shifted_operands_and_scratch_at_a_time(ops, monkeypatch):
     assert torch.equal(ops.linear(shifted(x), shifted(w), shifted(b), None, [600]), want)
     monkeypatch.setattr(ops, "F32_SPLIT_BYTES", 1)
     assert torch.equal(ops.linear(x, w, b, None, [600]), want)
+
+
+def attended(ops, num_new, lens_before, nheads, kvheads, hd, window=0, chunk=0, sink=None, seed=0, scale=None):
+    """A step's attention, its queries and the keys and values of every sequence in order."""
+    from test_kernels_gpu import make_cache_case
+
+    _, view, batch = make_cache_case(torch.float32, nheads, kvheads, hd, lens_before, num_new, seed, window)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    n = sum(num_new)
+    qkv = torch.randn(n, (nheads + 2 * kvheads) * hd, generator=g, device="cuda")
+    q = ops.rope_store(qkv, None, batch, view, nheads, kvheads, hd)
+    return ops.attention(q, batch, view, nheads, kvheads, hd, hd ** -0.5, window, sink, chunk), q, view, batch
+
+
+@pytest.mark.parametrize("nheads,kvheads,hd", [(4, 2, 64), (8, 2, 128)])
+@pytest.mark.parametrize("num_new,lens_before", [([17, 64, 65], [0, 0, 63]), ([128, 1, 16, 200], [5, 300, 64, 129])])
+@pytest.mark.parametrize("window,chunk,sinks", [(0, 0, False), (70, 0, True), (0, 96, False)])
+def test_attention_at_the_edges_of_its_tiles(ops, monkeypatch, nheads, kvheads, hd, num_new, lens_before, window, chunk, sinks):
+    """Remainders of 64 queries and of 64 keys, windows that skip blocks, sequences that stay on the CUDA cores beside others; everything
+    that no query sees is NaN.  Beside the CUDA cores' kernel: an output is an average of values, both sides' errors some 2^-24 of the
+    largest score's size and of the values' each."""
+    sink = torch.randn(nheads, device="cuda") if sinks else None
+    calls, entry = [], ops._call
+    monkeypatch.setattr(ops, "_call", lambda library, name, *a: (calls.append(name), entry(library, name, *a))[1])
+    got, q, view, batch = attended(ops, num_new, lens_before, nheads, kvheads, hd, window, chunk, sink)
+    assert "fms_attention_prefill_f32_split" in calls
+    monkeypatch.setattr(ops, "F32_SPLIT_ATTENTION_TOKENS", 1 << 30)
+    calls.clear()
+    want = ops.attention(q, batch, view, nheads, kvheads, hd, hd ** -0.5, window, sink, chunk)
+    assert "fms_attention_prefill_f32_split" not in calls
+    assert float((got - want).abs().max()) <= 2.0 ** -24 * 64 * float(want.abs().max())
+    assert float((got - want).norm()) <= 2.0 ** -24 * 16 * float(want.norm())
+    at = 0
+    for n in num_new:  # few rows: the same kernel, the same bits
+        if n < 17:
+            assert torch.equal(got[at:at + n], want[at:at + n])
+        at += n
+
+
+def test_attention_of_a_sequence_alone_and_among_others(ops):
+    """The same bits, also where a tile's other rows are other ones; and no further from 64 bits than the CUDA cores' kernel."""
+    nheads, kvheads, hd = 8, 2, 128
+    got, q, view, batch = attended(ops, [150, 40, 300], [10, 0, 100], nheads, kvheads, hd, seed=3)
+    from fms_b200.engine.batch import Batch
+
+    slots = batch.slots.tolist()
+    for i, (first, n, before) in enumerate(((0, 150, 10), (150, 40, 0), (190, 300, 100))):
+        alone = Batch.from_lists([slots[i]], [before], [[0] * n], [[]], "cuda")
+        assert torch.equal(ops.attention(q[first:first + n].contiguous(), alone, view, nheads, kvheads, hd, hd ** -0.5, 0), got[first:first + n])
+        rest = Batch.from_lists([slots[i]], [before + 13], [[0] * (n - 13)], [[]], "cuda")
+        assert torch.equal(ops.attention(q[first + 13:first + n].contiguous(), rest, view, nheads, kvheads, hd, hd ** -0.5, 0), got[first + 13:first + n])
+    table, errors = view.table.tolist(), []
+    keys, values = (torch.cat([t[b] for b in table[slots[2]][:7]], 1)[:, :400].double() for t in (view.keys, view.values))
+    scores = torch.einsum("thd,hkd->htk", q[190:].double().view(300, nheads, hd), keys.repeat_interleave(4, 0)) * hd ** -0.5
+    scores = scores.masked_fill(torch.arange(400, device="cuda")[None] > 100 + torch.arange(300, device="cuda")[:, None], -float("inf"))
+    want = torch.einsum("htk,hkd->thd", torch.softmax(scores, -1), values.repeat_interleave(4, 0)).flatten(1)
+    for least in (17, 1 << 30):
+        ops.F32_SPLIT_ATTENTION_TOKENS, kept = least, ops.F32_SPLIT_ATTENTION_TOKENS
+        try:
+            out = ops.attention(q, batch, view, nheads, kvheads, hd, hd ** -0.5, 0)[190:]
+        finally:
+            ops.F32_SPLIT_ATTENTION_TOKENS = kept
+        errors.append(float((out.double() - want).norm() / want.norm()))
+    assert errors[0] <= errors[1], errors
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 3e38])
+@pytest.mark.parametrize("what", ["query", "key", "value"])
+@pytest.mark.parametrize("window", [0, 70])
+def test_attention_keeps_what_does_not_split_to_the_rows_that_see_it(ops, what, value, window):
+    """The rows that do not see it come out as they do without it, bit for bit; the others as on the CUDA cores."""
+    nheads, kvheads, hd, n, before, at = 4, 2, 128, 200, 37, 120
+    clean, q, view, batch = attended(ops, [n], [before], nheads, kvheads, hd, window, seed=5)
+    q = q.clone()
+    if what == "query":
+        q[at, 2 * hd + 3] = value
+    else:
+        table = view.table[batch.slots[0]]
+        (view.keys if what == "key" else view.values)[table[(before + at) // 64], 1, (before + at) % 64, 3] = value
+    got, limit = ops.attention(q, batch, view, nheads, kvheads, hd, hd ** -0.5, window), ops.F32_SPLIT_ATTENTION_TOKENS
+    try:
+        ops.F32_SPLIT_ATTENTION_TOKENS = 1 << 30
+        want = ops.attention(q, batch, view, nheads, kvheads, hd, hd ** -0.5, window)
+    finally:
+        ops.F32_SPLIT_ATTENTION_TOKENS = limit
+    sees = torch.zeros(n, dtype=torch.bool, device="cuda")
+    sees[at: at + 1 if what == "query" else (at + window if window else n)] = True
+    assert torch.equal(got[~sees], clean[~sees])
+    assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+    fine = torch.isfinite(want)
+    assert float((got - want)[fine].abs().max()) <= 2.0 ** -24 * 64 * float(want[fine].abs().max())
