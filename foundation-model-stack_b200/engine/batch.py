@@ -14,6 +14,14 @@ from typing import List, Optional, Sequence
 import torch
 
 
+def int32_on(device, values) -> torch.Tensor:
+    """Whole numbers on the device, copied out of pinned memory (kept by torch until the copy is over) so that the host does not
+    wait for the stream: from pageable memory every such copy let the GPU run dry behind it.  A capture, which would read the
+    memory again at every replay, refuses the pageable copy that it gets."""
+    pinned = torch.device(device).type == "cuda" and not torch.cuda.is_current_stream_capturing()
+    return torch.tensor(values, dtype=torch.int32, pin_memory=pinned).to(device, non_blocking=pinned)
+
+
 class Batch:
     """Device arrays of one step.  Built by ``Batch.from_lists`` for a general step, or filled in place
     by the decode loop (``engine.step.DecodeState``) when every sequence brings one token."""
@@ -67,8 +75,7 @@ class Batch:
                 rows.append(base + j)
         len_after = [lb + n for lb, n in zip(len_before, b.num_new)]
         ids = [p + offsets[i] for p, i in zip(pos, seq)] if offsets is not None and any(offsets) else []
-        packed = torch.tensor(flat + pos + seq + first + list(slots) + len_after + ids + rows, dtype=torch.int32)
-        packed = packed.to(device)
+        packed = int32_on(device, flat + pos + seq + first + list(slots) + len_after + ids + rows)
         n, s = b.n_tokens, b.n_seqs
         o = 0
         b.tokens = packed[o:o + n]; o += n
@@ -97,7 +104,7 @@ class Batch:
                         rows.append((base + r, base + min(n, r + chunk)))
                 first.append(len(rows))
                 base += n
-            packed = torch.tensor([v for p in rows for v in p] + first, dtype=torch.int32).to(self.tokens.device)
+            packed = int32_on(self.tokens.device, [v for p in rows for v in p] + first)
             self._tiles[key] = (packed[: 2 * len(rows)].view(-1, 2), packed[2 * len(rows):])
         return self._tiles[key]
 
@@ -136,7 +143,7 @@ class Batch:
                 first.append(before + n - seen)
                 start.append(start[-1] + (seen if members is None or i in members else 0))
             base = [a - b for a, b in zip(start, first)]
-            packed = torch.tensor(start + first + base, dtype=torch.int32).to(self.tokens.device)
+            packed = int32_on(self.tokens.device, start + first + base)
             s = len(first)
             self._tiles[key] = (packed[: s + 1], packed[s + 1: 2 * s + 1], packed[2 * s + 1:], start[-1])
         return self._tiles[key]
@@ -151,7 +158,7 @@ class Batch:
             for i, n in enumerate(self.num_new):
                 if members is None or i in members:
                     t.extend((i, r) for r in range(0, n, tile_rows))
-            self._tiles[key] = torch.tensor(t, dtype=torch.int32).to(self.tokens.device)
+            self._tiles[key] = int32_on(self.tokens.device, t)
         return self._tiles[key]
 
     def _of(self, members: Optional[Sequence[int]]):

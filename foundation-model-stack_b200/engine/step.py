@@ -22,7 +22,7 @@ import torch
 
 from ..cache.cache import Cache
 from ..kernels import ops
-from .batch import Batch
+from .batch import Batch, int32_on
 
 # Tests that replace the kernels by plain restatements clear this to drive the host logic on the CPU.
 _REQUIRE_CUDA = True
@@ -181,8 +181,7 @@ class Engine:
         if buf.loaded != key or buf.lengths != lengths:
             offsets = [self.cache.offset(s) for s in slots]
             fill = rows - n
-            state = torch.tensor([list(slots) + [self.cache.spare_slot] * fill, lengths + [0] * fill, offsets + [0] * fill],
-                                 dtype=torch.int32)
+            state = int32_on(self.device, [list(slots) + [self.cache.spare_slot] * fill, lengths + [0] * fill, offsets + [0] * fill])
             buf.batch.slots.copy_(state[0])
             buf.batch.len_after.copy_(state[1])
             buf.offsets.copy_(state[2])
