@@ -356,29 +356,6 @@ template <int PARTS> __device__ __forceinline__ float group_sum(float v) {  // o
   for (int o = 1; o < PARTS; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// The same sums of N values (of several columns and tokens), value i's left on the lane `part` = i % PARTS in v[i / PARTS]: a lane
-// gives away the values that it does not keep, so that 16 values over 16 lanes take 15 shuffles instead of 64.  The same pairs are
-// added: the same bits.
-template <int N, int PARTS, int O = 1, int KEPT = N> __device__ __forceinline__ void scattered_sums(float (&v)[N], int part) {
-  static_assert((N & (N - 1)) == 0, "values");
-  if constexpr (O < PARTS) {
-    if constexpr (KEPT > 1) {
-#pragma unroll
-      for (int i = 0; i < KEPT / 2; ++i) {
-        const bool upper = part & O;
-        const float keep = upper ? v[2 * i + 1] : v[2 * i], give = upper ? v[2 * i] : v[2 * i + 1];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
-      }
-    } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
-    }
-    scattered_sums<N, PARTS, 2 * O, (KEPT > 1 ? KEPT / 2 : 1)>(v, part);
-  }
-}
-// Tokens whose outputs' sums are taken together.  Nothing waits for an output, but a warp's instructions go in order, and a
-// token's four shuffles in a row held the next token's up (120 tokens of one sequence and of four, 16 heads of 128 under the delta
-// rule 50 -> 39 and 68 -> 59 us, 32 heads under exponential gates 50 -> 38 and 74 -> 63, 128 heads of 64 state space 58 -> 42).
-constexpr int TOGETHER = 4;
 
 // ---- selective state-space scan ----------------------------------------------------------------------
 // xbc [tokens, inner + 2 groups * N] float32 (after the convolution): x | B | C;  dt_raw: column `head` of rows of
@@ -446,12 +423,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const floa
     const float* sB = smem + stage * STAGE;
     const float* sC = sB + CH * NPAD;
     const float* sx = sC + CH * NPAD;
-    auto token = [&](int t, float* acc) {
+    for (int t = 0; t < cn; ++t) {
       const float dec = sdec[t], dt = sdt[t];
-      float dtx[VP];
+      float xv[VP], dtx[VP], acc[VP];
 #pragma unroll
       for (int i = 0; i < VP; ++i) {
-        dtx[i] = dt * sx[t * VB + grp * VP + i];
+        xv[i] = sx[t * VB + grp * VP + i];
+        dtx[i] = dt * xv[i];
         acc[i] = 0.f;
       }
       float b[NP], c[NP];
@@ -466,30 +444,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) selective_scan_kernel(const floa
           acc[i] = fmaf(s[i][j], cj, acc[i]);
         }
       }
-    };
-    auto give = [&](int t, int column, float sum) {
-      const int v = v0 + grp * VP + column;
-      if (v < vdim) y[(size_t)(c0 + t) * inner + (size_t)head * vdim + v] = fmaf(D, sx[t * VB + grp * VP + column], sum);
-    };
-    // with four columns a thread the tokens' multiply-adds fill the wait (eight sequences of 120 tokens, 128 heads of 64: 195 us by fours)
-    constexpr int AT_ONCE = VP >= 4 ? 1 : TOGETHER;
-    int t = 0;
-    for (; t + AT_ONCE <= cn; t += AT_ONCE) {
-      float acc[AT_ONCE * VP];
 #pragma unroll
-      for (int u = 0; u < AT_ONCE; ++u) token(t + u, acc + u * VP);
-      scattered_sums<AT_ONCE * VP, PARTS>(acc, part);
-#pragma unroll
-      for (int i = 0; i < (AT_ONCE * VP + PARTS - 1) / PARTS; ++i) {
-        const int value = i * PARTS + part;
-        if (value < AT_ONCE * VP) give(t + value / VP, value % VP, acc[i]);
+      for (int i = 0; i < VP; ++i) {
+        acc[i] = group_sum<PARTS>(acc[i]);
+        const int v = v0 + grp * VP + i;
+        if (part == i && v < vdim) y[(size_t)(c0 + t) * inner + (size_t)head * vdim + v] = fmaf(D, xv[i], acc[i]);
       }
-    }
-    for (; t < cn; ++t) {
-      float acc[VP];
-      token(t, acc);
-      scattered_sums<VP, PARTS>(acc, part);
-      if (part < VP) give(t, part, acc[0]);
     }
     __syncthreads();  // this stage and sdt are free again
   }
@@ -601,26 +561,27 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_rule_scan_kernel(const flo
     const float* sg = sk + CH * NPAD;
     const float* sv = sg + CH * NPAD;
     const float* sbeta = sv + CH * VB;
-    auto token = [&](int t, float* acc) {
-      float q[NP], k[NP], g[NP], u[VP];
+    for (int t = 0; t < cn; ++t) {
+      float q[NP], k[NP], g[NP];
       load_run<NP>(sk + t * NPAD + part * RUN, k);
       load_run<NP>(sg + t * NPAD + part * RUN, g);
       load_run<NP>(sq + t * NPAD + part * RUN, q);
+      float acc[VP], u[VP];
 #pragma unroll
-      for (int i = 0; i < VP; ++i) u[i] = 0.f;
+      for (int i = 0; i < VP; ++i) acc[i] = 0.f;
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
         const float gj = g[j], kj = k[j];
 #pragma unroll
         for (int i = 0; i < VP; ++i) {
           s[i][j] *= gj;
-          u[i] = fmaf(s[i][j], kj, u[i]);
+          acc[i] = fmaf(s[i][j], kj, acc[i]);
         }
       }
       const float bt = sbeta[t];
 #pragma unroll
       for (int i = 0; i < VP; ++i) {
-        u[i] = bt * (sv[t * VB + grp * VP + i] - group_sum<PARTS>(u[i]));
+        u[i] = bt * (sv[t * VB + grp * VP + i] - group_sum<PARTS>(acc[i]));
         acc[i] = 0.f;
       }
 #pragma unroll
@@ -632,28 +593,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_rule_scan_kernel(const flo
           acc[i] = fmaf(s[i][j], qj, acc[i]);
         }
       }
-    };
-    auto give = [&](int t, int column, float sum) {
-      const int v = v0 + grp * VP + column;
-      if (v < vdim) o[(size_t)(c0 + t) * heads * vdim + (size_t)head * vdim + v] = sum;
-    };
-    int t = 0;
-    for (; t + TOGETHER <= cn; t += TOGETHER) {
-      float acc[TOGETHER * VP];
 #pragma unroll
-      for (int u = 0; u < TOGETHER; ++u) token(t + u, acc + u * VP);
-      scattered_sums<TOGETHER * VP, PARTS>(acc, part);
-#pragma unroll
-      for (int i = 0; i < (TOGETHER * VP + PARTS - 1) / PARTS; ++i) {
-        const int value = i * PARTS + part;
-        if (value < TOGETHER * VP) give(t + value / VP, value % VP, acc[i]);
+      for (int i = 0; i < VP; ++i) {
+        acc[i] = group_sum<PARTS>(acc[i]);
+        const int v = v0 + grp * VP + i;
+        if (part == i && v < vdim) o[(size_t)(c0 + t) * heads * vdim + (size_t)head * vdim + v] = acc[i];
       }
-    }
-    for (; t < cn; ++t) {
-      float acc[VP];
-      token(t, acc);
-      scattered_sums<VP, PARTS>(acc, part);
-      if (part < VP) give(t, part, acc[0]);
     }
     __syncthreads();  // this stage is free again
   }
@@ -901,9 +846,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) decay_scan_kernel(const float* q
     const float* sv = sk + CH * NPAD;
     const float* sg = sv + CH * VB;
     const float* sa = sg + CH * 4;
-    // two partial sums a column (even and odd rows): a token's loads and sums do not wait for the token before it, only its
-    // state values do
-    auto token = [&](int t, float* acc, float* nq_at) {
+    // two tokens an iteration and two partial sums a column (even and odd rows): a token's loads and sums do not
+    // wait for the token before it, only its state values do
+#pragma unroll 2
+    for (int t = 0; t < cn; ++t) {
       float q[NP], k[NP];
       load_run<NP>(sk + t * NPAD + part * RUN, k);
       load_run<NP>(sq + t * NPAD + part * RUN, q);
@@ -911,7 +857,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) decay_scan_kernel(const float* q
       float ch[CHANNEL ? NP : 1];
       if constexpr (CHANNEL) load_run<NP>(sa + t * NPAD + part * RUN, ch);
       const float b = GATED ? sg[t * 4 + 1] : 1.f;
-      float odd[VP], val[VP], nq = 0.f, nq_odd = 0.f;
+      float acc[VP], odd[VP], val[VP], nq = 0.f, nq_odd = 0.f;
 #pragma unroll
       for (int i = 0; i < VP; ++i) {
         acc[i] = odd[i] = 0.f;
@@ -935,35 +881,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) decay_scan_kernel(const float* q
           nq_odd = fmaf(nn[j + 1], q1, nq_odd);
         }
       }
+      float scale = 1.f;
+      if constexpr (GATED) scale = 1.f / (fmaxf(fabsf(group_sum<PARTS>(nq + nq_odd)), sg[t * 4 + 2]) + 1e-6f);
 #pragma unroll
-      for (int i = 0; i < VP; ++i) acc[i] += odd[i];
-      if constexpr (GATED) *nq_at = nq + nq_odd;
-    };
-    auto give = [&](int t, int column, float sum, float nq) {
-      const int v = v0 + grp * VP + column;
-      if (v < vdim)
-        o[(size_t)(c0 + t) * heads * vdim + (size_t)head * vdim + v] = GATED ? sum * (1.f / (fmaxf(fabsf(nq), sg[t * 4 + 2]) + 1e-6f)) : sum;
-    };
-    int t = 0;
-    for (; t + TOGETHER <= cn; t += TOGETHER) {
-      float acc[TOGETHER * VP], nq[TOGETHER];
-#pragma unroll
-      for (int u = 0; u < TOGETHER; ++u) token(t + u, acc + u * VP, nq + u);
-      scattered_sums<TOGETHER * VP, PARTS>(acc, part);
-      if constexpr (GATED) scattered_sums<TOGETHER, PARTS>(nq, part);
-#pragma unroll
-      for (int i = 0; i < (TOGETHER * VP + PARTS - 1) / PARTS; ++i) {
-        const int value = i * PARTS + part, u = value / VP % TOGETHER;
-        const float of_token = GATED ? __shfl_sync(0xffffffffu, nq[0], u, PARTS) : 0.f;
-        if (value < TOGETHER * VP) give(t + u, value % VP, acc[i], of_token);
+      for (int i = 0; i < VP; ++i) {
+        acc[i] = group_sum<PARTS>(acc[i] + odd[i]);
+        const int v = v0 + grp * VP + i;
+        if (part == i && v < vdim) o[(size_t)(c0 + t) * heads * vdim + (size_t)head * vdim + v] = acc[i] * scale;
       }
-    }
-    for (; t < cn; ++t) {
-      float acc[VP], nq = 0.f;
-      token(t, acc, &nq);
-      scattered_sums<VP, PARTS>(acc, part);
-      if constexpr (GATED) nq = group_sum<PARTS>(nq);
-      if (part < VP) give(t, part, acc[0], nq);
     }
     __syncthreads();  // this stage is free again
   }
@@ -1192,10 +1117,8 @@ FMS_API int fms_causal_conv(const void* x, int dtype, int stride, const float* w
 // How a scan is cut.  PARTS threads share a group of value columns and each holds NP of the state's rows: 8 threads
 // by default; 16 or 32 where a model has so few heads and value columns that a single sequence would leave most
 // multiprocessors idle (the choice looks at the model's sizes only, never at the batch, so a sequence's sums run in the
-// same order whatever it is batched with).  VP value columns a thread: as many as still leave every multiprocessor a
-// block, since columns share a token's loads and hide one another's latencies (the sums do not depend on it).  With four blocks a
-// multiprocessor instead, four sequences of 120 tokens took, before and after, 133 and 59 us under the delta rule (16 heads of 128),
-// 107 and 63 under exponential gates (32), 67 and 58 under fixed decays; two 110 and 57 in a state space of 128 heads of 64.
+// same order whatever it is batched with).  VP value columns a thread: as many as still leave every multiprocessor
+// four blocks, whose warps hide one another's latencies (the sums do not depend on it).
 struct ScanShape {
   int parts, np, vp;
 };
@@ -1216,10 +1139,10 @@ static ScanShape scan_shape(int n_seqs, int heads, int vdim, int rows, int few_d
   s.np = need <= 2 ? 2 : (need <= 4 ? 4 : (need <= 8 ? 8 : (need <= 16 ? 16 : 32)));
   const int groups = SCAN_THREADS / s.parts;
   s.vp = 1;
-  static int min_blocks = -1;  // FMS_B200_SCAN_BLOCKS: blocks that must remain for a thread to take more columns (148)
+  static int min_blocks = -1;  // FMS_B200_SCAN_BLOCKS: blocks that must remain for a thread to take more columns (592)
   if (min_blocks < 0) {
     const char* e = getenv("FMS_B200_SCAN_BLOCKS");
-    min_blocks = e ? atoi(e) : 148;
+    min_blocks = e ? atoi(e) : 592;
   }
   for (int vp = s.np >= 32 ? 2 : 4; vp > 1; vp >>= 1)
     if ((long)n_seqs * heads * ((vdim + groups * vp - 1) / (groups * vp)) >= min_blocks && vdim >= groups * vp) {

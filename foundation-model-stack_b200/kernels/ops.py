@@ -1005,12 +1005,13 @@ def causal_conv(x: torch.Tensor, offset: int, channels: int, weight: torch.Tenso
 CHUNK_STATE_BYTES = 64 << 20  # states of the runs of one pass (they are read back soon: within the second-level cache)
 # A sequence goes run by run through a scan under one decay a head from so many tokens of a step on: its own tokens decide, so that
 # its results do not depend on what else is in the step.  Whole layers, all walk / all by runs in us, under exponential gates with a
-# normalizer, fixed decays, state space with heads of 64, delta rule of 16 heads of 128: one prompt of 256 tokens 169 / 145, 139 / 144,
-# 238 / 191, 152 / 196; of 384 233 / 184, 188 / 163, 333 / 222, 204 / 191; of 512 294 / 207, 236 / 195, 418 / 254, 256 / 195; four of 256
-# 353 / 317, 283 / 306, 435 / 425, 250 / 284; of 384 504 / 446, 402 / 443, 629 / 657, 347 / 357.  The walk takes a sequence's tokens one
-# after the other, but many sequences fill the multiprocessors all the same, and a step that mixes both forms pays for both: so
-# the lines lie where a mixed step seldom takes longer than its walk, for the kinds whose runs gain least highest.
-CHUNK_SCAN_FROM = {"gated": 256, "fixed": 512, "space": 384, "delta": 352}
+# normalizer, fixed decays, state space with heads of 64, delta rule of 16 heads of 128: one prompt of 200 tokens 156 / 140, 125 / 137,
+# 192 / 178, 140 / 160; of 256 183 / 142, 140 / 140, 219 / 179, 165 / 158; of 512 329 / 201, 240 / 183, 389 / 245, 295 / 199; of 2,048
+# 1,327 / 607, 891 / 574, 1,455 / 782, 1,110 / 462; eight of 131 to 392 693 / 673, 598 / 652, 868 / 891, 566 / 468.  The walk takes a sequence's
+# tokens one after the other, but many sequences fill the multiprocessors all the same, and a step that mixes both forms pays for both
+# (eight of 131 to 392, those of 256 and more by runs: fixed decays 613, state space 902): so the lines lie where a mixed step seldom
+# takes longer than its walk, for the kinds whose runs gain least highest.
+CHUNK_SCAN_FROM = {"gated": 256, "fixed": 512, "space": 384, "delta": 256}
 
 
 def chunk_scan_pays(n: int, kind: str) -> bool:
