@@ -10,8 +10,9 @@
 // values are 192 KB.  Bound by the steps' order, some 12,000 cycles a block of keys, of which 3,800 are products.  Measured (three
 // prompts of 1,100 tokens together, 32 heads of 128 over 8): 95 us, the kernel on the CUDA cores 207; 64 tokens onto 1,000 cached ones
 // 125 and 271; 17 alone 27 and 29.
-// Operands that are not finite or beyond 2^100 do not split: zeros stand for them, and the rows that see them (or that they belong to)
-// go key by key on the CUDA cores instead.  Of values below 2^-110 the bits below 2^-133 are lost.  A row's result depends on its
+// Operands that are not finite or beyond 2^30 do not split: zeros stand for them, and the rows that see them (or that they belong to)
+// go on the CUDA cores instead, as do rows whose sum of probabilities is no number (a scale beyond 2^60 can make scores infinite):
+// a warp a row, a lane a key, every score by the multiply-adds of the kernel there in their order.  Of values below 2^-110 the bits below 2^-133 are lost.  A row's result depends on its
 // own keys only, block by block of the cache, whatever tile it lies in.
 #pragma once
 
@@ -28,7 +29,7 @@ __device__ __forceinline__ bool ft_put(unsigned char* p, int part, const float* 
   uint4 hi, mid, lo;
   uint32_t most = 0;
   split8(v, &hi, &mid, &lo, most);
-  const bool fine = !(kind_of(most) & 1u);
+  const bool fine = !beyond<30>(most);
   if (!fine) hi = mid = lo = make_uint4(0, 0, 0, 0);
   *reinterpret_cast<uint4*>(p) = hi;
   *reinterpret_cast<uint4*>(p + part) = mid;
@@ -216,6 +217,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
     }
   }
   sums[half][row] = l;
+  if (!(l == l)) odd_query[row] = 1;
   __syncthreads();
   auto odd = [&](int r) {
     const int at = p_first + (r & 63);
@@ -229,33 +231,45 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
 #pragma unroll
     for (int c = 0; c < HD / 2; c += 4) o[c / 4] = make_float4(acc[c] * inv, acc[c + 1] * inv, acc[c + 2] * inv, acc[c + 3] * inv);
   }
-  {  // the other rows: a warp a row, its lanes HD / 32 values each
+  {  // the other rows: a warp a row, a lane a key and HD / 32 of the results
     constexpr int PER = HD / 32;
     for (int r = warp; r < 128; r += FT_THREADS / 32) {
       if ((r & 63) >= rows_here || !odd(r)) continue;
       const int at = p_first + (r & 63), h = head0 + (r >> 6);
-      float qv[PER], o[PER], mr = -INFINITY, lr = 0.f;
-#pragma unroll
-      for (int d = 0; d < PER; ++d) {
-        qv[d] = q[(size_t)(r & 63) * a.q_stride + (r >> 6) * HD + lane * PER + d];
-        o[d] = 0.f;
-      }
-      for (int key = first_visible(a, at); key <= at; ++key) {
-        const int b = block_of(a, slot, key / BLK);
+      const float* qr = q + (size_t)(r & 63) * a.q_stride + (r >> 6) * HD;
+      const int first = first_visible(a, at);
+      float o[PER] = {}, mr = -INFINITY, lr = 0.f;
+      for (int base = first / 32 * 32; base <= at; base += 32) {
+        const int b = block_of(a, slot, base / BLK);
         if (b < 0) continue;
-        const size_t place = (((size_t)b * a.kvheads + kvh) * BLK + key % BLK) * HD + lane * PER;
-        float dot = 0.f;
-#pragma unroll
-        for (int d = 0; d < PER; ++d) dot = fmaf(qv[d], ((const float*)a.keys)[place + d], dot);
-        const float score = warp_sum(dot) * a.scale, m_new = fmaxf(mr, score), m_use = m_new == -INFINITY ? 0.f : m_new;
+        const size_t place = (((size_t)b * a.kvheads + kvh) * BLK + base % BLK) * HD;
+        const bool visible = base + lane >= first && base + lane <= at;
+        float score = -INFINITY;
+        if (visible) {
+          const float* key = (const float*)a.keys + place + (size_t)lane * HD;
+          float dot = 0.f;
+#pragma unroll 4
+          for (int d = 0; d < HD; d += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(qr + d), y = *reinterpret_cast<const float4*>(key + d);
+            dot = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, dot))));
+          }
+          score = dot * a.scale;
+        }
+        const float m_new = fmaxf(mr, warp_max(score)), m_use = m_new == -INFINITY ? 0.f : m_new;
         const float before = mr == -INFINITY ? 0.f : expf(mr - m_use), p = score == -INFINITY ? 0.f : expf(score - m_use);
-        lr = lr * before + p;
+        lr = lr * before + warp_sum(p);
         mr = m_new;
 #pragma unroll
-        for (int d = 0; d < PER; ++d) o[d] = fmaf(p, ((const float*)a.values)[place + d], o[d] * before);
+        for (int d = 0; d < PER; ++d) o[d] *= before;
+        const float* values = (const float*)a.values + place + lane * PER;
+        for (int j = max(first - base, 0); j <= min(at - base, 31); ++j) {
+          const float pj = __shfl_sync(0xffffffffu, p, j);
+#pragma unroll
+          for (int d = 0; d < PER; ++d) o[d] = fmaf(pj, values[j * HD + d], o[d]);
+        }
       }
       if (a.sink != nullptr) lr += expf(a.sink[h] - (mr == -INFINITY ? 0.f : mr));
-      const float inv = lr > 0.f ? 1.f / lr : (lr == lr ? 0.f : lr);
+      const float inv = lr > 0.f ? 1.f / lr : 0.f;  // where lr is no number, o is none
 #pragma unroll
       for (int d = 0; d < PER; ++d) ((float*)a.out)[(size_t)(row_begin + r0 + (r & 63)) * a.nheads * HD + (size_t)h * HD + lane * PER + d] = o[d] * inv;
     }

@@ -40,6 +40,13 @@ __device__ __forceinline__ void split8(const float* v, uint4* hi, uint4* mid, ui
   *mid = make_uint4(m[0], m[1], m[2], m[3]);
   *lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
+// Whether something is beyond 2^EXPONENT or no number, from the largest magnitudes.  Operands that stay below are split: their products'
+// sums are finite whatever their signs, where infinities of products of parts would meet in NaN.
+template <int EXPONENT>
+__device__ __forceinline__ bool beyond(uint32_t most) {
+  const uint32_t a = most & 0x7fffu, b = (most >> 16) & 0x7fffu;  // order of magnitudes is order of bits; NaN above all
+  return (a > b ? a : b) > ((127u + EXPONENT) << 7);
+}
 // What a row holds, from its largest magnitudes: bit 0 something beyond 2^100 or no number, bit 1 something but zeros, bit 2 something
 // from 2^-64 on.  Kinds of the parts of a row are or-ed; a row is split unless bit 0 is set, or bit 1 without bit 2.
 __device__ __forceinline__ unsigned kind_of(uint32_t most) {

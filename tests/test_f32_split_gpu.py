@@ -165,3 +165,32 @@ def test_attention_keeps_what_does_not_split_to_the_rows_that_see_it(ops, what, 
     assert torch.equal(torch.isfinite(got), torch.isfinite(want))
     fine = torch.isfinite(want)
     assert float((got - want)[fine].abs().max()) <= 2.0 ** -24 * 64 * float(want[fine].abs().max())
+
+
+def beside_the_cuda_cores(ops, monkeypatch, q, view, batch, nheads, kvheads, hd, window=0, scale=None):
+    """A step's attention as it is and on the CUDA cores."""
+    scale = hd ** -0.5 if scale is None else scale
+    got = ops.attention(q, batch, view, nheads, kvheads, hd, scale, window)
+    with monkeypatch.context() as m:
+        m.setattr(ops, "F32_SPLIT_ATTENTION_TOKENS", 1 << 30)
+        return got, ops.attention(q, batch, view, nheads, kvheads, hd, scale, window)
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("scale", [None, 3e38])
+def test_attention_of_scores_beyond_float32(ops, monkeypatch, sign, scale):
+    """A query and a key of 1e21, whose score overflows either way, and a scale that makes every score do so: no number where the
+    multiply-adds give none, weight zero where they give -inf; such a row equals theirs but for the order of its sums."""
+    nheads, kvheads, hd, n, before, at = 4, 2, 128, 200, 37, 120
+    _, q, view, batch = attended(ops, [n], [before], nheads, kvheads, hd, seed=6)
+    signs = torch.where(torch.randn(hd, device="cuda") < 0, -1.0, 1.0)
+    q = q.clone()
+    q[at, 2 * hd:3 * hd] = 1e21 * signs
+    block = view.table[batch.slots[0]][(before + at - 30) // 64]
+    view.keys[block, 1, (before + at - 30) % 64] = sign * 1e21 * signs
+    got, want = beside_the_cuda_cores(ops, monkeypatch, q, view, batch, nheads, kvheads, hd, scale=scale)
+    row = want[at, 2 * hd:3 * hd]
+    assert bool(torch.isnan(row).all() if sign > 0 or scale else (torch.isfinite(row) & (row != 0)).all())
+    assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+    fine = torch.isfinite(want)
+    assert scale or float((got - want)[fine].abs().max()) <= 2.0 ** -24 * 64 * float(want[fine].abs().max())
