@@ -65,21 +65,21 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   unsigned char *ks = qs + 3 * FT_QPART, *vs = ks + FT_KREGION;
   __shared__ uint64_t done_s, done_o;
   __shared__ uint32_t tmem_slot;
-  __shared__ int failed_flag, odd_first, odd_last;  // the first and the last position whose key or value does not split
-  __shared__ unsigned char odd_query[128];
+  __shared__ int failed_flag;
+  __shared__ unsigned odd_keys[2][2];  // by the parity of the step and by halves: the block's positions whose key or value does not split
+  __shared__ unsigned char odd[128];   // rows that go on the CUDA cores
   __shared__ float top[2][128], sums[2][128];
   volatile int* failed = &failed_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = warp >> 2, row = (warp & 3) * 32 + lane;
   pdl_launch_dependents();
   if (tid == 0) {
     failed_flag = 0;
-    odd_first = 0x7fffffff;
-    odd_last = -1;
     mbar_init(&done_s, 1);
     mbar_init(&done_o, 1);
     mbar_fence_init();
   }
-  if (tid < 128) odd_query[tid] = 0;
+  if (tid < 128) odd[tid] = 0;
+  if (tid < 4) odd_keys[tid >> 1][tid & 1] = 0;
   if (warp == 0) tmem_alloc(&tmem_slot, 512);
   __syncthreads();
   pdl_wait();
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
     const int r = i / FT_PER_ROW, c = i % FT_PER_ROW;
     float v[8];
     ft_read(v, q + (size_t)(r & 63) * a.q_stride + (r >> 6) * HD + 8 * c, (r & 63) < rows_here);
-    if (!ft_put(qs + (c >> 3) * (128 * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), FT_QPART, v)) odd_query[r] = 1;
+    if (!ft_put(qs + (c >> 3) * (128 * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), FT_QPART, v)) odd[r] = 1;
   }
   float x[FT_UNITS][8];
   auto read_block = [&](const void* cache, int kb, int blk) {
@@ -105,14 +105,12 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
 #pragma unroll
     for (int u = 0; u < FT_UNITS; ++u) ft_read(x[u], base + (size_t)(k_row + u * K_STEP) * HD + 8 * piece, kb * BLK + k_row + u * K_STEP < len);
   };
-  auto put_block = [&](unsigned char* to, int kb) {
+  auto put_block = [&](unsigned char* to, int parity) {
 #pragma unroll
     for (int u = 0; u < FT_UNITS; ++u) {
       const int r = k_row + u * K_STEP;
-      if (!ft_put(to + (piece >> 3) * (BLK * 128) + r * 128 + (((piece & 7) ^ (r & 7)) << 4), FT_KPART, x[u])) {
-        atomicMin(&odd_first, kb * BLK + r);
-        atomicMax(&odd_last, kb * BLK + r);
-      }
+      if (!ft_put(to + (piece >> 3) * (BLK * 128) + r * 128 + (((piece & 7) ^ (r & 7)) << 4), FT_KPART, x[u]))
+        atomicOr(&odd_keys[parity][r >> 5], 1u << (r & 31));
     }
   };
   // the next block of keys from kb on, or one behind the last (a block that left the window has no place in the cache)
@@ -130,9 +128,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   float m = -INFINITY, l = 0.f, acc[HD / 2];  // l: of this thread's half of the keys
 #pragma unroll
   for (int c = 0; c < HD / 2; ++c) acc[c] = 0.f;
-  bool ok = true;
+  bool ok = true, sees_odd = false;
   for (int it = 0; kb <= kb_hi; ++it) {
-    put_block(ks, kb);
+    put_block(ks, it & 1);
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();  // the keys' parts are there, and every row is done with the block before
@@ -148,7 +146,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
     }
     __syncwarp();
     read_block(a.values, kb, blk);
-    put_block(vs, kb);
+    put_block(vs, it & 1);
     const int this_kb = kb;
     kb = next_block(kb + 1, blk);
     if (kb <= kb_hi) read_block(a.keys, kb, blk);
@@ -174,7 +172,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
       most_here = fmaxf(most_here, s[j]);
     }
     top[half][row] = most_here;
+    if (tid < 2) odd_keys[(it + 1) & 1][tid] = 0;  // every row has read what the step before found
     __syncthreads();
+    // of this block's positions the row's own visible ones, so that nothing depends on the tile's other rows
+    const unsigned own = from < 32 && upto >= 0 ? (0xffffffffu << max(from, 0)) & (0xffffffffu >> (31 - min(upto, 31))) : 0u;
+    sees_odd |= (odd_keys[it & 1][half] & own) != 0;
     const float m_new = fmaxf(m, fmaxf(top[0][row], top[1][row])), m_use = m_new == -INFINITY ? 0.f : m_new;
     const float alpha = m == -INFINITY ? 0.f : expf(m - m_use);
     float psum = 0.f;
@@ -217,13 +219,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
     }
   }
   sums[half][row] = l;
-  if (!(l == l)) odd_query[row] = 1;
+  if (sees_odd || !(l == l)) odd[row] = 1;
   __syncthreads();
-  auto odd = [&](int r) {
-    const int at = p_first + (r & 63);
-    return odd_query[r] || (odd_first <= at && odd_last >= first_visible(a, at));
-  };
-  if (mine && !odd(row)) {
+  if (mine && !odd[row]) {
     float sum = sums[0][row] + sums[1][row];
     if (a.sink != nullptr) sum += expf(a.sink[head] - (m == -INFINITY ? 0.f : m));
     const float inv = sum > 0.f ? 1.f / sum : 0.f;
@@ -234,7 +232,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   {  // the other rows: a warp a row, a lane a key and HD / 32 of the results
     constexpr int PER = HD / 32;
     for (int r = warp; r < 128; r += FT_THREADS / 32) {
-      if ((r & 63) >= rows_here || !odd(r)) continue;
+      if ((r & 63) >= rows_here || !odd[r]) continue;
       const int at = p_first + (r & 63), h = head0 + (r >> 6);
       const float* qr = q + (size_t)(r & 63) * a.q_stride + (r >> 6) * HD;
       const int first = first_visible(a, at);

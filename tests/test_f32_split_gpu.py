@@ -194,3 +194,17 @@ def test_attention_of_scores_beyond_float32(ops, monkeypatch, sign, scale):
     assert torch.equal(torch.isfinite(got), torch.isfinite(want))
     fine = torch.isfinite(want)
     assert scale or float((got - want)[fine].abs().max()) <= 2.0 ** -24 * 64 * float(want[fine].abs().max())
+
+
+@pytest.mark.parametrize("what", ["key", "value"])
+@pytest.mark.parametrize("window,chunk", [(16, 0), (0, 16)])
+def test_attention_rows_between_positions_that_do_not_split(ops, what, window, chunk):
+    """Bad positions on both sides of what a row sees leave its bits as they are."""
+    nheads, kvheads, hd, n, bad = 4, 2, 64, 150, (5, 62, 127)
+    clean, q, view, batch = attended(ops, [n], [0], nheads, kvheads, hd, window, chunk, seed=7)
+    for at in bad:
+        (view.keys if what == "key" else view.values)[view.table[batch.slots[0]][at // 64], :, at % 64, 3] = float("nan")
+    got = ops.attention(q, batch, view, nheads, kvheads, hd, hd ** -0.5, window, None, chunk)
+    sees = torch.tensor([any(a <= p and (p - a < window if window else p // chunk == a // chunk) for a in bad) for p in range(n)], device="cuda")
+    assert torch.equal(got[~sees], clean[~sees])
+    assert bool(torch.isnan(got[sees]).any(1).all())
