@@ -12,8 +12,9 @@
 // 125 and 271; 17 alone 27 and 29.
 // Operands that are not finite or beyond 2^30 do not split: zeros stand for them, and the rows that see them (or that they belong to)
 // go on the CUDA cores instead, as do rows whose sum of probabilities is no number (a scale beyond 2^60 can make scores infinite):
-// a warp a row, a lane a key, every score by the multiply-adds of the kernel there in their order.  Of values below 2^-110 the bits below 2^-133 are lost.  A row's result depends on its
-// own keys only, block by block of the cache, whatever tile it lies in.
+// a warp a row, a lane a key, every score by the multiply-adds of the kernel there in their order.  All operands
+// are split times 2^SPLIT_SCALE, so that small ones lose nothing.  A row's result depends on its own keys only, block by block of
+// the cache, whatever tile it lies in.
 #pragma once
 
 constexpr int FT_THREADS = 256, FT_ATOMS = HD / 64;
@@ -24,12 +25,14 @@ constexpr int FT_O = 256;             // tensor memory: scores from column 0, re
 constexpr int FT_PER_ROW = HD / 8;    // threads a row of keys or values, eight values each
 constexpr int FT_UNITS = BLK * FT_PER_ROW / FT_THREADS;
 
+constexpr float FT_UNSCALE = power_of_two(-2 * SPLIT_SCALE);  // of a product of two operands
+
 // eight values to 16 bytes of each of three parts; whether they split (else zeros)
 __device__ __forceinline__ bool ft_put(unsigned char* p, int part, const float* v) {
   uint4 hi, mid, lo;
   uint32_t most = 0;
-  split8(v, &hi, &mid, &lo, most);
-  const bool fine = !beyond<30>(most);
+  split8<SPLIT_SCALE>(v, &hi, &mid, &lo, most);
+  const bool fine = !beyond<30 + SPLIT_SCALE>(most);
   if (!fine) hi = mid = lo = make_uint4(0, 0, 0, 0);
   *reinterpret_cast<uint4*>(p) = hi;
   *reinterpret_cast<uint4*>(p + part) = mid;
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
     const int from = my_first - (this_kb * BLK + half * 32), upto = mine ? my_pos - (this_kb * BLK + half * 32) : -1;  // visible: from .. upto
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-      s[j] = j >= from && j <= upto ? s[j] * a.scale : -INFINITY;
+      s[j] = j >= from && j <= upto ? s[j] * FT_UNSCALE * a.scale : -INFINITY;
       most_here = fmaxf(most_here, s[j]);
     }
     top[half][row] = most_here;
@@ -227,7 +230,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
     const float inv = sum > 0.f ? 1.f / sum : 0.f;
     float4* o = reinterpret_cast<float4*>((float*)a.out + (size_t)(row_begin + r0 + pos) * a.nheads * HD + (size_t)head * HD + half * (HD / 2));
 #pragma unroll
-    for (int c = 0; c < HD / 2; c += 4) o[c / 4] = make_float4(acc[c] * inv, acc[c + 1] * inv, acc[c + 2] * inv, acc[c + 3] * inv);
+    for (int c = 0; c < HD / 2; c += 4)
+      o[c / 4] = make_float4(acc[c] * inv * FT_UNSCALE, acc[c + 1] * inv * FT_UNSCALE, acc[c + 2] * inv * FT_UNSCALE, acc[c + 3] * inv * FT_UNSCALE);
   }
   {  // the other rows: a warp a row, a lane a key and HD / 32 of the results
     constexpr int PER = HD / 32;

@@ -1,6 +1,11 @@
 // float32 values as sums of three bfloat16 values, for products on the tensor cores that lose nothing of the operands (nearest, nearest
-// of the rest, the rest: 8 bits of mantissa each).  Included inside the anonymous namespace of the kernels that use it.
+// of the rest, the rest: 8 bits of mantissa each).  A part is exact while none of its bits lies below 2^-133: so for magnitudes from
+// 2^-110 on, and for every float32 value, subnormal ones too, where values are multiplied by 2^SPLIT_SCALE before (whose parts are
+// normal bfloat16 then).  Included inside the anonymous namespace of the kernels that use it.
 #pragma once
+
+constexpr int SPLIT_SCALE = 24;
+__host__ __device__ constexpr float power_of_two(int e) { return e < 0 ? 0.5f * power_of_two(e + 1) : e > 0 ? 2.f * power_of_two(e - 1) : 1.f; }
 
 __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {  // nearest bfloat16 of a in the low half, of b in the high half
   uint32_t r;
@@ -24,13 +29,25 @@ __device__ __forceinline__ float2 rest2(float2 v, uint32_t h) {
   asm("mov.b64 {%0, %1}, %2;\n" : "=f"(o.x), "=f"(o.y) : "l"(r));
   return o;
 }
-// eight values of consecutive k as three times 16 bytes; most: the largest magnitudes so far
+__device__ __forceinline__ float2 scaled2(float2 v, float by) {
+  unsigned long long r, a, b;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(a) : "f"(v.x), "f"(v.y));
+  asm("mov.b64 %0, {%1, %1};\n" : "=l"(b) : "f"(by));
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  float2 o;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(o.x), "=f"(o.y) : "l"(r));
+  return o;
+}
+// eight values of consecutive k, times 2^SCALE, as three times 16 bytes; most: the largest magnitudes so far
+template <int SCALE = 0>
 __device__ __forceinline__ void split8(const float* v, uint4* hi, uint4* mid, uint4* lo, uint32_t& most) {
   uint32_t h[4], m[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    h[i] = bf16_pair(v[2 * i], v[2 * i + 1]);
-    const float2 r = rest2(make_float2(v[2 * i], v[2 * i + 1]), h[i]);
+    float2 x = make_float2(v[2 * i], v[2 * i + 1]);
+    if constexpr (SCALE != 0) x = scaled2(x, power_of_two(SCALE));
+    h[i] = bf16_pair(x.x, x.y);
+    const float2 r = rest2(x, h[i]);
     m[i] = bf16_pair(r.x, r.y);
     const float2 t = rest2(r, m[i]);
     l[i] = bf16_pair(t.x, t.y);

@@ -208,3 +208,26 @@ def test_attention_rows_between_positions_that_do_not_split(ops, what, window, c
     sees = torch.tensor([any(a <= p and (p - a < window if window else p // chunk == a // chunk) for a in bad) for p in range(n)], device="cuda")
     assert torch.equal(got[~sees], clean[~sees])
     assert bool(torch.isnan(got[sees]).any(1).all())
+
+
+@pytest.mark.parametrize("small,gap", [(2.0 ** -126, 0.0), (1.0, 86.0)])
+def test_attention_of_small_values(ops, monkeypatch, small, gap):
+    """Values, and probabilities of e^-86 beside one whose value is zero, whose last bits lie below 2^-133: nothing of them is lost."""
+    nheads, kvheads, hd, n = 4, 2, 128, 130
+    _, q, view, batch = attended(ops, [n], [0], nheads, kvheads, hd, seed=8)
+    q = torch.zeros_like(q)
+    q.view(n, nheads, hd)[:, :, 0] = gap * hd ** 0.5
+    blocks = view.table[batch.slots[0]][:3].long()
+    view.keys[blocks] = 0.0
+    view.keys[blocks[0], :, 0, 0] = 1.0
+    view.values[blocks] *= small
+    view.values[blocks[0], :, 0] = 0.0
+    got, want = beside_the_cuda_cores(ops, monkeypatch, q, view, batch, nheads, kvheads, hd)
+    # both sides' sums of up to 130 terms and their exponentials: some 2^-24 of the terms' magnitudes each; a result's spacing
+    values = view.values[blocks].double().abs().transpose(0, 1).reshape(kvheads, -1, hd)[:, :n].repeat_interleave(nheads // kvheads, 0)
+    size = torch.cumsum(values, 1).transpose(0, 1) * float(torch.exp(torch.tensor(-gap).double()))
+    if not gap:
+        size /= torch.arange(1, n + 1, device="cuda")[:, None, None]
+    a, b = (t.view(n, nheads, hd).double() for t in (got, want))
+    assert float(b.abs().max()) > 2.0 ** -126
+    assert bool(((a - b).abs() <= 2.0 ** -24 * 64 * size + 2.0 ** -148).all())
