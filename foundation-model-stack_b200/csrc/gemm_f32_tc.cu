@@ -10,8 +10,10 @@
 // against 64 bits for normal values, K = 1,024 / 4,096 / 14,336: 5.6e-8 / 1.0e-7 / 1.9e-7 (multiply-adds of gemm_f32.cu 2.1e-7 /
 // 4.1e-7 / 7.6e-7).
 //
-// Values that are not finite or beyond 2^100, and rows without anything above 2^-64, do not split: a row of x or of w with
-// such values is noted while it is split, and its elements are made by multiply-adds instead.
+// x and w are split times 2^SPLIT_SCALE, and sums are scaled back when they are complete: parts of the smallest float32 values are
+// normal bfloat16 values then, and sums of products down to 2^-174 normal float32 ones (additions in memory flush what is smaller, the
+// others do so too).  Values that are not finite or beyond 2^30 do not split (products of parts of both signs could overflow where the
+// sum does not): a row of x or of w with such values is noted while it is split, and its elements are made by multiply-adds instead.
 //
 // x is split by a kernel of its own (it is read by every tile of w's rows; 27 MB written for 1,100 rows of 4,096).  w is split on
 // its way, since writing it split would take longer than the product reads it.  A block owns 128 rows of w (the instruction's
@@ -41,6 +43,8 @@ namespace cg = cooperative_groups;
 #include "split_f32.cuh"
 
 constexpr int RUNS = 4, BK = 32, WROWS = 128;
+constexpr int SPLIT_UP_TO = 30 + SPLIT_SCALE, MOST_K = 1 << 18;  // 2^18 products of two operands of 2^54 are below 2^127
+constexpr float UNSCALE = power_of_two(-2 * SPLIT_SCALE);
 constexpr int OTHER_REGS = 48;  // registers of the threads that neither split nor drain, where the kinds differ
 constexpr int W_PART = WROWS * BK * 2;  // bytes of one part of a stage's rows of w
 
@@ -61,6 +65,7 @@ struct Shape {
   static constexpr int NT = NT_, SUB = SUB_, CONV = CONV_, EPI = EPI_, STAGES = STAGES_, DEPTH = DEPTH_, AHEAD = AHEAD_;
   static constexpr int CONV_REGS = CONV_REGS_, EPI_REGS = EPI_REGS_;
   static constexpr int PIECE = NT > 128 ? 32 : 16;           // columns that a warp reads at a time
+  static constexpr int LAST = NT > 64 ? 16 : 8;              // sums of earlier runs that a thread reads at a time with the last
   static constexpr int SPAN = CONV * 8, UNITS = WROWS / SPAN;  // rows of w that the splitting warps take at a time, and how often
   static constexpr int MMA = EPI, TMA = EPI + 1, CONV_AT = EPI + 4;  // warps: first those that drain
   static constexpr int THREADS = 32 * (CONV_AT + CONV), COLS = NT / (EPI / 4);
@@ -73,7 +78,7 @@ struct Shape {
 struct Product {
   const float *x, *w, *bias;
   float* y;
-  const unsigned char* x_kinds;  // of every row of x
+  const unsigned char* x_whole;  // of every row of x: whether it stays whole
   int M, N, K, run_len, ranks, nt, tiles_x, tiles, vec;
   int* error_flag;
 };
@@ -89,14 +94,27 @@ __device__ __forceinline__ void umma_64(uint32_t tmem_d, uint32_t a, uint32_t b,
       "r"(a), "r"(b), "r"(idesc), "n"(ACCUMULATE ? 1 : 0), "r"((512u >> 4) | (1u << 14) | (4u << 29)), "r"(0u)
       : "memory");
 }
-// If wanted, *at = v, or *at += v where it lies, rounded to nearest; only this thread writes there, so its additions happen in their
-// order.  Under a predicate: a branch a column would cost more than the store
+// If wanted, *at = v, or *at += v where it lies, rounded to nearest, subnormal values as zeros; only this thread writes there, so its
+// additions happen in their order.  Under a predicate: a branch a column would cost more than the store
 template <bool ADD>
 __device__ __forceinline__ void put_to(float* at, float v, bool wanted) {
   if constexpr (ADD)
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %2, 0;\n@p red.relaxed.gpu.global.add.f32 [%0], %1;\n}\n" ::"l"(at), "f"(v), "r"((int)wanted) : "memory");
   else
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %2, 0;\n@p st.global.f32 [%0], %1;\n}\n" ::"l"(at), "f"(v), "r"((int)wanted) : "memory");
+}
+
+// what additions in memory have made of *at, if wanted, else 0
+__device__ __forceinline__ float sum_at(const float* at, bool wanted) {
+  float v = 0.f;
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %2, 0;\n@p ld.relaxed.gpu.global.f32 %0, [%1];\n}\n" : "+f"(v) : "l"(at), "r"((int)wanted) : "memory");
+  return v;
+}
+// a + b as additions in memory make it
+__device__ __forceinline__ float add_runs(float a, float b) {
+  float r;
+  asm("add.rn.ftz.f32 %0, %1, %2;\n" : "=f"(r) : "f"(a), "f"(b));
+  return r;
 }
 
 // Eight values from `at` on, if they are wanted; `left`: so many of them exist, the others are zeros.  vec: 2 rows of 32 bytes alignment, 1 of
@@ -132,14 +150,11 @@ __device__ __forceinline__ float whole_element(const float* __restrict__ x, cons
   return warp_sum(v);
 }
 
-// x as three matrices of bfloat16 parts [3][M][pitch], zeros behind K, and the kinds of its rows: a block a row
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, uint4* __restrict__ parts, unsigned char* __restrict__ kinds,
+// x as three matrices of bfloat16 parts [3][M][pitch], zeros behind K, and whether a row stays whole: a block a row
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, uint4* __restrict__ parts, unsigned char* __restrict__ whole,
                                                          int M, int K, int pitch, int vec) {
-  __shared__ unsigned all;
-  if (threadIdx.x == 0) all = 0;
   pdl_launch_dependents();
   pdl_wait();
-  __syncthreads();
   const int m = blockIdx.x;
   uint32_t most = 0;
   for (int k = threadIdx.x * 8; k < pitch; k += blockDim.x * 8) {
@@ -153,17 +168,15 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
       for (int j = 0; j < 8; ++j) v[j] = k + j < K ? at[j] : 0.f;
     }
     uint4 hi, mid, lo;
-    split8(v, &hi, &mid, &lo, most);
+    split8<SPLIT_SCALE>(v, &hi, &mid, &lo, most);
     const size_t part = (size_t)M * (pitch / 8), to = (size_t)m * (pitch / 8) + k / 8;
     if (!FMS_IN(to, part)) continue;
     parts[to] = hi;
     parts[part + to] = mid;
     parts[2 * part + to] = lo;
   }
-  const unsigned kind = __reduce_or_sync(0xffffffffu, kind_of(most));
-  if ((threadIdx.x & 31) == 0) atomicOr(&all, kind);
-  __syncthreads();
-  if (threadIdx.x == 0) kinds[m] = (unsigned char)all;
+  const int any = __syncthreads_or(beyond<SPLIT_UP_TO>(most));
+  if (threadIdx.x == 0) whole[m] = any ? 1 : 0;
 }
 
 template <typename S>
@@ -173,7 +186,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
   __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int failed_flag, whole_any;  // whole_any: some row of this block's run may have to stay whole
-  __shared__ unsigned char w_kinds[2][WROWS];  // by the parity of the block's tile
+  __shared__ unsigned char w_whole[2][WROWS];  // by the parity of the block's tile
   volatile int* failed = &failed_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int x_part = p.nt * BK * 2, sub_bytes = 3 * (W_PART + x_part), stage_bytes = S::SUB * sub_bytes;
@@ -269,7 +282,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
 #pragma unroll
               for (int h = 0; h < S::SUB; ++h) {
                 uint4 hi, mid, lo;
-                split8(v[d][u][h], &hi, &mid, &lo, most[u]);
+                split8<SPLIT_SCALE>(v[d][u][h], &hi, &mid, &lo, most[u]);
                 unsigned char* const place = stage + h * sub_bytes + u * S::SPAN * 64;
                 *reinterpret_cast<uint4*>(place) = hi;
                 *reinterpret_cast<uint4*>(place + W_PART) = mid;
@@ -290,7 +303,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
               for (int u = 0; u < S::UNITS; ++u) {
                 uint32_t m = most2(most[u], __shfl_xor_sync(0xffffffffu, most[u], 1));
                 m = most2(m, __shfl_xor_sync(0xffffffffu, m, 2));
-                if ((lane & 3) == 0) w_kinds[turn][u * S::SPAN + row] = (unsigned char)kind_of(m);
+                if ((lane & 3) == 0) w_whole[turn][u * S::SPAN + row] = beyond<SPLIT_UP_TO>(m) ? 1 : 0;
                 most[u] = 0;
               }
             }
@@ -404,24 +417,38 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
           const float b = end && p.bias && n < p.N ? p.bias[n] : 0.f;
           float* at = p.y + (size_t)(x0 + col0) * p.N + n;
           const int left = n < p.N ? min(cols, p.M - (x0 + col0)) : 0;
-          if (first_run) {
+          if (end) {
+#pragma unroll
+            for (int c0 = 0; c0 < S::COLS; c0 += S::LAST) {
+              float before[S::LAST];
+              float* from = at;
+#pragma unroll
+              for (int j = 0; j < S::LAST; ++j) {
+                before[j] = sum_at(from, !first_run && c0 + j < left && FMS_IN(from - p.y, (size_t)p.M * p.N));
+                from += p.N;
+                asm volatile("" : "+l"(from));  // one column after the other: no addresses kept for all of them
+              }
+#pragma unroll
+              for (int j = 0; j < S::LAST; ++j) {
+                put_to<false>(at, __fadd_rn(__fmul_rn(add_runs(before[j], acc[c0 + j]), UNSCALE), b), c0 + j < left && FMS_IN(at - p.y, (size_t)p.M * p.N));
+                at += p.N;
+                asm volatile("" : "+l"(at));
+              }
+            }
+          } else if (first_run) {
 #pragma unroll
             for (int c = 0; c < S::COLS; ++c) {
               put_to<false>(at, acc[c], c < left && FMS_IN(at - p.y, (size_t)p.M * p.N));
               at += p.N;
-              asm volatile("" : "+l"(at));  // one column after the other: no addresses kept for all of them
+              asm volatile("" : "+l"(at));
             }
           } else {
 #pragma unroll
             for (int c = 0; c < S::COLS; ++c) {
               put_to<true>(at, acc[c], c < left && FMS_IN(at - p.y, (size_t)p.M * p.N));
               at += p.N;
-              asm volatile("" : "+l"(at));  // one column after the other: no addresses kept for all of them
+              asm volatile("" : "+l"(at));
             }
-          }
-          if (end && p.bias) {
-            at = p.y + (size_t)(x0 + col0) * p.N + n;
-            for (int c = 0; c < left; ++c, at += p.N) put_to<true>(at, b, FMS_IN(at - p.y, (size_t)p.M * p.N));
           }
 #pragma unroll
           for (int c = 0; c < S::COLS; ++c) acc[c] = 0.f;
@@ -429,17 +456,17 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
           run_end += p.run_len / S::STEP;
           if (end) {
             bool any = false;
-            for (int j = lane; j < WROWS; j += 32) any |= stays_whole(w_kinds[turn][j]);
-            for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= stays_whole(p.x_kinds[x0 + j]);
+            for (int j = lane; j < WROWS; j += 32) any |= w_whole[turn][j] != 0;
+            for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_whole[x0 + j] != 0;
             if (__any_sync(0xffffffffu, any)) {
-              const bool whole_w = stays_whole(w_kinds[turn][my_row]);
+              const bool whole_w = w_whole[turn][my_row] != 0;
               for (int c = 0; c < cols && x0 + col0 + c < p.M; ++c) {
                 const int m = x0 + col0 + c;
-                unsigned rows = __ballot_sync(0xffffffffu, n < p.N && (whole_w || stays_whole(p.x_kinds[m])));
+                unsigned rows = __ballot_sync(0xffffffffu, n < p.N && (whole_w || p.x_whole[m]));
                 for (; rows; rows &= rows - 1) {
                   const int r = __ffs(rows) - 1;
                   const float v = whole_element(p.x + (size_t)m * p.K, p.w + (size_t)(w0 + quarter * 32 + r) * p.K, p.K, lane);
-                  if (lane == r) p.y[(size_t)m * p.N + n] = p.bias ? v + b : v;
+                  if (lane == r) p.y[(size_t)m * p.N + n] = v + b;
                 }
               }
             }
@@ -455,8 +482,8 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
           if (c < cols) own[(col0 + c) * WROWS + my_row] = acc[c];
         const int x0 = first_tile % p.tiles_x * p.nt;
         bool any = false;
-        for (int j = lane; j < WROWS; j += 32) any |= stays_whole(w_kinds[0][j]);
-        for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= stays_whole(p.x_kinds[x0 + j]);
+        for (int j = lane; j < WROWS; j += 32) any |= w_whole[0][j] != 0;
+        for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_whole[x0 + j] != 0;
         if (__any_sync(0xffffffffu, any) && lane == 0) whole_any = 1;
       }
       __syncwarp();
@@ -483,16 +510,16 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
         float4 q = t[0];
 #pragma unroll
         for (int s = 1; s < RUNS; ++s)
-          if (s < runs) q = make_float4(q.x + t[s].x, q.y + t[s].y, q.z + t[s].z, q.w + t[s].w);
-        float v[4] = {q.x, q.y, q.z, q.w};
+          if (s < runs) q = make_float4(add_runs(q.x, t[s].x), add_runs(q.y, t[s].y), add_runs(q.z, t[s].z), add_runs(q.w, t[s].w));
+        float v[4] = {__fmul_rn(q.x, UNSCALE), __fmul_rn(q.y, UNSCALE), __fmul_rn(q.z, UNSCALE), __fmul_rn(q.w, UNSCALE)};
         float* const at = p.y + (size_t)(x0 + c) * p.N + n;
         if (any) {
-          const unsigned kx = p.x_kinds[x0 + c];
+          const unsigned whole_x = p.x_whole[x0 + c];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            unsigned kw = 0;
-            for (int s = 0; s < runs; ++s) kw |= cluster.map_shared_rank(w_kinds[0], s)[row + j];
-            unsigned rows = __ballot_sync(0xffffffffu, n + j < p.N && (stays_whole(kw) || stays_whole(kx)));
+            unsigned whole = whole_x;
+            for (int s = 0; s < runs; ++s) whole |= cluster.map_shared_rank(w_whole[0], s)[row + j];
+            unsigned rows = __ballot_sync(0xffffffffu, n + j < p.N && whole);
             for (; rows; rows &= rows - 1) {
               const int r = __ffs(rows) - 1;
               const float t = whole_element(p.x + (size_t)(x0 + c) * p.K, p.w + (size_t)(n + j + (r - lane) * 4) * p.K, p.K, lane);
@@ -500,10 +527,9 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
             }
           }
         }
-        if (p.bias)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (n + j < p.N) v[j] += p.bias[n + j];
+        for (int j = 0; j < 4; ++j)
+          if (n + j < p.N) v[j] = __fadd_rn(v[j], p.bias ? p.bias[n + j] : 0.f);
         if (four && n + 3 < p.N) {
           if (FMS_IN(at + 3 - p.y, (size_t)p.M * p.N)) *reinterpret_cast<float4*>(at) = make_float4(v[0], v[1], v[2], v[3]);
         } else {
@@ -613,7 +639,7 @@ void plan(int M, int N, int K, Product& p) {
 FMS_API int fms_gemm_f32_tc(const float* x, const float* w, const float* bias, float* y, void* scratch, long long scratch_bytes, int M, int N,
                             int K, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0) return fms_fail("gemm_f32_tc: K %d", K);
+  if (K <= 0 || K > MOST_K) return fms_fail("gemm_f32_tc: K %d, at most %d", K, MOST_K);
   Product p = {};
   p.x = x; p.w = w; p.bias = bias; p.y = y;
   p.M = M; p.N = N; p.K = K;
@@ -628,10 +654,10 @@ FMS_API int fms_gemm_f32_tc(const float* x, const float* w, const float* bias, f
   if (3LL * M > 0x7fffffffLL) return fms_fail("gemm_f32_tc: %d rows", M);
   if (scratch == nullptr || ((uintptr_t)scratch & 127) || scratch_bytes < (long long)M * pitch_of(K) * 6 + M)
     return fms_fail("gemm_f32_tc: %lld bytes of scratch at %p", scratch_bytes, scratch);
-  unsigned char* kinds = (unsigned char*)scratch + (size_t)M * pitch * 6;
-  fms_launch(split_rows_kernel, dim3(M), dim3(256), 0, stream, x, (uint4*)scratch, kinds, M, K, pitch, p.vec);
+  unsigned char* whole = (unsigned char*)scratch + (size_t)M * pitch * 6;
+  fms_launch(split_rows_kernel, dim3(M), dim3(256), 0, stream, x, (uint4*)scratch, whole, M, K, pitch, p.vec);
   if (fms_launch_status("gemm_f32_tc")) return 1;
-  p.x_kinds = kinds;
+  p.x_whole = whole;
   if (make_parts_map(&map_x, scratch, 3L * M, pitch, p.nt)) return 1;
   if (p.nt <= 64) return launch_shape<Shape<64, 2, 16, 8, 3, 2, 4, 0, 0>>(p, map_x, stream);
   if (p.nt <= 128) return launch_shape<Shape<128, 2, 16, 8, 2, 1, 0, 56, 112>>(p, map_x, stream);

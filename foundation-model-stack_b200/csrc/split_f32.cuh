@@ -64,10 +64,3 @@ __device__ __forceinline__ bool beyond(uint32_t most) {
   const uint32_t a = most & 0x7fffu, b = (most >> 16) & 0x7fffu;  // order of magnitudes is order of bits; NaN above all
   return (a > b ? a : b) > ((127u + EXPONENT) << 7);
 }
-// What a row holds, from its largest magnitudes: bit 0 something beyond 2^100 or no number, bit 1 something but zeros, bit 2 something
-// from 2^-64 on.  Kinds of the parts of a row are or-ed; a row is split unless bit 0 is set, or bit 1 without bit 2.
-__device__ __forceinline__ unsigned kind_of(uint32_t most) {
-  const uint32_t a = most & 0x7fffu, b = (most >> 16) & 0x7fffu, m = a > b ? a : b;  // order of magnitudes is order of bits; NaN above all
-  return (m > (227u << 7) ? 1u : 0u) | (m ? 2u : 0u) | (m >= (63u << 7) ? 4u : 0u);
-}
-__device__ __forceinline__ bool stays_whole(unsigned kind) { return (kind & 1u) || (kind & 6u) == 2u; }

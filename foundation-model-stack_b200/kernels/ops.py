@@ -437,13 +437,14 @@ def cast_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 # 4,096 17 240 / 153, 64 335 / 175, 256 1,260 / 345; 4,096 x 14,336 17 120 / 81, 256 700 / 157; 4,096 x 4,096 16 33 / 34, 17 43 / 34;
 # 2,048 x 2,048 17 18 / 22, 33 37 / 22; 1,024 x 1,024 32 14 / 17, 33 18 / 17, 256 26 / 20.
 F32_SPLIT_SIZE, F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_SMALL = 12 << 20, 17, 33
+F32_SPLIT_MOST_K = 1 << 18  # terms of a sum, whose operands of up to 2^30 are split times 2^24
 F32_SPLIT_BYTES = 256 << 20  # of scratch that a product takes at a time for the parts of its rows (2,816 rows of 14,336 values)
 
 
 def f32_split_tokens(weight: torch.Tensor) -> int:
     """Tokens from which a sequence's rows go to the tensor cores; 0: never."""
     n, k = weight.shape
-    if min(n, k) < 1024:
+    if min(n, k) < 1024 or k > F32_SPLIT_MOST_K:
         return 0
     return F32_SPLIT_TOKENS if n * k >= F32_SPLIT_SIZE else F32_SPLIT_TOKENS_SMALL
 

@@ -231,3 +231,41 @@ def test_attention_of_small_values(ops, monkeypatch, small, gap):
     a, b = (t.view(n, nheads, hd).double() for t in (got, want))
     assert float(b.abs().max()) > 2.0 ** -126
     assert bool(((a - b).abs() <= 2.0 ** -24 * 64 * size + 2.0 ** -148).all())
+
+
+def split_product(ops, x, w, b=None):
+    """The product by ``gemm_f32_tc`` whatever the number of rows and the size of the matrix."""
+    m, (n, k) = x.shape[0], w.shape
+    y, scratch = torch.empty(m, n, device="cuda"), torch.empty(m * ((k + 63) // 64 * 64 * 6 + 1) + n, dtype=torch.uint8, device="cuda")
+    ops._call("gemm_f32_tc", "fms_gemm_f32_tc", x, w, b, y, scratch, scratch.numel(), m, n, k, ops.error_flag(x.device), ops._stream())
+    return y
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 1200, 1024), (300, 1200, 1024), (700, 6144, 1024)])
+def test_operands_of_any_size(ops, m, n, k):
+    """Products that overflow, operands near 2^63, rows of values below 2^-110, of subnormal ones, and results down to float32's
+    smallest: what multiply-adds give, with 2^-150 for every rounding of theirs.  Clusters, single blocks, and many tiles."""
+    x, w, _ = made(m, n, k, 9)
+    x[3], x[4], x[5], w[7], w[8] = x[3] * 1e21, x[4] * 2.0 ** 63, x[5] * 2.0 ** 28, w[7] * 1e21, w[8].sign() * 1.998 * 2.0 ** 63
+    x[6, 1:], x[9], x[10, ::2], w[11], w[12, ::2] = x[6, 1:] * 2.0 ** -120, x[9] * 2.0 ** -135, 0.0, w[11] * 2.0 ** -128, 0.0
+    x[10, 1::2] *= 2.0 ** -126
+    x[13], w[13], x[14] = x[13] * 2.0 ** -70, w[13] * 2.0 ** -70, x[14] * 2.0 ** -147
+    w[14, 0] = 0.0  # beside x[6]: what only the small values make
+    got, want = split_product(ops, x, w), ops.linear(x, w)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    fine, size = torch.isfinite(want), x.double().abs() @ w.double().abs().T
+    assert bool(((got.double() - want.double()).abs() <= 2e-6 * size + k * 2.0 ** -150)[fine].all())
+    few = split_product(ops, x[:33].contiguous(), w)  # another form: the same bits, those of subnormal results among them
+    assert torch.equal(few.nan_to_num(7.0), got[:33].nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 1024, 1024), (600, 1536, 4096)])
+def test_what_multiply_adds_make_exactly(ops, m, n, k):
+    """Rows that pick an element, whole numbers, equal terms: no sum that float32 holds is cut off."""
+    _, w, _ = made(m, n, k, 10)
+    at = torch.randint(0, k, (m,), device="cuda")
+    x = torch.nn.functional.one_hot(at, k).float()
+    assert torch.equal(split_product(ops, x, w), w[:, at].T)
+    x, w = torch.randint(-7, 8, (m, k), device="cuda").float(), torch.randint(-2047, 2048, (n, k), device="cuda").float()
+    assert torch.equal(split_product(ops, x, w).double(), x.double() @ w.double().T)
+    assert torch.equal(split_product(ops, torch.ones_like(x), torch.full_like(w, 1 + 2.0 ** -23)), torch.full((m, n), k * (1 + 2.0 ** -23), device="cuda"))
