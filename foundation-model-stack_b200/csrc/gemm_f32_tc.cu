@@ -13,7 +13,8 @@
 // x and w are split times 2^SPLIT_SCALE, and sums are scaled back when they are complete: parts of the smallest float32 values are
 // normal bfloat16 values then, and sums of products down to 2^-174 normal float32 ones (additions in memory flush what is smaller, the
 // others do so too).  Values that are not finite or beyond 2^30 do not split (products of parts of both signs could overflow where the
-// sum does not): a row of x or of w with such values is noted while it is split, and its elements are made by multiply-adds instead.
+// sum does not): a row of x or of w with such values is noted while it is split, and its elements are made by multiply-adds instead, by
+// persistent blocks once all their tiles are done (the other warps' waits are bounded, and many such rows take long).
 //
 // x is split by a kernel of its own (it is read by every tile of w's rows; 27 MB written for 1,100 rows of 4,096).  w is split on
 // its way, since writing it split would take longer than the product reads it.  A block owns 128 rows of w (the instruction's
@@ -78,7 +79,8 @@ struct Shape {
 struct Product {
   const float *x, *w, *bias;
   float* y;
-  const unsigned char* x_whole;  // of every row of x: whether it stays whole
+  const unsigned char* x_kinds;  // of every row of x (row_kind)
+  unsigned char* w_kinds;        // of every row of w, for a block's own use
   int M, N, K, run_len, ranks, nt, tiles_x, tiles, vec;
   int* error_flag;
 };
@@ -150,8 +152,8 @@ __device__ __forceinline__ float whole_element(const float* __restrict__ x, cons
   return warp_sum(v);
 }
 
-// x as three matrices of bfloat16 parts [3][M][pitch], zeros behind K, and whether a row stays whole: a block a row
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, uint4* __restrict__ parts, unsigned char* __restrict__ whole,
+// x as three matrices of bfloat16 parts [3][M][pitch], zeros behind K, and its rows' kinds: a block a row
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, uint4* __restrict__ parts, unsigned char* __restrict__ kinds,
                                                          int M, int K, int pitch, int vec) {
   pdl_launch_dependents();
   pdl_wait();
@@ -175,8 +177,9 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
     parts[part + to] = mid;
     parts[2 * part + to] = lo;
   }
-  const int any = __syncthreads_or(beyond<SPLIT_UP_TO>(most));
-  if (threadIdx.x == 0) whole[m] = any ? 1 : 0;
+  const unsigned char kind = row_kind<SPLIT_UP_TO>(most);
+  const int any = __syncthreads_or(kind != 0), none = __syncthreads_or(kind == 2);
+  if (threadIdx.x == 0) kinds[m] = none ? 2 : any ? 1 : 0;
 }
 
 template <typename S>
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
   __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int failed_flag, whole_any;  // whole_any: some row of this block's run may have to stay whole
-  __shared__ unsigned char w_whole[2][WROWS];  // by the parity of the block's tile
+  __shared__ unsigned char w_kinds[2][WROWS];  // by the parity of the block's tile
   volatile int* failed = &failed_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int x_part = p.nt * BK * 2, sub_bytes = 3 * (W_PART + x_part), stage_bytes = S::SUB * sub_bytes;
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
               for (int u = 0; u < S::UNITS; ++u) {
                 uint32_t m = most2(most[u], __shfl_xor_sync(0xffffffffu, most[u], 1));
                 m = most2(m, __shfl_xor_sync(0xffffffffu, m, 2));
-                if ((lane & 3) == 0) w_whole[turn][u * S::SPAN + row] = beyond<SPLIT_UP_TO>(m) ? 1 : 0;
+                if ((lane & 3) == 0) w_kinds[turn][u * S::SPAN + row] = row_kind<SPLIT_UP_TO>(m);
                 most[u] = 0;
               }
             }
@@ -387,6 +390,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
     pdl_wait();
     float acc[S::COLS];
     int it = 0, turn = 0;
+    bool some_whole = false;
     for (int tile = first_tile; tile < p.tiles && !*failed; tile += tile_step, turn ^= 1) {
       const int w0 = tile / p.tiles_x * WROWS, x0 = tile % p.tiles_x * p.nt, n = w0 + my_row;
 #pragma unroll
@@ -456,21 +460,27 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
           run_end += p.run_len / S::STEP;
           if (end) {
             bool any = false;
-            for (int j = lane; j < WROWS; j += 32) any |= w_whole[turn][j] != 0;
-            for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_whole[x0 + j] != 0;
-            if (__any_sync(0xffffffffu, any)) {
-              const bool whole_w = w_whole[turn][my_row] != 0;
-              for (int c = 0; c < cols && x0 + col0 + c < p.M; ++c) {
-                const int m = x0 + col0 + c;
-                unsigned rows = __ballot_sync(0xffffffffu, n < p.N && (whole_w || p.x_whole[m]));
-                for (; rows; rows &= rows - 1) {
-                  const int r = __ffs(rows) - 1;
-                  const float v = whole_element(p.x + (size_t)m * p.K, p.w + (size_t)(w0 + quarter * 32 + r) * p.K, p.K, lane);
-                  if (lane == r) p.y[(size_t)m * p.N + n] = v + b;
-                }
-              }
-            }
+            for (int j = lane; j < WROWS; j += 32) any |= w_kinds[turn][j] != 0;
+            for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_kinds[x0 + j] != 0;
+            some_whole |= __any_sync(0xffffffffu, any) != 0;
+            if (n < p.N) p.w_kinds[n] = w_kinds[turn][my_row];  // the same from every block that has the row
           }
+        }
+      }
+    }
+    // the rows that do not split, when no warp waits for this one any more
+    for (int tile = some_whole && !__any_sync(0xffffffffu, *failed) ? first_tile : p.tiles; tile < p.tiles; tile += tile_step) {
+      const int w0 = tile / p.tiles_x * WROWS, x0 = tile % p.tiles_x * p.nt, n = w0 + my_row;
+      const unsigned kind_w = n < p.N ? p.w_kinds[n] : 0;
+      const float b = p.bias && n < p.N ? p.bias[n] : 0.f;
+      for (int c = 0; c < cols && x0 + col0 + c < p.M; ++c) {
+        const int m = x0 + col0 + c;
+        const unsigned kind = max(kind_w, (unsigned)p.x_kinds[m]);
+        if (n < p.N && kind == 2) p.y[(size_t)m * p.N + n] = NAN;
+        for (unsigned rows = __ballot_sync(0xffffffffu, n < p.N && kind == 1); rows; rows &= rows - 1) {
+          const int r = __ffs(rows) - 1;
+          const float v = whole_element(p.x + (size_t)m * p.K, p.w + (size_t)(w0 + quarter * 32 + r) * p.K, p.K, lane);
+          if (lane == r) p.y[(size_t)m * p.N + n] = v + b;
         }
       }
     }
@@ -482,8 +492,8 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
           if (c < cols) own[(col0 + c) * WROWS + my_row] = acc[c];
         const int x0 = first_tile % p.tiles_x * p.nt;
         bool any = false;
-        for (int j = lane; j < WROWS; j += 32) any |= w_whole[0][j] != 0;
-        for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_whole[x0 + j] != 0;
+        for (int j = lane; j < WROWS; j += 32) any |= w_kinds[0][j] != 0;
+        for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_kinds[x0 + j] != 0;
         if (__any_sync(0xffffffffu, any) && lane == 0) whole_any = 1;
       }
       __syncwarp();
@@ -514,12 +524,13 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
         float v[4] = {__fmul_rn(q.x, UNSCALE), __fmul_rn(q.y, UNSCALE), __fmul_rn(q.z, UNSCALE), __fmul_rn(q.w, UNSCALE)};
         float* const at = p.y + (size_t)(x0 + c) * p.N + n;
         if (any) {
-          const unsigned whole_x = p.x_whole[x0 + c];
+          const unsigned kind_x = p.x_kinds[x0 + c];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            unsigned whole = whole_x;
-            for (int s = 0; s < runs; ++s) whole |= cluster.map_shared_rank(w_whole[0], s)[row + j];
-            unsigned rows = __ballot_sync(0xffffffffu, n + j < p.N && whole);
+            unsigned kind = kind_x;
+            for (int s = 0; s < runs; ++s) kind = max(kind, (unsigned)cluster.map_shared_rank(w_kinds[0], s)[row + j]);
+            if (kind == 2) v[j] = NAN;
+            unsigned rows = __ballot_sync(0xffffffffu, n + j < p.N && kind == 1);
             for (; rows; rows &= rows - 1) {
               const int r = __ffs(rows) - 1;
               const float t = whole_element(p.x + (size_t)(x0 + c) * p.K, p.w + (size_t)(n + j + (r - lane) * 4) * p.K, p.K, lane);
@@ -635,7 +646,7 @@ void plan(int M, int N, int K, Product& p) {
 }
 }  // namespace
 
-// scratch: 128-byte aligned, 6 bytes for every row and k (K rounded up to a multiple of 64) and one for every row: x split
+// scratch: 128-byte aligned, 6 bytes for every row of x and k (K rounded up to a multiple of 64) and one for every row of x and of w
 FMS_API int fms_gemm_f32_tc(const float* x, const float* w, const float* bias, float* y, void* scratch, long long scratch_bytes, int M, int N,
                             int K, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
@@ -652,12 +663,13 @@ FMS_API int fms_gemm_f32_tc(const float* x, const float* w, const float* bias, f
   CUtensorMap map_x = {};
   const int pitch = pitch_of(K);
   if (3LL * M > 0x7fffffffLL) return fms_fail("gemm_f32_tc: %d rows", M);
-  if (scratch == nullptr || ((uintptr_t)scratch & 127) || scratch_bytes < (long long)M * pitch_of(K) * 6 + M)
+  if (scratch == nullptr || ((uintptr_t)scratch & 127) || scratch_bytes < (long long)M * pitch_of(K) * 6 + M + N)
     return fms_fail("gemm_f32_tc: %lld bytes of scratch at %p", scratch_bytes, scratch);
-  unsigned char* whole = (unsigned char*)scratch + (size_t)M * pitch * 6;
-  fms_launch(split_rows_kernel, dim3(M), dim3(256), 0, stream, x, (uint4*)scratch, whole, M, K, pitch, p.vec);
+  unsigned char* kinds = (unsigned char*)scratch + (size_t)M * pitch * 6;
+  fms_launch(split_rows_kernel, dim3(M), dim3(256), 0, stream, x, (uint4*)scratch, kinds, M, K, pitch, p.vec);
   if (fms_launch_status("gemm_f32_tc")) return 1;
-  p.x_whole = whole;
+  p.x_kinds = kinds;
+  p.w_kinds = kinds + M;
   if (make_parts_map(&map_x, scratch, 3L * M, pitch, p.nt)) return 1;
   if (p.nt <= 64) return launch_shape<Shape<64, 2, 16, 8, 3, 2, 4, 0, 0>>(p, map_x, stream);
   if (p.nt <= 128) return launch_shape<Shape<128, 2, 16, 8, 2, 1, 0, 56, 112>>(p, map_x, stream);

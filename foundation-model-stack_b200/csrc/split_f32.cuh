@@ -64,3 +64,7 @@ __device__ __forceinline__ bool beyond(uint32_t most) {
   const uint32_t a = most & 0x7fffu, b = (most >> 16) & 0x7fffu;  // order of magnitudes is order of bits; NaN above all
   return (a > b ? a : b) > ((127u + EXPONENT) << 7);
 }
+// what becomes of a row whose largest magnitudes are `most`: 0 it is split, 1 it holds something beyond 2^EXPONENT, 2 something that is no
+// number (which every sum over the row then is)
+template <int EXPONENT>
+__device__ __forceinline__ unsigned char row_kind(uint32_t most) { return !beyond<EXPONENT>(most) ? 0 : beyond<128>(most) ? 2 : 1; }

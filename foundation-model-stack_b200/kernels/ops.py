@@ -469,7 +469,7 @@ def _linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
             continue
         size = (k + 63) // 64 * 64 * 6 + 1  # of a row of x in its parts
         step = max(256, F32_SPLIT_BYTES // size // 256 * 256)
-        scratch = torch.empty((min(count, step) * size,), dtype=torch.uint8, device=x.device)
+        scratch = torch.empty((min(count, step) * size + n,), dtype=torch.uint8, device=x.device)
         for first in range(at, at + count, step):
             some = min(step, at + count - first)
             _call("gemm_f32_tc", "fms_gemm_f32_tc", x[first:first + some], weight, bias, y[first:first + some], scratch, scratch.numel(),

@@ -269,3 +269,28 @@ def test_what_multiply_adds_make_exactly(ops, m, n, k):
     x, w = torch.randint(-7, 8, (m, k), device="cuda").float(), torch.randint(-2047, 2048, (n, k), device="cuda").float()
     assert torch.equal(split_product(ops, x, w).double(), x.double() @ w.double().T)
     assert torch.equal(split_product(ops, torch.ones_like(x), torch.full_like(w, 1 + 2.0 ** -23)), torch.full((m, n), k * (1 + 2.0 ** -23), device="cuda"))
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 28672, 4096), (2048, 4096, 14336)])
+def test_many_rows_that_do_not_split(ops, m, n, k):
+    """Several tiles a block, whose rows are none split: they are made behind all tiles, and no warp gives up waiting meanwhile."""
+    x, w, b = made(m, n, k, 11)
+    want = ops.linear(x, w, b, None, [m])
+    x[:, 0], rows = float("nan"), [5, m - 1]
+    x[rows, 0] = 1.0
+    x[rows[1], 1], w[:, 1] = 2e30, 0.0
+    got = ops.linear(x, w, b, None, [m])
+    ops.check_error_flag("cuda:0")
+    others = torch.ones(m, dtype=torch.bool, device="cuda")
+    others[rows] = False
+    assert bool(torch.isnan(got[others]).all()) and bool(torch.isfinite(got[rows]).all())
+    x[rows[1], 1] = 0.0
+    assert torch.equal(got[rows[0]], ops.linear(x[rows[0]].repeat(64, 1), w, b, None, [64])[0])
+    assert bool(((got[rows].double() - (x[rows].double() @ w.double().T + b.double())).abs() <= bound(x[rows], w, b) + 2e-6 * (x[rows].double().abs() @ w.double().abs().T)).all())
+    assert not torch.isnan(want).any()
+    x[:] = 2e30
+    w.fill_(1.0)
+    b.zero_()
+    got = ops.linear(x[:, :1024].contiguous(), w[:, :1024].contiguous(), b, None, [m])
+    ops.check_error_flag("cuda:0")
+    assert bool(((got.double() / (1024 * 2e30) - 1).abs() <= 2.0 ** -20).all())
