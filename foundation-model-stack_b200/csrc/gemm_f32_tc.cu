@@ -139,6 +139,12 @@ __device__ __forceinline__ void load8(float* v, const float* at, int vec, int le
   }
 }
 
+// A wait of a whole warp: its lanes look for themselves, so one can see the phase complete when another sees that a role gave up, and
+// what follows takes all of them
+__device__ __forceinline__ bool warp_waits(void* bar, uint32_t parity, volatile int* failed) {
+  return __all_sync(0xffffffffu, wait_or_abort(bar, parity, failed));
+}
+
 // asks for a run of bytes (16-byte aligned, a multiple of 16) to be brought into the second-level cache
 __device__ __forceinline__ void prefetch_l2_run(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
@@ -271,11 +277,13 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
 #pragma unroll
       for (int u = 0; u < S::UNITS; ++u) most[u] = 0;
       int i = 0, turn = 0, s = 0, round = 1;  // round: parity of the stage's phase
-      for (int it0 = 0; it0 < total && !*failed; it0 += S::DEPTH) {
+      bool go = true;
+      for (int it0 = 0; it0 < total && go; it0 += S::DEPTH) {
 #pragma unroll
         for (int d = 0; d < S::DEPTH; ++d) {
           if (it0 + d >= total) break;
-          if (!wait_or_abort(&empty[s], round, failed)) break;
+          go = warp_waits(&empty[s], round, failed);
+          if (!go) break;
           if (active) {
             unsigned char* const stage = to + s * stage_bytes;
             const int left = k_end - (k_begin + load_step * S::STEP + kk);
@@ -390,15 +398,16 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
     pdl_wait();
     float acc[S::COLS];
     int it = 0, turn = 0;
-    bool some_whole = false;
-    for (int tile = first_tile; tile < p.tiles && !*failed; tile += tile_step, turn ^= 1) {
+    bool some_whole = false, go = true;
+    for (int tile = first_tile; tile < p.tiles && go; tile += tile_step, turn ^= 1) {
       const int w0 = tile / p.tiles_x * WROWS, x0 = tile % p.tiles_x * p.nt, n = w0 + my_row;
 #pragma unroll
       for (int c = 0; c < S::COLS; ++c) acc[c] = 0.f;
       int run_end = alone ? p.run_len / S::STEP : steps;
       bool first_run = true;
       for (int i = 0; i < steps; ++i, ++it) {
-        if (!wait_or_abort(&acc_full[it & 1], (it >> 1) & 1, failed)) break;
+        go = warp_waits(&acc_full[it & 1], (it >> 1) & 1, failed);
+        if (!go) break;
         tc_fence_after();
 #pragma unroll
         for (int h = 0; h < S::SUB; ++h) {
@@ -469,7 +478,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
       }
     }
     // the rows that do not split, when no warp waits for this one any more
-    for (int tile = some_whole && !__any_sync(0xffffffffu, *failed) ? first_tile : p.tiles; tile < p.tiles; tile += tile_step) {
+    for (int tile = some_whole && go ? first_tile : p.tiles; tile < p.tiles; tile += tile_step) {
       const int w0 = tile / p.tiles_x * WROWS, x0 = tile % p.tiles_x * p.nt, n = w0 + my_row;
       const unsigned kind_w = n < p.N ? p.w_kinds[n] : 0;
       const float b = p.bias && n < p.N ? p.bias[n] : 0.f;
