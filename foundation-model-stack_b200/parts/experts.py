@@ -112,9 +112,7 @@ class RoutedExperts(Part):
         return self._routed(x)
 
     def _routed(self, x):
-        every = None
-        if self.shared is not None:  # whose rows they are is not known here
-            every = self.shared.forward(x, None) if getattr(self.shared, "takes_sequences", False) else self.shared.forward(x)
+        every = self.shared.forward(x) if self.shared is not None else None
         mode, further = self._ROUTE_MODES[self.scoring], {"bias": self._bias, "side": self.shared_gate, "experts": self.experts}
         if self.scoring == "sigmoid":
             routing = ops.route(x, self.router.tensor("weight"), self.top, mode, **further)

@@ -6,8 +6,8 @@ one matrix, gate first (fms/modules/feedforward.py:227-240 for the sizes, :288-2
 Interface of a feed-forward (what a block calls):
 
     forward(x) -> y          x, y: [tokens, dim] in the compute dtype
-    forward(x, sequences)    where ``takes_sequences`` is set: with the step's ``Batch``, or how many rows each sequence has (None:
-                             every row stands alone; left out: all rows are one sequence's): large float32 products choose by it
+    forward(x, sequences)    where ``takes_sequences`` is set: with the step's ``Batch``, or how many rows each sequence has, by which
+                             large float32 products choose their kernel (None, or left out: every row stands alone)
 
 A feed-forward with routing implements the same call and keeps router and experts inside.
 
@@ -31,9 +31,6 @@ ACTIVATIONS = {"silu": 0, "swish": 0, "gelu": 1, "gelu-tanh": 2, "gelu_pytorch_t
 UNGATED_ACTIVATIONS = dict(ACTIVATIONS, relu_squared=4)
 
 
-ONE_SEQUENCE = object()
-
-
 def feed_forward_of(part, x, batch):
     """A feed-forward's call in a step: the rows ``x`` are those of ``batch``."""
     return part.forward(x, batch) if getattr(part, "takes_sequences", False) else part.forward(x)
@@ -52,10 +49,12 @@ class GatedLinearUnit(Part):
 
     takes_sequences = True
 
-    def forward(self, x, sequences=ONE_SEQUENCE):
-        sequences = [x.shape[0]] if sequences is ONE_SEQUENCE else sequences
-        further = (sequences,) if self.gate_up.by_sequence() else ()
-        h = ops.gated_linear(x, self.gate_up.tensor("weight"), self.gate_up.tensor("bias"), self.activation, *further)
+    def forward(self, x, sequences=None):
+        product = (x, self.gate_up.tensor("weight"), self.gate_up.tensor("bias"), self.activation)
+        if sequences is not None and self.gate_up.by_sequence():
+            h = ops.gated_linear(*product, sequences)
+        else:
+            h = ops.gated_linear(*product)
         return self.down.forward(h, sequences=sequences)
 
     def kernel_libraries(self, dtype):
@@ -74,10 +73,12 @@ class PlainUnit(Part):
 
     takes_sequences = True
 
-    def forward(self, x, sequences=ONE_SEQUENCE):
-        sequences = [x.shape[0]] if sequences is ONE_SEQUENCE else sequences
-        further = (sequences,) if self.up.by_sequence() else ()
-        h = ops.activated_linear(x, self.up.tensor("weight"), self.up.tensor("bias"), self.activation, *further)
+    def forward(self, x, sequences=None):
+        product = (x, self.up.tensor("weight"), self.up.tensor("bias"), self.activation)
+        if sequences is not None and self.up.by_sequence():
+            h = ops.activated_linear(*product, sequences)
+        else:
+            h = ops.activated_linear(*product)
         return self.down.forward(h, sequences=sequences)
 
     def kernel_libraries(self, dtype):

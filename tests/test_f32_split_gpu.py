@@ -294,3 +294,51 @@ def test_many_rows_that_do_not_split(ops, m, n, k):
     got = ops.linear(x[:, :1024].contiguous(), w[:, :1024].contiguous(), b, None, [m])
     ops.check_error_flag("cuda:0")
     assert bool(((got.double() / (1024 * 2e30) - 1).abs() <= 2.0 ** -20).all())
+
+
+@pytest.mark.parametrize("kind", ["glu", "mlp"])
+def test_rows_of_a_feed_forward_stand_alone(ops, kind):
+    """Called as ``forward(x)`` a feed-forward does not know whose rows they are: 40 rows are what each is alone.  Told so, they
+    are a prompt's."""
+    from fms_b200.config.specs import FeedForwardSpec
+    from fms_b200.parts.registry import build_feed_forward
+
+    part = build_feed_forward(FeedForwardSpec(kind, dim=2048, hidden=4096))
+    g = torch.Generator(device="cuda").manual_seed(12)
+    for _, owner, local, d in list(part.named_decls()):
+        owner.set_tensor(local, torch.randn(d.shape, generator=g, device="cuda") * 0.02)
+    part.finalize("cuda", torch.float32)
+    x = torch.randn(40, 2048, generator=g, device="cuda")
+    got = part.forward(x)
+    assert torch.equal(torch.cat([part.forward(x[i:i + 1]) for i in range(40)]), got)
+    assert torch.equal(part.forward(x, [40]), part.forward(torch.cat([x, x]), [40, 40])[:40])
+    assert not torch.equal(part.forward(x, [40]), got)
+
+
+@pytest.mark.parametrize("lengths", [[33, 17, 2, 12], [70, 100, 65, 129, 80]])  # rows alone and together: up to 64, or more (the norms' forms)
+def test_requests_of_a_float32_model_together_and_alone(ops, lengths):
+    """A model whose products go to the tensor cores: a prompt's logits among other prompts, and a decode step's, are the
+    bits that each sequence gets alone."""
+    from fms_b200.models.llama import LLaMA, LLaMAConfig
+    from fms_b200.weights import RandomSource
+
+    model = LLaMA(LLaMAConfig(src_vocab_size=512, emb_dim=2048, nheads=16, kvheads=8, nlayers=2, hidden_dim=2048, multiple_of=1,
+                              max_expected_seq_len=512))
+    model.load(RandomSource(model.checkpoint_layout(), 13, dtype=torch.float32, device="cuda", std=0.05), "hf", "cuda", torch.float32)
+    prompts = [[(7 * i + 3 * j) % 512 for j in range(n)] for i, n in enumerate(lengths)]
+    calls, entry = [], ops._call
+    ops._call = lambda library, name, *a: (calls.append(name), entry(library, name, *a))[1]
+    try:
+        engine = model.new_engine(max_tokens=64 * 20, max_slots=20)
+        slots = engine.begin(len(lengths))
+        together = [engine.step(slots, prompts), engine.step(slots, [[i] for i in range(len(lengths))])]
+        engine.release(slots)
+    finally:
+        ops._call = entry
+    assert "fms_gemm_f32_tc" in calls and "fms_attention_prefill_f32_split" in calls
+    for i, prompt in enumerate(prompts):
+        slot = engine.begin(1)
+        alone = [engine.step(slot, [prompt]), engine.step(slot, [[i]])]
+        engine.release(slot)
+        assert all(torch.equal(t[i], a[0]) for t, a in zip(together, alone)), i
+    engine.check()
