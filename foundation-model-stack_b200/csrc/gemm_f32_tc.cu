@@ -574,6 +574,22 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
   if (threadIdx.x == 0 && *failed && p.error_flag) atomicExch(p.error_flag, 4);
 }
 
+// Rows of float32 out of or into places of a matrix of `extent` rows: a block a row, bound by what it copies
+template <bool INTO>
+__global__ void __launch_bounds__(256) copy_rows_kernel(const float* __restrict__ from, float* __restrict__ to, const int* __restrict__ places,
+                                                        int width, int extent, int vec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int place = places[blockIdx.x];
+  if (!FMS_IN(place, extent)) return;
+  const float* a = from + (size_t)(INTO ? (int)blockIdx.x : place) * width;
+  float* b = to + (size_t)(INTO ? place : (int)blockIdx.x) * width;
+  if (vec)
+    for (int i = threadIdx.x; i < width / 4; i += blockDim.x) reinterpret_cast<float4*>(b)[i] = reinterpret_cast<const float4*>(a)[i];
+  else
+    for (int i = threadIdx.x; i < width; i += blockDim.x) b[i] = a[i];
+}
+
 int multiprocessors() {
   static int sms = 0;
   if (sms == 0) {
@@ -683,4 +699,13 @@ FMS_API int fms_gemm_f32_tc(const float* x, const float* w, const float* bias, f
   if (p.nt <= 64) return launch_shape<Shape<64, 2, 16, 8, 3, 2, 4, 0, 0>>(p, map_x, stream);
   if (p.nt <= 128) return launch_shape<Shape<128, 2, 16, 8, 2, 1, 0, 56, 112>>(p, map_x, stream);
   return launch_shape<Shape<256, 1, 4, 8, 3, 1, 0, 88, 184>>(p, map_x, stream);
+}
+
+// to[r] = from[places[r]], or with `into` to[places[r]] = from[r], for r < rows; places lie within `extent` rows
+FMS_API int fms_copy_rows_f32(const float* from, float* to, const int* places, int rows, int width, int extent, int into, cudaStream_t stream) {
+  if (rows <= 0 || width <= 0) return 0;
+  const int vec = width % 4 == 0 && (((uintptr_t)from | (uintptr_t)to) & 15) == 0;
+  if (into) fms_launch(copy_rows_kernel<true>, dim3(rows), dim3(256), 0, stream, from, to, places, width, extent, vec);
+  else fms_launch(copy_rows_kernel<false>, dim3(rows), dim3(256), 0, stream, from, to, places, width, extent, vec);
+  return fms_launch_status("copy_rows_f32");
 }

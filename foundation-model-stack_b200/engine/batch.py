@@ -22,6 +22,28 @@ def int32_on(device, values) -> torch.Tensor:
     return torch.tensor(values, dtype=torch.int32, pin_memory=pinned).to(device, non_blocking=pinned)
 
 
+def row_sides(num_new: Sequence[int], least: int, device, in_runs: bool = False):
+    """A step's rows by whether their sequence brings ``least`` tokens: (whether it does, first row, rows, None) for rows that lie one
+    behind the other, (whether, 0, rows, their places: int32 on the device) for all of a side that does not; ``in_runs``: every run of
+    neighbours for itself, which needs nothing on the device."""
+    runs, at = {True: [], False: []}, 0
+    for n in num_new:
+        side = runs[n >= least]
+        if side and side[-1][1] == at:
+            side[-1][1] += n
+        elif n:
+            side.append([at, at + n])
+        at += n
+    out = []
+    for many, side in runs.items():
+        if len(side) > 1 and not in_runs:
+            places = [r for a, b in side for r in range(a, b)]
+            out.append((many, 0, len(places), int32_on(device, places)))
+        else:
+            out.extend((many, a, b - a, None) for a, b in side)
+    return out
+
+
 class Batch:
     """Device arrays of one step.  Built by ``Batch.from_lists`` for a general step, or filled in place
     by the decode loop (``engine.step.DecodeState``) when every sequence brings one token."""
@@ -147,6 +169,16 @@ class Batch:
             s = len(first)
             self._tiles[key] = (packed[: s + 1], packed[s + 1: 2 * s + 1], packed[2 * s + 1:], start[-1])
         return self._tiles[key]
+
+    def row_sides(self, least: int, in_runs: bool = False):
+        """``row_sides`` of the step's sequences; what the device needs for it is kept."""
+        key = ("sides", least)
+        if key in self._tiles:
+            return self._tiles[key]
+        out = row_sides(self.num_new, least, self.tokens.device, in_runs)
+        if not in_runs:
+            self._tiles[key] = out
+        return out
 
     def query_tiles(self, tile_rows: int, members: Optional[Sequence[int]] = None) -> torch.Tensor:
         """[tiles, 2] int32: (sequence index, first row of the tile within the sequence's new tokens), for

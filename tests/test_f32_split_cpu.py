@@ -32,3 +32,18 @@ def test_a_warp_waits_and_gives_up_as_one(name):
         assert any(a <= at < b for a, b in lanes) or "__all_sync(0xffffffffu, " in statement, text[at - 120:at + 60]
     for loop in re.finditer(r"for \([^;]*;[^;]*;[^)]*\)", text):  # nor may lanes leave a loop one by one
         assert "!*failed" not in loop.group() or any(a <= loop.start() < b for a, b in lanes), loop.group()
+
+
+def test_rows_of_either_side_of_a_limit():
+    """Which rows a float32 product takes together: neighbours as they lie, a side of several runs by its places."""
+    from fms_b200.engine.batch import Batch, row_sides
+
+    def plain(sides):
+        return [(many, first, rows, None if places is None else places.tolist()) for many, first, rows, places in sides]
+
+    assert plain(row_sides([3, 0, 4], 3, "cpu")) == [(True, 0, 7, None)]
+    assert plain(row_sides([3, 4, 1, 1], 3, "cpu")) == [(True, 0, 7, None), (False, 7, 2, None)]
+    assert plain(row_sides([1, 0, 3, 2, 4, 0], 3, "cpu")) == [(True, 0, 7, [1, 2, 3, 6, 7, 8, 9]), (False, 0, 3, [0, 4, 5])]
+    assert plain(row_sides([2, 3, 2], 3, "cpu", True)) == [(True, 2, 3, None), (False, 0, 2, None), (False, 5, 2, None)]
+    batch = Batch.from_lists([0, 1, 2], [0, 0, 0], [[1], [2, 3], [4]], [[], [], []], "cpu")
+    assert batch.row_sides(2, True) is not batch.row_sides(2) and batch.row_sides(2, True) is batch.row_sides(2)

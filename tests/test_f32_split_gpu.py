@@ -342,3 +342,26 @@ def test_requests_of_a_float32_model_together_and_alone(ops, lengths):
         engine.release(slot)
         assert all(torch.equal(t[i], a[0]) for t, a in zip(together, alone)), i
     engine.check()
+
+
+@pytest.mark.parametrize("k", [2048, 2051])
+def test_sequences_on_either_side_of_the_limit_in_turn(ops, monkeypatch, k):
+    """One product a side, whatever the order; each sequence's rows are what it gets alone; the same under capture."""
+    from fms_b200.engine.batch import Batch
+
+    counts = [33, 1, 40, 32, 32, 64, 2]
+    x, w, b = made(sum(counts), 2050, k, 14)
+    batch = Batch.from_lists(list(range(7)), [0] * 7, [[0] * c for c in counts], [[]] * 7, "cuda")
+    calls, entry = [], ops._call
+    monkeypatch.setattr(ops, "_call", lambda library, name, *a: (calls.append(name), entry(library, name, *a))[1])
+    got = ops.linear(x, w, b, None, counts)
+    assert calls.count("fms_gemm_f32_tc") == 1 and calls.count("fms_gemm_f32") == 1
+    graph, held = torch.cuda.CUDAGraph(), torch.empty_like(got)
+    with torch.cuda.graph(graph):
+        held.copy_(ops.linear(x, w, b, None, batch))
+    graph.replay()
+    assert torch.equal(held, got) and torch.equal(ops.linear(x, w, b, None, batch), got)
+    at = 0
+    for c in counts:
+        assert torch.equal(ops.linear(x[at:at + c].contiguous(), w, b, None, [c]), got[at:at + c])
+        at += c
