@@ -433,11 +433,16 @@ def cast_rows(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 
 # ---- linear ------------------------------------------------------------------------------------------
 # Tokens of a sequence from which the float32 products of its rows go to the tensor cores (gemm_f32_tc.cu: operands in three bfloat16
-# parts), where the matrix is large enough.  The sequence's own tokens decide, and what a row gets there does not depend on the other
+# parts), by the matrix' values.  The sequence's own tokens decide, and what a row gets there does not depend on the other
 # rows, so that a sequence's results do not depend on what else is in the step.  CUDA cores / tensor cores in us, by rows: w of 28,672 x
-# 4,096 17 240 / 153, 64 335 / 175, 256 1,260 / 345; 4,096 x 14,336 17 120 / 81, 256 700 / 157; 4,096 x 4,096 16 33 / 34, 17 43 / 34;
-# 2,048 x 2,048 17 18 / 22, 33 37 / 22; 1,024 x 1,024 32 14 / 17, 33 18 / 17, 256 26 / 20.
-F32_SPLIT_SIZE, F32_SPLIT_TOKENS, F32_SPLIT_TOKENS_SMALL = 12 << 20, 17, 33
+# 4,096 17 240 / 183, 64 645 / 200, 256 1,260 / 335; 4,096 x 14,336 17 121 / 91, 256 700 / 165; 4,096 x 4,096 16 33 / 34, 17 43 / 36;
+# 2,048 x 2,048 17 18 / 22, 33 37 / 24; 1,536 x 1,536 33 23 / 22, 257 50 / 40; 1,024 x 1,024 257 31 / 22, 2,048 111 / 54.  A step with
+# sequences on both sides reads the matrix twice, so from the line on a long sequence has to gain what some short ones beside it
+# lose: 257 tokens and 1 of 1,536 x 1,536 49 / 46, between eight and eight of 1 50 / 58 (33 and 1 23 / 28, 40 between eight and eight
+# 23 / 42); 2,000 between four and four of 1,024 x 1,024 111 / 87 (four of 200 and four of 300 in turn 111 / 189).  Larger
+# matrices: 33 and 1 of 2,048 x 2,048 37 / 30, 40 between eight and eight 37 / 48; of 28,672 x 4,096 17 and seven of 1 244 / 286, fifteen
+# of 17 and one of 16 1,570 / 501.
+F32_SPLIT_LINES = ((12 << 20, 17), (4 << 20, 33), (2 << 20, 257), (0, 1025))
 F32_SPLIT_MOST_K = 1 << 18  # terms of a sum, whose operands of up to 2^30 are split times 2^24
 F32_SPLIT_BYTES = 256 << 20  # of scratch that a product takes at a time for the parts of its rows (2,816 rows of 14,336 values)
 
@@ -447,7 +452,7 @@ def f32_split_tokens(weight: torch.Tensor) -> int:
     n, k = weight.shape
     if min(n, k) < 1024 or k > F32_SPLIT_MOST_K:
         return 0
-    return F32_SPLIT_TOKENS if n * k >= F32_SPLIT_SIZE else F32_SPLIT_TOKENS_SMALL
+    return next(tokens for size, tokens in F32_SPLIT_LINES if n * k >= size)
 
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], sequences) -> torch.Tensor:
@@ -456,7 +461,7 @@ def _linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     batch = sequences if hasattr(sequences, "num_new") else None
     if batch is not None:
         sequences = None if batch.decode else batch.num_new or None
-    least = f32_split_tokens(weight) if sequences is not None and m >= F32_SPLIT_TOKENS else 0
+    least = f32_split_tokens(weight) if sequences else 0
     if not least or max(sequences) < least or sum(sequences) != m:
         _call("gemm_f32", "fms_gemm_f32", x, weight, bias, y, m, n, k, _stream())
         return y

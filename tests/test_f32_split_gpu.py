@@ -365,3 +365,31 @@ def test_sequences_on_either_side_of_the_limit_in_turn(ops, monkeypatch, k):
     for c in counts:
         assert torch.equal(ops.linear(x[at:at + c].contiguous(), w, b, None, [c]), got[at:at + c])
         at += c
+
+
+@pytest.fixture
+def every_size(ops, monkeypatch):
+    """Matrices of fewer values go to the tensor cores from 33 tokens on as well."""
+    monkeypatch.setattr(ops, "F32_SPLIT_LINES", ((12 << 20, 17), (0, 33)))
+
+
+@pytest.mark.parametrize("n,k", [(1024, 1024), (1153, 1050), (1030, 2052)])
+@pytest.mark.parametrize("m", [33, 64, 65, 129, 256, 257, 600])
+def test_edges_with_small_matrices(ops, every_size, m, n, k):
+    test_edges_of_tiles_runs_and_steps(ops, m, n, k)
+
+
+@pytest.mark.parametrize("m", [40, 300])
+def test_values_that_do_not_split_with_small_matrices(ops, every_size, m):
+    test_values_that_do_not_split(ops, m)
+
+
+def test_shifted_operands_and_scratch_with_small_matrices(ops, every_size, monkeypatch):
+    test_shifted_operands_and_scratch_at_a_time(ops, monkeypatch)
+
+
+def test_lines_by_the_values_of_a_matrix(ops):
+    """The tokens from which a matrix' products change, at the edges of its sizes."""
+    shapes = {(1023, 1 << 20): 0, (1024, 1024): 1025, (1024, 2048): 257, (1024, 4096): 33, (3072, 4096): 17, (3071, 4096): 33, (1024, 1 << 18): 17,
+              (1024, (1 << 18) + 1): 0}
+    assert {s: ops.f32_split_tokens(torch.empty(s, device="meta")) for s in shapes} == shapes
