@@ -494,11 +494,19 @@ def _linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
 
 
 def _split_product(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], y: torch.Tensor) -> None:
-    """y = x weight^T (+ bias) on the tensor cores, some rows at a time: a row's result does not depend on those beside it."""
+    """y = x weight^T (+ bias) on the tensor cores, some rows at a time: a row's result does not depend on those beside it.  Where the
+    memory does not hold the scratch for as many rows, fewer are taken at a time."""
     m, (n, k) = x.shape[0], weight.shape
     size = (k + 63) // 64 * 64 * 6 + 1  # of a row of x in its parts
     step = max(256, F32_SPLIT_BYTES // size // 256 * 256)
-    scratch = torch.empty((min(m, step) * size + n,), dtype=torch.uint8, device=x.device)
+    while True:
+        try:
+            scratch = torch.empty((min(m, step) * size + n,), dtype=torch.uint8, device=x.device)
+            break
+        except torch.OutOfMemoryError:
+            if step <= 32:
+                raise
+            step = (min(m, step) // 2 + 31) // 32 * 32
     for first in range(0, m, step):
         some = min(step, m - first)
         _call("gemm_f32_tc", "fms_gemm_f32_tc", x[first:first + some], weight, bias, y[first:first + some], scratch, scratch.numel(),

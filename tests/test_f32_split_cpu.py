@@ -47,3 +47,36 @@ def test_rows_of_either_side_of_a_limit():
     assert plain(row_sides([2, 3, 2], 3, "cpu", True)) == [(True, 2, 3, None), (False, 0, 2, None), (False, 5, 2, None)]
     batch = Batch.from_lists([0, 1, 2], [0, 0, 0], [[1], [2, 3], [4]], [[], [], []], "cpu")
     assert batch.row_sides(2, True) is not batch.row_sides(2) and batch.row_sides(2, True) is batch.row_sides(2)
+
+
+def test_scratch_of_a_product_gives_way(monkeypatch):
+    """A card without room for a product's scratch takes fewer rows at a time, down to 32, and every row once."""
+    import torch
+
+    from fms_b200.kernels import ops
+
+    room, taken = [0], []
+    empty = torch.empty
+
+    def scratch(shape, dtype=None, device=None):
+        if shape[0] > room[0]:
+            raise torch.OutOfMemoryError("no room")
+        return empty(shape, dtype=dtype, device=device)
+
+    monkeypatch.setattr(ops, "error_flag", lambda device: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "_call", lambda library, name, x, w, b, y, s, have, rows, n, k, *_: (
+        taken.append((x.shape[0], rows)), y.fill_(1.0), have >= rows * (-(-k // 64) * 384 + 1) + n or pytest.fail("too little scratch")))
+    x, w = torch.zeros(1000, 128), torch.zeros(7, 128)
+    for at_a_time in (1000, 999, 300, 100, 32):
+        y = torch.zeros(1000, 7)
+        room[0], taken[:] = at_a_time * 769 + 7, []
+        monkeypatch.setattr(torch, "empty", scratch)
+        ops._split_product(x, w, None, y)
+        monkeypatch.setattr(torch, "empty", empty)
+        assert bool((y == 1).all()) and sum(r for _, r in taken) == 1000 and max(r for _, r in taken) <= at_a_time
+        assert all(a == r for a, r in taken)
+    monkeypatch.setattr(torch, "empty", scratch)
+    room[0] = 31 * 769 + 7
+    with pytest.raises(torch.OutOfMemoryError):
+        ops._split_product(x, w, None, torch.zeros(1000, 7))
