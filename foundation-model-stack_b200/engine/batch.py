@@ -14,12 +14,25 @@ from typing import List, Optional, Sequence
 import torch
 
 
+_copies = {}  # device -> the stream of its index arrays' copies
+
+
 def int32_on(device, values) -> torch.Tensor:
-    """Whole numbers on the device, copied out of pinned memory (kept by torch until the copy is over) so that the host does not
-    wait for the stream: from pageable memory every such copy let the GPU run dry behind it.  A capture, which would read the
-    memory again at every replay, refuses the pageable copy that it gets."""
-    pinned = torch.device(device).type == "cuda" and not torch.cuda.is_current_stream_capturing()
-    return torch.tensor(values, dtype=torch.int32, pin_memory=pinned).to(device, non_blocking=pinned)
+    """Whole numbers on the device, there when this returns, for use on any stream.  The copy has a stream of its own: on the current one
+    it would wait, and the host with it, for all that lies in front of it, and the GPU run dry behind it.  The memory is the copies'
+    stream's and is not given out again before what the current stream had been given when the tensor is freed is done.  A capture refuses the
+    copy."""
+    device = torch.device(device)
+    if device.type != "cuda" or torch.cuda.is_current_stream_capturing():
+        return torch.tensor(values, dtype=torch.int32).to(device)
+    current = torch.cuda.current_stream(device)
+    stream = _copies.get(current.device)
+    if stream is None:
+        stream = _copies.setdefault(current.device, torch.cuda.Stream(current.device))
+    with torch.cuda.stream(stream):
+        out = torch.tensor(values, dtype=torch.int32).to(current.device)
+    out.record_stream(current)
+    return out
 
 
 def row_sides(num_new: Sequence[int], least: int, device, in_runs: bool = False):
