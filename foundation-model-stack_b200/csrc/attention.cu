@@ -831,7 +831,9 @@ FMS_API int fms_attn_f32_split_takes(int nheads, int kvheads) {
 FMS_API int fms_attention_prefill_f32_split(const void* q, void* out, const void* keys, const void* values, const int* table, int table_stride,
                                             int block_tokens, const int* slots, const int* first_row, const int* len_after, const int* tiles,
                                             int n_tiles, int nheads, int kvheads, int head_dim, float scale, int window, int pool_blocks,
-                                            int table_rows, int* error_flag, const float* sink, int chunk, long q_stride, cudaStream_t stream) {
+                                            int table_rows, int* error_flag, const float* sink, int chunk, long q_stride, int n_seqs, int n_rows,
+                                            cudaStream_t stream) {
+  // n_seqs, n_rows: extents of the sequences' arrays and of q and out, for the bounds-checked build (0: not known)
   if (n_tiles <= 0) return 0;
 #if FMS_ATTENTION_TC
   if (check_args("attention_prefill_f32_split", nheads, kvheads, head_dim, block_tokens)) return 1;
@@ -850,7 +852,7 @@ FMS_API int fms_attention_prefill_f32_split(const void* q, void* out, const void
   }
   const long blocks = (long)n_tiles * (nheads / 2);
   if (blocks > 0x7fffffffL) return fms_fail("attention_prefill_f32_split: %ld thread blocks", blocks);
-  fms_launch(attn_prefill_f32_tc_kernel, dim3((unsigned)blocks), dim3(FT_THREADS), FT_SMEM, stream, a, tiles, n_tiles, error_flag);
+  fms_launch(attn_prefill_f32_tc_kernel, dim3((unsigned)blocks), dim3(FT_THREADS), FT_SMEM, stream, a, tiles, n_tiles, n_seqs, n_rows, error_flag);
   return fms_launch_status("attention_prefill_f32_split");
 #else
   return fms_fail("attention_prefill_f32_split: head size %d has no tcgen05 kernel", HD);

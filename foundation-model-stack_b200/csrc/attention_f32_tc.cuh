@@ -62,7 +62,7 @@ __device__ __forceinline__ void ft_accumulate(uint32_t d, uint64_t a, uint64_t b
 }
 
 __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(AttnArgs a, const int* __restrict__ tiles, int n_tiles,
-                                                                             int* __restrict__ error_flag) {
+                                                                             int n_seqs, int n_rows, int* __restrict__ error_flag) {
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* qs = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
   unsigned char *ks = qs + 3 * FT_QPART, *vs = ks + FT_KREGION;
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   __syncthreads();
   pdl_wait();
   const int pairs = a.nheads / 2, pair = blockIdx.x % pairs, tile = n_tiles - 1 - blockIdx.x / pairs;  // the longest tiles first
-  const int seq = tiles[2 * tile], r0 = tiles[2 * tile + 1];
+  const int seq = FMS_IN(tiles[2 * tile], n_seqs) ? tiles[2 * tile] : 0, r0 = tiles[2 * tile + 1];
   const int row_begin = a.first_row[seq], n_new = a.first_row[seq + 1] - row_begin, len = a.len_after[seq];
   const int rows_here = min(TQ, n_new - r0), slot = a.slots[seq], p_first = len - n_new + r0, p_last = p_first + rows_here - 1;
   const int head0 = 2 * pair, kvh = head0 / (a.nheads / a.kvheads), head = head0 + (row >> 6), pos = row & 63, my_pos = p_first + pos;
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   for (int i = tid; i < 128 * FT_PER_ROW; i += FT_THREADS) {
     const int r = i / FT_PER_ROW, c = i % FT_PER_ROW;
     float v[8];
-    ft_read(v, q + (size_t)(r & 63) * a.q_stride + (r >> 6) * HD + 8 * c, (r & 63) < rows_here);
+    ft_read(v, q + (size_t)(r & 63) * a.q_stride + (r >> 6) * HD + 8 * c, (r & 63) < rows_here && FMS_IN(row_begin + r0 + (r & 63), n_rows));
     if (!ft_put(qs + (c >> 3) * (128 * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), FT_QPART, v)) odd[r] = 1;
   }
   float x[FT_UNITS][8];
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   sums[half][row] = l;
   if (sees_odd || !(l == l)) odd[row] = 1;
   __syncthreads();
-  if (mine && !odd[row]) {
+  if (mine && !odd[row] && FMS_IN(row_begin + r0 + pos, n_rows)) {
     float sum = sums[0][row] + sums[1][row];
     if (a.sink != nullptr) sum += expf(a.sink[head] - (m == -INFINITY ? 0.f : m));
     const float inv = sum > 0.f ? 1.f / sum : 0.f;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_prefill_f32_tc_kernel(Attn
   {  // the other rows: a warp a row, a lane a key and HD / 32 of the results
     constexpr int PER = HD / 32;
     for (int r = warp; r < 128; r += FT_THREADS / 32) {
-      if ((r & 63) >= rows_here || !odd[r]) continue;
+      if ((r & 63) >= rows_here || !odd[r] || !FMS_IN(row_begin + r0 + (r & 63), n_rows)) continue;
       const int at = p_first + (r & 63), h = head0 + (r >> 6);
       const float* qr = q + (size_t)(r & 63) * a.q_stride + (r >> 6) * HD;
       const int first = first_visible(a, at);

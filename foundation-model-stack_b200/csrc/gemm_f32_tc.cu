@@ -250,6 +250,8 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
         if (load_tile < p.tiles) aim();
       }
     };
+    // for the bounds-checked build: what is read of a row of w lies in the matrix
+    auto inside = [&](const float* from, int left) { return left <= 0 || FMS_IN(from - p.w + min(left, 8) - 1, (size_t)p.N * p.K); };
     if (first_tile < p.tiles) {  // w may be what the kernel in front makes: only asked for
       const int n = first_tile / p.tiles_x * WROWS + member * 32 + lane;
       for (int s = 0; s < S::DEPTH; ++s)
@@ -270,7 +272,10 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
 #pragma unroll
             for (int u = 0; u < S::UNITS; ++u)
 #pragma unroll
-              for (int h = 0; h < S::SUB; ++h) load8<fast>(v[d][u][h], at[u] + h * BK, p.vec, k_end - (k_begin + load_step * S::STEP + h * BK + kk), true);
+              for (int h = 0; h < S::SUB; ++h) {
+                const int left = k_end - (k_begin + load_step * S::STEP + h * BK + kk);
+                load8<fast>(v[d][u][h], at[u] + h * BK, p.vec, left, inside(at[u] + h * BK, left));
+              }
             loaded();
           }
       }
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
                 *reinterpret_cast<uint4*>(place) = hi;
                 *reinterpret_cast<uint4*>(place + W_PART) = mid;
                 *reinterpret_cast<uint4*>(place + 2 * W_PART) = lo;
-                load8<fast>(v[d][u][h], at[u] + h * BK, p.vec, left - h * BK, more);
+                load8<fast>(v[d][u][h], at[u] + h * BK, p.vec, left - h * BK, more && inside(at[u] + h * BK, left - h * BK));
               }
             }
             if (more) {
@@ -472,7 +477,7 @@ __global__ void __launch_bounds__(S::THREADS, 1) gemm_f32_split_kernel(const Pro
             for (int j = lane; j < WROWS; j += 32) any |= w_kinds[turn][j] != 0;
             for (int j = lane; j < min(p.nt, p.M - x0); j += 32) any |= p.x_kinds[x0 + j] != 0;
             some_whole |= __any_sync(0xffffffffu, any) != 0;
-            if (n < p.N) p.w_kinds[n] = w_kinds[turn][my_row];  // the same from every block that has the row
+            if (n < p.N && FMS_IN(n, p.N)) p.w_kinds[n] = w_kinds[turn][my_row];  // the same from every block that has the row
           }
         }
       }

@@ -116,7 +116,7 @@ _SIGNATURES = {
     "fms_gated_group_rmsnorm": [_P, _P, _I, _I, _I, _P, _I, _F, _F, _P, _I, _I, _I, _P],
     "fms_argmax": [_P, _P, _I, _I, _P],
     "fms_sample": [_P, _P, _I, _I, _F, _I, _U64, _P, _I, _P],
-    "fms_attention_prefill_f32_split": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _L, _P],
+    "fms_attention_prefill_f32_split": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _L, _I, _I, _P],
     "fms_attention_prefill": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P],
     "fms_attention_decode": [_P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I, _I, _I, _L, _P, _P,
                              _P],
@@ -953,7 +953,7 @@ def attention(q: torch.Tensor, batch, view, nheads: int, kvheads: int, head_dim:
                 tiles = batch.query_tiles(tile_rows, long)
                 _call(lib, "fms_attention_prefill_f32_split", q, out, view.keys, view.values, view.table, view.table.shape[1], view.block_tokens,
                       batch.slots, batch.first_row, batch.len_after, tiles, tiles.shape[0], nheads, kvheads, head_dim, float(scale), int(window),
-                      view.keys.shape[0], view.table.shape[0], error_flag(q.device), sink, int(chunk), q.shape[1], _stream())
+                      view.keys.shape[0], view.table.shape[0], error_flag(q.device), sink, int(chunk), q.shape[1], batch.n_seqs, q.shape[0], _stream())
                 if len(long) == batch.n_seqs:
                     return out
                 members = [i for i, n in enumerate(batch.num_new) if 0 < n < F32_SPLIT_ATTENTION_TOKENS]

@@ -9,6 +9,7 @@ loaded; they are compiled at first use, beside the ordinary ones.
 2. A tiny model generates through the entry point and equals the plain implementation, with no index recorded.
 3. The kernel tests run under the flag (small cases: the slowest, many-sequence ones are left out); a fixture in
    conftest.py fails any of them that records an index.
+4. So do those of float32 work on the tensor cores.
 """
 import os
 import subprocess
@@ -114,3 +115,16 @@ def test_the_kernel_tests_pass_under_the_index_checks():
                         "-k", "not streams_the_cache and not every_batch_size and not 128256 and not long_context"],
                        env=ENV, capture_output=True, text=True, timeout=3000, cwd=ROOT)
     assert r.returncode == 0, (r.stdout + r.stderr)[-3000:]
+
+
+def test_the_float32_tensor_core_tests_pass_under_the_index_checks():
+    code = """
+import sys, pytest
+assert pytest.main([sys.argv[1] + "/tests/test_f32_split_gpu.py", "-q", "-x", "-m", "gpu"]) == 0
+from fms_b200.kernels import build
+names = [lib._name for lib in build.loaded_libraries().values()]
+assert all(any(n + "_checked_" in name for name in names) for n in ("gemm_f32_tc", "attention_hd64", "attention_hd128")), names
+print("checked")
+"""
+    r = subprocess.run([sys.executable, "-c", code, ROOT], env=ENV, capture_output=True, text=True, timeout=3000, cwd=ROOT)
+    assert r.returncode == 0 and "checked" in r.stdout, (r.stdout + r.stderr)[-3000:]
