@@ -18,7 +18,8 @@ Llama-2-7B and Llama-2-13B shapes, decode at batch 8 in float32); ``points_frac`
 roofline (copy bandwidth for decode, the dtype's arithmetic peak for prefill).  Weights (15 GB a step) are
 larger than L2, so no flush is needed between steps.
 
-``--dtype fp32`` measures the true 32-bit path (FFMA products, float32 cache) in the same line format.
+``--dtype fp32`` measures the true 32-bit path (float32 weights, activations and cache; prompts' products as six products of bfloat16
+parts) in the same line format; a prefill's fraction is of a sixth of the bfloat16 peak.
 ``--points main`` leaves the further configurations out; ``--points long`` adds decode at batch 64 with
 7,000 to 8,000 cached tokens a request (a prefill of half a million tokens comes before it).
 ``--only decode_b<N>`` or ``--only prefill`` prints that part alone (for profilers); ``--only gemm_rows``,
@@ -63,8 +64,7 @@ def choose_model(name):
     PROMPT_MIN, PROMPT_MAX = MODEL["prompts"]
 
 
-# float32 on the CUDA cores: 148 multiprocessors x 128 lanes x 2 flops x 1.965 GHz (nominal; nobody measured it here)
-FP32_TFLOPS_NOMINAL = 148 * 128 * 2 * 1.965e9 / 1e12
+FP32_PRODUCTS = 6  # bfloat16 products on the tensor cores that make one float32 product of a prompt's rows
 REGIONS = 5  # timed regions of --steps steps each; the median counts
 
 
@@ -362,7 +362,7 @@ class Measured:
         return decode_bytes(self.nlayers, context, self.m, self.itemsize) / (ms_step / 1e3) / 1e9 / pk["hbm_gbs"]
 
     def prefill_frac(self, ms, tokens, pk):
-        peak = pk["bf16_tflops"] if self.dtype == "bf16" else FP32_TFLOPS_NOMINAL
+        peak = pk["bf16_tflops"] / (1 if self.dtype == "bf16" else FP32_PRODUCTS)
         return prefill_flops(self.nlayers, tokens, self.m) / (ms / 1e3) / (peak * 1e12)
 
 
@@ -449,7 +449,7 @@ def run_ours(args):
             "weights": "random N(0,0.02), seed 0",
             "l2": f"weights read per step ({decode_bytes(nlayers, 0, MODEL, run.itemsize) / 1e9:.0f} GB) exceed L2; no flush",
             "timed": f"median of {REGIONS} regions of {args.steps} steps", "cache_block_tokens": 64,
-            "peaks": pk["source"] + ("" if dtype == "bf16" else f"; fp32 arithmetic {FP32_TFLOPS_NOMINAL:.1f} TFLOP/s nominal"),
+            "peaks": pk["source"] + ("" if dtype == "bf16" else f"; float32 prefill: the bfloat16 rate / {FP32_PRODUCTS}"),
         },
         "clocks": sampler.summary(),
         "e2e": {"value": round(e2e, 1), "unit": "tok/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},

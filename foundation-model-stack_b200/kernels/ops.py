@@ -496,6 +496,7 @@ def _linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
 def _split_product(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], y: torch.Tensor) -> None:
     """y = x weight^T (+ bias) on the tensor cores, some rows at a time: a row's result does not depend on those beside it.  Where the
     memory does not hold the scratch for as many rows, fewer are taken at a time."""
+    global launches
     m, (n, k) = x.shape[0], weight.shape
     size = (k + 63) // 64 * 64 * 6 + 1  # of a row of x in its parts
     step = max(256, F32_SPLIT_BYTES // size // 256 * 256)
@@ -511,6 +512,7 @@ def _split_product(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
         some = min(step, m - first)
         _call("gemm_f32_tc", "fms_gemm_f32_tc", x[first:first + some], weight, bias, y[first:first + some], scratch, scratch.numel(),
               some, n, k, error_flag(x.device), _stream())
+        launches += 1  # the kernel that splits the rows
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -809,7 +811,11 @@ def qkv_rope_store(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
               weight.shape[1], nheads, kvheads, head_dim, 1 if writes_cache else 0, error_flag(x.device),
               batch.slots.shape[0], view.table.shape[0], view.keys.shape[0], _stream())
         return q
-    return rope_store(linear(x, weight, bias, *((None, batch) if weight.dtype == torch.float32 and f32_split_tokens(weight) else ())), inv_freq, batch, view, nheads, kvheads, head_dim, writes_cache)
+    if weight.dtype == torch.float32 and f32_split_tokens(weight):
+        qkv = linear(x, weight, bias, sequences=batch)
+    else:
+        qkv = linear(x, weight, bias)
+    return rope_store(qkv, inv_freq, batch, view, nheads, kvheads, head_dim, writes_cache)
 
 
 def _attention_library(head_dim: int) -> str:
