@@ -916,9 +916,11 @@ int launch_states(const ChunkArgs& g, cudaStream_t stream) {
   return 0;
 }
 
-// A block walks a sequence's runs one by one: 32 columns a block where 64 would give most multiprocessors no second block, whose
-// instructions fill the gaps of the first's (two prompts of 32 heads, 128 blocks of 64 or 256 of 32: 94 -> 78 us of 1,700 tokens;
-// one of 128 heads of 64 values: 167 -> 161 of 2,048).
+// A block walks a sequence's runs one by one: 32 columns a block instead of 64 give twice the blocks, whose instructions fill the gaps
+// of one another (two prompts of 32 heads, 128 blocks of 64 or 256 of 32: 94 -> 78 us of 1,700 tokens; one of 128 heads of 64 values:
+// 167 -> 161 of 2,048).  Whole layers, 16 blocks of 64 a sequence, 32 columns' time over that of 64, in the three kinds alike: 64 blocks
+// 0.86-0.99 (2,048 and 640 tokens), 128 0.92-1.00, 144 0.86-0.98, 160 0.94-0.98, 224 0.94-0.96, 384 0.89-0.98, 448 0.87-1.03 (1,100 and 520
+// tokens), 1,024 0.85-1.00, 1,536 0.84-1.02.  So the line has nothing slower on its side; beyond it 32 would mostly win as well.
 bool columns_32(const ChunkArgs& g, int vdim) { return (long)g.n_seqs * g.heads * vdim / 64 <= 148; }
 
 template <int VDIM, int KIND>
