@@ -26,9 +26,10 @@
 // A step fills two accumulators (nt 256: one, for there is no more tensor memory), while the epilogue drains those of the step
 // before: handing over costs 600 cycles, whatever a step holds (w of 4,096 x 14,336 and 64 rows: 124 us by single accumulators, 91 so).
 // Few tiles: the blocks of a cluster take a run each and add their sums through distributed shared memory.  Many: persistent
-// blocks take all runs of a tile and add a run's sums to y where it lies, which nobody waits for.
-// Measured (us, before / now; six products of bfloat16 at the tensor cores' rate would be 279 TFLOP/s): 1,100 rows of 6,144 x 4,096
-// 1,217 / 296 (187 TFLOP/s), 4,096 x 4,096 824 / 240; 2,048 of 4,096 x 14,336 4,870 / 1,150 (209); 64 of 28,672 x 4,096 335 / 175.
+// blocks take all runs of a tile and add a run's sums to y where it lies, which nobody waits for; the last run's meet them in registers.
+// Measured (us, CUDA cores / here; six products of bfloat16 at the tensor cores' rate would be 279 TFLOP/s): 1,100 rows of 6,144 x 4,096
+// 1,217 / 304 (182 TFLOP/s), 4,096 x 4,096 824 / 241; 2,048 of 4,096 x 14,336 4,870 / 1,183 (203); 64 of 28,672 x 4,096 645 / 200.  The scale
+// costs 1% of that, the last run's way through registers 1 to 3%.
 // What is left: tiles of 128 x 256 read 96 bytes of shared memory a cycle for the products and 48 for what is brought in, of 128;
 // the last round of tiles; adding a run to y stalls the products by a tenth.
 #include <cooperative_groups.h>
